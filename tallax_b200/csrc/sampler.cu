@@ -1225,6 +1225,7 @@ __device__ __forceinline__ int classify_row(const SampleParams& p, int64_t row, 
 }  // namespace tlx
 #include "sampler_wide.cuh"
 #include "sampler_stream.cuh"
+#include "sampler_cluster.cuh"
 #include "sampler_rows.cuh"
 namespace tlx {
 
@@ -1785,7 +1786,7 @@ __device__ __forceinline__ uint32_t ld_acquire_sys_u32(const uint32_t* p) {
   asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ unsigned long long global_timer_ns() {
+__device__ __forceinline__ unsigned long long exchange_timer_ns() {
   unsigned long long t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
   return t;
@@ -1842,11 +1843,11 @@ __global__ void __launch_bounds__(kMergeThreads) merge_and_sample_kernel(MergePa
     }
     if (threadIdx.x == 0) {
       // every rank's block of this row has arrived when the word reads `world`; two seconds at most
-      const unsigned long long t0 = global_timer_ns();
+      const unsigned long long t0 = exchange_timer_ns();
       bool ok = false;
       for (int it = 0; it < (1 << 24); ++it) {
         if (ld_acquire_sys_u32(flag) >= (uint32_t)p.world) { ok = true; break; }
-        if (global_timer_ns() - t0 > 2000000000ull) break;
+        if (exchange_timer_ns() - t0 > 2000000000ull) break;
         __nanosleep(100);
       }
       if (!ok) {
@@ -2219,6 +2220,64 @@ static int launch_rows_path(cudaStream_t st, const SampleParams& sp) {
   return TLX_OK;
 }
 
+// ---- cluster path (sampler_cluster.cuh) -----------------------------------------------------------------------
+// CTAs per row: parts of at most 32 KB, so that four CTAs fit an SM; more and smaller ones, down to 8 KB, while two
+// per SM would not be reached (a few rows: the part's copy and passes are then the shorter).
+static int cluster_size(int64_t rows, int64_t vocab, int elem_bytes) {
+  const int64_t row_bytes = vocab * elem_bytes;
+  int c = vocab > kRcListCap ? 2 : 1;
+  while (c < kRcMaxCluster && row_bytes > (int64_t)c * 32768) c *= 2;
+  while (c < kRcMaxCluster && rows * c * 2 <= 592 && row_bytes > (int64_t)c * 8192) c *= 2;
+  return c;
+}
+
+template <int DT>
+static int launch_cluster_path(cudaStream_t st, const SampleParams& sp) {
+  const int es = (int)sizeof(typename Elem<DT>::type), vec = 16 / es;
+  RcSampleParams p{};
+  p.sp = sp;
+  p.cluster = cluster_size(sp.rows, sp.vocab, es);
+  if (const char* f = getenv("TLX_CLUSTER")) p.cluster = atoi(f);
+  p.part_len = ((sp.vocab + p.cluster - 1) / p.cluster + vec - 1) / vec * vec;
+  if (p.part_len > kRcMaxPart) { p.cluster = 1; p.part_len = 0; }   // longer than a cluster holds: rc_slow_row
+  size_t part_bytes = (size_t)p.part_len * es + 32;
+  if (part_bytes < kRcMinPartBytes) part_bytes = kRcMinPartBytes;
+  const size_t smem = RcLayout(p.cluster, true).off_part + part_bytes;
+  int rc;
+  if ((rc = ensure_smem((const void*)sample_cluster_kernel<DT>, smem, "sample")) != TLX_OK) return rc;
+  {
+    static std::mutex mu;
+    static bool done[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < 0 || dev >= 64 || !done[dev]) {
+      cudaError_t e = cudaFuncSetAttribute((const void*)sample_cluster_kernel<DT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute((const void*)sample_cluster_kernel<DT>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "sample: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+      if (dev >= 0 && dev < 64) done[dev] = true;
+    }
+  }
+#ifdef TLX_TIMELINE
+  p.sp.timeline = (long long*)sp.counters;   // timeline builds: the caller's workspace receives the stamps
+#endif
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(sp.rows * p.cluster));
+  cfg.blockDim = dim3(kRcThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)p.cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<DT>, p);
+  if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "sample: %s", cudaGetErrorString(e)); }
+  count_launch();
+  return TLX_OK;
+}
+
 static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* workspace) {
   const StreamLayout l = stream_layout(sp.rows, sp.vocab);
   const int stages = debug_stages() & 15;
@@ -2352,6 +2411,8 @@ static int sample_impl(void* stream, const void* logits, int dtype, int64_t rows
   p.rowstate = reinterpret_cast<RowState*>((unsigned char*)workspace + 256);
   p.records = (unsigned char*)workspace + counters_bytes(rows);
 
+  if (const char* f = getenv("TLX_SAMPLE_PATH"); f && f[0] == 'c')
+    return dtype == TLX_BF16 ? launch_cluster_path<TLX_BF16>(st, p) : launch_cluster_path<TLX_F32>(st, p);
   if (stream_path_serves(dtype, rows, vocab, row_stride, logits)) {
     // the rows are split over the CTAs; the row-per-CTA kernel is kept for comparison (diagnostic switch
     // TLX_SAMPLE_PATH=rows): it is faster on batches without wide rows and much slower with them

@@ -1,0 +1,1006 @@
+// Fused sampler, one kernel: a row is spread over a thread-block cluster (row_cluster.cuh), included by sampler.cu.
+//
+// Rows with 1 <= top_k <= 1024 (greedy rows are top_k = 1): every CTA filters its part against the cluster's bound,
+// scores its candidates (x / T + Gumbel of the noise there) and leaves them in its list; the leader gathers the
+// lists over distributed shared memory, cuts them to the top-k set (radix descent over the keys) and decides.
+//
+// Decision.  A token is kept if the softmax mass of the greater values of the set is below top_p, so nothing has to
+// be sorted: the best score of the set wins if the mass above its value is below top_p * Z; otherwise no lower
+// value is kept either, and the best score among the greater values is tried.  One or two rounds as a rule.
+//
+// Rows without top-k: every CTA publishes its greatest element and that element's score.  An element can only win if
+// no greater (or equal) element has a greater score, because a greater value is kept whenever the smaller one is;
+// so what the published pairs dominate is out, and before its noise is even looked at an element is out if its
+// value plus the greatest Gumbel term there is would not do.  The survivors (a handful) go to the leader, and the
+// mass above its best ones comes from one more pass over the parts, which are still in shared memory.
+//
+// Anything these lists cannot hold (huge groups of equal values, top_k > 1024), and rows without a finite maximum,
+// takes rc_slow_row: exact, any top-k, by passes over the row in global memory.
+#pragma once
+#include "row_cluster.cuh"
+
+namespace tlx {
+
+struct RcSampleParams {
+  SampleParams sp;
+  int cluster;
+  int64_t part_len;   // elements of a part, a multiple of a 16-byte vector
+};
+
+// Warp 0: the bin of a 256-bin histogram that holds the need-th element counted from the top; out[0] = bin,
+// out[1] = elements in higher bins, out[2] = elements in the bin.
+__device__ __forceinline__ void rc_pick_bin(const uint32_t* h, int need, int* out) {
+  const int lane = lane_id();
+  const int hi = 255 - 8 * lane;
+  uint32_t local = 0;
+#pragma unroll 1
+  for (int j = 0; j < 8; ++j) local += h[hi - j];
+  uint32_t incl = local;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+    if (lane >= o) incl += up;
+  }
+  uint32_t run = incl - local;
+  if (run < (uint32_t)need && incl >= (uint32_t)need) {
+#pragma unroll 1
+    for (int j = 0; j < 8; ++j) {
+      const uint32_t c = h[hi - j];
+      if (run + c >= (uint32_t)need) { out[0] = hi - j; out[1] = (int)run; out[2] = (int)c; break; }
+      run += c;
+    }
+  }
+}
+
+// Key of a score for an unsigned maximum; NaN is below everything.
+__device__ __forceinline__ uint32_t rc_score_key(float a) { return a == a ? f32_key(a) : 0u; }
+__device__ __forceinline__ float rc_cut(float smax) {
+  return fabsf(smax) < INFINITY ? smax - (kGumbelSlack + 1e-5f * fabsf(smax)) : smax;
+}
+__device__ __forceinline__ unsigned long long rc_win_make(float y, int64_t tok) {
+  return ((unsigned long long)rc_score_key(y) << 32) | (uint32_t)(0x7FFFFFFF - (int32_t)tok);
+}
+
+// One row by passes over global memory, any top-k, ties or NaNs.  Returns the token.
+template <int DT>
+static __device__ __noinline__ int rc_slow_row(const typename Elem<DT>::type* __restrict__ row, int64_t n, int64_t K, float p,
+                                               float T_, const NoiseSrc& noise, int64_t nrow, RcShared& s) {
+  using T = typename Elem<DT>::type;
+  int tog = 0;
+  auto composite = [](T v, int64_t c) { return ((uint64_t)Elem<DT>::key(v) << 32) | (uint32_t)(0x7FFFFFFF - (int32_t)c); };
+  auto block_max = [&](uint64_t v) {
+    const uint32_t hi = rc_max_u32((uint32_t)(v >> 32), s, tog);
+    const uint32_t lo = rc_max_u32((uint32_t)(v >> 32) == hi ? (uint32_t)v : 0u, s, tog);
+    return ((uint64_t)hi << 32) | lo;
+  };
+  __syncthreads();
+  uint64_t best = 0;
+  for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) { const uint64_t x = composite(v, c); best = x > best ? x : best; });
+  const uint64_t top = block_max(best);
+  const int top_col = 0x7FFFFFFF - (int)(uint32_t)top;
+  if (T_ < kSamplingEps) return top_col;
+  const float xmax = key_f32((uint32_t)(top >> 32));
+  uint64_t least = 0;   // least composite of the top-k set
+  if (K < n) {
+    int need = (int)K;
+#pragma unroll 1
+    for (int sh = 56; sh >= 0; sh -= 8) {
+      s.hist[threadIdx.x] = 0;
+      __syncthreads();
+      for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
+        const uint64_t x = composite(v, c);
+        if (sh == 56 || ((x ^ least) >> (sh + 8)) == 0) atomicAdd(&s.hist[(x >> sh) & 255], 1u);
+      });
+      __syncthreads();
+      if (warp_id() == 0) rc_pick_bin(s.hist, need, s.pick);
+      __syncthreads();
+      least |= (uint64_t)(uint32_t)s.pick[0] << sh;
+      need -= s.pick[1];
+      if (s.pick[2] == need) break;   // the whole bin belongs to the set
+    }
+  }
+  double z = 0.0, unused = 0.0;
+  for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
+    if (composite(v, c) >= least) z += (double)expf(elem_as_float<DT>(v) - xmax);
+  });
+  rc_sum2_f64(z, unused, s, tog);
+  float above = -INFINITY;   // only values above this one are still in question
+  bool first = true;
+#pragma unroll 1
+  for (int round = 0; round < 4096; ++round) {
+    auto eligible = [&](T v, int64_t c) { return composite(v, c) >= least && (first || elem_as_float<DT>(v) > above); };
+    uint32_t a = 0;
+    for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
+      if (eligible(v, c)) a = max(a, rc_score_key(__fdiv_rn(elem_as_float<DT>(v), T_) + gumbel_screen(noise.at(nrow, c))));
+    });
+    const uint32_t ak = rc_max_u32(a, s, tog);
+    if (ak == 0) return top_col;   // nothing has a score
+    const float cut = rc_cut(key_f32(ak));
+    uint64_t w = 0;
+    for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
+      if (eligible(v, c)) {
+        const float u = noise.at(nrow, c), q = __fdiv_rn(elem_as_float<DT>(v), T_);
+        if (q + gumbel_screen(u) >= cut) { const uint64_t x = rc_win_make(q + gumbel_exact(u), c); w = x > w ? x : w; }
+      }
+    });
+    w = block_max(w);
+    const int tok = 0x7FFFFFFF - (int)(uint32_t)w;
+    const float wx = elem_as_float<DT>(row[tok]);
+    double mass = 0.0, count = 0.0;
+    for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
+      const float x = elem_as_float<DT>(v);
+      if (x > wx && composite(v, c) >= least) { mass += (double)expf(x - xmax); count += 1.0; }
+    });
+    rc_sum2_f64(mass, count, s, tog);
+    if (count == 0.0 || !(mass / z >= (double)p)) return tok;
+    above = wx;
+    first = false;
+  }
+  return top_col;
+}
+
+// Leader: cuts the gathered list to the top-K set.  Elements outside it lose their score (-inf) and their weight
+// (value -inf).  K-th greatest key by radix descent from the first bit in which the keys differ; ties at the K-th
+// key are admitted by ascending column.
+static __device__ __noinline__ void rc_cut_to_k(RcShared& s, int m, int K, int64_t part_len, float* lx, float* ls,
+                                                const unsigned short* lpos, uint32_t* bins) {
+  int tog = 2;
+  uint32_t kmax = 0, kmin_inv = 0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < m; i += kRcThreads) {
+    const uint32_t k = f32_key(lx[i]);
+    kmax = max(kmax, k);
+    kmin_inv = max(kmin_inv, ~k);
+  }
+  kmax = rc_max_u32(kmax, s, tog);
+  const uint32_t kmin = ~rc_max_u32(kmin_inv, s, tog);
+  // One histogram of 2048 bins over the range of the keys; the K-th key's bin then holds a few elements, which are
+  // ranked by counting.
+  {
+    const uint32_t range = kmax - kmin;
+    const int shift = range >> 11 ? 21 - __clz(range) : 0;
+    uint4* b4 = reinterpret_cast<uint4*>(bins);
+    b4[threadIdx.x] = make_uint4(0, 0, 0, 0);
+    b4[threadIdx.x + kRcThreads] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x == 0) s.pick[3] = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int i = threadIdx.x; i < m; i += kRcThreads) atomicAdd(&bins[(kRcBins - 1) - ((f32_key(lx[i]) - kmin) >> shift)], 1u);
+    __syncthreads();
+    const uint4 c0 = b4[2 * threadIdx.x], c1 = b4[2 * threadIdx.x + 1];
+    const int sum = (int)(c0.x + c0.y + c0.z + c0.w + c1.x + c1.y + c1.z + c1.w);
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane_id() >= o) incl += up;
+    }
+    if (lane_id() == 31) s.red_u32[0][warp_id()] = (uint32_t)incl;
+    __syncthreads();
+#pragma unroll 1
+    for (int w = 0; w < warp_id(); ++w) incl += (int)s.red_u32[0][w];
+    if (incl - sum < K && incl >= K) {
+      int run = incl - sum;
+#pragma unroll 1
+      for (int j = 0; j < 8; ++j) {
+        const int c = (int)bins[8 * threadIdx.x + j];
+        if (run + c >= K) { s.pick[0] = 8 * threadIdx.x + j; s.pick[1] = run; s.pick[2] = c; break; }
+        run += c;
+      }
+    }
+    __syncthreads();
+    const int bin = s.pick[0], need = K - s.pick[1], in_bin = s.pick[2];
+    if (in_bin <= 256) {
+      uint64_t* list = reinterpret_cast<uint64_t*>(bins);   // (the histogram has been read)
+#pragma unroll 1
+      for (int i = threadIdx.x; i < m; i += kRcThreads) {
+        const uint32_t k = f32_key(lx[i]);
+        const int b = (kRcBins - 1) - (int)((k - kmin) >> shift);
+        if (b > bin) { lx[i] = -INFINITY; ls[i] = -INFINITY; }
+        else if (b == bin)
+          list[atomicAdd(&s.pick[3], 1)] = ((uint64_t)k << 32) | (uint32_t)i;
+      }
+      __syncthreads();
+      if ((int)threadIdx.x < in_bin) {
+        const uint64_t c = list[threadIdx.x];
+        const int i = (int)(c & 2047u);
+        const int64_t col = rc_column(s, lpos, i, part_len);
+        int before = 0;
+#pragma unroll 1
+        for (int j = 0; j < in_bin; ++j) {
+          const uint64_t o = list[j];
+          if ((o >> 32) > (c >> 32)) ++before;
+          else if ((o >> 32) == (c >> 32) && o != c && rc_column(s, lpos, (int)(o & 2047u), part_len) < col) ++before;
+        }
+        if (before >= need) { lx[i] = -INFINITY; ls[i] = -INFINITY; }
+      }
+      __syncthreads();
+      return;
+    }
+  }
+  int need = K, ties = m;
+  uint32_t vk = kmax;          // prefix of the K-th key; bits below `top` are still to be found
+  int top = kmax == kmin ? 0 : 32 - __clz(kmax ^ kmin);
+  if (top < 32) vk &= ~((1u << top) - 1u); else vk = 0;
+#pragma unroll 1
+  while (top > 0) {
+    const int sh = top > 8 ? top - 8 : 0;
+    s.hist[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int i = threadIdx.x; i < m; i += kRcThreads) {
+      const uint32_t k = f32_key(lx[i]);
+      if (top == 32 || ((k ^ vk) >> top) == 0) atomicAdd(&s.hist[(k >> sh) & ((1u << (top - sh)) - 1u)], 1u);
+    }
+    __syncthreads();
+    if (warp_id() == 0) rc_pick_bin(s.hist, need, s.pick);
+    __syncthreads();
+    vk |= (uint32_t)s.pick[0] << sh;
+    need -= s.pick[1];
+    ties = s.pick[2];
+    top = sh;
+    __syncthreads();
+    if (ties == need) break;   // everything in the bin belongs to the set: vk is its lower end
+  }
+  // ties at the K-th key (vk is complete then): the `need` lowest columns stay.  Up to 256 ties are listed first.
+  const bool cut_ties = need < ties;
+  const bool listed = cut_ties && ties <= 256;
+  if (threadIdx.x == 0) s.pick[3] = 0;
+  __syncthreads();
+  if (listed) {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < m; i += kRcThreads)
+      if (f32_key(lx[i]) == vk) s.hist[atomicAdd(&s.pick[3], 1)] = (uint32_t)rc_column(s, lpos, i, part_len);
+    __syncthreads();
+  }
+#pragma unroll 1
+  for (int i = threadIdx.x; i < m; i += kRcThreads) {
+    const uint32_t k = f32_key(lx[i]);
+    bool out = k < vk;
+    if (cut_ties && k == vk) {
+      const uint32_t col = (uint32_t)rc_column(s, lpos, i, part_len);
+      int before = 0;
+#pragma unroll 1
+      for (int j = 0; j < (listed ? ties : m); ++j)
+        if (listed ? s.hist[j] < col : f32_key(lx[j]) == vk && (uint32_t)rc_column(s, lpos, j, part_len) < col) ++before;
+      out = before >= need;
+    }
+    if (out) ls[i] = __int_as_float(0x7FC00001);   // marked; the values are still being compared by other threads
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int i = threadIdx.x; i < m; i += kRcThreads)
+    if (__float_as_uint(ls[i]) == 0x7FC00001u) { ls[i] = -INFINITY; lx[i] = -INFINITY; }
+  __syncthreads();
+}
+
+// Leader: the best element of the gathered list among those above `above` (all of them if first): its column, its
+// value in s.win_x.  -1 if none has a score.
+template <int DT>
+static __device__ __noinline__ int rc_best_of_list(RcShared& s, int m, bool first, float above, int64_t part_len,
+                                                   const float* lx, const float* ls, const unsigned short* lpos, float T_,
+                                                   const NoiseSrc& noise, int64_t nrow) {
+  int tog = 2;
+  uint32_t a = 0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < m; i += kRcThreads)
+    if (first || lx[i] > above) a = max(a, rc_score_key(ls[i]));
+  const uint32_t ak = rc_max_u32(a, s, tog);
+  if (ak <= 0x007FFFFFu) return -1;   // NaN or -inf
+  const float cut = rc_cut(key_f32(ak));
+  uint32_t near_ = 0;
+  if (threadIdx.x == 0) s.win = 0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < m; i += kRcThreads)
+    if ((first || lx[i] > above) && ls[i] >= cut) ++near_;
+  near_ = rc_sum_u32(near_, s, tog);
+#pragma unroll 1
+  for (int i = threadIdx.x; i < m; i += kRcThreads) {
+    if ((first || lx[i] > above) && ls[i] >= cut) {
+      const int64_t col = rc_column(s, lpos, i, part_len);
+      // several within the screening slack of the best: decided on the f64-evaluated noise
+      float y = 0.f;
+      if (near_ > 1) y = __fdiv_rn(lx[i], T_) + gumbel_exact(noise.at(nrow, col));
+      atomicMax(&s.win, rc_win_make(y, col));
+    }
+  }
+  __syncthreads();
+  const int tok = 0x7FFFFFFF - (int)(uint32_t)s.win;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < m; i += kRcThreads)
+    if ((first || lx[i] > above) && ls[i] >= cut && rc_column(s, lpos, i, part_len) == tok) s.win_x = lx[i];
+  __syncthreads();
+  return tok;
+}
+
+// Leader: at most 256 candidates.  Every thread ranks one by counting, which sorts the top-K set; one warp then takes
+// the softmax prefix, the top-p threshold and the best score among the kept ones.  Returns the token, -1 if no kept
+// one has a score.
+constexpr int kRcSmall = 256;
+static __device__ __noinline__ int rc_decide_small(RcShared& s, int m, int K, float pp, int64_t part_len, const float* lx,
+                                                   const float* ls, const unsigned short* lpos, unsigned char* scratch,
+                                                   float T_, const NoiseSrc& noise, int64_t nrow) {
+  uint64_t* comp = reinterpret_cast<uint64_t*>(scratch);
+  float* sx = reinterpret_cast<float*>(comp + kRcSmall);
+  float* ss = sx + kRcSmall;
+  int* scol = reinterpret_cast<int*>(ss + kRcSmall);
+  const int i = threadIdx.x;
+  uint64_t mine = 0;
+  float x = 0.f, a = 0.f;
+  if (i < m) {
+    x = lx[i];
+    a = ls[i];
+    mine = ((uint64_t)f32_key(x) << 32) | (uint32_t)(0x7FFFFFFF - (int32_t)rc_column(s, lpos, i, part_len));
+  }
+  comp[i] = mine;
+  __syncthreads();
+  if (i < m) {
+    int rank = 0;
+    const ulonglong2* c2 = reinterpret_cast<const ulonglong2*>(comp);
+#pragma unroll 4
+    for (int j = 0; j < (m + 1) / 2; ++j) {
+      const ulonglong2 c = c2[j];
+      rank += (c.x > mine ? 1 : 0) + (c.y > mine ? 1 : 0);
+    }
+    if (rank < K) {
+      sx[rank] = x;
+      ss[rank] = a;
+      scol[rank] = 0x7FFFFFFF - (int)(uint32_t)mine;
+    }
+  }
+  __syncthreads();
+  if (warp_id() == 0) {
+    const int lane = lane_id(), n = min(m, K), per = (n + 31) / 32;
+    const int i0 = lane * per, i1 = min(i0 + per, n);
+    const float x0 = sx[0];
+    double acc = 0.0;
+#pragma unroll 1
+    for (int j = i0; j < i1; ++j) acc += (double)expf(sx[j] - x0);
+    double incl = acc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const double up = shfl_up_f64(incl, o);
+      if (lane >= o) incl += up;
+    }
+    const double Z = __hiloint2double(__shfl_sync(0xFFFFFFFFu, __double2hiint(incl), 31),
+                                      __shfl_sync(0xFFFFFFFFu, __double2loint(incl), 31));
+    double run = incl - acc;
+    int below = 0;
+#pragma unroll 1
+    for (int j = i0; j < i1; ++j) {
+      run += (double)expf(sx[j] - x0);
+      below += run / Z < (double)pp ? 1 : 0;
+    }
+    below = __reduce_add_sync(0xFFFFFFFFu, below);
+    // a sum that is not a number keeps everything
+    const float thr = Z == Z ? sx[min(below, n - 1)] : -INFINITY;
+    uint32_t best = 0;
+#pragma unroll 1
+    for (int j = i0; j < i1; ++j)
+      if (sx[j] >= thr) best = max(best, rc_score_key(ss[j]));
+    best = __reduce_max_sync(0xFFFFFFFFu, best);
+    int tok = -1;
+    if (best > 0x007FFFFFu) {
+      const float cut = rc_cut(key_f32(best));
+      int near_ = 0;
+      uint32_t hi = 0, lo = 0;
+#pragma unroll 1
+      for (int j = i0; j < i1; ++j)
+        if (sx[j] >= thr && ss[j] >= cut) { ++near_; lo = max(lo, (uint32_t)(0x7FFFFFFF - scol[j])); }
+      near_ = __reduce_add_sync(0xFFFFFFFFu, near_);
+      if (near_ > 1) {   // several within the screening slack of the best: decided on the f64-evaluated noise
+        lo = 0;
+#pragma unroll 1
+        for (int j = i0; j < i1; ++j)
+          if (sx[j] >= thr && ss[j] >= cut) {
+            const uint32_t k = rc_score_key(__fdiv_rn(sx[j], T_) + gumbel_exact(noise.at(nrow, scol[j])));
+            const uint32_t c = (uint32_t)(0x7FFFFFFF - scol[j]);
+            if (k > hi || (k == hi && c > lo)) { hi = k; lo = c; }
+          }
+        const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, hi);
+        if (hi != top) lo = 0;
+      }
+      lo = __reduce_max_sync(0xFFFFFFFFu, lo);
+      tok = 0x7FFFFFFF - (int)lo;
+    }
+    if (lane == 0) s.pick[0] = tok;
+  }
+  __syncthreads();
+  return s.pick[0];
+}
+
+// ---- rows without top-k ------------------------------------------------------------------------------------------
+constexpr int kRcWideCap = 512;     // survivors of a CTA
+constexpr int kRcWideSend = 32;     // survivors a CTA may hand to the leader
+constexpr int kRcQueue = 384;       // positions a warp has noted and not yet scored (up to 127 + 32 lanes x 8)
+static_assert(kRcWarps * kRcQueue * 2 + kRcWideCap * 4 <= kRcListCap * 4, "the queues lie behind the scores");
+static_assert(kRcMaxCluster * kRcWideSend == 512, "the leader's copies of the survivors");
+
+// The places of the survivors in the list's space: this CTA's own ones, and (leader) those that the CTAs have sent,
+// kRcWideSend places each.
+struct RcWideLists {
+  unsigned short *pos, *queue;
+  float *x, *s, *all_x, *all_s;
+  int* all_col;
+  __device__ __forceinline__ RcWideLists(unsigned char* smem, const RcLayout& l) {
+    pos = reinterpret_cast<unsigned short*>(smem + l.off_pos);
+    all_s = reinterpret_cast<float*>(smem + l.off_pos + kRcWideCap * 2);
+    x = reinterpret_cast<float*>(smem + l.off_x);
+    all_x = x + kRcWideCap;
+    all_col = reinterpret_cast<int*>(all_x + kRcMaxCluster * kRcWideSend);
+    s = reinterpret_cast<float*>(smem + l.off_s);
+    queue = reinterpret_cast<unsigned short*>(s + kRcWideCap);
+  }
+};
+
+// What the passes over a row without top-k need of it.
+struct RcWideRow {
+  int64_t col0, nrow;
+  float rt, xmax;            // 1 / T; the row's greatest value
+  const float* dense;        // the part's noise, or null: the key
+  uint32_t k0, k1, ctr0;     // key; counter of the part's first element
+};
+
+// The least score of a survivor, by its value.
+struct RcLow {
+  float bx, bs, ms;   // at or below bx: bs; above it: ms
+  __device__ __forceinline__ float of(float x) const { return x <= bx ? bs : ms; }
+};
+// Whether an element can reach the score `cut`: its Gumbel term -log(-log u) is at most -log(1 - u).
+__device__ __forceinline__ bool rc_may_reach(float x, float u, float rt, float cut) {
+  return 1.0f - u <= __expf(fmaf(x, rt, -cut)) * 1.0001f;
+}
+template <int DT>
+__device__ __forceinline__ void rc_keep_survivor(float x, float u, int i, const RcWideRow& r, RcShared& s, const RcWideLists& w) {
+  const float a = fmaf(x, r.rt, gumbel_screen(u));
+  bool out = !(a > -INFINITY);
+#pragma unroll 1
+  for (int j = 0; j < 6; ++j) out = out || (x <= s.cut_x[j] && a < s.cut_s[j]);
+  if (!out) {
+    const int slot = atomicAdd(&s.n_list, 1);
+    if (slot < kRcWideCap) { w.x[slot] = x; w.s[slot] = a; w.pos[slot] = (unsigned short)i; }
+  }
+}
+
+// Noise from a key.  Scores `count` (at most 128) noted elements, four per lane: four interleaved chains of dependent
+// rounds (with the two warps that a scheduler has here, one chain would leave it idle).
+template <int DT>
+__device__ __forceinline__ void rc_score_noted(const RcPart<DT>& part, const unsigned short* queue, int count, const RcLow& low,
+                                               const RcWideRow& r, RcShared& s, const RcWideLists& w) {
+  int at[4];
+  float u[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int q = lane_id() + 32 * k;
+    at[k] = q < count ? queue[q] : -1;
+    u[k] = fmaxf(threefry_uniform01(r.k0, r.k1, r.ctr0 + (uint32_t)at[k]), kF32Tiny);
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (at[k] < 0) continue;
+    const float x = elem_as_float<DT>(part.elem(at[k]));
+    if (rc_may_reach(x, u[k], r.rt, low.of(x))) rc_keep_survivor<DT>(x, u[k], at[k], r, s, w);
+  }
+}
+
+// The part's survivors (see the top of the file) into the CTA's list; with `mass`, also the part's share of the softmax
+// denominator (returned).
+//   From a key: a warp notes the positions whose value allows a survivor at all and makes their noise 128 at a time.
+//   From a tensor: the noise is read beside the values, and a vector is looked into if its greatest value with its
+//   greatest noise could survive.
+template <int DT>
+__device__ __forceinline__ double rc_survivors(const RcPart<DT>& part, const RcLow& low, float xcut, bool mass, const RcWideRow& r,
+                                               RcShared& s, const RcWideLists& l) {
+  using T = typename Elem<DT>::type;
+  constexpr int VEC = RcPart<DT>::VEC;
+  const int lane = lane_id();
+  unsigned short* queue = l.queue + warp_id() * kRcQueue;
+  const bool aligned = r.dense && (reinterpret_cast<uintptr_t>(r.dense - part.off) & 15) == 0;
+  double z = 0.0;
+  int waiting = 0;
+#pragma unroll 1
+  for (int v0 = 0; v0 < part.nvec; v0 += kRcThreads) {
+    const int v = v0 + threadIdx.x;
+    const bool last = v0 + kRcThreads >= part.nvec;
+    uint32_t mask = 0;
+    float u[VEC];
+    if (v < part.nvec) {
+      const uint4 w = part.vec[v];
+      const T* e = reinterpret_cast<const T*>(&w);
+      const int i0 = v * VEC - part.off;
+      if (r.dense) {
+        if (aligned && i0 >= 0 && i0 + VEC <= part.n) {
+#pragma unroll
+          for (int j = 0; j < VEC; j += 4) {
+            const float4 q = __ldcs(reinterpret_cast<const float4*>(r.dense + i0 + j));
+            u[j] = q.x; u[j + 1] = q.y; u[j + 2] = q.z; u[j + 3] = q.w;
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < VEC; ++j) u[j] = i0 + j >= 0 && i0 + j < part.n ? __ldg(r.dense + i0 + j) : 0.f;
+        }
+      }
+      if (mass) {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) z += (double)expf(elem_as_float<DT>(e[j]) - r.xmax);
+      }
+      if (r.dense) {
+        float xm = elem_as_float<DT>(e[0]), um = u[0];
+#pragma unroll
+        for (int j = 1; j < VEC; ++j) { xm = fmaxf(xm, elem_as_float<DT>(e[j])); um = fmaxf(um, u[j]); }
+        if (rc_may_reach(xm, um, r.rt, low.of(xm))) {
+#pragma unroll
+          for (int j = 0; j < VEC; ++j) {
+            const float x = elem_as_float<DT>(e[j]);
+            if (x > -INFINITY && rc_may_reach(x, u[j], r.rt, low.of(x))) rc_keep_survivor<DT>(x, u[j], i0 + j, r, s, l);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < VEC; ++j) mask |= elem_as_float<DT>(e[j]) >= xcut ? 1u << j : 0u;
+        if (xcut == -INFINITY) {   // nothing is ruled out by its value: leave out what lies outside the part
+          for (int j = 0; j < VEC; ++j)
+            if (i0 + j < 0 || i0 + j >= part.n) mask &= ~(1u << j);
+        }
+      }
+    }
+    if (r.dense) continue;
+    if (__ballot_sync(0xFFFFFFFFu, mask != 0)) {
+      int incl = __popc(mask);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      int at = waiting + incl - __popc(mask);
+      while (mask) {
+        const int j = __ffs(mask) - 1;
+        mask &= mask - 1;
+        queue[at++] = (unsigned short)(v * VEC + j - part.off);
+      }
+      waiting += __shfl_sync(0xFFFFFFFFu, incl, 31);
+      __syncwarp();
+    }
+    while (waiting >= 128 || (last && waiting > 0)) {
+      const int count = min(waiting, 128);
+      waiting -= count;
+      rc_score_noted<DT>(part, queue + waiting, count, low, r, s, l);
+    }
+    __syncwarp();
+  }
+  return z;
+}
+
+// Warp 0: the best entry of a list of m among those above `above` (all of them if `first`): its index, -1 if none has
+// a score.  col_of(i) is the column of entry i.
+template <typename ColOf>
+__device__ __forceinline__ int rc_warp_best(int m, bool first, float above, const float* lx, const float* ls, float T_,
+                                            const NoiseSrc& noise, int64_t nrow, ColOf col_of) {
+  uint32_t a = 0;
+#pragma unroll 1
+  for (int i = lane_id(); i < m; i += 32)
+    if (first || lx[i] > above) a = max(a, rc_score_key(ls[i]));
+  a = __reduce_max_sync(0xFFFFFFFFu, a);
+  if (a <= 0x007FFFFFu) return -1;
+  const float cut = rc_cut(key_f32(a));
+  int near_ = 0, idx = -1;
+#pragma unroll 1
+  for (int i = lane_id(); i < m; i += 32)
+    if ((first || lx[i] > above) && ls[i] >= cut) { ++near_; idx = i; }
+  near_ = __reduce_add_sync(0xFFFFFFFFu, near_);
+  if (near_ > 1) {
+    uint32_t hi = 0, lo = 0;
+    idx = -1;
+#pragma unroll 1
+    for (int i = lane_id(); i < m; i += 32)
+      if ((first || lx[i] > above) && ls[i] >= cut) {
+        const int64_t col = col_of(i);
+        const uint32_t k = rc_score_key(__fdiv_rn(lx[i], T_) + gumbel_exact(noise.at(nrow, col)));
+        const uint32_t c = (uint32_t)(0x7FFFFFFF - (int32_t)col);
+        if (k > hi || (k == hi && c > lo)) { hi = k; lo = c; idx = i; }
+      }
+    const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, hi);
+    const uint32_t low = __reduce_max_sync(0xFFFFFFFFu, hi == top ? lo : 0u);
+    if (hi != top || lo != low) idx = -1;
+  }
+  return __reduce_max_sync(0xFFFFFFFFu, idx);
+}
+
+// Warp 0: more than kRcWideSend survivors: drops those that another one dominates, in place.
+__device__ __forceinline__ int rc_thin_out(int m, float* lx, float* ls, unsigned short* lpos) {
+  const int lane = lane_id();
+  float above = -INFINITY;
+  bool first = true;
+  // marks are collected in the scores' sign of life: a dominated entry gets the score -inf
+#pragma unroll 1
+  for (int round = 0; round < 2 * kRcWideSend; ++round) {
+    uint32_t a = 0;
+#pragma unroll 1
+    for (int i = lane; i < m; i += 32) if (first || lx[i] > above) a = max(a, rc_score_key(ls[i]));
+    a = __reduce_max_sync(0xFFFFFFFFu, a);
+    if (a <= 0x007FFFFFu) break;
+    uint32_t xk = 0;
+#pragma unroll 1
+    for (int i = lane; i < m; i += 32)
+      if ((first || lx[i] > above) && rc_score_key(ls[i]) == a) xk = max(xk, f32_key(lx[i]));
+    const float x = key_f32(__reduce_max_sync(0xFFFFFFFFu, xk)), cut = rc_cut(key_f32(a));
+#pragma unroll 1
+    for (int i = lane; i < m; i += 32)
+      if ((first || lx[i] > above) && lx[i] <= x && ls[i] < cut) ls[i] = -INFINITY;
+    __syncwarp();
+    above = x;
+    first = false;
+  }
+  int kept = 0;
+#pragma unroll 1
+  for (int i0 = 0; i0 < m; i0 += 32) {
+    const int i = i0 + lane;
+    const float x = i < m ? lx[i] : 0.f, a = i < m ? ls[i] : -INFINITY;
+    const unsigned short q = i < m ? lpos[i] : 0;
+    const unsigned live = __ballot_sync(0xFFFFFFFFu, a > -INFINITY);
+    const int to = kept + __popc(live & ((1u << lane) - 1u));
+    if (a > -INFINITY) { lx[to] = x; ls[to] = a; lpos[to] = q; }
+    kept += __popc(live);
+    __syncwarp();
+  }
+  return kept;
+}
+
+// The thread's share of the softmax mass above two values (q0 <= q1).
+template <int DT>
+__device__ __forceinline__ void rc_mass_above(const RcPart<DT>& part, float xmax, float q0, float q1, double& m0, double& m1) {
+  using T = typename Elem<DT>::type;
+  constexpr int VEC = RcPart<DT>::VEC;
+#pragma unroll 1
+  for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) {
+    const uint4 w = part.vec[v];
+    if (!rc_any_at_least<DT>(w, q0)) continue;
+    const T* e = reinterpret_cast<const T*>(&w);
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+      const float x = elem_as_float<DT>(e[j]);
+      const double y = (double)(x > q0 ? expf(x - xmax) : 0.f);
+      m0 += y;
+      m1 += x > q1 ? y : 0.0;
+    }
+  }
+}
+
+// Rows with 1 <= top_k <= 1024 and greedy rows.  Returns the token in the leader (rank 0), -1 if the row has to be
+// answered by rc_slow_row; the other CTAs return -1 when they may leave.
+template <int DT>
+__device__ __forceinline__ int rc_normal_row(const RcSampleParams& p, const RcPart<DT>& part, int64_t col0, uint32_t rank, int K,
+                                             float pp, float T_, int64_t nrow, RcShared& s, const RcLayout& l,
+                                             unsigned char* smem, int& tog) {
+  float* lx = reinterpret_cast<float*>(smem + l.off_x);
+  float* ls = reinterpret_cast<float*>(smem + l.off_s);
+  unsigned short* lpos = reinterpret_cast<unsigned short*>(smem + l.off_pos);
+  uint32_t* bound = reinterpret_cast<uint32_t*>(smem + l.off_bound);
+  const bool greedy = T_ < kSamplingEps;
+  float thr = key_f32(0x80u << 16);
+  if (p.sp.vocab > kRcListCap) {
+    GroupMax<DT> gm;
+    gm.init();
+#pragma unroll 2
+    for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) gm.add(part.vec[v]);
+    rc_publish_maxima<DT>(gm, l.bound_words, bound);
+    cl_sync();
+    TLX_STAMP(p.sp, 2);
+    thr = key_f32(rc_bound_key16(bound, l.bound_words, K, s) << 16);
+  } else {
+    cl_sync();
+  }
+  TLX_STAMP(p.sp, 3);
+  rc_filter<DT>(part, thr, s, lx, lpos);
+  __syncthreads();
+  TLX_STAMP(p.sp, 4);
+  const int nl = min(s.n_list, kRcListCap);
+#pragma unroll 1
+  for (int i = threadIdx.x; i < nl; i += kRcThreads) {
+    float a = 0.f;
+    if (!greedy) a = __fdiv_rn(lx[i], T_) + gumbel_screen(p.sp.noise.at(nrow, col0 + lpos[i]));
+    ls[i] = a;
+  }
+  TLX_STAMP(p.sp, 5);
+  cl_sync();
+  TLX_STAMP(p.sp, 6);
+  if (rank != 0) {
+    cl_sync();
+    return -1;
+  }
+  const int m = rc_gather(s, p.cluster, lx, ls, lpos);
+  cl_arrive();   // the other CTAs may leave
+  TLX_STAMP(p.sp, 7);
+  int tok = -1;
+  if (m > 0 && greedy) {
+    if (threadIdx.x == 0) s.win = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int i = threadIdx.x; i < m; i += kRcThreads)
+      atomicMax(&s.win, ((unsigned long long)f32_key(lx[i]) << 32) |
+                            (uint32_t)(0x7FFFFFFF - (int32_t)rc_column(s, lpos, i, p.part_len)));
+    __syncthreads();
+    tok = 0x7FFFFFFF - (int)(uint32_t)s.win;
+  } else if (m > 0 && m <= kRcSmall) {
+    tok = rc_decide_small(s, m, K, pp, p.part_len, lx, ls, lpos, smem + l.off_part, T_, p.sp.noise, nrow);
+  } else if (m > 0) {
+    if (m > K) rc_cut_to_k(s, m, K, p.part_len, lx, ls, lpos, reinterpret_cast<uint32_t*>(smem + l.off_part));
+    TLX_STAMP(p.sp, 8);
+    uint32_t k0 = 0;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < m; i += kRcThreads) k0 = max(k0, f32_key(lx[i]));
+    const float x0 = key_f32(rc_max_u32(k0, s, tog));
+    float above = -INFINITY;
+    bool first = true;
+#pragma unroll 1
+    for (int round = 0; round < kRcListCap; ++round) {
+      const int t = rc_best_of_list<DT>(s, m, first, above, p.part_len, lx, ls, lpos, T_, p.sp.noise, nrow);
+      if (t < 0) break;
+      const float wx = s.win_x;
+      double mass = 0.0, z = 0.0;
+#pragma unroll 1
+      for (int i = threadIdx.x; i < m; i += kRcThreads) {
+        const double w = (double)expf(lx[i] - x0);
+        z += w;
+        if (lx[i] > wx) mass += w;
+      }
+      rc_sum2_f64(mass, z, s, tog);
+      if (mass == 0.0 || !(mass / z >= (double)pp)) { tok = t; break; }
+      above = wx;
+      first = false;
+    }
+  }
+  cl_wait();
+  TLX_STAMP(p.sp, 9);
+  return tok;
+}
+
+// Rows without top-k.  Returns the token in the leader, -1 if the row has to be answered by rc_slow_row.
+template <int DT>
+__device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart<DT>& part, int64_t col0, uint32_t rank, float pp,
+                                           float T_, int64_t nrow, RcShared& s, const RcLayout& layout, unsigned char* smem,
+                                           int& tog) {
+  using T = typename Elem<DT>::type;
+  constexpr int VEC = RcPart<DT>::VEC;
+  const RcWideLists l(smem, layout);
+  const NoiseSrc& noise = p.sp.noise;
+  RcWideRow r;
+  r.col0 = col0;
+  r.nrow = nrow;
+  r.rt = __frcp_rn(T_);
+  r.dense = noise.dense ? noise.dense_row(nrow) + col0 : nullptr;
+  r.k0 = r.k1 = r.ctr0 = 0;
+  if (!r.dense) {
+    r.k0 = noise.key_dev ? __ldg(noise.key_dev) : noise.k0;
+    r.k1 = noise.key_dev ? __ldg(noise.key_dev + 1) : noise.k1;
+    r.ctr0 = (uint32_t)(noise.row_of(nrow) * noise.vocab + col0);
+  }
+  // every thread's greatest element and its score; of the CTA: the greatest element and the best-scored one of these
+  GroupMax<DT> gm;
+  gm.init();
+#pragma unroll 2
+  for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) gm.add(part.vec[v]);
+  float x = -INFINITY, a = -INFINITY;
+#pragma unroll
+  for (int j = 0; j < GroupMax<DT>::kSlots; ++j) x = fmaxf(x, gm.slot(j));
+  if (x > -INFINITY) {
+    int at = 0;
+#pragma unroll 1
+    for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) {
+      if (!rc_any_at_least<DT>(part.vec[v], x)) continue;
+      const T* e = reinterpret_cast<const T*>(part.vec + v);
+#pragma unroll 1
+      for (int j = 0; j < VEC; ++j)
+        if (elem_as_float<DT>(e[j]) == x) at = v * VEC + j - part.off;
+    }
+    const float u = r.dense ? __ldg(r.dense + at) : fmaxf(threefry_uniform01(r.k0, r.k1, r.ctr0 + (uint32_t)at), kF32Tiny);
+    a = fmaf(x, r.rt, gumbel_screen(u));
+    if (!(a == a)) a = -INFINITY;
+  }
+  {
+    const uint32_t xk = f32_key(x), ak = rc_score_key(a);
+    const uint32_t xm = rc_max_u32(xk, s, tog), am = rc_max_u32(ak, s, tog);
+    const uint32_t xa = rc_max_u32(xk == xm ? ak : 0u, s, tog), ax = rc_max_u32(ak == am ? xk : 0u, s, tog);
+    if (threadIdx.x == 0) {
+      s.query[0] = key_f32(xm); s.query[1] = key_f32(xa);   // (the queries' place, not used yet)
+      s.query[2] = key_f32(ax); s.query[3] = key_f32(am);
+    }
+    if (rank == 0) {
+#pragma unroll 1
+      for (int i = threadIdx.x; i < kRcMaxCluster * kRcWideSend; i += kRcThreads) l.all_s[i] = -INFINITY;
+    }
+  }
+  cl_sync();
+  TLX_STAMP(p.sp, 2);
+  if ((int)threadIdx.x < p.cluster) {
+    const uint32_t q = cl_map(s.query, threadIdx.x);
+    const float v0 = cl_ld_f32(q), v1 = cl_ld_f32(q + 4), v2 = cl_ld_f32(q + 8), v3 = cl_ld_f32(q + 12);
+    s.dom_x[2 * threadIdx.x] = v0; s.dom_s[2 * threadIdx.x] = v1;
+    s.dom_x[2 * threadIdx.x + 1] = v2; s.dom_s[2 * threadIdx.x + 1] = v3;
+  }
+  __syncthreads();
+  float xmax = -INFINITY, ms = -INFINITY, bx = -INFINITY, bs = -INFINITY;
+#pragma unroll 1
+  for (int i = 0; i < 2 * p.cluster; ++i) {
+    const float dx = s.dom_x[i], ds = s.dom_s[i];
+    if (dx > xmax) { xmax = dx; ms = ds; }
+    else if (dx == xmax) ms = fmaxf(ms, ds);
+    if (ds > bs || (ds == bs && dx > bx)) { bs = ds; bx = dx; }
+  }
+  r.xmax = xmax;
+  // the same in every CTA: no finite maximum, or no score for it
+  const bool lost = !(fabsf(xmax) < INFINITY) || !(fabsf(ms) < INFINITY) || !(fabsf(bs) < INFINITY);
+  double z = 0.0;
+  if (!lost) {
+    // [0]: the published element with the best score; [1]: the row's greatest element; [2..4]: filled below
+    if (threadIdx.x < 6) {
+      s.cut_x[threadIdx.x] = threadIdx.x == 0 ? bx : xmax;
+      s.cut_s[threadIdx.x] = rc_cut(threadIdx.x == 0 ? bs : ms);
+    }
+    __syncthreads();
+    RcLow low{bx, rc_cut(bs), rc_cut(ms)};
+#pragma unroll 1
+    for (int attempt = 0;; ++attempt) {
+      // from a key the greatest Gumbel term is that of 1 - 2^-23: 15.943
+      const double zz = rc_survivors<DT>(part, low, (low.bs - 15.95f) * T_, attempt == 0, r, s, l);
+      if (attempt == 0) z = zz;
+      __syncthreads();
+      if (attempt == 0) { TLX_STAMP(p.sp, 10); }
+      if (s.n_list <= kRcWideCap || attempt == 4) break;
+      // too many (a flat row): the best of those that were kept, the best among the greater ones and the best
+      // among those that are greater again dominate nearly all of them
+      float above = -INFINITY;
+#pragma unroll 1
+      for (int j = 0; j < 3; ++j) {
+        uint32_t bk = 0, xk = 0;
+#pragma unroll 1
+        for (int i = threadIdx.x; i < kRcWideCap; i += kRcThreads) if (j == 0 || l.x[i] > above) bk = max(bk, rc_score_key(l.s[i]));
+        bk = rc_max_u32(bk, s, tog);
+        if (bk == 0) break;
+#pragma unroll 1
+        for (int i = threadIdx.x; i < kRcWideCap; i += kRcThreads)
+          if ((j == 0 || l.x[i] > above) && rc_score_key(l.s[i]) == bk) xk = max(xk, f32_key(l.x[i]));
+        above = key_f32(rc_max_u32(xk, s, tog));
+        const float cut = rc_cut(key_f32(bk));
+        if (threadIdx.x == 0) { s.cut_x[2 + j] = above; s.cut_s[2 + j] = cut; }
+        if (j == 0 && cut > low.bs) { low.bs = cut; low.bx = above; }
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) s.n_list = 0;
+      __syncthreads();
+    }
+    double unused = 0.0;
+    rc_sum2_f64(z, unused, s, tog);
+    if (warp_id() == 0) {
+      // to the leader: the survivors (those that others dominate are left out if there are many), the mass
+      const int lane = lane_id();
+      int k = s.n_list;
+      if (k > kRcWideCap) k = kRcWideSend + 1;   // given up: rc_slow_row
+      else if (k > kRcWideSend) k = rc_thin_out(k, l.x, l.s, l.pos);
+      if (lane < k && k <= kRcWideSend) {
+        const int i = rank * kRcWideSend + lane;
+        cl_st_f32(cl_map(l.all_x + i, 0), l.x[lane]);
+        cl_st_f32(cl_map(l.all_s + i, 0), l.s[lane]);
+        cl_st_u32(cl_map(l.all_col + i, 0), (uint32_t)(col0 + l.pos[lane]));
+      }
+      if (lane == 0) {
+        cl_st_u32(cl_map(s.sent + rank, 0), (uint32_t)k);
+        cl_st_f64(cl_map(s.z + rank, 0), z);
+      }
+    }
+  }
+  TLX_STAMP(p.sp, 5);
+  cl_sync();
+  TLX_STAMP(p.sp, 6);
+  if (lost) return -1;
+  int tok = -1;
+  double Z = 0.0;
+  float above = -INFINITY;
+  bool first = true, going = true;
+  if (rank == 0 && warp_id() == 0) {
+    const int lane = lane_id();
+    going = !__any_sync(0xFFFFFFFFu, lane < p.cluster && s.sent[lane] > kRcWideSend);
+    Z = lane < p.cluster ? s.z[lane] : 0.0;
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) Z += shfl_xor_f64(Z, o);
+  }
+#pragma unroll 1
+  for (int round = 0; round < kRcListCap; ++round) {
+    if (rank == 0 && warp_id() == 0) {
+      // the tokens in question: the best score, and the best score among greater values
+      const int lane = lane_id();
+      int nq = 0;
+      float q[2] = {INFINITY, INFINITY};
+#pragma unroll 1
+      while (going && nq < 2) {
+        const int i = rc_warp_best(p.cluster * kRcWideSend, first, above, l.all_x, l.all_s, T_, noise, nrow,
+                                   [&](int j) { return (int64_t)l.all_col[j]; });
+        if (i < 0) { going = false; break; }
+        above = l.all_x[i];
+        first = false;
+        if (lane == 0) s.query_tok[nq] = l.all_col[i];
+        if (nq == 0) q[0] = above; else q[1] = above;
+        ++nq;
+        if (above == xmax) going = false;   // nothing lies above it: kept whatever top_p is
+      }
+      __syncwarp();
+      if (nq > 0 && tok < 0 && q[0] == xmax) { tok = s.query_tok[0]; nq = 0; }
+      if (lane < p.cluster) {
+        cl_st_f32(cl_map(s.query, lane), q[0]);
+        cl_st_f32(cl_map(s.query + 1, lane), q[1]);
+        cl_st_u32(cl_map(&s.n_query, lane), (uint32_t)nq);
+      }
+    }
+    if (round == 0) { TLX_STAMP(p.sp, 12); }
+    cl_sync();
+    const int nq = s.n_query;
+    if (nq == 0) break;
+    double m0 = 0.0, m1 = 0.0;
+    rc_mass_above<DT>(part, xmax, s.query[0], s.query[1], m0, m1);
+    rc_sum2_f64(m0, m1, s, tog);
+    if (threadIdx.x == 0) {
+      cl_st_f64(cl_map(&s.msum[rank][0], 0), m0);
+      cl_st_f64(cl_map(&s.msum[rank][1], 0), m1);
+    }
+    if (round == 0) { TLX_STAMP(p.sp, 13); }
+    cl_sync();
+    if (round == 0) { TLX_STAMP(p.sp, 14); }
+    if (rank == 0 && warp_id() == 0) {
+#pragma unroll 1
+      for (int j = 0; j < nq && tok < 0; ++j) {
+        double mass = lane_id() < p.cluster ? s.msum[lane_id()][j] : 0.0;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) mass += shfl_xor_f64(mass, o);
+        mass = __hiloint2double(__shfl_sync(0xFFFFFFFFu, __double2hiint(mass), 0), __shfl_sync(0xFFFFFFFFu, __double2loint(mass), 0));
+        if (mass == 0.0 || !(mass / Z >= (double)pp)) tok = s.query_tok[j];
+        tok = __shfl_sync(0xFFFFFFFFu, tok, 0);
+      }
+      if (tok >= 0) going = false;
+    }
+  }
+  if (threadIdx.x == 0) s.pick[0] = tok;
+  __syncthreads();
+  TLX_STAMP(p.sp, 9);
+  return s.pick[0];
+}
+
+// One cluster per row.
+template <int DT>
+__global__ void __launch_bounds__(kRcThreads, 4) sample_cluster_kernel(const __grid_constant__ RcSampleParams p) {
+  using T = typename Elem<DT>::type;
+  extern __shared__ __align__(128) unsigned char smem[];
+  RcShared& s = *reinterpret_cast<RcShared*>(smem);
+  const RcLayout l(p.cluster, true);
+  const uint32_t rank = cl_rank();
+  const int64_t row = blockIdx.x / p.cluster;
+  const int64_t n = p.sp.vocab;
+  const T* rowp = reinterpret_cast<const T*>(p.sp.logits) + row * p.sp.row_stride;
+  const RcPart<DT> part(rowp, n, p.part_len, rank, smem + l.off_part);
+  part.copy_in();
+  TLX_STAMP(p.sp, 0);
+  const float T_ = p.sp.temperature[row], pp = p.sp.top_p[row];
+  int64_t K = p.sp.top_k[row];
+  if (K <= 0 || K > n) K = n;
+  if (T_ < kSamplingEps) K = 1;
+  const bool wide = K >= n && n > 1 && p.part_len > 0, large = !wide && (K > kRcMaxK || p.part_len == 0);
+  if (threadIdx.x == 0) s.n_list = 0;
+  part.copy_wait();
+  __syncthreads();
+  TLX_STAMP(p.sp, 1);
+  const int64_t col0 = (int64_t)rank * p.part_len, nrow = row + p.sp.dim0_offset;
+  int tok = -1, tog = 0;
+  if (wide) tok = rc_wide_row<DT>(p, part, col0, rank, pp, T_, nrow, s, l, smem, tog);
+  else if (!large) tok = rc_normal_row<DT>(p, part, col0, rank, (int)K, pp, T_, nrow, s, l, smem, tog);
+  if (rank != 0) return;
+  int status = wide || large ? kStatusGeneral : 0;
+  if (tok < 0) {
+    tok = rc_slow_row<DT>(rowp, n, K, pp, T_, p.sp.noise, nrow, s);
+    status |= large ? 0 : kStatusRedone;
+  }
+  if (threadIdx.x == 0) {
+    p.sp.out_tokens[row] = tok;
+    if (p.sp.out_status) p.sp.out_status[row] = status;
+  }
+}
+
+}  // namespace tlx

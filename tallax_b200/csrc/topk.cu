@@ -1,7 +1,7 @@
 // Row-wise exact / single-pass top-k and the per-shard candidate stage of the
 // vocab-sharded sampler.  One CTA per row: the streaming collector leaves a superset of
 // the top-k in shared memory, a bitonic network orders it by (value desc, index asc).
-#include "select.cuh"
+#include "row_cluster.cuh"
 #include "exchange.cuh"
 
 #include <cstdlib>
@@ -151,59 +151,6 @@ __global__ void __launch_bounds__(kTopkThreads) topk_kernel(TopkParams p) {
 constexpr int kShortThreads = 128;
 constexpr int kShortCap = 1024;
 constexpr int kShortMaxK = 128;
-
-template <int DT> struct GroupMax;
-template <> struct GroupMax<TLX_BF16> {
-  static constexpr int kSlots = 8;
-  __nv_bfloat162 m[4];
-  __device__ __forceinline__ void init() {
-    const __nv_bfloat16 ninf = __float2bfloat16_rn(-INFINITY);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = __halves2bfloat162(ninf, ninf);
-  }
-  __device__ __forceinline__ void add(const uint4& v) {
-    const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = __hmax2(m[j], e[j]);
-  }
-  __device__ __forceinline__ void add_one(__nv_bfloat16 x) { m[0] = __hmax2(m[0], __halves2bfloat162(x, m[0].y)); }
-  __device__ __forceinline__ float slot(int j) const {
-    return (j & 1) ? __high2float(m[j >> 1]) : __low2float(m[j >> 1]);
-  }
-};
-template <> struct GroupMax<TLX_F16> {
-  static constexpr int kSlots = 8;
-  __half2 m[4];
-  __device__ __forceinline__ void init() {
-    const __half ninf = __float2half_rn(-INFINITY);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = __halves2half2(ninf, ninf);
-  }
-  __device__ __forceinline__ void add(const uint4& v) {
-    const __half2* e = reinterpret_cast<const __half2*>(&v);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = __hmax2(m[j], e[j]);
-  }
-  __device__ __forceinline__ void add_one(__half x) { m[0] = __hmax2(m[0], __halves2half2(x, __high2half(m[0]))); }
-  __device__ __forceinline__ float slot(int j) const {
-    return (j & 1) ? __high2float(m[j >> 1]) : __low2float(m[j >> 1]);
-  }
-};
-template <> struct GroupMax<TLX_F32> {
-  static constexpr int kSlots = 4;
-  float m[4];
-  __device__ __forceinline__ void init() {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = -INFINITY;
-  }
-  __device__ __forceinline__ void add(const uint4& v) {
-    const float* e = reinterpret_cast<const float*>(&v);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) m[j] = fmaxf(m[j], e[j]);
-  }
-  __device__ __forceinline__ void add_one(float x) { m[0] = fmaxf(m[0], x); }
-  __device__ __forceinline__ float slot(int j) const { return m[j]; }
-};
 
 // Row traversal by 16-byte vectors: fv(vector, first column) in the aligned body, kU loads in flight per
 // thread; fs(element, column) for the unaligned head and tail.  sub > 1 visits only every sub-th run of
