@@ -48,10 +48,9 @@ const char* tlx_last_error(void);
  * benchmark count launches per call instead of assuming them). */
 unsigned long long tlx_kernel_launches(void);
 
-/* Optional.  Touches `device` once (so that no later call makes its first query of the device
- * inside a stream capture) and, with TLX_INIT_SIDE_STREAM, creates the calling thread's helper
- * stream and events on it and lets tlx_sample use them.  Without this call the library creates no
- * CUDA stream or event of its own, ever.                                                       */
+/* Optional.  Touches `device` once, so that no later call makes its first query of the device
+ * inside a stream capture.  The library creates no CUDA stream or event of its own, ever;
+ * TLX_INIT_SIDE_STREAM is accepted and has no effect.                                          */
 #define TLX_INIT_SIDE_STREAM 1u
 int tlx_init(int device, unsigned flags);
 
@@ -216,9 +215,8 @@ int tlx_top_p_and_sample_dev(void* stream, const void* topk_logits, int dtype, c
  * out_status (nullable, device int32[rows]): bit 0 = the row took a path for rows without
  * (or with a very large) top-k, bit 1 = a bounded wait gave up (result invalid), bit 2 = the
  * row needed a second pass (first threshold too high, or candidate list overflow).
- * All of the call's work is ordered on `stream`.  Only after tlx_init(device,
- * TLX_INIT_SIDE_STREAM) may part of it run on a stream owned by the library, forked from
- * `stream` and joined back to it inside the call (also when a launch or an event call fails).
+ * All of the call's work is ordered on `stream`.  `workspace` is used by large calls only
+ * (tlx_sample_workspace_bytes); without it, or with a smaller one, they take the form that needs none.
  * Replaces the whole of tallax/_src/sampling.py:331-343 (`sample`), i.e. the
  * top_dynamic_k kernel (top_k.py:482-506) followed by _top_p_and_sample.            */
 size_t tlx_sample_workspace_bytes(int64_t rows, int64_t vocab);

@@ -132,6 +132,8 @@ struct __align__(16) RcShared {
   int sent[kRcMaxCluster];
   double z[kRcMaxCluster], msum[kRcMaxCluster][4];
   int first[kRcMaxCluster + 1];         // leader: first candidate of every CTA in the gathered list
+  uint32_t key_lo, key_hi;              // range of the candidates' keys (from the bound's search)
+  int n_near;
   unsigned long long win;               // winner of a round of the decision
   float win_x;
   int fail;
@@ -305,6 +307,16 @@ __device__ __forceinline__ uint32_t rc_bound_key16(const uint32_t* bound, int wo
     for (int j = 1; j < 32; ++j) { hi = __hmax2(hi, rc_bf162(w[j])); lo = __hmin2(lo, rc_bf162(w[j])); }
     const uint32_t kmax = __reduce_max_sync(0xFFFFFFFFu, rc_key16(fmaxf(__low2float(hi), __high2float(hi))));
     const uint32_t kmin = __reduce_min_sync(0xFFFFFFFFu, rc_key16(fminf(__low2float(lo), __high2float(lo))));
+    // a few of many: fewer and larger groups give as tight a bound (512 groups: 53 elements for K = 50)
+    const int n = K <= 64 ? 8 : K <= 256 ? 16 : 32;
+    if (n <= 16) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) w[j] = rc_bits(__hmax2(rc_bf162(w[j]), rc_bf162(w[j + 16])));
+      if (n <= 8) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) w[j] = rc_bits(__hmax2(rc_bf162(w[j]), rc_bf162(w[j + 8])));
+      }
+    }
     uint32_t t = kmin;
     if (kmax > kmin) {
       int bit = 31 - __clz(kmax ^ kmin);
@@ -315,6 +327,7 @@ __device__ __forceinline__ uint32_t rc_bound_key16(const uint32_t* bound, int wo
         __nv_bfloat162 c0 = __hge2(rc_bf162(w[0]), p), c1 = __hge2(rc_bf162(w[1]), p);
 #pragma unroll
         for (int j = 2; j < 32; j += 2) {
+          if ((j == 8 && n == 8) || (j == 16 && n == 16)) break;
           c0 = __hadd2(c0, __hge2(rc_bf162(w[j]), p));
           c1 = __hadd2(c1, __hge2(rc_bf162(w[j + 1]), p));
         }
@@ -323,7 +336,7 @@ __device__ __forceinline__ uint32_t rc_bound_key16(const uint32_t* bound, int wo
         if (c >= K) t |= 1u << bit;
       }
     }
-    if (lane_id() == 0) s.pick[0] = (int)(t < 0x80u ? 0x80u : t);
+    if (lane_id() == 0) { s.pick[0] = (int)(t < 0x80u ? 0x80u : t); s.key_lo = (uint32_t)s.pick[0] << 16; s.key_hi = (kmax << 16) | 0xFFFFu; }
   }
   __syncthreads();
   return (uint32_t)s.pick[0];

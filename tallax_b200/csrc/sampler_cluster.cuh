@@ -104,11 +104,21 @@ static __device__ __noinline__ int rc_slow_row(const typename Elem<DT>::type* __
     if (composite(v, c) >= least) z += (double)expf(elem_as_float<DT>(v) - xmax);
   });
   rc_sum2_f64(z, unused, s, tog);
-  float above = -INFINITY;   // only values above this one are still in question
-  bool first = true;
+  // softmax mass of the set's elements whose key is above `key`, and whether there is one
+  bool none_above = false;
+  auto mass_above = [&](uint32_t key) {
+    double mass = 0.0, count = 0.0;
+    for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
+      if (Elem<DT>::key(v) > key && composite(v, c) >= least) { mass += (double)expf(elem_as_float<DT>(v) - xmax); count += 1.0; }
+    });
+    rc_sum2_f64(mass, count, s, tog);
+    none_above = count == 0.0;
+    return mass;
+  };
+  uint32_t from = 0;   // least key still in question
 #pragma unroll 1
-  for (int round = 0; round < 4096; ++round) {
-    auto eligible = [&](T v, int64_t c) { return composite(v, c) >= least && (first || elem_as_float<DT>(v) > above); };
+  for (int round = 0; round < 8; ++round) {
+    auto eligible = [&](T v, int64_t c) { return Elem<DT>::key(v) >= from && composite(v, c) >= least; };
     uint32_t a = 0;
     for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
       if (eligible(v, c)) a = max(a, rc_score_key(__fdiv_rn(elem_as_float<DT>(v), T_) + gumbel_screen(noise.at(nrow, c))));
@@ -125,16 +135,20 @@ static __device__ __noinline__ int rc_slow_row(const typename Elem<DT>::type* __
     });
     w = block_max(w);
     const int tok = 0x7FFFFFFF - (int)(uint32_t)w;
-    const float wx = elem_as_float<DT>(row[tok]);
-    double mass = 0.0, count = 0.0;
-    for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
-      const float x = elem_as_float<DT>(v);
-      if (x > wx && composite(v, c) >= least) { mass += (double)expf(x - xmax); count += 1.0; }
-    });
-    rc_sum2_f64(mass, count, s, tog);
-    if (count == 0.0 || !(mass / z >= (double)p)) return tok;
-    above = wx;
-    first = false;
+    const uint32_t wk = Elem<DT>::key(row[tok]);
+    const double mass = mass_above(wk);
+    if (none_above || !(mass / z >= (double)p)) return tok;
+    from = wk + 1;
+    if (round == 6) {
+      // many records in a row: the least key that is kept, by bisection; the next round is then the last
+      uint32_t hi = (uint32_t)(top >> 32);
+#pragma unroll 1
+      while (from < hi) {
+        const uint32_t mid = from + (hi - from) / 2;
+        const double m = mass_above(mid);
+        if (none_above || !(m / z >= (double)p)) hi = mid; else from = mid + 1;
+      }
+    }
   }
   return top_col;
 }
@@ -145,27 +159,20 @@ static __device__ __noinline__ int rc_slow_row(const typename Elem<DT>::type* __
 static __device__ __noinline__ void rc_cut_to_k(RcShared& s, int m, int K, int64_t part_len, float* lx, float* ls,
                                                 const unsigned short* lpos, uint32_t* bins) {
   int tog = 2;
-  uint32_t kmax = 0, kmin_inv = 0;
-#pragma unroll 1
-  for (int i = threadIdx.x; i < m; i += kRcThreads) {
-    const uint32_t k = f32_key(lx[i]);
-    kmax = max(kmax, k);
-    kmin_inv = max(kmin_inv, ~k);
-  }
-  kmax = rc_max_u32(kmax, s, tog);
-  const uint32_t kmin = ~rc_max_u32(kmin_inv, s, tog);
+  uint32_t kmin = s.key_lo, kmax = s.key_hi;   // (a NaN lies above: the top bin takes it)
   // One histogram of 2048 bins over the range of the keys; the K-th key's bin then holds a few elements, which are
   // ranked by counting.
   {
-    const uint32_t range = kmax - kmin;
+    const uint32_t range = kmax > kmin ? kmax - kmin : 0;
     const int shift = range >> 11 ? 21 - __clz(range) : 0;
+    auto bin_of = [&](float x) { return (kRcBins - 1) - (int)min((f32_key(x) - kmin) >> shift, (uint32_t)kRcBins - 1); };
     uint4* b4 = reinterpret_cast<uint4*>(bins);
     b4[threadIdx.x] = make_uint4(0, 0, 0, 0);
     b4[threadIdx.x + kRcThreads] = make_uint4(0, 0, 0, 0);
     if (threadIdx.x == 0) s.pick[3] = 0;
     __syncthreads();
 #pragma unroll 1
-    for (int i = threadIdx.x; i < m; i += kRcThreads) atomicAdd(&bins[(kRcBins - 1) - ((f32_key(lx[i]) - kmin) >> shift)], 1u);
+    for (int i = threadIdx.x; i < m; i += kRcThreads) atomicAdd(&bins[bin_of(lx[i])], 1u);
     __syncthreads();
     const uint4 c0 = b4[2 * threadIdx.x], c1 = b4[2 * threadIdx.x + 1];
     const int sum = (int)(c0.x + c0.y + c0.z + c0.w + c1.x + c1.y + c1.z + c1.w);
@@ -192,32 +199,45 @@ static __device__ __noinline__ void rc_cut_to_k(RcShared& s, int m, int K, int64
     const int bin = s.pick[0], need = K - s.pick[1], in_bin = s.pick[2];
     if (in_bin <= 256) {
       uint64_t* list = reinterpret_cast<uint64_t*>(bins);   // (the histogram has been read)
+      unsigned short* at = reinterpret_cast<unsigned short*>(list + 256);
+      if ((int)threadIdx.x >= in_bin) list[threadIdx.x] = 0;
 #pragma unroll 1
       for (int i = threadIdx.x; i < m; i += kRcThreads) {
-        const uint32_t k = f32_key(lx[i]);
-        const int b = (kRcBins - 1) - (int)((k - kmin) >> shift);
+        const int b = bin_of(lx[i]);
         if (b > bin) { lx[i] = -INFINITY; ls[i] = -INFINITY; }
-        else if (b == bin)
-          list[atomicAdd(&s.pick[3], 1)] = ((uint64_t)k << 32) | (uint32_t)i;
+        else if (b == bin) {
+          const int slot = atomicAdd(&s.pick[3], 1);
+          list[slot] = ((uint64_t)f32_key(lx[i]) << 32) | (uint32_t)(0x7FFFFFFF - (int32_t)rc_column(s, lpos, i, part_len));
+          at[slot] = (unsigned short)i;
+        }
       }
       __syncthreads();
       if ((int)threadIdx.x < in_bin) {
         const uint64_t c = list[threadIdx.x];
-        const int i = (int)(c & 2047u);
-        const int64_t col = rc_column(s, lpos, i, part_len);
+        const ulonglong2* l2 = reinterpret_cast<const ulonglong2*>(list);
         int before = 0;
-#pragma unroll 1
-        for (int j = 0; j < in_bin; ++j) {
-          const uint64_t o = list[j];
-          if ((o >> 32) > (c >> 32)) ++before;
-          else if ((o >> 32) == (c >> 32) && o != c && rc_column(s, lpos, (int)(o & 2047u), part_len) < col) ++before;
+#pragma unroll 4
+        for (int j = 0; j < (in_bin + 1) / 2; ++j) {
+          const ulonglong2 o = l2[j];
+          before += (o.x > c ? 1 : 0) + (o.y > c ? 1 : 0);
         }
-        if (before >= need) { lx[i] = -INFINITY; ls[i] = -INFINITY; }
+        if (before >= need) { lx[at[threadIdx.x]] = -INFINITY; ls[at[threadIdx.x]] = -INFINITY; }
       }
       __syncthreads();
       return;
     }
   }
+  // keys so spread, or so many equal ones, that the bin holds more than that: digit by digit
+  kmax = 0;
+  uint32_t kmin_inv = 0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < m; i += kRcThreads) {
+    const uint32_t k = f32_key(lx[i]);
+    kmax = max(kmax, k);
+    kmin_inv = max(kmin_inv, ~k);
+  }
+  kmax = rc_max_u32(kmax, s, tog);
+  kmin = ~rc_max_u32(kmin_inv, s, tog);
   int need = K, ties = m;
   uint32_t vk = kmax;          // prefix of the K-th key; bits below `top` are still to be found
   int top = kmax == kmin ? 0 : 32 - __clz(kmax ^ kmin);
@@ -274,43 +294,72 @@ static __device__ __noinline__ void rc_cut_to_k(RcShared& s, int m, int K, int64
   __syncthreads();
 }
 
-// Leader: the best element of the gathered list among those above `above` (all of them if first): its column, its
-// value in s.win_x.  -1 if none has a score.
-template <int DT>
-static __device__ __noinline__ int rc_best_of_list(RcShared& s, int m, bool first, float above, int64_t part_len,
-                                                   const float* lx, const float* ls, const unsigned short* lpos, float T_,
-                                                   const NoiseSrc& noise, int64_t nrow) {
+// Leader: the decision (top of the file) over more than kRcSmall candidates, cut to the top-K set.  A round has three
+// barriers.  Returns the token, -1 if no kept element has a score.
+static __device__ __noinline__ int rc_decide_large(RcShared& s, int m, float pp, int64_t part_len, const float* lx,
+                                                   const float* ls, const unsigned short* lpos, float T_, const NoiseSrc& noise,
+                                                   int64_t nrow) {
   int tog = 2;
-  uint32_t a = 0;
+  float above = -INFINITY, x0 = 0.f;
+  bool first = true;
 #pragma unroll 1
-  for (int i = threadIdx.x; i < m; i += kRcThreads)
-    if (first || lx[i] > above) a = max(a, rc_score_key(ls[i]));
-  const uint32_t ak = rc_max_u32(a, s, tog);
-  if (ak <= 0x007FFFFFu) return -1;   // NaN or -inf
-  const float cut = rc_cut(key_f32(ak));
-  uint32_t near_ = 0;
-  if (threadIdx.x == 0) s.win = 0;
+  for (int round = 0; round < kRcListCap; ++round) {
+    uint32_t a = 0, xk = 0;
 #pragma unroll 1
-  for (int i = threadIdx.x; i < m; i += kRcThreads)
-    if ((first || lx[i] > above) && ls[i] >= cut) ++near_;
-  near_ = rc_sum_u32(near_, s, tog);
-#pragma unroll 1
-  for (int i = threadIdx.x; i < m; i += kRcThreads) {
-    if ((first || lx[i] > above) && ls[i] >= cut) {
-      const int64_t col = rc_column(s, lpos, i, part_len);
-      // several within the screening slack of the best: decided on the f64-evaluated noise
-      float y = 0.f;
-      if (near_ > 1) y = __fdiv_rn(lx[i], T_) + gumbel_exact(noise.at(nrow, col));
-      atomicMax(&s.win, rc_win_make(y, col));
+    for (int i = threadIdx.x; i < m; i += kRcThreads) {
+      const float x = lx[i];
+      if (first) xk = max(xk, f32_key(x));
+      if (first || x > above) a = max(a, rc_score_key(ls[i]));
     }
-  }
-  __syncthreads();
-  const int tok = 0x7FFFFFFF - (int)(uint32_t)s.win;
+    a = __reduce_max_sync(0xFFFFFFFFu, a);
+    if (first) xk = __reduce_max_sync(0xFFFFFFFFu, xk);
+    if (lane_id() == 0) { s.red_u32[2][warp_id()] = a; s.red_u32[3][warp_id()] = xk; }
+    if (threadIdx.x == 0) { s.win = 0; s.n_near = 0; }
+    __syncthreads();
+    a = __reduce_max_sync(0xFFFFFFFFu, s.red_u32[2][lane_id() & (kRcWarps - 1)]);
+    if (first) x0 = key_f32(__reduce_max_sync(0xFFFFFFFFu, s.red_u32[3][lane_id() & (kRcWarps - 1)]));
+    if (a <= 0x007FFFFFu) return -1;   // NaN or -inf
+    const float cut = rc_cut(key_f32(a));
 #pragma unroll 1
-  for (int i = threadIdx.x; i < m; i += kRcThreads)
-    if ((first || lx[i] > above) && ls[i] >= cut && rc_column(s, lpos, i, part_len) == tok) s.win_x = lx[i];
-  __syncthreads();
-  return tok;
+    for (int i = threadIdx.x; i < m; i += kRcThreads)
+      if ((first || lx[i] > above) && ls[i] >= cut) {
+        atomicAdd(&s.n_near, 1);
+        s.win = (unsigned long long)i;
+      }
+    __syncthreads();
+    int at = (int)s.win;
+    if (s.n_near > 1) {   // several within the screening slack of the best: decided on the f64-evaluated noise
+      __syncthreads();
+      if (threadIdx.x == 0) s.win = 0;
+      __syncthreads();
+#pragma unroll 1
+      for (int i = threadIdx.x; i < m; i += kRcThreads)
+        if ((first || lx[i] > above) && ls[i] >= cut) {
+          const int64_t col = rc_column(s, lpos, i, part_len);
+          atomicMax(&s.win, rc_win_make(__fdiv_rn(lx[i], T_) + gumbel_exact(noise.at(nrow, col)), col));
+        }
+      __syncthreads();
+      const int tok = 0x7FFFFFFF - (int)(uint32_t)s.win;
+#pragma unroll 1
+      for (int i = threadIdx.x; i < m; i += kRcThreads)
+        if ((first || lx[i] > above) && ls[i] >= cut && rc_column(s, lpos, i, part_len) == tok) s.n_near = i;
+      __syncthreads();
+      at = s.n_near;
+    }
+    const float wx = lx[at];
+    double mass = 0.0, z = 0.0;
+#pragma unroll 1
+    for (int i = threadIdx.x; i < m; i += kRcThreads) {
+      const double w = (double)expf(lx[i] - x0);
+      z += w;
+      if (lx[i] > wx) mass += w;
+    }
+    rc_sum2_f64(mass, z, s, tog);
+    if (mass == 0.0 || !(mass / z >= (double)pp)) return (int)rc_column(s, lpos, at, part_len);
+    above = wx;
+    first = false;
+  }
+  return -1;
 }
 
 // Leader: at most 256 candidates.  Every thread ranks one by counting, which sorts the top-K set; one warp then takes
@@ -436,7 +485,7 @@ struct RcWideLists {
 // What the passes over a row without top-k need of it.
 struct RcWideRow {
   int64_t col0, nrow;
-  float rt, xmax;            // 1 / T; the row's greatest value
+  float rt;                  // 1 / T
   const float* dense;        // the part's noise, or null: the key
   uint32_t k0, k1, ctr0;     // key; counter of the part's first element
 };
@@ -483,20 +532,18 @@ __device__ __forceinline__ void rc_score_noted(const RcPart<DT>& part, const uns
   }
 }
 
-// The part's survivors (see the top of the file) into the CTA's list; with `mass`, also the part's share of the softmax
-// denominator (returned).
+// The part's survivors (see the top of the file) into the CTA's list.
 //   From a key: a warp notes the positions whose value allows a survivor at all and makes their noise 128 at a time.
 //   From a tensor: the noise is read beside the values, and a vector is looked into if its greatest value with its
 //   greatest noise could survive.
 template <int DT>
-__device__ __forceinline__ double rc_survivors(const RcPart<DT>& part, const RcLow& low, float xcut, bool mass, const RcWideRow& r,
+__device__ __forceinline__ void rc_survivors(const RcPart<DT>& part, const RcLow& low, float xcut, const RcWideRow& r,
                                                RcShared& s, const RcWideLists& l) {
   using T = typename Elem<DT>::type;
   constexpr int VEC = RcPart<DT>::VEC;
   const int lane = lane_id();
   unsigned short* queue = l.queue + warp_id() * kRcQueue;
   const bool aligned = r.dense && (reinterpret_cast<uintptr_t>(r.dense - part.off) & 15) == 0;
-  double z = 0.0;
   int waiting = 0;
 #pragma unroll 1
   for (int v0 = 0; v0 < part.nvec; v0 += kRcThreads) {
@@ -519,10 +566,6 @@ __device__ __forceinline__ double rc_survivors(const RcPart<DT>& part, const RcL
 #pragma unroll
           for (int j = 0; j < VEC; ++j) u[j] = i0 + j >= 0 && i0 + j < part.n ? __ldg(r.dense + i0 + j) : 0.f;
         }
-      }
-      if (mass) {
-#pragma unroll
-        for (int j = 0; j < VEC; ++j) z += (double)expf(elem_as_float<DT>(e[j]) - r.xmax);
       }
       if (r.dense) {
         float xm = elem_as_float<DT>(e[0]), um = u[0];
@@ -568,42 +611,41 @@ __device__ __forceinline__ double rc_survivors(const RcPart<DT>& part, const RcL
     }
     __syncwarp();
   }
-  return z;
 }
 
-// Warp 0: the best entry of a list of m among those above `above` (all of them if `first`): its index, -1 if none has
-// a score.  col_of(i) is the column of entry i.
-template <typename ColOf>
-__device__ __forceinline__ int rc_warp_best(int m, bool first, float above, const float* lx, const float* ls, float T_,
-                                            const NoiseSrc& noise, int64_t nrow, ColOf col_of) {
+// Leader, warp 0: the best of the survivors that the CTAs have sent, among those above `above` (all of them if `first`):
+// its place, -1 if none has a score.  `most`: the greatest number that a CTA has sent.
+__device__ __forceinline__ int rc_best_sent(int most, bool first, float above, const RcWideLists& l, float T_,
+                                            const NoiseSrc& noise, int64_t nrow) {
+  const int i0 = (lane_id() & 15) * kRcWideSend + (lane_id() >> 4), i1 = i0 + (most + 1) / 2 * 2;   // every other place
   uint32_t a = 0;
 #pragma unroll 1
-  for (int i = lane_id(); i < m; i += 32)
-    if (first || lx[i] > above) a = max(a, rc_score_key(ls[i]));
+  for (int i = i0; i < i1; i += 2)
+    if (first || l.all_x[i] > above) a = max(a, rc_score_key(l.all_s[i]));
   a = __reduce_max_sync(0xFFFFFFFFu, a);
   if (a <= 0x007FFFFFu) return -1;
   const float cut = rc_cut(key_f32(a));
-  int near_ = 0, idx = -1;
+  int near_ = 0, at = -1;
 #pragma unroll 1
-  for (int i = lane_id(); i < m; i += 32)
-    if ((first || lx[i] > above) && ls[i] >= cut) { ++near_; idx = i; }
+  for (int i = i0; i < i1; i += 2)
+    if ((first || l.all_x[i] > above) && l.all_s[i] >= cut) { ++near_; at = i; }
   near_ = __reduce_add_sync(0xFFFFFFFFu, near_);
-  if (near_ > 1) {
+  if (near_ > 1) {   // several within the screening slack: decided on the f64-evaluated noise
     uint32_t hi = 0, lo = 0;
-    idx = -1;
+    at = -1;
 #pragma unroll 1
-    for (int i = lane_id(); i < m; i += 32)
-      if ((first || lx[i] > above) && ls[i] >= cut) {
-        const int64_t col = col_of(i);
-        const uint32_t k = rc_score_key(__fdiv_rn(lx[i], T_) + gumbel_exact(noise.at(nrow, col)));
-        const uint32_t c = (uint32_t)(0x7FFFFFFF - (int32_t)col);
-        if (k > hi || (k == hi && c > lo)) { hi = k; lo = c; idx = i; }
+    for (int i = i0; i < i1; i += 2)
+      if ((first || l.all_x[i] > above) && l.all_s[i] >= cut) {
+        const int col = l.all_col[i];
+        const uint32_t k = rc_score_key(__fdiv_rn(l.all_x[i], T_) + gumbel_exact(noise.at(nrow, col)));
+        const uint32_t c = (uint32_t)(0x7FFFFFFF - col);
+        if (k > hi || (k == hi && c > lo)) { hi = k; lo = c; at = i; }
       }
     const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, hi);
     const uint32_t low = __reduce_max_sync(0xFFFFFFFFu, hi == top ? lo : 0u);
-    if (hi != top || lo != low) idx = -1;
+    if (hi != top || lo != low) at = -1;
   }
-  return __reduce_max_sync(0xFFFFFFFFu, idx);
+  return __reduce_max_sync(0xFFFFFFFFu, at);
 }
 
 // Warp 0: more than kRcWideSend survivors: drops those that another one dominates, in place.
@@ -646,24 +688,34 @@ __device__ __forceinline__ int rc_thin_out(int m, float* lx, float* ls, unsigned
   return kept;
 }
 
-// The thread's share of the softmax mass above two values (q0 <= q1).
+// The thread's share of the softmax denominator and of the mass above two values (q0 <= q1).  Four sums of each: f64
+// additions are a chain of latencies.
 template <int DT>
-__device__ __forceinline__ void rc_mass_above(const RcPart<DT>& part, float xmax, float q0, float q1, double& m0, double& m1) {
+__device__ __forceinline__ void rc_masses(const RcPart<DT>& part, float xmax, float q0, float q1, double& z, double& m0, double& m1) {
   using T = typename Elem<DT>::type;
   constexpr int VEC = RcPart<DT>::VEC;
+  double zs[4] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
   for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) {
     const uint4 w = part.vec[v];
-    if (!rc_any_at_least<DT>(w, q0)) continue;
     const T* e = reinterpret_cast<const T*>(&w);
+    const bool any = rc_any_at_least<DT>(w, q0);
+    double y[VEC];
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
-      const float x = elem_as_float<DT>(e[j]);
-      const double y = (double)(x > q0 ? expf(x - xmax) : 0.f);
-      m0 += y;
-      m1 += x > q1 ? y : 0.0;
+      y[j] = (double)expf(elem_as_float<DT>(e[j]) - xmax);
+      zs[j & 3] += y[j];
+    }
+    if (any) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const float x = elem_as_float<DT>(e[j]);
+        if (x > q0) m0 += y[j];
+        if (x > q1) m1 += y[j];
+      }
     }
   }
+  z = (zs[0] + zs[1]) + (zs[2] + zs[3]);
 }
 
 // Rows with 1 <= top_k <= 1024 and greedy rows.  Returns the token in the leader (rank 0), -1 if the row has to be
@@ -688,6 +740,7 @@ __device__ __forceinline__ int rc_normal_row(const RcSampleParams& p, const RcPa
     TLX_STAMP(p.sp, 2);
     thr = key_f32(rc_bound_key16(bound, l.bound_words, K, s) << 16);
   } else {
+    if (threadIdx.x == 0) { s.key_lo = 0x80u << 16; s.key_hi = 0xFFFFFFFFu; }
     cl_sync();
   }
   TLX_STAMP(p.sp, 3);
@@ -726,29 +779,7 @@ __device__ __forceinline__ int rc_normal_row(const RcSampleParams& p, const RcPa
   } else if (m > 0) {
     if (m > K) rc_cut_to_k(s, m, K, p.part_len, lx, ls, lpos, reinterpret_cast<uint32_t*>(smem + l.off_part));
     TLX_STAMP(p.sp, 8);
-    uint32_t k0 = 0;
-#pragma unroll 1
-    for (int i = threadIdx.x; i < m; i += kRcThreads) k0 = max(k0, f32_key(lx[i]));
-    const float x0 = key_f32(rc_max_u32(k0, s, tog));
-    float above = -INFINITY;
-    bool first = true;
-#pragma unroll 1
-    for (int round = 0; round < kRcListCap; ++round) {
-      const int t = rc_best_of_list<DT>(s, m, first, above, p.part_len, lx, ls, lpos, T_, p.sp.noise, nrow);
-      if (t < 0) break;
-      const float wx = s.win_x;
-      double mass = 0.0, z = 0.0;
-#pragma unroll 1
-      for (int i = threadIdx.x; i < m; i += kRcThreads) {
-        const double w = (double)expf(lx[i] - x0);
-        z += w;
-        if (lx[i] > wx) mass += w;
-      }
-      rc_sum2_f64(mass, z, s, tog);
-      if (mass == 0.0 || !(mass / z >= (double)pp)) { tok = t; break; }
-      above = wx;
-      first = false;
-    }
+    tok = rc_decide_large(s, m, pp, p.part_len, lx, ls, lpos, T_, p.sp.noise, nrow);
   }
   cl_wait();
   TLX_STAMP(p.sp, 9);
@@ -827,10 +858,8 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
     else if (dx == xmax) ms = fmaxf(ms, ds);
     if (ds > bs || (ds == bs && dx > bx)) { bs = ds; bx = dx; }
   }
-  r.xmax = xmax;
   // the same in every CTA: no finite maximum, or no score for it
   const bool lost = !(fabsf(xmax) < INFINITY) || !(fabsf(ms) < INFINITY) || !(fabsf(bs) < INFINITY);
-  double z = 0.0;
   if (!lost) {
     // [0]: the published element with the best score; [1]: the row's greatest element; [2..4]: filled below
     if (threadIdx.x < 6) {
@@ -842,8 +871,7 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
 #pragma unroll 1
     for (int attempt = 0;; ++attempt) {
       // from a key the greatest Gumbel term is that of 1 - 2^-23: 15.943
-      const double zz = rc_survivors<DT>(part, low, (low.bs - 15.95f) * T_, attempt == 0, r, s, l);
-      if (attempt == 0) z = zz;
+      rc_survivors<DT>(part, low, (low.bs - 15.95f) * T_, r, s, l);
       __syncthreads();
       if (attempt == 0) { TLX_STAMP(p.sp, 10); }
       if (s.n_list <= kRcWideCap || attempt == 4) break;
@@ -869,10 +897,8 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
       if (threadIdx.x == 0) s.n_list = 0;
       __syncthreads();
     }
-    double unused = 0.0;
-    rc_sum2_f64(z, unused, s, tog);
     if (warp_id() == 0) {
-      // to the leader: the survivors (those that others dominate are left out if there are many), the mass
+      // to the leader: the survivors (those that others dominate are left out if there are many)
       const int lane = lane_id();
       int k = s.n_list;
       if (k > kRcWideCap) k = kRcWideSend + 1;   // given up: rc_slow_row
@@ -883,26 +909,20 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
         cl_st_f32(cl_map(l.all_s + i, 0), l.s[lane]);
         cl_st_u32(cl_map(l.all_col + i, 0), (uint32_t)(col0 + l.pos[lane]));
       }
-      if (lane == 0) {
-        cl_st_u32(cl_map(s.sent + rank, 0), (uint32_t)k);
-        cl_st_f64(cl_map(s.z + rank, 0), z);
-      }
+      if (lane == 0) cl_st_u32(cl_map(s.sent + rank, 0), (uint32_t)k);
     }
   }
   TLX_STAMP(p.sp, 5);
   cl_sync();
   TLX_STAMP(p.sp, 6);
   if (lost) return -1;
-  int tok = -1;
-  double Z = 0.0;
+  int tok = -1, most = 0;
   float above = -INFINITY;
   bool first = true, going = true;
   if (rank == 0 && warp_id() == 0) {
     const int lane = lane_id();
     going = !__any_sync(0xFFFFFFFFu, lane < p.cluster && s.sent[lane] > kRcWideSend);
-    Z = lane < p.cluster ? s.z[lane] : 0.0;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) Z += shfl_xor_f64(Z, o);
+    most = __reduce_max_sync(0xFFFFFFFFu, lane < p.cluster ? s.sent[lane] : 0);
   }
 #pragma unroll 1
   for (int round = 0; round < kRcListCap; ++round) {
@@ -913,8 +933,7 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
       float q[2] = {INFINITY, INFINITY};
 #pragma unroll 1
       while (going && nq < 2) {
-        const int i = rc_warp_best(p.cluster * kRcWideSend, first, above, l.all_x, l.all_s, T_, noise, nrow,
-                                   [&](int j) { return (int64_t)l.all_col[j]; });
+        const int i = rc_best_sent(most, first, above, l, T_, noise, nrow);
         if (i < 0) { going = false; break; }
         above = l.all_x[i];
         first = false;
@@ -935,10 +954,12 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
     cl_sync();
     const int nq = s.n_query;
     if (nq == 0) break;
-    double m0 = 0.0, m1 = 0.0;
-    rc_mass_above<DT>(part, xmax, s.query[0], s.query[1], m0, m1);
+    double z = 0.0, unused = 0.0, m0 = 0.0, m1 = 0.0;
+    rc_masses<DT>(part, xmax, s.query[0], s.query[1], z, m0, m1);
     rc_sum2_f64(m0, m1, s, tog);
+    rc_sum2_f64(z, unused, s, tog);
     if (threadIdx.x == 0) {
+      cl_st_f64(cl_map(&s.z[rank], 0), z);
       cl_st_f64(cl_map(&s.msum[rank][0], 0), m0);
       cl_st_f64(cl_map(&s.msum[rank][1], 0), m1);
     }
@@ -946,12 +967,14 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
     cl_sync();
     if (round == 0) { TLX_STAMP(p.sp, 14); }
     if (rank == 0 && warp_id() == 0) {
+      double Z = lane_id() < p.cluster ? s.z[lane_id()] : 0.0;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) Z += shfl_xor_f64(Z, o);
 #pragma unroll 1
       for (int j = 0; j < nq && tok < 0; ++j) {
         double mass = lane_id() < p.cluster ? s.msum[lane_id()][j] : 0.0;
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) mass += shfl_xor_f64(mass, o);
-        mass = __hiloint2double(__shfl_sync(0xFFFFFFFFu, __double2hiint(mass), 0), __shfl_sync(0xFFFFFFFFu, __double2loint(mass), 0));
         if (mass == 0.0 || !(mass / Z >= (double)pp)) tok = s.query_tok[j];
         tok = __shfl_sync(0xFFFFFFFFu, tok, 0);
       }

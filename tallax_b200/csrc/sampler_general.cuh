@@ -1,12 +1,7 @@
-// Whole-row ("general") sampler paths that work on a row in global memory, whatever
-// its top-k: the exact fallback of the sliced sampler and the path for rows whose top-k
-// filter is disabled or larger than the single-pass limit.
-//   bf16 : windowed histogram over the full 16-bit key.  The softmax mass of a value
-//          group is count * exp(value - max), so counts alone give the exact top-k
-//          boundary, the denominator and the top-p threshold.
-//   f32  : 12/12/8-bit radix passes, counts for the top-k boundary and f64 mass bins
-//          for the top-p threshold.
-// Both end with a streaming Gumbel arg-max over the kept elements.
+// Whole-row sampler routines of the streaming form (sampler_stream.cuh): a bf16 row in global memory, whatever its
+// top-k.  Windowed histograms over the full 16-bit key: the softmax mass of a value group is count * exp(value - max),
+// so counts alone give the exact top-k boundary, the denominator and the top-p threshold; a streaming Gumbel arg-max
+// over the kept elements follows.
 #pragma once
 #include "select.cuh"
 
@@ -298,108 +293,6 @@ static __device__ __noinline__ int general_row_bf16(const __nv_bfloat16* __restr
   const uint32_t vstar32 = vstar16 == 0 ? 0u : key16_to_key32((uint32_t)vstar16);
   const bool ordered = bounded && vstar16 == vk16 && ties_admitted < ties_total;
   return final_argmax<TLX_BF16>(row, n, T_, vstar32, bounded, vk32, ties_admitted, ordered, noise, nrow, s);
-}
-
-// ---- any float dtype: 32-bit keys, radix digits of 12 / 12 / 8 bits -----------------------
-// `mass` holds kHistBins doubles; blockDim.x must divide kHistBins.
-template <int DT>
-static __device__ __noinline__ int general_row_radix(const typename Elem<DT>::type* __restrict__ row, int64_t n, int K,
-                                                 float p_row, float T_, const NoiseSrc& noise, int64_t nrow,
-                                                 SelectShared& s, double* mass) {
-  using T = typename Elem<DT>::type;
-  const int kPer = kHistBins / (int)blockDim.x;
-  const int shifts[3] = {20, 8, 0};
-  const int bits[3] = {12, 12, 8};
-  const bool bounded = (int64_t)K < n;
-  const uint64_t top = row_argmax<DT>(row, n, s);
-  const float xmax = key_f32((uint32_t)(top >> 32));
-
-  // phase A: K-th largest key and the number of admitted ties, by counting passes
-  uint32_t vk = 0, ties_admitted = 0, ties_total = 0;
-  if (bounded) {
-    uint32_t prefix = 0, prefix_mask = 0;
-    int need = K;
-    for (int d = 0; d < 3; ++d) {
-      const int nb = 1 << bits[d], sh = shifts[d];
-      for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) s.hist[i] = 0;
-      __syncthreads();
-      for_each_elem<DT>(row, 0, n, [&](T v, int64_t) {
-        const uint32_t key = Elem<DT>::key(v);
-        if ((key & prefix_mask) == prefix) atomicAdd(&s.hist[(key >> sh) & (nb - 1)], 1u);
-      });
-      __syncthreads();
-      find_threshold_bin(s, need, 0);
-      const int b = s.bin, above = s.above;
-      const uint32_t cb = s.hist[b];
-      __syncthreads();
-      prefix |= (uint32_t)b << sh;
-      prefix_mask |= (uint32_t)(nb - 1) << sh;
-      need -= above;
-      ties_total = cb;
-    }
-    vk = prefix;
-    ties_admitted = (uint32_t)need;
-  }
-
-  // phase B: softmax denominator over the top-k set
-  double Z = stream_mass<DT>(row, n, xmax, bounded, vk, s);
-  const double wk = bounded ? (double)expf(key_f32(vk) - xmax) : 0.0;
-  if (bounded) Z += (double)ties_admitted * wk;
-  const double target = (double)p_row * Z;
-
-  // phase C: radix descent on cumulative mass
-  uint32_t vstar;
-  {
-    uint32_t prefix = 0, prefix_mask = 0;
-    double cum = 0.0;
-    bool fell_through = false;
-    for (int d = 0; d < 3 && !fell_through; ++d) {
-      const int nb = 1 << bits[d], sh = shifts[d];
-      for (int i = threadIdx.x; i < kHistBins; i += blockDim.x) mass[i] = 0.0;
-      __syncthreads();
-      for_each_elem<DT>(row, 0, n, [&](T v, int64_t) {
-        const uint32_t key = Elem<DT>::key(v);
-        if ((key & prefix_mask) == prefix && (!bounded || key > vk))
-          atomicAdd(&mass[(key >> sh) & (nb - 1)], (double)expf(elem_as_float<DT>(v) - xmax));
-      });
-      __syncthreads();
-      if (threadIdx.x == 0 && bounded && (vk & prefix_mask) == prefix)
-        mass[(vk >> sh) & (nb - 1)] += (double)ties_admitted * wk;
-      if (threadIdx.x == 0) s.tmp_i[3] = -1;
-      __syncthreads();
-      // thread t owns bins [hi - kPer + 1, hi] in descending order
-      const int hi = kHistBins - 1 - threadIdx.x * kPer;
-      double local = 0.0;
-      for (int j = 0; j < kPer; ++j) local += mass[hi - j];
-      double total;
-      const double incl = block_scan_incl<double>(local, s.scan_f64, &total, ShflUpF64());
-      const double before = cum + incl - local;
-      if (before < target && before + local >= target) {
-        double run = before;
-        for (int j = 0; j < kPer; ++j) {
-          const double mj = mass[hi - j];
-          if (mj > 0.0 && run + mj >= target) {
-            s.tmp_i[3] = hi - j;
-            s.scan_f64[36] = run;
-            break;
-          }
-          run += mj;
-        }
-      }
-      __syncthreads();
-      const int found = s.tmp_i[3];
-      const double cum_before = s.scan_f64[36];
-      __syncthreads();
-      if (found < 0) { fell_through = true; break; }
-      prefix |= (uint32_t)found << sh;
-      prefix_mask |= (uint32_t)(nb - 1) << sh;
-      cum = cum_before;
-    }
-    // Mass short of the target (top_p ~ 1 and rounding): keep the whole top-k set.
-    vstar = fell_through ? (bounded ? vk : 0u) : prefix;
-  }
-  const bool ordered = bounded && vstar == vk && ties_admitted < ties_total;
-  return final_argmax<DT>(row, n, T_, vstar, bounded, vk, ties_admitted, ordered, noise, nrow, s);
 }
 
 }  // namespace tlx

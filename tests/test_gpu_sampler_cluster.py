@@ -1,0 +1,41 @@
+"""GPU: the sampler's cluster kernel (a row resident in a cluster's shared memory) at the sizes where its parts, its lists
+and its bound can go wrong, against the oracle."""
+import numpy as np
+import pytest
+
+from oracle import tallax_oracle as o
+from tallax_b200._src import ops
+from tests.conftest import to_dev, to_np
+
+pytestmark = pytest.mark.gpu
+
+
+# one element; a vector and a remainder; all elements candidates (<= 2048) and just not; parts that end inside a vector;
+# odd row starts; two, eight and sixteen CTAs; longer than a cluster holds
+@pytest.mark.parametrize("V", [1, 2, 129, 2048, 2049, 8191, 40961, 131072, 327681, 800001])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("from_key", [False, True])
+def test_cluster_sampler_sizes(cuda, dtype, V, from_key):
+    B = 8 if V < 300000 else 4
+    x, tk, tp, T, noise = o.make_sampling_inputs(B=B, V=max(V, 64), seed=V, dtype=dtype)
+    x, noise = np.ascontiguousarray(x[:, :V]), np.ascontiguousarray(noise[:, :V])
+    xf = x.astype(np.float32)
+    tk[:] = ([1024, 0, 50, 257, 0, 1, 0, 1500])[:B]
+    T[B - 3] = 0.0                                             # greedy
+    if B == 8:
+        xf[1] = 0.25 * (np.arange(V) % 3)                      # three values: far more survivors than the lists hold
+        xf[2] = np.round(xf[2])                                # ties at the k-th value
+        xf[3, V // 2:] = -np.inf                               # masked half
+        xf[4] *= 0.01                                          # flat
+        xf[6] = -np.inf
+        xf[6, V // 3] = -3.0                                   # a single token left
+        xf[7] = np.sort(xf[7])                                 # the set sits in one CTA's part
+    x = xf.astype(x.dtype)
+    key = (17, V)
+    kw = dict(rng_key=key) if from_key else dict(noise=noise)
+    exp, flags = o.sample(x, tk, tp, T, return_flags=True, **kw)
+    dkw = dict(rng_key=key) if from_key else dict(noise=to_dev(noise, cuda))
+    tok, status = ops.sample(to_dev(x, cuda), to_dev(tk, cuda), to_dev(tp, cuda), to_dev(T, cuda), return_status=True, **dkw)
+    bad = (to_np(tok) != exp) & ~flags
+    assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
+    assert (to_np(status) & 2 == 0).all()
