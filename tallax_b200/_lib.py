@@ -66,7 +66,14 @@ SIGNATURES = {
     "tlx_exchange_merge_and_sample": (_i32, [_vp, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _vp, _vp]),
 }
 
+BINDING_PATH = os.path.join(_HERE, "lib", "_tlx_torch.so")
+# the library functions that the binding calls
+_BOUND = ("tlx_sample", "tlx_sample_workspace_bytes", "tlx_top_k", "tlx_top_k_workspace_bytes", "tlx_sort",
+          "tlx_sort_workspace_bytes", "tlx_take_along_axis", "tlx_cumsum", "tlx_exchange_shard_candidates",
+          "tlx_exchange_merge_and_sample")
+
 _lib = None
+_native = None
 
 
 class TallaxLibraryError(RuntimeError):
@@ -105,3 +112,23 @@ def check(rc: int):
     if rc == TLX_ERR_UNSUPPORTED:
         raise NotImplementedError(msg)
     raise RuntimeError(f"tallax_b200 error {rc}: {msg}")
+
+
+def native():
+    """The CPython binding of the hot entry points (csrc/torch_binding.cpp), bound to the loaded library.  Its functions
+    return NotImplemented for arguments that need converting first."""
+    global _native
+    if _native is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (the binding's symbols come from torch's libraries)
+        lib = load()
+        if not os.path.exists(BINDING_PATH):
+            raise TallaxLibraryError(f"{BINDING_PATH} is missing: build it with `python -m tallax_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_tlx_torch", BINDING_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("_tlx_torch", loader))
+        loader.exec_module(mod)
+        mod.init(check, {name: C.cast(getattr(lib, name), C.c_void_p).value for name in _BOUND})
+        _native = mod
+    return _native

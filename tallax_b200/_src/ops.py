@@ -2,7 +2,10 @@
 
 PyTorch is used for device memory and streams only: every function allocates its
 outputs (and workspace) as torch CUDA tensors and passes raw pointers plus the current
-stream to libtallax_b200.so.
+stream to libtallax_b200.so.  The functions of the hot paths first offer their arguments to
+the CPython binding (`_lib.native()`), which serves contiguous CUDA tensors of the right types
+with a few hundred nanoseconds of host work; what it declines is converted here and goes
+through ctypes.
 """
 from __future__ import annotations
 
@@ -104,6 +107,9 @@ def offset_operand(dim0_offset):
 
 # ---------------------------------------------------------------------------------------
 def take_along_axis(values: torch.Tensor, indices: torch.Tensor, axis: int) -> torch.Tensor:
+    out = _lib.native().take_along_axis(values, indices, axis)
+    if out is not NotImplemented:
+        return out
     values, indices = _dev(values), _dev(indices)
     if values.ndim != 2 or indices.ndim != 2:
         raise ValueError("Only 2D inputs supported")
@@ -117,6 +123,9 @@ def take_along_axis(values: torch.Tensor, indices: torch.Tensor, axis: int) -> t
 
 
 def cumsum(arr: torch.Tensor, axis: int, reverse: bool = False) -> torch.Tensor:
+    out = _lib.native().cumsum(arr, axis, reverse)
+    if out is not NotImplemented:
+        return out
     arr = _dev(arr)
     if arr.ndim != 2:
         raise ValueError("Only 2D inputs supported")
@@ -147,6 +156,9 @@ def argmax(keys: torch.Tensor, axis: int) -> torch.Tensor:
 def argsort_rows(keys: torch.Tensor, descending: bool = False, in_perm: torch.Tensor | None = None,
                  want_keys: bool = True, want_perm: bool = True):
     """Stable argsort of every row; returns (sorted_keys | None, perm | None)."""
+    out = _lib.native().argsort_rows(keys, descending, in_perm, want_keys, want_perm)
+    if out is not NotImplemented:
+        return out
     keys = _dev(keys)
     rows, n = keys.shape
     lib = _lib.load()
@@ -161,6 +173,10 @@ def argsort_rows(keys: torch.Tensor, descending: bool = False, in_perm: torch.Te
 
 def top_k(x: torch.Tensor, k_max: int, k_per_row=None, replace_val=None, single_pass: bool = False):
     """Returns (vals, idx) or, with single_pass, (vals, idx, valid, depths, cutoff)."""
+    if not single_pass:
+        out = _lib.native().top_k(x, k_max, k_per_row, replace_val)
+        if out is not NotImplemented:
+            return out
     x = _dev(x)
     if x.ndim != 2:
         raise ValueError("Only 2D inputs supported")
@@ -208,7 +224,8 @@ def top_p_mask(topk_logits, p, replace_val):
         x = x.float()
     k, batch = x.shape
     out = torch.empty_like(x)
-    check(_lib.load().tlx_top_p_mask(_stream(), _ptr(x), _ptr(_f32vec(p, batch, x.device)), k, batch,
+    p = _f32vec(p, batch, x.device)
+    check(_lib.load().tlx_top_p_mask(_stream(), _ptr(x), _ptr(p), k, batch,
                                      float(replace_val), _ptr(out)))
     return out
 
@@ -243,20 +260,21 @@ def top_p_and_sample(topk_logits, topk_idx, top_p, temperature, *, vocab_size, r
     elif rng_key is None:
         raise ValueError("either rng_key or noise is required")
     out = torch.empty(rows, dtype=torch.int32, device=dev)
+    top_p, temperature = _f32vec(top_p, rows, dev), _f32vec(temperature, rows, dev)   # alive until the launch
     kd, od = key_operand(rng_key), offset_operand(dim0_offset)
     if kd is not None or od is not None:
         if kd is None and noise is None:
             kd = torch.tensor(key_pair(rng_key), dtype=torch.int64, device=dev).to(torch.int32)
         check(_lib.load().tlx_top_p_and_sample_dev(
             _stream(), _ptr(topk_logits), dtype_code(topk_logits), _ptr(topk_idx), rows, k,
-            _ptr(_f32vec(top_p, rows, dev)), _ptr(_f32vec(temperature, rows, dev)), _ptr(noise),
+            _ptr(top_p), _ptr(temperature), _ptr(noise),
             noise.shape[1] if noise is not None else 0, _ptr(kd), int(vocab_size), float(replace_val),
             _ptr(od if od is not None else _host_offset(dim0_offset, dev)), _ptr(out)))
         return out
     k0, k1 = key_pair(rng_key)
     check(_lib.load().tlx_top_p_and_sample(
-        _stream(), _ptr(topk_logits), dtype_code(topk_logits), _ptr(topk_idx), rows, k, _ptr(_f32vec(top_p, rows, dev)),
-        _ptr(_f32vec(temperature, rows, dev)), _ptr(noise), noise.shape[1] if noise is not None else 0, k0, k1,
+        _stream(), _ptr(topk_logits), dtype_code(topk_logits), _ptr(topk_idx), rows, k, _ptr(top_p),
+        _ptr(temperature), _ptr(noise), noise.shape[1] if noise is not None else 0, k0, k1,
         int(vocab_size), float(replace_val), int(dim0_offset), _ptr(out)))
     return out
 
@@ -275,6 +293,10 @@ class SampleWorkspace:
 def sample(logits, top_k_, top_p, temperature, *, rng_key=None, noise=None, dim0_offset=0, workspace=None,
            return_status=False):
     """Fused sampler: logits [B, V] -> int32 tokens [B]."""
+    if workspace is None and not return_status:
+        out = _lib.native().sample(logits, top_k_, top_p, temperature, rng_key, noise, dim0_offset)
+        if out is not NotImplemented:
+            return out
     logits = _dev(logits)
     if logits.ndim != 2:
         raise ValueError("Only 2D inputs supported")
@@ -287,22 +309,24 @@ def sample(logits, top_k_, top_p, temperature, *, rng_key=None, noise=None, dim0
     elif rng_key is None:
         raise ValueError("either rng_key or noise is required")
     w = workspace if workspace is not None else SampleWorkspace(rows, vocab, dev)
+    # converted copies have to live until the launch: a freed one's memory goes to the next
+    top_k_, top_p, temperature = _i32vec(top_k_, rows, dev), _f32vec(top_p, rows, dev), _f32vec(temperature, rows, dev)
     kd, od = key_operand(rng_key), offset_operand(dim0_offset)
     if kd is not None or od is not None:
         # key and/or offset live on the device: they are handed over as device operands
         if kd is None and noise is None:
             kd = torch.tensor(key_pair(rng_key), dtype=torch.int64, device=dev).to(torch.int32)
         check(_lib.load().tlx_sample_dev(
-            _stream(), _ptr(logits), dtype_code(logits), rows, vocab, vocab, _ptr(_i32vec(top_k_, rows, dev)),
-            _ptr(_f32vec(top_p, rows, dev)), _ptr(_f32vec(temperature, rows, dev)), _ptr(noise),
+            _stream(), _ptr(logits), dtype_code(logits), rows, vocab, vocab, _ptr(top_k_),
+            _ptr(top_p), _ptr(temperature), _ptr(noise),
             noise.shape[1] if noise is not None else 0, _ptr(kd),
             _ptr(od if od is not None else _host_offset(dim0_offset, dev)), _ptr(w.tokens), _ptr(w.status),
             _ptr(w.ws), w.ws.numel()))
         return (w.tokens, w.status) if return_status else w.tokens
     k0, k1 = key_pair(rng_key)
     check(_lib.load().tlx_sample(
-        _stream(), _ptr(logits), dtype_code(logits), rows, vocab, vocab, _ptr(_i32vec(top_k_, rows, dev)),
-        _ptr(_f32vec(top_p, rows, dev)), _ptr(_f32vec(temperature, rows, dev)), _ptr(noise),
+        _stream(), _ptr(logits), dtype_code(logits), rows, vocab, vocab, _ptr(top_k_),
+        _ptr(top_p), _ptr(temperature), _ptr(noise),
         noise.shape[1] if noise is not None else 0, k0, k1, int(dim0_offset), _ptr(w.tokens), _ptr(w.status),
         _ptr(w.ws), w.ws.numel()))
     if return_status:
@@ -351,11 +375,12 @@ def merge_and_sample(gathered, top_k_, top_p, temperature, out=None):
     dev = gathered.device
     if out is None:
         out = torch.empty(rows, dtype=torch.int32, device=dev)
+    top_k_, top_p, temperature = _i32vec(top_k_, rows, dev), _f32vec(top_p, rows, dev), _f32vec(temperature, rows, dev)
     block = 3 * rows * k
     check(_lib.load().tlx_merge_and_sample(
         _stream(), gathered[0, 0].data_ptr(), gathered[0, 1].data_ptr(), gathered[0, 2].data_ptr(), rows,
-        n_shards * k, k, block, k, _ptr(_i32vec(top_k_, rows, dev)), _ptr(_f32vec(top_p, rows, dev)),
-        _ptr(_f32vec(temperature, rows, dev)), _ptr(out)))
+        n_shards * k, k, block, k, _ptr(top_k_), _ptr(top_p),
+        _ptr(temperature), _ptr(out)))
     return out
 
 
@@ -373,7 +398,8 @@ class Exchange:
         self.rank = None
         self.own = None          # device address of this rank's buffer
         self.handle = None
-        self.peers = None        # ctypes array of `world` device addresses
+        self.peers = None        # ctypes array of `world` device addresses ...
+        self.peers_address = 0   # ... and where it lies
         self._opened = []
         self.status = None
 
@@ -409,6 +435,7 @@ class Exchange:
                 self._opened.append(peer.value)
                 ptrs.append(peer.value)
         self.peers = (ctypes.c_void_p * self.world)(*ptrs)
+        self.peers_address = ctypes.addressof(self.peers)
         return self
 
     @classmethod
@@ -418,6 +445,7 @@ class Exchange:
         for r, e in enumerate(group):
             e.rank = r
             e.peers = (ctypes.c_void_p * world)(*[g.own for g in group])
+            e.peers_address = ctypes.addressof(e.peers)
         return group
 
     def state(self):
@@ -468,13 +496,29 @@ def exchange_shard_candidates(logits_shard, col_offset: int, exchange: Exchange,
         exchange.rank, exchange.world, exchange.peers))
 
 
+def exchange_step(logits_shard, col_offset: int, exchange: Exchange, top_k_, top_p, temperature, *, noise_shard=None,
+                  rng_key=None, vocab_total=None, dim0_offset=0, out=None):
+    """Both stages of a step on this rank: the candidates into every rank's buffer, then merge and sample."""
+    vocab_total = logits_shard.shape[1] if vocab_total is None else vocab_total
+    if getattr(exchange, "peers_address", 0) and exchange.own and logits_shard.shape[0] == exchange.rows:
+        got = _lib.native().exchange_step(logits_shard, col_offset, vocab_total, rng_key, noise_shard, dim0_offset,
+                                          exchange.k_cand, exchange.rank, exchange.world, exchange.peers_address, exchange.own,
+                                          exchange.status, top_k_, top_p, temperature, out)
+        if got is not NotImplemented:
+            return got
+    exchange_shard_candidates(logits_shard, col_offset, exchange, noise_shard=noise_shard, rng_key=rng_key,
+                              vocab_total=vocab_total, dim0_offset=dim0_offset)
+    return exchange_merge_and_sample(exchange, top_k_, top_p, temperature, out=out)
+
+
 def exchange_merge_and_sample(exchange: Exchange, top_k_, top_p, temperature, out=None):
     """Stage 2 on this rank's exchange buffer: waits per row for all ranks' candidates, merges, samples."""
     rows = exchange.rows
     dev = exchange.device
     if out is None:
         out = torch.empty(rows, dtype=torch.int32, device=dev)
+    top_k_, top_p, temperature = _i32vec(top_k_, rows, dev), _f32vec(top_p, rows, dev), _f32vec(temperature, rows, dev)
     check(_lib.load().tlx_exchange_merge_and_sample(
-        _stream(), exchange.own, rows, exchange.k_cand, exchange.world, _ptr(_i32vec(top_k_, rows, dev)),
-        _ptr(_f32vec(top_p, rows, dev)), _ptr(_f32vec(temperature, rows, dev)), _ptr(out), _ptr(exchange.status)))
+        _stream(), exchange.own, rows, exchange.k_cand, exchange.world, _ptr(top_k_),
+        _ptr(top_p), _ptr(temperature), _ptr(out), _ptr(exchange.status)))
     return out

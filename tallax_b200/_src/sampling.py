@@ -107,10 +107,9 @@ def sample_vocab_sharded(rng_key, logits_shard, tpu_sampling_metadata, *, group=
     if exchange is not None:
         if exchange.world != world or exchange.rank != rank:
             raise ValueError("exchange was made for another group")
-        ops.exchange_shard_candidates(logits_shard, rank * v_local, exchange, noise_shard=noise_shard, rng_key=rng_key,
-                                      vocab_total=v_local * world, dim0_offset=dim0_offset)
-        return ops.exchange_merge_and_sample(exchange, md.top_k, md.top_p, md.temperature,
-                                             out=workspace.tokens if workspace is not None else None)
+        return ops.exchange_step(logits_shard, rank * v_local, exchange, md.top_k, md.top_p, md.temperature,
+                                 noise_shard=noise_shard, rng_key=rng_key, vocab_total=v_local * world,
+                                 dim0_offset=dim0_offset, out=workspace.tokens if workspace is not None else None)
     if k_cand is None:
         k_cand = 128
     k_cand = min(k_cand, v_local)

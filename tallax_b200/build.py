@@ -9,6 +9,9 @@
     python -m tallax_b200.build --timeline # libtallax_b200_timeline.so: the streaming sampler's kernels
                                            # record global-timer stamps per CTA (sampler.cu, TLX_STAMP)
 
+Next to the library the torch binding (csrc/torch_binding.cpp -> lib/_tlx_torch.so) is compiled with g++ against the
+installed torch's headers.
+
 Every .cu file is compiled to an object of its own (in parallel) under lib/obj, so that a change to one
 kernel file does not rebuild the others.
 """
@@ -25,6 +28,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 OBJ_DIR = os.path.join(LIB_DIR, "obj")
 LIB_PATH = os.path.join(LIB_DIR, "libtallax_b200.so")
+BINDING_SRC = os.path.join(CSRC, "torch_binding.cpp")
+BINDING_PATH = os.path.join(LIB_DIR, "_tlx_torch.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -48,6 +53,29 @@ def _newer(path, deps):
         return True
     t = os.path.getmtime(path)
     return any(os.path.getmtime(d) > t for d in deps)
+
+
+def build_binding(force: bool = False) -> str:
+    """lib/_tlx_torch.so, the CPython binding on torch tensors."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    header = os.path.join(HERE, "..", "include", "tallax_b200.h")
+    if not force and not _newer(BINDING_PATH, [BINDING_SRC, header]):
+        return BINDING_PATH
+    os.makedirs(LIB_DIR, exist_ok=True)
+    cuda = os.environ.get("CUDA_HOME") or "/usr/local/cuda"
+    includes = [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-w", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *(f"-I{p}" for p in includes), BINDING_SRC, "-o", BINDING_PATH,
+           *(f"-L{p}" for p in cpp_extension.library_paths()), "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch",
+           "-lc10_cuda", "-lc10"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed: " + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    return BINDING_PATH
 
 
 def build(force: bool = False, verbose: bool = False, checked: bool = False, timeline: bool = False) -> str:
@@ -87,6 +115,8 @@ def build(force: bool = False, verbose: bool = False, checked: bool = False, tim
     def run(cmd):
         return cmd, subprocess.run(cmd, capture_output=True, text=True)
 
+    if not (checked or timeline):
+        build_binding(force)
     if jobs:
         with ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:
             for cmd, res in ex.map(run, jobs):
