@@ -1,6 +1,6 @@
 // Gather (take_along_axis), cumsum, arg-max and counter-based uniform noise.
 // All four are plain HBM-bound streaming kernels: one read, one write, coalesced.
-#include "tlx_common.cuh"
+#include "row_cluster.cuh"
 
 #include <atomic>
 
@@ -104,49 +104,246 @@ static int launch_gather(cudaStream_t st, const void* values, const int32_t* idx
 // ---------------------------------------------------------------------------------
 // cumsum
 // ---------------------------------------------------------------------------------
-template <typename T, typename Shfl>
-__global__ void cumsum_axis1_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t cols, int reverse) {
-  constexpr int ITEMS = 4;
-  __shared__ T scratch[33];
-  const T* src = in + blockIdx.x * cols;
-  T* dst = out + blockIdx.x * cols;
+// Along rows.  HBM-bound: one read, one write.  A CTA sums tiles of 256 threads x V vectors of four; a row's tiles go
+// round the CTAs of a cluster (as many CTAs as it takes to fill the GPU) and every turn carries the sum on.  What
+// keeps the memory system busy is a ring of kStages tiles per CTA, filled by asynchronous copies that run ahead of
+// the scans, the barriers and the stores: without it the cluster's barrier of every turn was paid in full (f32
+// [256, 128256] 81 us).  A thread copies and reads the same vectors, so the ring needs no barrier of its own.
+//   A warp owns V runs of 32 vectors, scanned independently and chained afterwards; warp totals meet in shared memory,
+// CTA totals in distributed shared memory, and the sums go out from registers.  Reversed sums walk the same vectors
+// from the end.  f32 [64, 128256]: 143 us with one CTA per row and a block scan per 1024 elements.
+constexpr int kCumsumThreads = 256;
+template <typename T, typename Idx, int V, int kStages>
+__global__ void __launch_bounds__(kCumsumThreads)
+cumsum_axis1_kernel(const T* __restrict__ in, T* __restrict__ out, Idx cols, int reverse, int cluster, int same_phase) {
+  constexpr int kThreads = kCumsumThreads, kWarps = kThreads / 32, kPer = kThreads * V;
+  __shared__ __align__(16) uint4 ring[kStages][kPer];
+  __shared__ T warp_total[2][kWarps];
+  __shared__ T cta_total[2];           // alternating, so that a slow reader of the last turn is not overtaken
+  const int rank = cluster > 1 ? (int)cl_rank() : 0;
+  const int64_t row = blockIdx.x / cluster;
+  const T* src = in + row * (int64_t)cols;
+  T* dst = out + row * (int64_t)cols;
+  const int off = (int)((reinterpret_cast<uintptr_t>(src) & 15) / sizeof(T));
+  const Idx nvec = (off + cols + 3) / 4;
+  const int lane = lane_id(), w = warp_id();
+  const int slot0 = w * 32 * V + lane;
+  const Idx stride = (Idx)kPer * cluster;
+  auto fetch = [&](Idx v0, int stage) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const Idx v = v0 + 32 * k;
+      if (v < nvec) {
+        const Idx c = (reverse ? nvec - 1 - v : v) * 4 - off;
+        uint4* d = &ring[stage][slot0 + 32 * k];
+        if (c >= 0 && c + 4 <= cols) {
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(d)), "l"(src + c) : "memory");
+        } else {
+          T e[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) e[j] = c + j >= 0 && c + j < cols ? src[c + j] : T(0);
+          memcpy(d, e, 16);
+        }
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  Idx v0 = (Idx)rank * kPer + slot0;   // in the order of summation
+#pragma unroll
+  for (int i = 0; i < kStages - 1; ++i) fetch(v0 + i * stride, i);
   T carry = T(0);
-  const int64_t chunk = (int64_t)blockDim.x * ITEMS;
-  for (int64_t base = 0; base < cols; base += chunk) {
-    T v[ITEMS];
+  int turn = 0, stage = 0;
+  for (Idx base = 0; base < nvec; base += stride, v0 += stride, turn ^= 1) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2) : "memory");
+    T x[V][4];
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      T e[4] = {T(0), T(0), T(0), T(0)};
+      if (v0 + 32 * k < nvec) memcpy(e, &ring[stage][slot0 + 32 * k], 16);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[k][j] = reverse ? e[3 - j] : e[j];
+    }
+    fetch(v0 + (kStages - 1) * stride, stage == 0 ? kStages - 1 : stage - 1);   // the slot that was read a turn ago
+    stage = stage + 1 == kStages ? 0 : stage + 1;
+    T incl[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+#pragma unroll
+      for (int j = 1; j < 4; ++j) x[k][j] += x[k][j - 1];
+      incl[k] = x[k][3];
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) {
+        const T up = __shfl_up_sync(0xFFFFFFFFu, incl[k], o);
+        if (lane >= o) incl[k] += up;
+      }
+    }
     T run = T(0);
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-      const int64_t c = base + (int64_t)threadIdx.x * ITEMS + j;
-      const int64_t cc = reverse ? (cols - 1 - c) : c;
-      T x = (c < cols) ? src[cc] : T(0);
-      run += x;
-      v[j] = run;
+    for (int k = 0; k < V; ++k) {
+      const T total = __shfl_sync(0xFFFFFFFFu, incl[k], 31);
+      incl[k] = run + (incl[k] - x[k][3]);    // sum before this vector, inside the warp
+      run += total;
     }
-    T total;
-    T incl = block_scan_incl<T>(run, scratch, &total, Shfl());
-    const T offs = carry + (incl - run);
+    if (lane == 0) warp_total[turn][w] = run;
+    __syncthreads();
+    T before = T(0), cta = T(0);
 #pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-      const int64_t c = base + (int64_t)threadIdx.x * ITEMS + j;
-      const int64_t cc = reverse ? (cols - 1 - c) : c;
-      if (c < cols) dst[cc] = v[j] + offs;
+    for (int i = 0; i < kWarps; ++i) {
+      const T t = warp_total[turn][i];
+      if (i < w) before += t;
+      cta += t;
     }
-    carry += total;
+    T all = cta;
+    if (cluster > 1) {
+      if (threadIdx.x == 0) cta_total[turn] = cta;
+      cl_sync();
+      all = T(0);
+      T mine = T(0);
+      const uint32_t bits = lane < cluster ? cl_ld_u32(cl_map(&cta_total[turn], (uint32_t)lane)) : 0u;
+      T t;
+      memcpy(&t, &bits, 4);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const T ti = __shfl_sync(0xFFFFFFFFu, t, i);
+        if (i < cluster) {
+          if (i < rank) mine += ti;
+          all += ti;
+        }
+      }
+      before += mine;
+    }
+    before += carry;
+    carry += all;
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const Idx v = v0 + 32 * k, c = (reverse ? nvec - 1 - v : v) * 4 - off;
+      if (v >= nvec) continue;
+      const T add = before + incl[k];
+      T e[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) e[j] = x[k][reverse ? 3 - j : j] + add;
+      if (same_phase && c >= 0 && c + 4 <= cols) {
+        uint4 q;
+        memcpy(&q, e, 16);
+        __stcs(reinterpret_cast<uint4*>(dst + c), q);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (c + j >= 0 && c + j < cols) dst[c + j] = e[j];
+      }
+    }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  if (cluster > 1) cl_sync();   // nobody leaves while its total may still be read
 }
 
+// Along columns.  A CTA takes 32 columns (128-byte rows of the matrix per warp) and kAxis0Warps x kAxis0Rows rows at a
+// time: every warp sums its own consecutive rows, the totals meet in shared memory, the sums go out from registers.
+// Few columns: the rows of a turn are cut over the CTAs of a cluster, whose totals meet in distributed shared memory.
+// One thread per column with one load in flight took 130 us for f32 [1024, 500].
+constexpr int kAxis0Warps = 16, kAxis0Rows = 16, kAxis0Turn = kAxis0Warps * kAxis0Rows;
 template <typename T>
-__global__ void cumsum_axis0_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t rows, int64_t cols,
-                                    int reverse) {
-  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  T acc = T(0);
-  for (int64_t r = 0; r < rows; ++r) {
-    const int64_t rr = reverse ? (rows - 1 - r) : r;
-    acc += in[rr * cols + c];
-    out[rr * cols + c] = acc;
+__global__ void __launch_bounds__(kAxis0Warps * 32) cumsum_axis0_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t rows,
+                                                                         int64_t cols, int reverse, int cluster) {
+  __shared__ T total[2][kAxis0Warps][32];
+  __shared__ T cta_total[2][32];
+  const int rank = cluster > 1 ? (int)cl_rank() : 0;
+  const int lane = lane_id(), w = warp_id();
+  const int64_t c = blockIdx.x / cluster * 32ll + lane;
+  const bool live = c < cols;
+  T carry = T(0);
+  int turn = 0;
+  for (int64_t base = 0; base < rows; base += (int64_t)kAxis0Turn * cluster, turn ^= 1) {
+    const int64_t r0 = base + rank * kAxis0Turn + w * kAxis0Rows;
+    T x[kAxis0Rows];
+#pragma unroll
+    for (int k = 0; k < kAxis0Rows; ++k) {
+      const int64_t r = r0 + k;
+      x[k] = live && r < rows ? __ldcs(in + (reverse ? rows - 1 - r : r) * cols + c) : T(0);
+    }
+#pragma unroll
+    for (int k = 1; k < kAxis0Rows; ++k) x[k] += x[k - 1];
+    total[turn][w][lane] = x[kAxis0Rows - 1];
+    __syncthreads();
+    T before = carry, cta = T(0);
+#pragma unroll
+    for (int i = 0; i < kAxis0Warps; ++i) {
+      const T t = total[turn][i][lane];
+      if (i < w) before += t;
+      cta += t;
+    }
+    T all = cta;
+    if (cluster > 1) {
+      if (w == 0) cta_total[turn][lane] = cta;
+      cl_sync();
+      all = T(0);
+      for (int i = 0; i < cluster; ++i) {
+        const uint32_t bits = cl_ld_u32(cl_map(&cta_total[turn][lane], (uint32_t)i));
+        T t;
+        memcpy(&t, &bits, 4);
+        if (i < rank) before += t;
+        all += t;
+      }
+    }
+    carry += all;
+#pragma unroll
+    for (int k = 0; k < kAxis0Rows; ++k) {
+      const int64_t r = r0 + k;
+      if (live && r < rows) __stcs(out + (reverse ? rows - 1 - r : r) * cols + c, x[k] + before);
+    }
   }
+  if (cluster > 1) cl_sync();   // nobody leaves while its totals may still be read
+}
+
+template <typename... Params, typename... Args>
+static int launch_cluster(void (*kernel)(Params...), unsigned grid, unsigned block, int cluster, cudaStream_t st, const char* what,
+                          Args... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = cluster > 1 ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+  if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e)); }
+  count_launch();
+  return TLX_OK;
+}
+
+template <typename T, typename Idx, int V, int kStages>
+static int launch_cumsum_rows(cudaStream_t st, const T* in, T* out, int64_t rows, int64_t cols, int reverse, int cluster) {
+  const int same = ((reinterpret_cast<uintptr_t>(in) ^ reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  return launch_cluster(cumsum_axis1_kernel<T, Idx, V, kStages>, (unsigned)(rows * cluster), kCumsumThreads, cluster, st, "cumsum", in,
+                        out, cols, reverse, cluster, same);
+}
+
+// One vector a thread for rows of up to 1024 elements; beyond that two tiles of 4096 elements (32 KB: six CTAs fit an SM)
+// and as many CTAs per row, up to eight and up to its tiles, as give 740 in all (five per SM): a barrier across CTAs
+// every turn costs more than it brings once the rows fill the GPU.  Measured, f32, with the ring: [64, 128256] 15.7 us,
+// [167, 27252] 10.1, [256, 128256] 54, [1024, 31000] 48 (5.3 TB/s).
+template <typename T>
+static int launch_cumsum(cudaStream_t st, const void* in, void* out, int64_t rows, int64_t cols, int axis, int reverse) {
+  const T* x = (const T*)in;
+  T* y = (T*)out;
+  if (axis == 0) {
+    const int64_t strips = (cols + 31) / 32;
+    int cluster = 1;
+    while (cluster < 8 && strips * cluster * 2 <= 592 && (int64_t)cluster * kAxis0Turn < rows) cluster *= 2;
+    return launch_cluster(cumsum_axis0_kernel<T>, (unsigned)(strips * cluster), kAxis0Warps * 32, cluster, st, "cumsum", x, y, rows, cols,
+                          reverse, cluster);
+  }
+  const int64_t n = cols + 3;   // the first vector may be a partial one
+  if (n <= 1024) return launch_cumsum_rows<T, int, 1, 2>(st, x, y, rows, cols, reverse, 1);
+  int cluster = 1;
+  while (cluster < 8 && rows * cluster * 2 <= 740 && cluster * 4096ll < n) cluster *= 2;
+  if (cols < (1ll << 30)) return launch_cumsum_rows<T, int, 4, 2>(st, x, y, rows, cols, reverse, cluster);
+  return launch_cumsum_rows<T, int64_t, 4, 2>(st, x, y, rows, cols, reverse, cluster);
 }
 
 // ---------------------------------------------------------------------------------
@@ -275,20 +472,8 @@ int tlx_cumsum(void* stream, const void* in, void* out, int64_t rows, int64_t co
   TLX_CHECK_ARG(in && out, "cumsum: null pointer");
   if (dtype != TLX_F32 && dtype != TLX_I32)
     return set_error(TLX_ERR_UNSUPPORTED, "cumsum: dtype %d not supported (f32, i32)", dtype);
-  if (axis == 1) {
-    if (dtype == TLX_F32)
-      cumsum_axis1_kernel<float, ShflUpF32><<<(unsigned)rows, 256, 0, st>>>((const float*)in, (float*)out, cols, reverse);
-    else
-      cumsum_axis1_kernel<int, ShflUpI32><<<(unsigned)rows, 256, 0, st>>>((const int*)in, (int*)out, cols, reverse);
-  } else {
-    const unsigned blocks = (unsigned)((cols + 127) / 128);
-    if (dtype == TLX_F32)
-      cumsum_axis0_kernel<float><<<blocks, 128, 0, st>>>((const float*)in, (float*)out, rows, cols, reverse);
-    else
-      cumsum_axis0_kernel<int><<<blocks, 128, 0, st>>>((const int*)in, (int*)out, rows, cols, reverse);
-  }
-  TLX_CHECK_LAUNCH("cumsum");
-  return TLX_OK;
+  return dtype == TLX_F32 ? launch_cumsum<float>(st, in, out, rows, cols, axis, reverse)
+                          : launch_cumsum<int>(st, in, out, rows, cols, axis, reverse);
 }
 
 int tlx_argmax(void* stream, const void* keys, int dtype, int64_t rows, int64_t cols, int axis, int32_t* out_idx) {

@@ -1,0 +1,22 @@
+"""GPU: cumsum at the edges of its tiles, rings and clusters (odd row starts, one element over a tile, several turns)."""
+import numpy as np
+import pytest
+
+from tallax_b200 import tax
+from tests.conftest import to_dev, to_np
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape,axis", [((5, 1021), 1), ((5, 1022), 1), ((3, 4095), 1), ((2, 4098), 1), ((7, 16385), 1), ((3, 70001), 1),
+                                        ((400, 5003), 1), ((1, 1), 1), ((256, 33), 0), ((257, 31), 0), ((2049, 5), 0), ((5000, 70), 0)])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_cumsum_sizes(cuda, shape, axis, reverse):
+    rng = np.random.default_rng(shape[1])
+    x = rng.integers(-1000, 1000, shape).astype(np.int32)
+    y = np.flip(np.cumsum(np.flip(x, axis), axis=axis, dtype=np.int32), axis) if reverse else np.cumsum(x, axis=axis, dtype=np.int32)
+    assert np.array_equal(to_np(tax.cumsum(to_dev(x, cuda), axis, reverse=reverse)), y)
+    # whole numbers, so that f32 sums are exact in any order
+    f = (x % 8).astype(np.float32)
+    g = np.flip(np.cumsum(np.flip(f, axis), axis=axis), axis) if reverse else np.cumsum(f, axis=axis)
+    assert np.array_equal(to_np(tax.cumsum(to_dev(f, cuda), axis, reverse=reverse)), g)
