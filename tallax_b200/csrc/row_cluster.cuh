@@ -48,6 +48,7 @@ __device__ __forceinline__ uint32_t cl_ld_u16(uint32_t a) {
 }
 __device__ __forceinline__ void cl_st_u32(uint32_t a, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void cl_st_f32(uint32_t a, float v) { cl_st_u32(a, __float_as_uint(v)); }
+__device__ __forceinline__ void cl_st_u64(uint32_t a, uint64_t v) { asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }
 __device__ __forceinline__ void cl_st_f64(uint32_t a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
 __device__ __forceinline__ float cl_ld_f32(uint32_t a) { return __uint_as_float(cl_ld_u32(a)); }
 __device__ __forceinline__ double cl_ld_f64(uint32_t a) {
@@ -377,9 +378,10 @@ __device__ __forceinline__ void rc_filter(const RcPart<DT>& part, float thr, RcS
 #pragma unroll
     for (int j = 0; j < VEC; ++j) {
       const float x = elem_as_float<DT>(e[j]);
-      if (!(x < thr)) {
+      const int i = v * VEC + j - part.off;
+      if (!(x < thr) && (unsigned)i < (unsigned)part.n) {
         const int slot = atomicAdd(&s.n_list, 1);
-        if (slot < kRcListCap) { lx[slot] = x; lpos[slot] = (unsigned short)(v * VEC + j - part.off); }
+        if (slot < kRcListCap) { lx[slot] = x; lpos[slot] = (unsigned short)i; }
       }
     }
   }
@@ -423,6 +425,23 @@ __device__ __forceinline__ int64_t rc_column(const RcShared& s, const unsigned s
   int r = 0;
   while (i >= s.first[r + 1]) ++r;
   return (int64_t)r * part_len + lpos[i];
+}
+
+// CTAs per row: parts of at most 40 KB (three or four CTAs fit an SM), eight CTAs at most: clusters of sixteen find
+// their place on the GPU so much later that they are only worth it for a few rows, where the shorter parts count.
+// A few rows take more and smaller parts, down to 8 KB, while there is an SM for every two CTAs.
+inline int rc_cluster_size(int64_t rows, int64_t n, int elem_bytes) {
+  const int64_t row_bytes = n * elem_bytes;
+  int c = n > kRcListCap ? 2 : 1;
+  while (c < 8 && row_bytes > (int64_t)c * 40960) c *= 2;
+  while (c < kRcMaxCluster && rows * c * 2 <= 296 && row_bytes > (int64_t)c * 8192) c *= 2;
+  if (c < kRcMaxCluster && n > (int64_t)c * kRcMaxPart) c = kRcMaxCluster;
+  return c;
+}
+// Elements of a part, a multiple of a 16-byte vector.
+inline int64_t rc_part_len(int64_t n, int cluster, int elem_bytes) {
+  const int vec = 16 / elem_bytes;
+  return ((n + cluster - 1) / cluster + vec - 1) / vec * vec;
 }
 
 }  // namespace tlx

@@ -716,25 +716,13 @@ static int launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned b
 }
 
 // ---- cluster path (sampler_cluster.cuh) -----------------------------------------------------------------------
-// CTAs per row: parts of at most 40 KB (three or four CTAs fit an SM), eight CTAs at most: clusters of sixteen find
-// their place on the GPU so much later that they are only worth it for a few rows, where the shorter parts count.
-// A few rows take more and smaller parts, down to 8 KB, while there is an SM for every two CTAs.
-static int cluster_size(int64_t rows, int64_t vocab, int elem_bytes) {
-  const int64_t row_bytes = vocab * elem_bytes;
-  int c = vocab > kRcListCap ? 2 : 1;
-  while (c < 8 && row_bytes > (int64_t)c * 40960) c *= 2;
-  while (c < kRcMaxCluster && rows * c * 2 <= 296 && row_bytes > (int64_t)c * 8192) c *= 2;
-  if (c < kRcMaxCluster && vocab > (int64_t)c * kRcMaxPart) c = kRcMaxCluster;
-  return c;
-}
-
 template <int DT>
 static int launch_cluster_path(cudaStream_t st, const SampleParams& sp) {
-  const int es = (int)sizeof(typename Elem<DT>::type), vec = 16 / es;
+  const int es = (int)sizeof(typename Elem<DT>::type);
   RcSampleParams p{};
   p.sp = sp;
-  p.cluster = cluster_size(sp.rows, sp.vocab, es);
-  p.part_len = ((sp.vocab + p.cluster - 1) / p.cluster + vec - 1) / vec * vec;
+  p.cluster = rc_cluster_size(sp.rows, sp.vocab, es);
+  p.part_len = rc_part_len(sp.vocab, p.cluster, es);
   if (p.part_len > kRcMaxPart) { p.cluster = 1; p.part_len = 0; }   // longer than a cluster holds: rc_slow_row
   size_t part_bytes = (size_t)p.part_len * es + 32;
   if (part_bytes < kRcMinPartBytes) part_bytes = kRcMinPartBytes;

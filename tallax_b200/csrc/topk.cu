@@ -47,7 +47,7 @@ __device__ __forceinline__ typename Elem<DT>::type cast_replace(double v) {
 // Writes a row's results from its sorted candidate list (m valid entries, the first K are the answer).
 template <int DT>
 __device__ __forceinline__ void emit_row(const TopkParams& p, int64_t r, const typename Elem<DT>::type* __restrict__ row,
-                                         const uint64_t* cand, int m, const SelectShared& s) {
+                                         const uint64_t* cand, int m, int refinements = 0, int bin = 0) {
   using T = typename Elem<DT>::type;
   const int K = p.k_max;
   const int k_row = p.k_per_row ? p.k_per_row[r] : K;
@@ -103,12 +103,12 @@ __device__ __forceinline__ void emit_row(const TopkParams& p, int64_t r, const t
     }
   }
   if (threadIdx.x == 0) {
-    if (p.out_depths) p.out_depths[r] = s.refinements;
+    if (p.out_depths) p.out_depths[r] = refinements;
     if (p.out_cutoff) {
       if constexpr (DT == TLX_I32 || DT == TLX_U32)
-        reinterpret_cast<int32_t*>(p.out_cutoff)[r] = (int32_t)Elem<TLX_I32>::from_key((uint32_t)s.bin << kHistShift);
+        reinterpret_cast<int32_t*>(p.out_cutoff)[r] = (int32_t)Elem<TLX_I32>::from_key((uint32_t)bin << kHistShift);
       else
-        reinterpret_cast<float*>(p.out_cutoff)[r] = bin_lower_value(s.bin);
+        reinterpret_cast<float*>(p.out_cutoff)[r] = bin_lower_value(bin);
     }
   }
 }
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(kTopkThreads) topk_kernel(TopkParams p) {
   const int m = min(s.fill, CAP);
   sort_candidates(cand, m);
 
-  emit_row<DT>(p, r, row, cand, m, s);
+  emit_row<DT>(p, r, row, cand, m, s.refinements, s.bin);
 }
 
 // ---- many short rows ---------------------------------------------------------------------------------
@@ -395,11 +395,143 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
       placed[below] = c;
     }
     __syncthreads();
-    emit_row<DT>(p, r, row, placed, m, s);
+    emit_row<DT>(p, r, row, placed, m);
   } else {
     sort_candidates(cand, m);
-    emit_row<DT>(p, r, row, cand, m, s);
+    emit_row<DT>(p, r, row, cand, m);
   }
+}
+
+// ---- fewer rows: a row over the CTAs of a cluster -------------------------------------------------------------------------
+// (row_cluster.cuh)  The cluster's bound leaves a few more than K candidates, which the leader gathers and orders: up to
+// 256 by counting the greater ones of each, more by the bitonic network.  Too many candidates (huge groups of equal
+// values) or fewer than K finite elements: the exact radix select.  One CTA per row, or a row cut into "rows" with a
+// second call over their results, took three launches and 18 us for f32 [8, 32768], k = 64.
+template <int DT>
+__global__ void __launch_bounds__(kRcThreads, 4) topk_cluster_kernel(const __grid_constant__ TopkParams p, int cluster, int64_t part_len) {
+  using T = typename Elem<DT>::type;
+  extern __shared__ __align__(128) unsigned char smem[];
+  RcShared& s = *reinterpret_cast<RcShared*>(smem);
+  const RcLayout l(cluster, false);
+  const uint32_t rank = cl_rank();
+  const int64_t r = blockIdx.x / cluster;
+  const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
+  const RcPart<DT> part(row, p.n, part_len, rank, smem + l.off_part);
+  part.copy_in();
+  // exchange mode: the merge kernel that follows waits for the rows' arrival counts, not for this kernel
+  if (p.ex.world > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int K = p.k_max;
+  float* lx = reinterpret_cast<float*>(smem + l.off_x);
+  unsigned short* lpos = reinterpret_cast<unsigned short*>(smem + l.off_pos);
+  if (threadIdx.x == 0) s.n_list = 0;
+  part.copy_wait();
+  __syncthreads();
+  float thr = -INFINITY;
+  if (p.n > kRcListCap) {
+    uint32_t* bound = reinterpret_cast<uint32_t*>(smem + l.off_bound);
+    GroupMax<DT> gm;
+    gm.init();
+#pragma unroll 2
+    for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) gm.add(part.vec[v]);
+    rc_publish_maxima<DT>(gm, l.bound_words, bound);
+    cl_sync();
+    thr = key_f32(rc_bound_key16(bound, l.bound_words, K, s) << 16);
+  } else {
+    cl_sync();
+  }
+  rc_filter<DT>(part, thr, s, lx, lpos);
+  cl_sync();
+  if (rank != 0) {
+    cl_sync();
+    return;
+  }
+  int m = rc_gather(s, cluster, lx, nullptr, lpos);
+  cl_arrive();   // the other CTAs may leave
+  uint64_t* cand = reinterpret_cast<uint64_t*>(smem + l.off_part);   // the part is not needed any more
+  if (m < K) {   // (or -1)
+    SelectShared& sel = *reinterpret_cast<SelectShared*>(smem + l.off_part + (size_t)kRcListCap * 8);
+    exact_select_row<DT>(row, p.n, K, sel, cand);
+    m = K;
+    sort_candidates(cand, m);
+  } else {
+#pragma unroll 1
+    for (int i = threadIdx.x; i < m; i += kRcThreads) cand[i] = cand_make(f32_key(lx[i]), (uint32_t)rc_column(s, lpos, i, part_len));
+    if (m <= kRcThreads) {
+      uint64_t* placed = cand + kRcThreads;
+      if ((int)threadIdx.x >= m) cand[threadIdx.x] = ~0ull;
+      __syncthreads();
+      if ((int)threadIdx.x < m) {
+        const uint64_t mine = cand[threadIdx.x];
+        const ulonglong2* c2 = reinterpret_cast<const ulonglong2*>(cand);
+        int below = 0;
+#pragma unroll 4
+        for (int j = 0; j < (m + 1) / 2; ++j) {
+          const ulonglong2 c = c2[j];
+          below += (c.x < mine ? 1 : 0) + (c.y < mine ? 1 : 0);
+        }
+        placed[below] = mine;
+      }
+      __syncthreads();
+      cand = placed;
+    } else {
+      __syncthreads();
+      sort_candidates(cand, m);
+    }
+  }
+  emit_row<DT>(p, r, row, cand, m);
+  cl_wait();
+}
+
+// Whether it serves a call: floating-point rows that a cluster holds, exact mode without the diagnostics of the one-pass
+// kernel, fewer rows than the kernel of many short rows wants, and not more than 64 MB, beyond which the kernels with a CTA
+// per row move more bytes per second (f32 [204, 39024] 22 us against 30, bf16 [225, 130894] 40 against 49, f32
+// [128, 262144] 117 against 62).
+static bool cluster_rows_apply(int dtype, const TopkParams& p) {
+  if (dtype != TLX_F32 && dtype != TLX_BF16 && dtype != TLX_F16) return false;
+  if (p.k_max > kRcMaxK || p.mode != 0 || p.out_valid || p.out_depths || p.out_cutoff) return false;
+  static const bool forced = getenv("TLX_TOPK_PATH") != nullptr;   // comparison runs of the other two kernels
+  return !forced && p.rows < 256 && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart && p.rows * p.n * dtype_bytes(dtype) <= (64ll << 20);
+}
+
+template <int DT>
+static int launch_topk_cluster(cudaStream_t st, const TopkParams& p) {
+  const int es = (int)sizeof(typename Elem<DT>::type);
+  const int cluster = rc_cluster_size(p.rows, p.n, es);
+  const int64_t part_len = rc_part_len(p.n, cluster, es);
+  size_t part_bytes = (size_t)part_len * es + 32;
+  const size_t least = (size_t)kRcListCap * 8 + sizeof(SelectShared);   // of the exact select
+  if (part_bytes < least) part_bytes = least;
+  const size_t smem = RcLayout(cluster, false).off_part + part_bytes;
+  {
+    static std::mutex mu;
+    static size_t raised[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lock(mu);
+    if (dev < 0 || dev >= 64 || raised[dev] < smem) {
+      const void* f = (const void*)topk_cluster_kernel<DT>;
+      cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+      if (dev >= 0 && dev < 64) raised[dev] = smem;
+    }
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(p.rows * cluster));
+  cfg.blockDim = dim3(kRcThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = (unsigned)cluster;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, topk_cluster_kernel<DT>, p, cluster, part_len);
+  if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "top_k: %s", cudaGetErrorString(e)); }
+  count_launch();
+  return TLX_OK;
 }
 
 // Whether the two-pass kernel serves a call: floating-point rows, K <= 128, exact mode without the
@@ -470,6 +602,13 @@ static int launch_topk(cudaStream_t st, const TopkParams& p) {
 }
 
 static int dispatch_topk(cudaStream_t st, int dtype, const TopkParams& p, const char* what) {
+  if (cluster_rows_apply(dtype, p)) {
+    switch (dtype) {
+      case TLX_F32: return launch_topk_cluster<TLX_F32>(st, p);
+      case TLX_BF16: return launch_topk_cluster<TLX_BF16>(st, p);
+      default: return launch_topk_cluster<TLX_F16>(st, p);
+    }
+  }
   if (short_rows_apply(dtype, p)) {
     switch (dtype) {
       case TLX_F32: return launch_topk_short<TLX_F32>(st, p);
@@ -553,7 +692,11 @@ int tlx_top_k(void* stream, const void* x, int dtype, int64_t rows, int64_t n, i
   // few long rows, exact mode, no diagnostics asked for, and scratch given: split the rows over CTAs
   const int es = dtype == TLX_BF16 || dtype == TLX_F16 ? 2 : 4;
   const SplitPlan sp = split_plan(rows, n, k_max, es);
-  if (sp.parts && mode == 0 && !out_valid && !out_depths && !out_cutoff && row_stride == n && workspace &&
+  TopkParams p{};
+  p.x = x; p.rows = rows; p.n = n; p.row_stride = row_stride; p.k_max = k_max; p.k_per_row = k_per_row;
+  p.use_replace = use_replace; p.replace_val = replace_val; p.mode = mode; p.out_vals = out_vals;
+  p.out_idx = out_idx; p.out_valid = out_valid; p.out_depths = out_depths; p.out_cutoff = out_cutoff;
+  if (sp.parts && !cluster_rows_apply(dtype, p) && mode == 0 && !out_valid && !out_depths && !out_cutoff && row_stride == n && workspace &&
       workspace_bytes >= sp.bytes && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     unsigned char* ws = (unsigned char*)workspace;
@@ -574,10 +717,6 @@ int tlx_top_k(void* stream, const void* x, int dtype, int64_t rows, int64_t n, i
     TLX_CHECK_LAUNCH("top_k (index map)");
     return TLX_OK;
   }
-  TopkParams p{};
-  p.x = x; p.rows = rows; p.n = n; p.row_stride = row_stride; p.k_max = k_max; p.k_per_row = k_per_row;
-  p.use_replace = use_replace; p.replace_val = replace_val; p.mode = mode; p.out_vals = out_vals;
-  p.out_idx = out_idx; p.out_valid = out_valid; p.out_depths = out_depths; p.out_cutoff = out_cutoff;
   return dispatch_topk(st, dtype, p, "top_k");
 }
 

@@ -167,7 +167,8 @@ PyObject* py_top_k(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (replace == -1.0 && PyErr_Occurred()) { PyErr_Clear(); TLX_NOT_MINE; }
   }
   at::Tensor vals = empty({rows, k}, x->scalar_type(), dev), idx = empty({rows, k}, at::kInt, dev), ws;
-  const size_t ws_bytes = lib.top_k_workspace_bytes(rows, cols, (int)k);
+  // (floating-point rows need the workspace only beyond what a cluster holds)
+  const size_t ws_bytes = dt == TLX_I32 || cols > 700000 ? lib.top_k_workspace_bytes(rows, cols, (int)k) : 0;
   if (ws_bytes) ws = empty({(int64_t)ws_bytes}, at::kByte, dev);
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
   int rc;
