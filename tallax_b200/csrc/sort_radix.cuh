@@ -1,0 +1,274 @@
+// Stable row-wise argsort by radix: least significant digit first, eight bits a pass, a row in the shared memory of one
+// CTA (up to 16384 elements) or of a cluster of CTAs (up to 131072).  Included by sort.cu.
+//
+// What bounds it: integer instructions, which issue at half rate, about 100 of them an element and pass; four passes for
+// 32-bit keys and two for 16-bit ones, against 50 to 70 compare-exchanges of ten instructions an element of a bitonic
+// network on 64-bit composites.  Every pass keeps the order of equal digits, so the position need not be compared: it
+// travels beside the key.
+//
+// A pass.  A warp owns consecutive elements, 32 at a time; lanes with the same digit find each other with one ballot per
+// digit bit (__match_any_sync took half as long again), their number goes into the warp's own counter of the digit and
+// gives every lane its rank among the warp's equal digits.  The counters of all warps are turned into places (digit
+// first, then warp), the elements are scattered to them and read again in order.
+//   In a cluster the scatter first goes to the CTA's own shared memory, so that runs of equal digits lie together; then
+// the CTAs exchange their digit counts and every run is copied to where it belongs in the row, in whichever CTA that
+// is: the copies over distributed shared memory are contiguous.
+// Digits in which all keys of the row agree (small integers) are skipped.
+#pragma once
+#include "row_cluster.cuh"
+
+namespace tlx {
+
+constexpr int kRadixMaxThreads = 1024;
+constexpr int kRadixTile = 16384;            // elements per CTA at most
+constexpr int kRadixMaxRow = 8 * kRadixTile; // elements per row at most
+
+// Order-preserving key of a type in its own number of bits, and back (-0 comes back as +0, NaN as the one NaN).
+template <int DT> struct RadixKey {
+  static constexpr int kBits = 32;
+  using T = typename Elem<DT>::type;
+  static __device__ __forceinline__ uint32_t make(T v) { return Elem<DT>::key(v); }
+  static __device__ __forceinline__ T back(uint32_t k) { return Elem<DT>::from_key(k); }
+};
+__device__ __forceinline__ uint32_t radix_key_half(uint32_t b, uint32_t inf) {
+  uint32_t k = (b & 0x8000u) ? (~b & 0xFFFFu) : (b | 0x8000u);
+  if (b == 0x8000u) k = 0x8000u;
+  return (b & 0x7FFFu) > inf ? 0xFFFFu : k;
+}
+__device__ __forceinline__ unsigned short radix_half_back(uint32_t k) {
+  return (unsigned short)(k == 0xFFFFu ? 0x7FFFu : (k & 0x8000u) ? (k & 0x7FFFu) : (~k & 0xFFFFu));
+}
+template <> struct RadixKey<TLX_BF16> {
+  static constexpr int kBits = 16;
+  static __device__ __forceinline__ uint32_t make(__nv_bfloat16 v) { return radix_key_half(__bfloat16_as_ushort(v), 0x7F80u); }
+  static __device__ __forceinline__ __nv_bfloat16 back(uint32_t k) { return __ushort_as_bfloat16(radix_half_back(k)); }
+};
+template <> struct RadixKey<TLX_F16> {
+  static constexpr int kBits = 16;
+  static __device__ __forceinline__ uint32_t make(__half v) { return radix_key_half(__half_as_ushort(v), 0x7C00u); }
+  static __device__ __forceinline__ __half back(uint32_t k) { return __ushort_as_half(radix_half_back(k)); }
+};
+
+struct __align__(16) RadixShared {
+  uint32_t total[256];    // elements of every digit in this CTA
+  int shift_by[256];      // cluster: place in the row - place in the CTA
+  uint32_t warp[32];
+};
+
+static_assert(sizeof(RadixShared) % 16 == 0, "the counters behind it are cleared 16 bytes at a time");
+
+// Exclusive sum over the 256 digits of one value each (thread d < 256 holds digit d's), all threads call.
+__device__ __forceinline__ uint32_t radix_scan256(uint32_t v, uint32_t* warp_sum) {
+  uint32_t incl = v;
+  if (threadIdx.x < 256) {
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+      if (lane_id() >= o) incl += up;
+    }
+    if (lane_id() == 31) warp_sum[warp_id()] = incl;
+  }
+  __syncthreads();
+  uint32_t base = 0;
+  if (threadIdx.x < 256) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) base += i < warp_id() ? warp_sum[i] : 0u;
+  }
+  return base + incl - v;
+}
+
+// By digits.  k, p: element w * 32 * IPT + 32 j + lane of the CTA in k[j], p[j]; diff: the bits in which the row's keys
+// differ.  Leaves the CTA's part of the sorted row in k, p: element i of it (returned by place(j)) in k[j], p[j].
+template <int IPT, int kBits, bool CL, typename Pos>
+__device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p)[IPT], uint32_t diff, int rank, int cluster,
+                                                RadixShared& s, unsigned short* count, uint32_t* sk, Pos* sp) {
+  const int nt = blockDim.x, nw = nt >> 5, cap = nt * IPT;
+  const int lane = lane_id(), w = warp_id();
+  bool scattered = false;
+#pragma unroll 1
+  for (int sh = 0; sh < kBits; sh += 8) {
+    if (((diff >> sh) & 255u) == 0) continue;
+    if (scattered) {
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) {
+        const int i = w * 32 * IPT + 32 * j + lane;
+        k[j] = sk[i];
+        p[j] = sp[i];
+      }
+    }
+    // ranks among the warp's equal digits
+    unsigned short* mine = count + w * 256;
+    reinterpret_cast<uint4*>(mine)[lane] = make_uint4(0, 0, 0, 0);
+    __syncwarp();
+    unsigned short at[IPT];
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      const uint32_t d = (k[j] >> sh) & 255u;
+      uint32_t peers = 0xFFFFFFFFu;
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        const bool one = (d >> b) & 1u;
+        const uint32_t v = __ballot_sync(0xFFFFFFFFu, one);
+        peers &= one ? v : ~v;
+      }
+      const int before = __popc(peers & ((1u << lane) - 1u));
+      const uint32_t old = mine[d];
+      __syncwarp();
+      if (before == 0) mine[d] = (unsigned short)(old + __popc(peers));
+      __syncwarp();
+      at[j] = (unsigned short)(old + before);
+    }
+    __syncthreads();
+    // counters -> places: digit first, then warp.  Groups of 256 threads take the warps in equal shares.
+    {
+      const int groups = nt >> 8, g = threadIdx.x >> 8, d = threadIdx.x & 255;
+      const int share = (nw + groups - 1) / groups, w0 = g * share, w1 = min(w0 + share, nw);
+      uint32_t sum = 0;
+      if (g < groups)
+        for (int i = w0; i < w1; ++i) sum += count[i * 256 + d];
+      if (groups > 1) {
+        // the groups' totals meet in the scatter area, which nobody reads now
+        if (g < groups) sk[g * 256 + d] = sum;
+        __syncthreads();
+      }
+      uint32_t total = sum, before = 0;
+      if (groups > 1 && g < groups) {
+        total = 0;
+        for (int i = 0; i < groups; ++i) {
+          const uint32_t t = sk[i * 256 + d];
+          if (i < g) before += t;
+          total += t;
+        }
+      }
+      const uint32_t base = radix_scan256(total, s.warp);
+      if (threadIdx.x < 256) { s.total[d] = total; s.shift_by[d] = (int)base; }
+      __syncthreads();
+      if (g < groups) {
+        uint32_t run = (uint32_t)s.shift_by[d] + before;
+        for (int i = w0; i < w1; ++i) {
+          const uint32_t c = count[i * 256 + d];
+          count[i * 256 + d] = (unsigned short)run;
+          run += c;
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      const int to = mine[(k[j] >> sh) & 255u] + at[j];
+      sk[to] = k[j];
+      sp[to] = (Pos)p[j];
+    }
+    __syncthreads();
+    if constexpr (CL) {
+      // read back in the CTA's order; then (nobody's area is needed any more) every element to its place in the row
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) {
+        const int i = threadIdx.x + j * nt;
+        k[j] = sk[i];
+        p[j] = sp[i];
+      }
+      cl_sync();
+      uint32_t all = 0, before = 0;
+      if (threadIdx.x < 256) {
+#pragma unroll 8
+        for (int r = 0; r < cluster; ++r) {
+          const uint32_t t = cl_ld_u32(cl_map(&s.total[threadIdx.x], (uint32_t)r));
+          if (r < rank) before += t;
+          all += t;
+        }
+      }
+      const uint32_t base = radix_scan256(all, s.warp);
+      if (threadIdx.x < 256) s.shift_by[threadIdx.x] = (int)(base + before) - s.shift_by[threadIdx.x];
+      __syncthreads();
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) {
+        const int to = threadIdx.x + j * nt + s.shift_by[(k[j] >> sh) & 255u];
+        const int r = to / cap, i = to - r * cap;
+        cl_st_u32(cl_map(sk + i, (uint32_t)r), k[j]);
+        cl_st_u32(cl_map(sp + i, (uint32_t)r), p[j]);
+      }
+      cl_sync();
+    }
+    scattered = true;
+  }
+  if (scattered) {
+#pragma unroll
+    for (int j = 0; j < IPT; ++j) {
+      const int i = threadIdx.x + j * nt;
+      k[j] = sk[i];
+      p[j] = sp[i];
+    }
+  }
+  return scattered;
+}
+
+// Digit-wise difference of the CTA's keys from the row's first one, in every thread.
+__device__ __forceinline__ uint32_t radix_diff(uint32_t diff, RadixShared& s) {
+  diff = __reduce_or_sync(0xFFFFFFFFu, diff);
+  if (lane_id() == 0) s.warp[warp_id()] = diff;
+  __syncthreads();
+  return __reduce_or_sync(0xFFFFFFFFu, lane_id() < (int)(blockDim.x >> 5) ? s.warp[lane_id()] : 0u);
+}
+
+// Dynamic shared memory: RadixShared, counters [warps][256] u16, keys [cap] u32, positions [cap] u16 or (cluster) u32.
+__host__ __device__ __forceinline__ size_t radix_smem(int threads, int cap, bool cluster) {
+  return sizeof(RadixShared) + (size_t)(threads / 32) * 512 + (size_t)cap * (cluster ? 8 : 6);
+}
+
+template <int DT, int IPT, bool CL>
+__global__ void __launch_bounds__(kRadixMaxThreads) sort_radix_kernel(
+    const typename Elem<DT>::type* __restrict__ keys, const int32_t* __restrict__ in_perm, int64_t n, int descending,
+    typename Elem<DT>::type* __restrict__ out_keys, int32_t* __restrict__ out_perm, int cluster) {
+  using RK = RadixKey<DT>;
+  using Pos = typename std::conditional<CL, uint32_t, unsigned short>::type;
+  extern __shared__ __align__(16) unsigned char radix_raw[];
+  const int nt = blockDim.x, nw = nt >> 5, cap = nt * IPT;
+  RadixShared& s = *reinterpret_cast<RadixShared*>(radix_raw);
+  unsigned short* count = reinterpret_cast<unsigned short*>(radix_raw + sizeof(RadixShared));
+  uint32_t* sk = reinterpret_cast<uint32_t*>(count + nw * 256);
+  Pos* sp = reinterpret_cast<Pos*>(sk + cap);
+  const int rank = CL ? (int)cl_rank() : 0;
+  const int64_t row = CL ? blockIdx.x / cluster : blockIdx.x;
+  const int64_t c0 = (int64_t)rank * cap;
+  const auto* krow = keys + row * n;
+  const int32_t* prow = in_perm ? in_perm + row * n : nullptr;
+  const uint32_t ones = RK::kBits == 32 ? 0xFFFFFFFFu : 0xFFFFu, flip = descending ? ones : 0u;
+
+  // element w * 32 * IPT + 32 j + lane of the CTA; those past the row's end carry the greatest key and stay last
+  const int i0 = warp_id() * 32 * IPT + lane_id();
+  uint32_t k[IPT], p[IPT];
+  const uint32_t first = RK::make(krow[prow ? prow[0] : 0]) ^ flip;
+  uint32_t diff = 0;
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    const int64_t c = c0 + i0 + 32 * j;
+    k[j] = ones;
+    if (c < n) {
+      k[j] = RK::make(krow[prow ? (int64_t)prow[c] : c]) ^ flip;
+      diff |= k[j] ^ first;
+    }
+    p[j] = (uint32_t)c;
+  }
+  diff = radix_diff(diff, s);
+  if constexpr (CL) {
+    if (threadIdx.x == 0) s.total[0] = diff;
+    cl_sync();
+    diff = __reduce_or_sync(0xFFFFFFFFu, cl_ld_u32(cl_map(&s.total[0], (uint32_t)(lane_id() < cluster ? lane_id() : 0))));
+    cl_sync();
+  } else {
+    __syncthreads();
+  }
+  const bool scattered = radix_by_digits<IPT, RK::kBits, CL, Pos>(k, p, diff, rank, cluster, s, count, sk, sp);
+  if constexpr (CL) cl_sync();   // (nobody leaves while another one may still read its counts)
+#pragma unroll
+  for (int j = 0; j < IPT; ++j) {
+    const int64_t c = c0 + (scattered ? (int)threadIdx.x + j * nt : i0 + 32 * j);
+    if (c < n) {
+      if (out_keys) out_keys[row * n + c] = RK::back(k[j] ^ flip);
+      if (out_perm) out_perm[row * n + c] = prow ? prow[p[j]] : (int32_t)p[j];
+    }
+  }
+}
+
+}  // namespace tlx

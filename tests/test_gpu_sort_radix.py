@@ -1,0 +1,42 @@
+"""GPU: the radix sort at the edges of its CTAs and clusters, with ties, -0, NaNs, infinities and small integers."""
+import numpy as np
+import pytest
+
+from oracle import tallax_oracle as o
+from tallax_b200 import tax
+from tests.conftest import exact_match, to_dev, to_np
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1025, 8192, 8193, 16384, 16385, 32769, 131072, 131073])
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16", "i32"])
+@pytest.mark.parametrize("descending", [False, True])
+def test_radix_sort_sizes(cuda, dtype, n, descending):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((4, n)).astype(np.float32) * 3
+    x[1] = np.round(x[1])
+    x[2] = 1.0
+    if dtype == "i32":
+        x = (x * 1000).astype(np.int32)
+        x[3] = rng.integers(-2**31, 2**31 - 1, n)
+    else:
+        x[3, ::7] = 0.0
+        x[3, 1::7] = -0.0
+        x[3, 2::7] = np.nan
+        x[3, 3::7] = np.inf
+        x[3, 4::7] = -np.inf
+        x = x.astype({"f32": np.float32, "f16": np.float16, "bf16": o.bfloat16}[dtype])
+    first = rng.integers(0, 5, x.shape).astype(np.int32)
+    for operands, keys in (([x], 1), ([first, x], 2)):
+        got = tax.sort([to_dev(a, cuda) for a in operands], num_keys=keys, is_stable=True, return_argsort=True, descending=descending)
+        exp = o.sort(operands, keys, is_stable=True, return_argsort=True, descending=descending)
+        for g, e in zip(got, exp):
+            assert exact_match(to_np(g), e)
+
+
+@pytest.mark.parametrize("rows", [1, 300])
+def test_radix_sort_row_counts(cuda, rows):
+    x = np.random.default_rng(rows).standard_normal((rows, 3001)).astype(np.float32)
+    keys, perm = tax.sort([to_dev(x, cuda)], num_keys=1, return_argsort=True)
+    assert np.array_equal(to_np(perm), np.argsort(x, axis=1, kind="stable")) and np.array_equal(to_np(keys), np.sort(x, axis=1))
