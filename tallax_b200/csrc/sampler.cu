@@ -664,10 +664,11 @@ static bool stream_path_serves(int dtype, int64_t rows, int64_t vocab, int64_t r
 
 // Whether it is the faster one for a call that both forms serve.  The clusters' time grows with the bytes (four CTAs an
 // SM take turns of about 10 us); the stream starts from the 25 us of its three kernels and then moves more bytes per
-// second.  Requests with mixed parameters, us stream / cluster: a noise tensor, [32, 128256] 28/25, [64, 128256] 30/29,
-// [32, 200064] 29/31; a key, whose noise the stream makes element by element, [64, 128256] 39/39, [64, 200064] 45/57.
+// second.  Where they meet depends on the parameters, which the host does not know; us stream / cluster, requests with
+// mixed parameters, with one usual top_k and without top-k: a noise tensor, [64, 128256] 30/29, 21/13, 38/32 and
+// [96, 128256] 32/38, 24/22, 51/47; a key, [32, 128256] 31/34, 20/11, 36/33 and [64, 200064] 41/56, 27/22, 66/66.
 static bool stream_path_wanted(int64_t rows, int64_t vocab, bool dense) {
-  return rows * vocab * 2 > (dense ? (10ll << 20) : (18ll << 20));
+  return rows * vocab * 2 > (dense ? (16ll << 20) : (9ll << 20));
 }
 
 // Diagnostic switch for timing the stages of the streaming path one by one (environment variable

@@ -917,13 +917,13 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
         const int v = st_wide_threshold(p, row, key16, p.sp.top_p[row], area, ctl.wide);
         if (threadIdx.x == 0) {
           // The row's greatest element is always kept: its screened score (the very expression its final item
-          // will evaluate) seeds the row's best score, so that the final items' test bites from their first
-          // chunk on.  Threshold and seed become visible together (one 8-byte store).
+          // will evaluate) seeds the row's best score, so that the test of the final items (of the final pass) bites from
+          // their first chunk on.  Threshold and seed become visible together (one 8-byte store).
           uint32_t seed = f32_key(-INFINITY);
           const unsigned long long wb = __ldcg(&p.wbest[row]);
           const int64_t pos = (int64_t)(uint32_t)wb;
           const float T_ = p.sp.temperature[row];
-          if (v >= 0 && p.fin_items > 0 && pos < p.sp.vocab && (wb >> 32) < 65536ull) {
+          if (v >= 0 && pos < p.sp.vocab && (wb >> 32) < 65536ull) {
             const uint32_t bits = reinterpret_cast<const unsigned short*>(p.sp.logits)[(int64_t)row * p.sp.row_stride + pos];
             const float u = p.sp.noise.at(row + p.sp.dim0_offset, pos);
             seed = f32_key(fmaf(__uint_as_float(bits << 16), 1.0f / T_, gumbel_screen(u)));
@@ -1499,7 +1499,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
     if (threadIdx.x == 0) {
       for (int s = 0; s < kFinSlots; ++s) mbar_init(&ctl.mbar[s], 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-      ctl.best_key = f32_key(-INFINITY);
+      ctl.best_key = __ldcg(&ws->best_key);   // of the whole row so far
       for (int s = 0; s < kFinSlots; ++s) fin_issue(p, row, c_begin + s, c_end, dense != 0, ring, ctl.mbar, s);
     }
     __syncthreads();
@@ -1522,7 +1522,70 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
       const unsigned char* buf = ring + (size_t)slot * kFinSlotBytes;
       const float* nbuf = reinterpret_cast<const float*>(buf + kFinChunk);
       const int nvec = (c == p.nfin - 1) ? last_nvec : kFinChunk / 16;
-      if (!(p.debug & 2)) {
+      if (!dense && !(p.debug & 2)) {
+        // noise element by element: only for values that could reach the best known score with the greatest noise
+        // there is (of 1 - 2^-23 from a key, 1 - 2^-24 in a tensor); the warp notes their places and then takes them
+        // 128 at a time, four a lane, so that the dependent rounds of four keys (or four reads) overlap
+        const float low = cb - 2.0f * (kGumbelSlack + 1e-5f * fabsf(cb));
+        const float xcut = fmaxf(tvf, (low - (sp.noise.dense ? 16.65f : 15.95f)) * T_);
+        unsigned short* noted = reinterpret_cast<unsigned short*>(ring + (size_t)slot * kFinSlotBytes + kFinChunk) +
+                                warp * (kFinVecPerThread * 32 * 8);
+        int n = 0;
+#pragma unroll 1
+        for (int jv = 0; jv < kFinVecPerThread; ++jv) {
+          const int v = (int)threadIdx.x + jv * kStThreads;
+          uint32_t mask = 0;
+          if (v < nvec) {
+            const uint4 x = *reinterpret_cast<const uint4*>(buf + (size_t)v * 16);
+            const uint32_t wd[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+              const float xf = __uint_as_float((e & 1) ? (wd[e >> 1] & 0xFFFF0000u) : (wd[e >> 1] << 16));
+              mask |= xf >= xcut ? 1u << e : 0u;
+            }
+          }
+          int incl = __popc(mask);
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += up;
+          }
+          int at = n + incl - __popc(mask);
+          while (mask) {
+            const int e = __ffs(mask) - 1;
+            mask &= mask - 1;
+            noted[at++] = (unsigned short)(v * 8 + e);
+          }
+          n += __shfl_sync(0xFFFFFFFFu, incl, 31);
+        }
+        __syncwarp();
+        const uint32_t k0 = sp.noise.key_dev ? __ldg(sp.noise.key_dev) : sp.noise.k0;
+        const uint32_t k1 = sp.noise.key_dev ? __ldg(sp.noise.key_dev + 1) : sp.noise.k1;
+        const uint32_t ctr0 = (uint32_t)(sp.noise.row_of(nrow) * sp.noise.vocab) + (uint32_t)(c * kFinChunkElems);
+#pragma unroll 1
+        for (int q0 = 0; q0 < n; q0 += 128) {
+          int at[4];
+          float un[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int q = q0 + lane + 32 * k;
+            at[k] = q < n ? noted[q] : -1;
+            if (sp.noise.dense) un[k] = at[k] >= 0 ? __ldg(sp.noise.dense_row(nrow) + c * kFinChunkElems + at[k]) : 0.5f;
+            else un[k] = fmaxf(threefry_uniform01(k0, k1, ctr0 + (uint32_t)at[k]), kF32Tiny);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            if (at[k] < 0) continue;
+            const uint32_t b = reinterpret_cast<const unsigned short*>(buf)[at[k]];
+            const float xf = __uint_as_float(b << 16);
+            // -log(-log u) <= -log(1 - u): most that were noted stop here
+            if (!(1.0f - un[k] <= __expf(fmaf(xf, inv_T, -low)) * 1.0001f)) continue;
+            const float a = fmaf(xf, inv_T, gumbel_screen(un[k]));
+            if (a > a1) { a2 = a1; a1 = a; u1 = un[k]; b1 = b; t1 = c * kFinChunkElems + at[k]; }
+            else a2 = fmaxf(a2, a);
+          }
+        }
+      } else if (!(p.debug & 2)) {
 #pragma unroll 1
         for (int jv = 0; jv < kFinVecPerThread; ++jv) {
           const int v = (int)threadIdx.x + jv * kStThreads;
@@ -1534,7 +1597,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
               // eight independent screened scores, then their best two
               const uint32_t wd[4] = {x.x, x.y, x.z, x.w};
               float un[8];
-              if (dense) {
+              {
                 const float4 n0 = *reinterpret_cast<const float4*>(nbuf + v * 8);
                 const float4 n1 = *reinterpret_cast<const float4*>(nbuf + v * 8 + 4);
                 un[0] = n0.x; un[1] = n0.y; un[2] = n0.z; un[3] = n0.w;
@@ -1550,7 +1613,6 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
                 const uint32_t hi = (e & 1) ? (wd[e >> 1] & 0xFFFF0000u) : (wd[e >> 1] << 16);
                 const float xf = __uint_as_float(hi);
                 bool keep = !(xf < tvf);
-                if (!dense) un[e] = keep ? sp.noise.at(nrow, c * kFinChunkElems + v * 8 + e) : 0.5f;
                 keep = keep && 1.0f - un[e] <= eps;
                 sc[e] = keep ? fmaf(xf, inv_T, gumbel_screen(un[e])) : -INFINITY;
                 const float lo = fminf(v1, sc[e]);
