@@ -153,10 +153,9 @@ constexpr int kShortCap = 1024;
 constexpr int kShortMaxK = 128;
 
 // Row traversal by 16-byte vectors: fv(vector, first column) in the aligned body, kU loads in flight per
-// thread; fs(element, column) for the unaligned head and tail.  sub > 1 visits only every sub-th run of
-// blockDim vectors (a sample of the row in contiguous 2 KB pieces).
+// thread; fs(element, column) for the unaligned head and tail.
 template <int DT, int kU, typename FV, typename FS>
-__device__ __forceinline__ void for_each_vec(const typename Elem<DT>::type* __restrict__ row, int64_t n, int sub, FV&& fv,
+__device__ __forceinline__ void for_each_vec(const typename Elem<DT>::type* __restrict__ row, int64_t n, FV&& fv,
                                              FS&& fs) {
   using T = typename Elem<DT>::type;
   constexpr int VEC = 16 / (int)sizeof(T);
@@ -166,7 +165,7 @@ __device__ __forceinline__ void for_each_vec(const typename Elem<DT>::type* __re
   for (int64_t c = threadIdx.x; c < head; c += blockDim.x) fs(row[c], c);
   const int64_t nvec = (n - head) / VEC;
   const uint4* vp = reinterpret_cast<const uint4*>(row + head);
-  const int64_t step = (int64_t)blockDim.x * sub;
+  const int64_t step = (int64_t)blockDim.x;
   int64_t i = threadIdx.x;
   for (; i + (int64_t)(kU - 1) * step < nvec; i += (int64_t)kU * step) {
     uint4 v[kU];
@@ -226,23 +225,178 @@ __device__ __forceinline__ void warp_pick_bin(const uint32_t* h, int need, int* 
   }
 }
 
-static __device__ __noinline__ uint32_t kth_largest_u16(const uint16_t* keys, int G, int K, uint32_t* hist, int* pick) {
+template <typename KeyOf>
+__device__ __forceinline__ uint32_t kth_largest_key16(KeyOf key_of, int G, int K, uint32_t* hist, int* pick) {
   for (int i = threadIdx.x; i < 512; i += blockDim.x) hist[i] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < G; i += blockDim.x) atomicAdd(&hist[keys[i] >> 8], 1u);
+  for (int i = threadIdx.x; i < G; i += blockDim.x) atomicAdd(&hist[key_of(i) >> 8], 1u);
   __syncthreads();
   if (warp_id() == 0) warp_pick_bin(hist, K, pick);
   __syncthreads();
   const uint32_t top = (uint32_t)pick[0];
   const int need = K - pick[1];
   for (int i = threadIdx.x; i < G; i += blockDim.x) {
-    const uint32_t k = keys[i];
+    const uint32_t k = key_of(i);
     if ((k >> 8) == top) atomicAdd(&hist[256 + (k & 255u)], 1u);
   }
   __syncthreads();
   if (warp_id() == 0) warp_pick_bin(hist + 256, need, pick + 2);
   __syncthreads();
   return (top << 8) | (uint32_t)pick[2];
+}
+static __device__ __noinline__ uint32_t kth_largest_u16(const uint16_t* keys, int G, int K, uint32_t* hist, int* pick) {
+  return kth_largest_key16([&](int i) { return (uint32_t)keys[i]; }, G, K, hist, pick);
+}
+
+// 16-bit key of the greatest element of a vector (a NaN has the greatest key).
+template <int DT>
+__device__ __forceinline__ uint32_t vector_key16(const uint4& v) {
+  if constexpr (DT == TLX_BF16) {
+    const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
+    const __nv_bfloat162 a = __hmax2_nan(__hmax2_nan(e[0], e[1]), __hmax2_nan(e[2], e[3]));
+    return f32_key(__bfloat162float(__hmax_nan(__low2bfloat16(a), __high2bfloat16(a)))) >> 16;
+  } else {
+    using T = typename Elem<DT>::type;
+    const T* e = reinterpret_cast<const T*>(&v);
+    uint32_t k = 0;
+#pragma unroll
+    for (int j = 0; j < 16 / (int)sizeof(T); ++j) k = max(k, Elem<DT>::key(e[j]));
+    return k >> 16;
+  }
+}
+
+// ---- many long rows ------------------------------------------------------------------------------------------------------
+// Rows of more than 128 KB, which L2 would not keep between two passes: the bound comes from every sixteenth 2 KB piece of
+// the row, whose vectors leave the 16-bit keys of their greatest elements in shared memory, so that every byte of the
+// row is read once.  A sixteenth of the row bounds loosely (about 2400 vectors hold an element at or above the bound for
+// K = 128 of f32 rows): the vectors are noted with their keys, the K-th greatest of these keys is a second, tight bound
+// (K vectors hold an element at or above it), and only the vectors that reach it are looked into.
+// HBM-bound; f32 [1024, 262144], k = 128: 285 us with the bound from a quarter of the row and the whole row read again.
+constexpr int kSampledNotes = kHistBins;              // noted vectors, in the fallback's histogram space
+constexpr int64_t kSampledVecs = 65536;               // vectors of a row at most: 4096 of them are sampled
+template <int DT>
+__global__ void __launch_bounds__(kShortThreads, 8) topk_sampled_kernel(TopkParams p) {
+  using T = typename Elem<DT>::type;
+  constexpr int kSlots = GroupMax<DT>::kSlots, G = kShortThreads * kSlots, VEC = 16 / (int)sizeof(T), kSub = 16;
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  SelectShared& s = *reinterpret_cast<SelectShared*>(smem_raw);
+  uint64_t* cand = reinterpret_cast<uint64_t*>(smem_raw + ((sizeof(SelectShared) + 15) & ~size_t(15)));
+  uint16_t* gkeys = reinterpret_cast<uint16_t*>(s.hist);            // G * 2 bytes <= 2 KB
+  uint16_t* vkeys = reinterpret_cast<uint16_t*>(cand);               // the sampled vectors' keys, 8 KB
+  static_assert(kSampledVecs / kSub * 2 <= kShortCap * 8, "the sampled vectors' keys lie in the candidate list's space");
+  const int64_t r = blockIdx.x;
+  const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
+  const int K = p.k_max, n = (int)p.n, tid = threadIdx.x;
+  if (p.ex.world > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int head = (int)(((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / sizeof(T));
+  const int nvec = (n - head) / VEC;
+  const uint4* vp = reinterpret_cast<const uint4*>(row + head);
+  constexpr int kGroup = kShortThreads * kSub;                       // vectors of sixteen pieces; the first piece is sampled
+  GroupMax<DT> gm;
+  gm.init();
+#pragma unroll 1
+  for (int g0 = 0; g0 * kGroup < nvec; g0 += 8) {
+    uint4 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if ((g0 + u) * kGroup + tid < nvec) v[u] = __ldcs(vp + (g0 + u) * kGroup + tid);
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if ((g0 + u) * kGroup + tid < nvec) {
+        gm.add(v[u]);
+        vkeys[(g0 + u) * kShortThreads + tid] = (uint16_t)vector_key16<DT>(v[u]);
+      }
+  }
+#pragma unroll
+  for (int j = 0; j < kSlots; ++j) gkeys[tid * kSlots + j] = (uint16_t)(f32_key(gm.slot(j)) >> 16);
+  if (tid == 0) { s.fill = 0; s.bin = 0; s.above = 0; s.refinements = 0; }
+  __syncthreads();
+  const uint32_t t16 = kth_largest_u16(gkeys, G, K, s.hist + 1024, s.tmp_i);
+  const float thr = key_f32(t16 << 16);   // (a NaN pattern, the bin of -inf, admits everything)
+  int* nnoted = &s.above;
+  auto note = [&](uint32_t key, int i) {
+    const int slot = atomicAdd(nnoted, 1);
+    if (slot < kSampledNotes) s.hist[slot] = (key << 16) | (uint32_t)i;
+  };
+#pragma unroll 1
+  for (int g = 0; g * kGroup + tid < nvec; ++g) {
+    const uint32_t k = vkeys[g * kShortThreads + tid];
+    if (k >= t16) note(k, g * kGroup + tid);
+  }
+  auto look = [&](const uint4& v, int i) {
+    bool any;
+    if constexpr (DT == TLX_BF16) {
+      const __nv_bfloat16 tb = __ushort_as_bfloat16((unsigned short)(__float_as_uint(thr) >> 16));
+      const __nv_bfloat162 t2 = __halves2bfloat162(tb, tb);
+      const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
+      any = !(__hblt2(e[0], t2) && __hblt2(e[1], t2) && __hblt2(e[2], t2) && __hblt2(e[3], t2));
+    } else {
+      any = rc_any_at_least<DT>(v, thr);
+    }
+    if (any) note(vector_key16<DT>(v), i);
+  };
+#pragma unroll 1
+  for (int g = 0; g * kGroup < nvec; ++g) {
+    const int i0 = g * kGroup + tid;
+    if ((g + 1) * kGroup <= nvec) {
+#pragma unroll
+      for (int h = 1; h < kSub; h += 8) {   // eight loads in flight, then seven
+        uint4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) if (h + u < kSub) v[u] = __ldcs(vp + i0 + (h + u) * kShortThreads);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) if (h + u < kSub) look(v[u], i0 + (h + u) * kShortThreads);
+      }
+    } else {
+#pragma unroll 1
+      for (int h = 1; h < kSub; ++h)
+        if (i0 + h * kShortThreads < nvec) look(__ldcs(vp + i0 + h * kShortThreads), i0 + h * kShortThreads);
+    }
+  }
+  __syncthreads();   // the sampled vectors' keys have been used: the candidate list may begin
+  auto push_one = [&](T x, int c) {
+    const uint32_t key = Elem<DT>::key(x);
+    if ((key >> 16) >= t16) {
+      const int slot = atomicAdd(&s.fill, 1);
+      if (slot < kShortCap) cand[slot] = cand_make(key, (uint32_t)c);
+    }
+  };
+  if (tid < head) push_one(row[tid], tid);
+  if (tid >= 32 && head + nvec * VEC + tid - 32 < n) push_one(row[head + nvec * VEC + tid - 32], head + nvec * VEC + tid - 32);
+  const int nn = *nnoted;
+  __syncthreads();
+  if (nn > kSampledNotes) {
+    if (tid == 0) s.fill = kShortCap + 1;   // more vectors than the list holds: the exact fallback
+  } else {
+    uint32_t t2 = t16;
+    if (nn > K) t2 = kth_largest_key16([&](int i) { return s.hist[i] >> 16; }, nn, K, reinterpret_cast<uint32_t*>(cand + kShortCap / 2), s.tmp_i);
+    const float thr2 = key_f32(t2 << 16);
+    for (int l = tid; l < nn; l += kShortThreads) {
+      const uint32_t w = s.hist[l];
+      if ((w >> 16) < t2) continue;
+      const int i = (int)(w & 0xFFFFu);
+      push_vector<DT>(__ldg(vp + i), head + (int64_t)i * VEC, t2, thr2, &s.fill, cand, kShortCap);
+    }
+  }
+  __syncthreads();
+  if (s.fill > kShortCap) exact_select_row<DT>(row, n, K, s, cand);   // huge groups of equal values
+  const int m = min(s.fill, kShortCap);
+  if (m <= 2 * kShortThreads) {
+    // every thread counts the composites below its own ones (they are distinct) and puts them at their places
+    uint64_t* placed = reinterpret_cast<uint64_t*>(s.hist);
+    for (int i = tid; i < m; i += kShortThreads) {
+      const uint64_t c = cand[i];
+      int below = 0;
+#pragma unroll 4
+      for (int j = 0; j < m; ++j) below += cand[j] < c ? 1 : 0;
+      placed[below] = c;
+    }
+    __syncthreads();
+    emit_row<DT>(p, r, row, placed, m);
+  } else {
+    sort_candidates(cand, m);
+    emit_row<DT>(p, r, row, cand, m);
+  }
 }
 
 template <int DT>
@@ -263,8 +417,6 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   // exchange mode: the merge kernel that follows waits for the rows' arrival counts, not for this kernel
   if (p.ex.world > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  // rows that L2 would not keep between the passes give their bound from a quarter of the row
-  const int sub = n * (int64_t)sizeof(T) > (128 << 10) ? 4 : 1;
   // bf16 rows of up to 4096 vectors (64 KB) read in full by pass 1: pass 1 also leaves every vector's greatest
   // element (NaN if it holds one) in shared memory, in the candidate list's space, and pass 2 reads those
   // 2 bytes per vector instead of the row
@@ -273,7 +425,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   if (head > n) head = n;
   const int64_t nvec = (n - head) / VEC;
   bool vec_maxima = false;
-  if constexpr (DT == TLX_BF16) vec_maxima = sub == 1 && nvec <= kShortCap * 4;
+  if constexpr (DT == TLX_BF16) vec_maxima = nvec <= kShortCap * 4;
   __nv_bfloat16* vmax = reinterpret_cast<__nv_bfloat16*>(cand);
   GroupMax<DT> gm;
   gm.init();
@@ -281,7 +433,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
     if (vec_maxima) {
       const __nv_bfloat16 ninf = __float2bfloat16_rn(-INFINITY);
       for (int64_t i = nvec + threadIdx.x; i < ((nvec + 7) & ~(int64_t)7); i += blockDim.x) vmax[i] = ninf;
-      for_each_vec<DT, 10>(row, n, 1,
+      for_each_vec<DT, 10>(row, n,
         [&](const uint4& v, int64_t cb) {
           gm.add(v);
           const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
@@ -292,7 +444,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
     }
   }
   if (!vec_maxima)
-    for_each_vec<DT, 10>(row, n, sub, [&](const uint4& v, int64_t) { gm.add(v); }, [&](T x, int64_t) { gm.add_one(x); });
+    for_each_vec<DT, 10>(row, n, [&](const uint4& v, int64_t) { gm.add(v); }, [&](T x, int64_t) { gm.add_one(x); });
 #pragma unroll
   for (int j = 0; j < kSlots; ++j) gkeys[threadIdx.x * kSlots + j] = (uint16_t)(f32_key(gm.slot(j)) >> 16);
   if (threadIdx.x == 0) { s.fill = 0; s.bin = 0; s.above = 0; s.refinements = 0; }
@@ -339,7 +491,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
         }
       }
     } else {
-      for_each_vec<DT, 10>(row, n, 1,
+      for_each_vec<DT, 10>(row, n,
         [&](const uint4& v, int64_t cb) {
           const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
           // __hblt2: both halves less than the bound (false when either is a NaN)
@@ -348,7 +500,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
         push_one);
     }
   } else if constexpr (DT == TLX_F16) {
-    for_each_vec<DT, 10>(row, n, 1,
+    for_each_vec<DT, 10>(row, n,
       [&](const uint4& v, int64_t cb) {
         const __half2* e = reinterpret_cast<const __half2*>(&v);
         bool any = false;
@@ -361,7 +513,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
       },
       push_one);
   } else {
-    for_each_vec<DT, 10>(row, n, 1,
+    for_each_vec<DT, 10>(row, n,
       [&](const uint4& v, int64_t cb) {
         const float* e = reinterpret_cast<const float*>(&v);
         if (!(e[0] < thr) || !(e[1] < thr) || !(e[2] < thr) || !(e[3] < thr)) note(cb);
@@ -534,6 +686,11 @@ static int launch_topk_cluster(cudaStream_t st, const TopkParams& p) {
   return TLX_OK;
 }
 
+// Rows of more than 128 KB take the kernel that reads them once, if it can number their vectors in 16 bits.
+constexpr int64_t kLongRowBytes = 128 << 10;
+static bool long_rows_apply(int dtype, const TopkParams& p) {
+  return p.n * dtype_bytes(dtype) > kLongRowBytes && p.n * dtype_bytes(dtype) / 16 <= kSampledVecs;
+}
 // Whether the two-pass kernel serves a call: floating-point rows, K <= 128, exact mode without the
 // diagnostics of the one-pass kernel, and enough rows to fill the eight CTAs per SM.
 static bool short_rows_apply(int dtype, const TopkParams& p) {
@@ -542,11 +699,11 @@ static bool short_rows_apply(int dtype, const TopkParams& p) {
   if (p.k_max > kShortMaxK || p.mode != 0 || p.out_valid || p.out_depths || p.out_cutoff) return false;
   if (force && !strcmp(force, "short")) return true;
   if (force && !strcmp(force, "long")) return false;
-  return p.rows >= 256 && p.n >= 2048;
+  return p.rows >= 256 && p.n >= 2048 && (p.n * dtype_bytes(dtype) <= kLongRowBytes || long_rows_apply(dtype, p));
 }
 
 template <int DT>
-static int launch_topk_short(cudaStream_t st, const TopkParams& p) {
+static int launch_topk_short(cudaStream_t st, const TopkParams& p, bool long_rows) {
   const size_t smem = ((sizeof(SelectShared) + 15) & ~size_t(15)) + (size_t)kShortCap * 8;
   // eight CTAs of 25 KB per SM need the large shared-memory configuration: asked for once per device
   static std::mutex mu;
@@ -558,11 +715,15 @@ static int launch_topk_short(cudaStream_t st, const TopkParams& p) {
     if (dev < 0 || dev >= 64 || !asked[dev]) {
       cudaError_t e = cudaFuncSetAttribute(topk_short_kernel<DT>, cudaFuncAttributePreferredSharedMemoryCarveout,
                                            (int)cudaSharedmemCarveoutMaxShared);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(topk_sampled_kernel<DT>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                 (int)cudaSharedmemCarveoutMaxShared);
       if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
       if (dev >= 0 && dev < 64) asked[dev] = true;
     }
   }
-  topk_short_kernel<DT><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
+  if (long_rows) topk_sampled_kernel<DT><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
+  else topk_short_kernel<DT><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
   TLX_CHECK_LAUNCH("top_k (short rows)");
   return TLX_OK;
 }
@@ -610,10 +771,11 @@ static int dispatch_topk(cudaStream_t st, int dtype, const TopkParams& p, const 
     }
   }
   if (short_rows_apply(dtype, p)) {
+    const bool long_rows = long_rows_apply(dtype, p);
     switch (dtype) {
-      case TLX_F32: return launch_topk_short<TLX_F32>(st, p);
-      case TLX_BF16: return launch_topk_short<TLX_BF16>(st, p);
-      default: return launch_topk_short<TLX_F16>(st, p);
+      case TLX_F32: return launch_topk_short<TLX_F32>(st, p, long_rows);
+      case TLX_BF16: return launch_topk_short<TLX_BF16>(st, p, long_rows);
+      default: return launch_topk_short<TLX_F16>(st, p, long_rows);
     }
   }
   switch (dtype) {
