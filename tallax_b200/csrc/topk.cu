@@ -225,27 +225,23 @@ __device__ __forceinline__ void warp_pick_bin(const uint32_t* h, int need, int* 
   }
 }
 
-template <typename KeyOf>
-__device__ __forceinline__ uint32_t kth_largest_key16(KeyOf key_of, int G, int K, uint32_t* hist, int* pick) {
+static __device__ __noinline__ uint32_t kth_largest_u16(const uint16_t* keys, int G, int K, uint32_t* hist, int* pick) {
   for (int i = threadIdx.x; i < 512; i += blockDim.x) hist[i] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < G; i += blockDim.x) atomicAdd(&hist[key_of(i) >> 8], 1u);
+  for (int i = threadIdx.x; i < G; i += blockDim.x) atomicAdd(&hist[keys[i] >> 8], 1u);
   __syncthreads();
   if (warp_id() == 0) warp_pick_bin(hist, K, pick);
   __syncthreads();
   const uint32_t top = (uint32_t)pick[0];
   const int need = K - pick[1];
   for (int i = threadIdx.x; i < G; i += blockDim.x) {
-    const uint32_t k = key_of(i);
+    const uint32_t k = keys[i];
     if ((k >> 8) == top) atomicAdd(&hist[256 + (k & 255u)], 1u);
   }
   __syncthreads();
   if (warp_id() == 0) warp_pick_bin(hist + 256, need, pick + 2);
   __syncthreads();
   return (top << 8) | (uint32_t)pick[2];
-}
-static __device__ __noinline__ uint32_t kth_largest_u16(const uint16_t* keys, int G, int K, uint32_t* hist, int* pick) {
-  return kth_largest_key16([&](int i) { return (uint32_t)keys[i]; }, G, K, hist, pick);
 }
 
 // 16-bit key of the greatest element of a vector (a NaN has the greatest key).
@@ -265,25 +261,58 @@ __device__ __forceinline__ uint32_t vector_key16(const uint4& v) {
   }
 }
 
+// Orders m distinct composites: four lanes count the ones below a composite, which is its place.
+__device__ __forceinline__ void order_by_count(const uint64_t* cand, int m, uint64_t* placed) {
+  const int part = threadIdx.x & 3;
+  for (int i0 = 0; i0 < m; i0 += blockDim.x / 4) {
+    const int i = i0 + threadIdx.x / 4;
+    const uint64_t c = cand[min(i, m - 1)];
+    int below = 0;
+#pragma unroll 4
+    for (int j = part; j < m; j += 4) below += cand[j] < c ? 1 : 0;
+    below += __shfl_xor_sync(0xFFFFFFFFu, below, 1);
+    below += __shfl_xor_sync(0xFFFFFFFFu, below, 2);
+    if (part == 0 && i < m) placed[below] = c;
+  }
+}
+
 // ---- many long rows ------------------------------------------------------------------------------------------------------
-// Rows of more than 128 KB, which L2 would not keep between two passes: the bound comes from every sixteenth 2 KB piece of
+// Rows of more than 128 KB, which L2 would not keep between two passes: the bound comes from every eighth 4 KB piece of
 // the row, whose vectors leave the 16-bit keys of their greatest elements in shared memory, so that every byte of the
-// row is read once.  A sixteenth of the row bounds loosely (about 2400 vectors hold an element at or above the bound for
-// K = 128 of f32 rows): the vectors are noted with their keys, the K-th greatest of these keys is a second, tight bound
-// (K vectors hold an element at or above it), and only the vectors that reach it are looked into.
-// HBM-bound; f32 [1024, 262144], k = 128: 285 us with the bound from a quarter of the row and the whole row read again.
-constexpr int kSampledNotes = kHistBins;              // noted vectors, in the fallback's histogram space
-constexpr int64_t kSampledVecs = 65536;               // vectors of a row at most: 4096 of them are sampled
+// row is read once.  An eighth of the row bounds loosely (about 1200 vectors hold an element at or above the bound for
+// K = 128): the vectors are noted with their keys, a list per warp, the K-th greatest of these keys is a second, tight
+// bound (K vectors hold an element at or above it), and only the vectors that reach it are looked into.
+// HBM-bound; f32 [1024, 262144], k = 128: 285 us with the bound from a quarter of the row and the whole row read again,
+// 234 us with one list of noted vectors per CTA of 128 threads, 204 us so (the bytes alone: 164 us).
+constexpr int kSampledSub = 8;
+constexpr int kSampledThreads = 256;   // (of 128: 213 us at that size, 33.5 us against 26.7 us for 300 rows of 60000)
+constexpr int64_t kSampledVecs = 65536;   // vectors of a row at most: their numbers have 16 bits
 template <int DT>
-__global__ void __launch_bounds__(kShortThreads, 8) topk_sampled_kernel(TopkParams p) {
+__device__ __forceinline__ bool vector_reaches(const uint4& v, float thr) {   // (true also for vectors somewhat below)
+  if constexpr (DT == TLX_F16) {
+    const __half2 t2 = __half2half2(__float2half_rd(thr));
+    const __half2* e = reinterpret_cast<const __half2*>(&v);
+    return !(__hblt2(e[0], t2) && __hblt2(e[1], t2) && __hblt2(e[2], t2) && __hblt2(e[3], t2));
+  } else {
+    return rc_any_at_least<DT>(v, thr);
+  }
+}
+template <int DT>
+__global__ void __launch_bounds__(kSampledThreads, 1024 / kSampledThreads) topk_sampled_kernel(TopkParams p) {
   using T = typename Elem<DT>::type;
-  constexpr int kSlots = GroupMax<DT>::kSlots, G = kShortThreads * kSlots, VEC = 16 / (int)sizeof(T), kSub = 16;
+  constexpr int TH = kSampledThreads;
+  constexpr int kSlots = GroupMax<DT>::kSlots, G = TH * kSlots, VEC = 16 / (int)sizeof(T);
+  constexpr int kGroup = TH * kSampledSub;   // vectors of eight pieces; the first piece is sampled
+  constexpr int kSampledNotes = kShortCap * 2 / (TH / 32);           // noted vectors of a warp, in the candidates' space
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SelectShared& s = *reinterpret_cast<SelectShared*>(smem_raw);
   uint64_t* cand = reinterpret_cast<uint64_t*>(smem_raw + ((sizeof(SelectShared) + 15) & ~size_t(15)));
-  uint16_t* gkeys = reinterpret_cast<uint16_t*>(s.hist);            // G * 2 bytes <= 2 KB
-  uint16_t* vkeys = reinterpret_cast<uint16_t*>(cand);               // the sampled vectors' keys, 8 KB
-  static_assert(kSampledVecs / kSub * 2 <= kShortCap * 8, "the sampled vectors' keys lie in the candidate list's space");
+  uint16_t* vkeys = reinterpret_cast<uint16_t*>(s.hist);            // the sampled vectors' keys; later
+  uint64_t* list = reinterpret_cast<uint64_t*>(s.hist);             // the candidates, and behind them
+  uint32_t* hist8 = s.hist + kShortCap * 2;                         // the second bound's histogram
+  uint16_t* sel = reinterpret_cast<uint16_t*>(hist8 + 256);         // the vectors to look into
+  uint16_t* gkeys = reinterpret_cast<uint16_t*>(cand);              // the groups' maxima, 4 KB at most; later the noted vectors
+  static_assert(kSampledVecs / kSampledSub * 2 <= sizeof(s.hist) && kShortCap * 3 + 256 <= kHistBins && G <= kShortCap * 2, "");
   const int64_t r = blockIdx.x;
   const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
   const int K = p.k_max, n = (int)p.n, tid = threadIdx.x;
@@ -291,7 +320,6 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_sampled_kernel(TopkPara
   const int head = (int)(((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / sizeof(T));
   const int nvec = (n - head) / VEC;
   const uint4* vp = reinterpret_cast<const uint4*>(row + head);
-  constexpr int kGroup = kShortThreads * kSub;                       // vectors of sixteen pieces; the first piece is sampled
   GroupMax<DT> gm;
   gm.init();
 #pragma unroll 1
@@ -304,98 +332,119 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_sampled_kernel(TopkPara
     for (int u = 0; u < 8; ++u)
       if ((g0 + u) * kGroup + tid < nvec) {
         gm.add(v[u]);
-        vkeys[(g0 + u) * kShortThreads + tid] = (uint16_t)vector_key16<DT>(v[u]);
+        vkeys[(g0 + u) * TH + tid] = (uint16_t)vector_key16<DT>(v[u]);
       }
   }
 #pragma unroll
   for (int j = 0; j < kSlots; ++j) gkeys[tid * kSlots + j] = (uint16_t)(f32_key(gm.slot(j)) >> 16);
+  // while the bound is found, what is streamed next comes into L2
+#pragma unroll
+  for (int g = 0; g < 2; ++g)
+    if (tid < TH - TH / kSampledSub && (g + 1) * kGroup <= nvec)
+      asm volatile("prefetch.global.L2 [%0];" :: "l"(vp + g * kGroup + TH + tid * 8));
   if (tid == 0) { s.fill = 0; s.bin = 0; s.above = 0; s.refinements = 0; }
   __syncthreads();
-  const uint32_t t16 = kth_largest_u16(gkeys, G, K, s.hist + 1024, s.tmp_i);
+  const uint32_t t16 = kth_largest_u16(gkeys, G, K, reinterpret_cast<uint32_t*>(cand + kShortCap / 2), s.tmp_i);
   const float thr = key_f32(t16 << 16);   // (a NaN pattern, the bin of -inf, admits everything)
-  int* nnoted = &s.above;
-  auto note = [&](uint32_t key, int i) {
-    const int slot = atomicAdd(nnoted, 1);
-    if (slot < kSampledNotes) s.hist[slot] = (key << 16) | (uint32_t)i;
-  };
-#pragma unroll 1
-  for (int g = 0; g * kGroup + tid < nvec; ++g) {
-    const uint32_t k = vkeys[g * kShortThreads + tid];
-    if (k >= t16) note(k, g * kGroup + tid);
-  }
-  auto look = [&](const uint4& v, int i) {
-    bool any;
-    if constexpr (DT == TLX_BF16) {
-      const __nv_bfloat16 tb = __ushort_as_bfloat16((unsigned short)(__float_as_uint(thr) >> 16));
-      const __nv_bfloat162 t2 = __halves2bfloat162(tb, tb);
-      const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
-      any = !(__hblt2(e[0], t2) && __hblt2(e[1], t2) && __hblt2(e[2], t2) && __hblt2(e[3], t2));
-    } else {
-      any = rc_any_at_least<DT>(v, thr);
+
+  // (key, number) of the vectors that may hold an element at or above the bound, in the warp's list
+  uint32_t* noted = reinterpret_cast<uint32_t*>(cand) + warp_id() * kSampledNotes;
+  const unsigned below_me = (1u << lane_id()) - 1;
+  int nn = 0;
+  auto look = [&](bool reaches, auto key16, int i) {
+    const unsigned b = __ballot_sync(0xFFFFFFFFu, reaches);
+    if (b) {
+      const int slot = nn + __popc(b & below_me);
+      if (reaches && slot < kSampledNotes) noted[slot] = (key16() << 16) | (uint32_t)i;
+      nn += __popc(b);
     }
-    if (any) note(vector_key16<DT>(v), i);
   };
 #pragma unroll 1
   for (int g = 0; g * kGroup < nvec; ++g) {
+    const int i = g * kGroup + tid;
+    const uint32_t k = i < nvec ? vkeys[g * TH + tid] : 0u;
+    look(i < nvec && k >= t16, [&] { return k; }, i);
+  }
+#pragma unroll 1
+  for (int g = 0; g * kGroup < nvec; ++g) {
     const int i0 = g * kGroup + tid;
+    uint4 v[kSampledSub];
     if ((g + 1) * kGroup <= nvec) {
 #pragma unroll
-      for (int h = 1; h < kSub; h += 8) {   // eight loads in flight, then seven
-        uint4 v[8];
+      for (int u = 1; u < kSampledSub; ++u) v[u] = __ldcs(vp + i0 + u * TH);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) if (h + u < kSub) v[u] = __ldcs(vp + i0 + (h + u) * kShortThreads);
-#pragma unroll
-        for (int u = 0; u < 8; ++u) if (h + u < kSub) look(v[u], i0 + (h + u) * kShortThreads);
-      }
+      for (int u = 1; u < kSampledSub; ++u)
+        look(vector_reaches<DT>(v[u], thr), [&] { return vector_key16<DT>(v[u]); }, i0 + u * TH);
     } else {
 #pragma unroll 1
-      for (int h = 1; h < kSub; ++h)
-        if (i0 + h * kShortThreads < nvec) look(__ldcs(vp + i0 + h * kShortThreads), i0 + h * kShortThreads);
+      for (int u = 1; u < kSampledSub; ++u) {
+        const int i = i0 + u * TH;
+        const uint4 w = i < nvec ? __ldcs(vp + i) : make_uint4(0, 0, 0, 0);
+        look(i < nvec && vector_reaches<DT>(w, thr), [&] { return vector_key16<DT>(w); }, i);
+      }
     }
   }
-  __syncthreads();   // the sampled vectors' keys have been used: the candidate list may begin
-  auto push_one = [&](T x, int c) {
+  if (lane_id() == 0) s.scan_u32[warp_id()] = (uint32_t)nn;
+  __syncthreads();   // the sampled vectors' keys have been used: their space is free
+  int most = 0, total = 0;
+#pragma unroll
+  for (int w = 0; w < TH / 32; ++w) {
+    most = max(most, (int)s.scan_u32[w]);
+    total += (int)s.scan_u32[w];
+  }
+  auto push_one = [&](int c) {
+    const T x = row[c];
     const uint32_t key = Elem<DT>::key(x);
-    if ((key >> 16) >= t16) {
-      const int slot = atomicAdd(&s.fill, 1);
-      if (slot < kShortCap) cand[slot] = cand_make(key, (uint32_t)c);
-    }
+    if ((key >> 16) >= t16) list[atomicAdd(&s.fill, 1)] = cand_make(key, (uint32_t)c);
   };
-  if (tid < head) push_one(row[tid], tid);
-  if (tid >= 32 && head + nvec * VEC + tid - 32 < n) push_one(row[head + nvec * VEC + tid - 32], head + nvec * VEC + tid - 32);
-  const int nn = *nnoted;
-  __syncthreads();
-  if (nn > kSampledNotes) {
-    if (tid == 0) s.fill = kShortCap + 1;   // more vectors than the list holds: the exact fallback
-  } else {
+  if (tid < head) push_one(tid);
+  if (tid >= 32 && head + nvec * VEC + tid - 32 < n) push_one(head + nvec * VEC + tid - 32);
+  bool exact = most > kSampledNotes;   // more vectors than a list holds
+  if (!exact) {
     uint32_t t2 = t16;
-    if (nn > K) t2 = kth_largest_key16([&](int i) { return s.hist[i] >> 16; }, nn, K, reinterpret_cast<uint32_t*>(cand + kShortCap / 2), s.tmp_i);
+    if (total > K) {
+      // the keys lie close above the bound as a rule: one histogram of their distances from it, and only if the K-th
+      // greatest key is 255 or more away (two octaves) a second, coarse one of the keys from there on
+      for (int shift = 0;; shift = 8) {
+        for (int i = tid; i < 256; i += TH) hist8[i] = 0;
+        __syncthreads();
+        for (int l = lane_id(); l < nn; l += 32) {
+          const uint32_t key = max(noted[l] >> 16, t16);
+          if (key >= t2) atomicAdd(&hist8[min((key - t2) >> shift, 255u)], 1u);
+        }
+        __syncthreads();
+        if (warp_id() == 0) warp_pick_bin(hist8, K, s.tmp_i);
+        __syncthreads();
+        t2 += (uint32_t)s.tmp_i[0] << shift;
+        if (shift != 0 || s.tmp_i[0] < 255) break;
+      }
+    }
+    for (int l = lane_id(); l < nn; l += 32)
+      if ((noted[l] >> 16) >= t2) sel[atomicAdd(&s.above, 1)] = (uint16_t)noted[l];
+    __syncthreads();
     const float thr2 = key_f32(t2 << 16);
-    for (int l = tid; l < nn; l += kShortThreads) {
-      const uint32_t w = s.hist[l];
-      if ((w >> 16) < t2) continue;
-      const int i = (int)(w & 0xFFFFu);
-      push_vector<DT>(__ldg(vp + i), head + (int64_t)i * VEC, t2, thr2, &s.fill, cand, kShortCap);
+    for (int l = tid; l < s.above; l += TH) {
+      const int i = sel[l];
+      push_vector<DT>(__ldg(vp + i), head + (int64_t)i * VEC, t2, thr2, &s.fill, list, kShortCap);
     }
   }
   __syncthreads();
-  if (s.fill > kShortCap) exact_select_row<DT>(row, n, K, s, cand);   // huge groups of equal values
-  const int m = min(s.fill, kShortCap);
-  if (m <= 2 * kShortThreads) {
-    // every thread counts the composites below its own ones (they are distinct) and puts them at their places
-    uint64_t* placed = reinterpret_cast<uint64_t*>(s.hist);
-    for (int i = tid; i < m; i += kShortThreads) {
-      const uint64_t c = cand[i];
-      int below = 0;
-#pragma unroll 4
-      for (int j = 0; j < m; ++j) below += cand[j] < c ? 1 : 0;
-      placed[below] = c;
-    }
+  exact = exact || s.fill > kShortCap;   // huge groups of equal values, or keys far above the bound
+  if (exact) {
     __syncthreads();
-    emit_row<DT>(p, r, row, placed, m);
-  } else {
+    exact_select_row<DT>(row, n, K, s, cand);
+    const int m = min(s.fill, kShortCap);
     sort_candidates(cand, m);
     emit_row<DT>(p, r, row, cand, m);
+  } else if (s.fill <= 256) {
+    const int m = s.fill;
+    order_by_count(list, m, cand);
+    __syncthreads();
+    emit_row<DT>(p, r, row, cand, m);
+  } else {
+    const int m = s.fill;
+    sort_candidates(list, m);
+    emit_row<DT>(p, r, row, list, m);
   }
 }
 
@@ -536,16 +585,9 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   __syncthreads();
   if (s.fill > kShortCap) exact_select_row<DT>(row, n, K, s, cand);   // huge groups of equal values
   const int m = min(s.fill, kShortCap);
-  if (m <= 96) {
-    // a handful of candidates: every thread counts the composites below its own (they are distinct) and
-    // puts it at that place; no network, no barriers in between
-    uint64_t* placed = reinterpret_cast<uint64_t*>(s.hist + 2048);   // 96 slots in the fallback's histogram space
-    if ((int)threadIdx.x < m) {
-      const uint64_t c = cand[threadIdx.x];
-      int below = 0;
-      for (int i = 0; i < m; ++i) below += cand[i] < c ? 1 : 0;
-      placed[below] = c;
-    }
+  if (m <= 256) {   // (the network's barriers cost more up to there)
+    uint64_t* placed = reinterpret_cast<uint64_t*>(s.hist);
+    order_by_count(cand, m, placed);
     __syncthreads();
     emit_row<DT>(p, r, row, placed, m);
   } else {
@@ -722,7 +764,7 @@ static int launch_topk_short(cudaStream_t st, const TopkParams& p, bool long_row
       if (dev >= 0 && dev < 64) asked[dev] = true;
     }
   }
-  if (long_rows) topk_sampled_kernel<DT><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
+  if (long_rows) topk_sampled_kernel<DT><<<(unsigned)p.rows, kSampledThreads, smem, st>>>(p);
   else topk_short_kernel<DT><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
   TLX_CHECK_LAUNCH("top_k (short rows)");
   return TLX_OK;
