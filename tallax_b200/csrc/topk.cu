@@ -276,16 +276,17 @@ __device__ __forceinline__ void order_by_count(const uint64_t* cand, int m, uint
   }
 }
 
-// ---- many long rows ------------------------------------------------------------------------------------------------------
-// Rows of more than 128 KB, which L2 would not keep between two passes: the bound comes from every eighth 4 KB piece of
-// the row, whose vectors leave the 16-bit keys of their greatest elements in shared memory, so that every byte of the
+// ---- long rows -----------------------------------------------------------------------------------------------------------
+// A CTA per row, for rows that L2 would not keep between two passes: the bound comes from every eighth of the row's pieces
+// of a vector per thread, whose vectors leave the 16-bit keys of their greatest elements in shared memory, so that every byte of the
 // row is read once.  An eighth of the row bounds loosely (about 1200 vectors hold an element at or above the bound for
 // K = 128): the vectors are noted with their keys, a list per warp, the K-th greatest of these keys is a second, tight
 // bound (K vectors hold an element at or above it), and only the vectors that reach it are looked into.
 // HBM-bound; f32 [1024, 262144], k = 128: 285 us with the bound from a quarter of the row and the whole row read again,
-// 234 us with one list of noted vectors per CTA of 128 threads, 204 us so (the bytes alone: 164 us).
+// 234 us with one list of noted vectors per CTA of 128 threads, 205 us with a list per warp of a CTA of 256 threads, 171 us
+// with no more shared memory taken from L1 than it needs (the bytes alone: 164 us).
 constexpr int kSampledSub = 8;
-constexpr int kSampledThreads = 256;   // (of 128: 213 us at that size, 33.5 us against 26.7 us for 300 rows of 60000)
+constexpr int kSampledNotes = 256;   // noted vectors of a warp
 constexpr int64_t kSampledVecs = 65536;   // vectors of a row at most: their numbers have 16 bits
 template <int DT>
 __device__ __forceinline__ bool vector_reaches(const uint4& v, float thr) {   // (true also for vectors somewhat below)
@@ -297,13 +298,11 @@ __device__ __forceinline__ bool vector_reaches(const uint4& v, float thr) {   //
     return rc_any_at_least<DT>(v, thr);
   }
 }
-template <int DT>
-__global__ void __launch_bounds__(kSampledThreads, 1024 / kSampledThreads) topk_sampled_kernel(TopkParams p) {
+template <int DT, int TH>
+__global__ void __launch_bounds__(TH, 1024 / TH) topk_sampled_kernel(TopkParams p) {
   using T = typename Elem<DT>::type;
-  constexpr int TH = kSampledThreads;
   constexpr int kSlots = GroupMax<DT>::kSlots, G = TH * kSlots, VEC = 16 / (int)sizeof(T);
   constexpr int kGroup = TH * kSampledSub;   // vectors of eight pieces; the first piece is sampled
-  constexpr int kSampledNotes = kShortCap * 2 / (TH / 32);           // noted vectors of a warp, in the candidates' space
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SelectShared& s = *reinterpret_cast<SelectShared*>(smem_raw);
   uint64_t* cand = reinterpret_cast<uint64_t*>(smem_raw + ((sizeof(SelectShared) + 15) & ~size_t(15)));
@@ -311,8 +310,8 @@ __global__ void __launch_bounds__(kSampledThreads, 1024 / kSampledThreads) topk_
   uint64_t* list = reinterpret_cast<uint64_t*>(s.hist);             // the candidates, and behind them
   uint32_t* hist8 = s.hist + kShortCap * 2;                         // the second bound's histogram
   uint16_t* sel = reinterpret_cast<uint16_t*>(hist8 + 256);         // the vectors to look into
-  uint16_t* gkeys = reinterpret_cast<uint16_t*>(cand);              // the groups' maxima, 4 KB at most; later the noted vectors
-  static_assert(kSampledVecs / kSampledSub * 2 <= sizeof(s.hist) && kShortCap * 3 + 256 <= kHistBins && G <= kShortCap * 2, "");
+  uint16_t* gkeys = reinterpret_cast<uint16_t*>(cand);              // the groups' maxima and a histogram; later the noted vectors, TH * 32 bytes
+  static_assert(kSampledVecs / kSampledSub * 2 <= sizeof(s.hist) && kShortCap * 3 + 256 <= kHistBins && G * 2 + 2048 <= TH * 32, "");
   const int64_t r = blockIdx.x;
   const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
   const int K = p.k_max, n = (int)p.n, tid = threadIdx.x;
@@ -344,7 +343,7 @@ __global__ void __launch_bounds__(kSampledThreads, 1024 / kSampledThreads) topk_
       asm volatile("prefetch.global.L2 [%0];" :: "l"(vp + g * kGroup + TH + tid * 8));
   if (tid == 0) { s.fill = 0; s.bin = 0; s.above = 0; s.refinements = 0; }
   __syncthreads();
-  const uint32_t t16 = kth_largest_u16(gkeys, G, K, reinterpret_cast<uint32_t*>(cand + kShortCap / 2), s.tmp_i);
+  const uint32_t t16 = kth_largest_u16(gkeys, G, K, reinterpret_cast<uint32_t*>(gkeys + G), s.tmp_i);
   const float thr = key_f32(t16 << 16);   // (a NaN pattern, the bin of -inf, admits everything)
 
   // (key, number) of the vectors that may hold an element at or above the bound, in the warp's list
@@ -420,10 +419,14 @@ __global__ void __launch_bounds__(kSampledThreads, 1024 / kSampledThreads) topk_
       }
     }
     for (int l = lane_id(); l < nn; l += 32)
-      if ((noted[l] >> 16) >= t2) sel[atomicAdd(&s.above, 1)] = (uint16_t)noted[l];
+      if ((noted[l] >> 16) >= t2) {
+        const int slot = atomicAdd(&s.above, 1);
+        if (slot < kShortCap * 2) sel[slot] = (uint16_t)noted[l];
+      }
     __syncthreads();
+    exact = s.above > kShortCap * 2;
     const float thr2 = key_f32(t2 << 16);
-    for (int l = tid; l < s.above; l += TH) {
+    for (int l = tid; !exact && l < s.above; l += TH) {
       const int i = sel[l];
       push_vector<DT>(__ldg(vp + i), head + (int64_t)i * VEC, t2, thr2, &s.fill, list, kShortCap);
     }
@@ -453,12 +456,15 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   using T = typename Elem<DT>::type;
   constexpr int kSlots = GroupMax<DT>::kSlots;
   constexpr int G = kShortThreads * kSlots;
+  constexpr int kU = DT == TLX_F32 ? 9 : 10;   // loads in flight per thread (of f32 the tenth would spill)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   SelectShared& s = *reinterpret_cast<SelectShared*>(smem_raw);
-  uint64_t* cand = reinterpret_cast<uint64_t*>(smem_raw + ((sizeof(SelectShared) + 15) & ~size_t(15)));
-  // the group keys and the small histogram live in the big histogram's space, which only the fallback uses
+  // all of it lives in the big histogram's space, which only the fallback uses (its candidates, too, are written when the
+  // histogram has been read): 4 KB for the group keys and the small histogram, and later the noted vectors, and later the
+  // ordered candidates; 8 KB for the candidates
+  uint64_t* cand = reinterpret_cast<uint64_t*>(s.hist + 1024);
   uint16_t* gkeys = reinterpret_cast<uint16_t*>(s.hist);            // G * 2 bytes <= 2 KB
-  uint32_t* hist8 = s.hist + 1024;                                    // 512 words
+  uint32_t* hist8 = s.hist + 512;                                     // 512 words
   const int64_t r = blockIdx.x;
   const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
   const int K = p.k_max;
@@ -482,7 +488,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
     if (vec_maxima) {
       const __nv_bfloat16 ninf = __float2bfloat16_rn(-INFINITY);
       for (int64_t i = nvec + threadIdx.x; i < ((nvec + 7) & ~(int64_t)7); i += blockDim.x) vmax[i] = ninf;
-      for_each_vec<DT, 10>(row, n,
+      for_each_vec<DT, kU>(row, n,
         [&](const uint4& v, int64_t cb) {
           gm.add(v);
           const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
@@ -493,7 +499,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
     }
   }
   if (!vec_maxima)
-    for_each_vec<DT, 10>(row, n, [&](const uint4& v, int64_t) { gm.add(v); }, [&](T x, int64_t) { gm.add_one(x); });
+    for_each_vec<DT, kU>(row, n, [&](const uint4& v, int64_t) { gm.add(v); }, [&](T x, int64_t) { gm.add_one(x); });
 #pragma unroll
   for (int j = 0; j < kSlots; ++j) gkeys[threadIdx.x * kSlots + j] = (uint16_t)(f32_key(gm.slot(j)) >> 16);
   if (threadIdx.x == 0) { s.fill = 0; s.bin = 0; s.above = 0; s.refinements = 0; }
@@ -513,7 +519,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   };
   // The streaming loop only notes which vectors hold an element at or above the bound (about one per
   // candidate); the noted vectors are then read again, one per thread, and their elements pushed.
-  uint32_t* noted = s.hist + 2048;          // up to kShortCap first columns, in the fallback's histogram space
+  uint32_t* noted = s.hist;                 // up to kShortCap first columns
   int* nnoted = &s.above;                   // (tmp_i holds the bound's picks, which threads may still be reading)
   if (threadIdx.x == 0) *nnoted = 0;
   __syncthreads();
@@ -540,7 +546,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
         }
       }
     } else {
-      for_each_vec<DT, 10>(row, n,
+      for_each_vec<DT, kU>(row, n,
         [&](const uint4& v, int64_t cb) {
           const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
           // __hblt2: both halves less than the bound (false when either is a NaN)
@@ -549,7 +555,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
         push_one);
     }
   } else if constexpr (DT == TLX_F16) {
-    for_each_vec<DT, 10>(row, n,
+    for_each_vec<DT, kU>(row, n,
       [&](const uint4& v, int64_t cb) {
         const __half2* e = reinterpret_cast<const __half2*>(&v);
         bool any = false;
@@ -562,7 +568,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
       },
       push_one);
   } else {
-    for_each_vec<DT, 10>(row, n,
+    for_each_vec<DT, kU>(row, n,
       [&](const uint4& v, int64_t cb) {
         const float* e = reinterpret_cast<const float*>(&v);
         if (!(e[0] < thr) || !(e[1] < thr) || !(e[2] < thr) || !(e[3] < thr)) note(cb);
@@ -585,9 +591,16 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   __syncthreads();
   if (s.fill > kShortCap) exact_select_row<DT>(row, n, K, s, cand);   // huge groups of equal values
   const int m = min(s.fill, kShortCap);
-  if (m <= 256) {   // (the network's barriers cost more up to there)
+  if (m <= 96) {
+    // a handful of candidates: every thread counts the composites below its own (they are distinct) and
+    // puts it at that place; no network, no barriers in between
     uint64_t* placed = reinterpret_cast<uint64_t*>(s.hist);
-    order_by_count(cand, m, placed);
+    if ((int)threadIdx.x < m) {
+      const uint64_t c = cand[threadIdx.x];
+      int below = 0;
+      for (int i = 0; i < m; ++i) below += cand[i] < c ? 1 : 0;
+      placed[below] = c;
+    }
     __syncthreads();
     emit_row<DT>(p, r, row, placed, m);
   } else {
@@ -676,15 +689,35 @@ __global__ void __launch_bounds__(kRcThreads, 4) topk_cluster_kernel(const __gri
   cl_wait();
 }
 
-// Whether it serves a call: floating-point rows that a cluster holds, exact mode without the diagnostics of the one-pass
-// kernel, fewer rows than the kernel of many short rows wants, and not more than 64 MB, beyond which the kernels with a CTA
-// per row move more bytes per second (f32 [204, 39024] 22 us against 30, bf16 [225, 130894] 40 against 49, f32
-// [128, 262144] 117 against 62).
+// Exact mode of floating-point rows without the diagnostics of the one-pass kernel, and not a comparison run of that one.
+static bool float_rows(int dtype, const TopkParams& p) {
+  return (dtype == TLX_F32 || dtype == TLX_BF16 || dtype == TLX_F16) && p.mode == 0 && !p.out_valid && !p.out_depths && !p.out_cutoff;
+}
+static const char* forced_path() {   // "short" / "long": comparison runs of the two-pass and of the one-pass kernel
+  static const char* force = getenv("TLX_TOPK_PATH");
+  return force;
+}
+
+// Whether the long-row kernel serves a call: rows whose vectors have 16-bit numbers, and either
+// - fewer than 256 rows of more bytes in all than the shared memory of the clusters that run at the same time holds, about
+//   14 MB: beyond it the cluster form takes several waves (f32 [148, 33000] 18 us against 12, [100, 131072] 43 against 18,
+//   [148, 262144] 57 against 30; below it f32 [100, 33000] 11.4 against 11.5, [20, 131072] 11.8 against 16.6); or
+// - rows of more than 80 KB, more than 30 MB in all, whose second reading by the two-pass kernel L2 no longer serves (f32
+//   [1024, 24500] 51 us against 40, [450, 24500] 26 against 22, [300, 24500] 16.8 against 18.2; of 64 KB [1024, 16384] 27
+//   against 28); 70 MB where 592 CTAs of 256 threads do not run all the rows at once ([600, 24000]
+//   25 us both, [600, 30000] 31 against 27).
+static bool long_rows_apply(int dtype, const TopkParams& p) {
+  const int64_t row = p.n * dtype_bytes(dtype), all = row * p.rows;
+  if (!float_rows(dtype, p) || p.k_max > kShortMaxK || row / 16 > kSampledVecs || forced_path()) return false;
+  if (p.rows < 256) return all > (14ll << 20);
+  return row > (80 << 10) && all > ((p.rows > 4 * 148 ? 70ll : 30ll) << 20);
+}
+
+// Whether the cluster form serves a call: fewer rows than the kernels with a CTA per row want, rows that a cluster holds, and
+// not more than 64 MB, beyond which several waves of clusters take longer than the one-pass kernel.
 static bool cluster_rows_apply(int dtype, const TopkParams& p) {
-  if (dtype != TLX_F32 && dtype != TLX_BF16 && dtype != TLX_F16) return false;
-  if (p.k_max > kRcMaxK || p.mode != 0 || p.out_valid || p.out_depths || p.out_cutoff) return false;
-  static const bool forced = getenv("TLX_TOPK_PATH") != nullptr;   // comparison runs of the other two kernels
-  return !forced && p.rows < 256 && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart && p.rows * p.n * dtype_bytes(dtype) <= (64ll << 20);
+  if (!float_rows(dtype, p) || p.k_max > kRcMaxK || forced_path() || long_rows_apply(dtype, p)) return false;
+  return p.rows < 256 && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart && p.rows * p.n * dtype_bytes(dtype) <= (64ll << 20);
 }
 
 template <int DT>
@@ -728,46 +761,63 @@ static int launch_topk_cluster(cudaStream_t st, const TopkParams& p) {
   return TLX_OK;
 }
 
-// Rows of more than 128 KB take the kernel that reads them once, if it can number their vectors in 16 bits.
-constexpr int64_t kLongRowBytes = 128 << 10;
-static bool long_rows_apply(int dtype, const TopkParams& p) {
-  return p.n * dtype_bytes(dtype) > kLongRowBytes && p.n * dtype_bytes(dtype) / 16 <= kSampledVecs;
-}
-// Whether the two-pass kernel serves a call: floating-point rows, K <= 128, exact mode without the
-// diagnostics of the one-pass kernel, and enough rows to fill the eight CTAs per SM.
+// Whether the two-pass kernel serves a call: K <= 128 and enough rows to fill the eight CTAs per SM.
 static bool short_rows_apply(int dtype, const TopkParams& p) {
-  static const char* force = getenv("TLX_TOPK_PATH");   // "short" / "long": comparison runs
-  if (dtype != TLX_F32 && dtype != TLX_BF16 && dtype != TLX_F16) return false;
-  if (p.k_max > kShortMaxK || p.mode != 0 || p.out_valid || p.out_depths || p.out_cutoff) return false;
-  if (force && !strcmp(force, "short")) return true;
-  if (force && !strcmp(force, "long")) return false;
-  return p.rows >= 256 && p.n >= 2048 && (p.n * dtype_bytes(dtype) <= kLongRowBytes || long_rows_apply(dtype, p));
+  if (!float_rows(dtype, p) || p.k_max > kShortMaxK) return false;
+  if (forced_path()) return !strcmp(forced_path(), "short");
+  return p.rows >= 256 && p.n >= 2048 && p.n * dtype_bytes(dtype) <= (128 << 10);
+}
+
+// The shared memory that `ctas` CTAs of an SM need (1 KB each is the system's), asked for once per device, and not more: what
+// is left is L1, without which fewer loads are in flight (f32 [1024, 262144], k = 128: 171 us, and 205 us with all
+// of it shared memory).
+template <typename F>
+static cudaError_t ask_shared_memory(std::mutex& mu, bool (&asked)[64], F* kernel, size_t smem, int ctas) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(mu);
+  if (dev >= 0 && dev < 64 && asked[dev]) return cudaSuccess;
+  const size_t percent = ((smem + 1024) * ctas * 100 + (228 << 10) - 1) / (228 << 10);
+  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, (int)(percent < 100 ? percent : 100));
+  if (e == cudaSuccess && smem > (48 << 10)) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) asked[dev] = true;
+  return e;
 }
 
 template <int DT>
-static int launch_topk_short(cudaStream_t st, const TopkParams& p, bool long_rows) {
-  const size_t smem = ((sizeof(SelectShared) + 15) & ~size_t(15)) + (size_t)kShortCap * 8;
-  // eight CTAs of 25 KB per SM need the large shared-memory configuration: asked for once per device
+static int launch_topk_short(cudaStream_t st, const TopkParams& p) {
+  const size_t smem = sizeof(SelectShared);
   static std::mutex mu;
   static bool asked[64] = {};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (dev < 0 || dev >= 64 || !asked[dev]) {
-      cudaError_t e = cudaFuncSetAttribute(topk_short_kernel<DT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                           (int)cudaSharedmemCarveoutMaxShared);
-      if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(topk_sampled_kernel<DT>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared);
-      if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-      if (dev >= 0 && dev < 64) asked[dev] = true;
-    }
-  }
-  if (long_rows) topk_sampled_kernel<DT><<<(unsigned)p.rows, kSampledThreads, smem, st>>>(p);
-  else topk_short_kernel<DT><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
+  cudaError_t e = ask_shared_memory(mu, asked, topk_short_kernel<DT>, smem, 1024 / kShortThreads);
+  if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  topk_short_kernel<DT><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
   TLX_CHECK_LAUNCH("top_k (short rows)");
   return TLX_OK;
+}
+
+template <int DT, int TH>
+static int launch_topk_sampled_threads(cudaStream_t st, const TopkParams& p) {
+  const size_t smem = ((sizeof(SelectShared) + 15) & ~size_t(15)) + TH * 32;
+  static std::mutex mu;
+  static bool asked[64] = {};
+  cudaError_t e = ask_shared_memory(mu, asked, topk_sampled_kernel<DT, TH>, smem, 1024 / TH);
+  if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
+  topk_sampled_kernel<DT, TH><<<(unsigned)p.rows, TH, smem, st>>>(p);
+  TLX_CHECK_LAUNCH("top_k (long rows)");
+  return TLX_OK;
+}
+// 1024 threads per SM in any case: one, two, four or eight rows at a time, by which of them has every row running at once (f32
+// [128, 262144]: 27.4 us with CTAs of 1024 threads, 31 of 512, 49 of 256; [200, 100000]: 32, 24, 30; [500, 100000]: 65, 47,
+// 42; bf16 [800, 60000]: 34 us of 256, 27.5 us of 128).  CTAs of 128 threads have lists for twice the vectors that reach the
+// bound as a rule only up to K = 64.
+template <int DT>
+static int launch_topk_sampled(cudaStream_t st, const TopkParams& p) {
+  constexpr int sms = 148;
+  if (p.rows <= sms) return launch_topk_sampled_threads<DT, 1024>(st, p);
+  if (p.rows <= 2 * sms) return launch_topk_sampled_threads<DT, 512>(st, p);
+  if (p.rows > 4 * sms && p.k_max <= 64) return launch_topk_sampled_threads<DT, 128>(st, p);
+  return launch_topk_sampled_threads<DT, 256>(st, p);
 }
 
 template <int DT, int CAP>
@@ -812,12 +862,18 @@ static int dispatch_topk(cudaStream_t st, int dtype, const TopkParams& p, const 
       default: return launch_topk_cluster<TLX_F16>(st, p);
     }
   }
-  if (short_rows_apply(dtype, p)) {
-    const bool long_rows = long_rows_apply(dtype, p);
+  if (long_rows_apply(dtype, p)) {
     switch (dtype) {
-      case TLX_F32: return launch_topk_short<TLX_F32>(st, p, long_rows);
-      case TLX_BF16: return launch_topk_short<TLX_BF16>(st, p, long_rows);
-      default: return launch_topk_short<TLX_F16>(st, p, long_rows);
+      case TLX_F32: return launch_topk_sampled<TLX_F32>(st, p);
+      case TLX_BF16: return launch_topk_sampled<TLX_BF16>(st, p);
+      default: return launch_topk_sampled<TLX_F16>(st, p);
+    }
+  }
+  if (short_rows_apply(dtype, p)) {
+    switch (dtype) {
+      case TLX_F32: return launch_topk_short<TLX_F32>(st, p);
+      case TLX_BF16: return launch_topk_short<TLX_BF16>(st, p);
+      default: return launch_topk_short<TLX_F16>(st, p);
     }
   }
   switch (dtype) {
@@ -900,7 +956,7 @@ int tlx_top_k(void* stream, const void* x, int dtype, int64_t rows, int64_t n, i
   p.x = x; p.rows = rows; p.n = n; p.row_stride = row_stride; p.k_max = k_max; p.k_per_row = k_per_row;
   p.use_replace = use_replace; p.replace_val = replace_val; p.mode = mode; p.out_vals = out_vals;
   p.out_idx = out_idx; p.out_valid = out_valid; p.out_depths = out_depths; p.out_cutoff = out_cutoff;
-  if (sp.parts && !cluster_rows_apply(dtype, p) && mode == 0 && !out_valid && !out_depths && !out_cutoff && row_stride == n && workspace &&
+  if (sp.parts && !cluster_rows_apply(dtype, p) && !long_rows_apply(dtype, p) && mode == 0 && !out_valid && !out_depths && !out_cutoff && row_stride == n && workspace &&
       workspace_bytes >= sp.bytes && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 &&
       (reinterpret_cast<uintptr_t>(x) & 15) == 0) {
     unsigned char* ws = (unsigned char*)workspace;
