@@ -689,9 +689,10 @@ static int debug_stages() {
 // launch): the kernel does whatever needs none of the predecessor's results and then executes
 // griddepcontrol.wait, which returns when the predecessor has finished and its writes are visible.  Where
 // the attribute is not accepted the kernel is launched in plain stream order (the wait is then a no-op).
+// carveout: the share of an SM's memory it prefers as shared memory, in percent; -1: as set for the kernel.
 template <typename... Params, typename... Args>
 static int launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                            const char* what, Args... args) {
+                            const char* what, int carveout, Args... args) {
   static bool programmatic = getenv("TLX_NO_DEPENDENT_LAUNCH") == nullptr;
   if (programmatic) {
     cudaLaunchConfig_t cfg{};
@@ -699,11 +700,13 @@ static int launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned b
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+    attr[1].val.sharedMemCarveout = (unsigned)carveout;
+    cfg.attrs = attr;
+    cfg.numAttrs = carveout >= 0 ? 2 : 1;
     if (cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess) {
       count_launch();
       return TLX_OK;
@@ -824,11 +827,11 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   if (stages < 2) return TLX_OK;
   const int64_t sgrid = items < 4ll * sms ? items : 4ll * sms;
   TLX_TIMELINE_KERNEL(1);
-  if ((rc = launch_dependent(sample_stream_kernel, (unsigned)sgrid, kStThreads, st_smem, st, "sample (stream)", p)) != TLX_OK) return rc;
+  if ((rc = launch_dependent(sample_stream_kernel, (unsigned)sgrid, kStThreads, st_smem, st, "sample (stream)", -1, p)) != TLX_OK) return rc;
   if (stages < 3) return TLX_OK;
   TLX_TIMELINE_KERNEL(2);
   return launch_dependent(sample_finish_kernel, (unsigned)(p.fin_ctas + sp.rows), kStThreads, fin_smem, st,
-                          "sample (finish)", p, dense);
+                          "sample (finish)", -1, p, dense);
 }
 
 }  // namespace tlx
@@ -1032,7 +1035,12 @@ static int launch_merge(cudaStream_t st, const MergeParams& p, int64_t rows) {
     // exchange mode: the rows' arrival counts order this kernel after the candidate kernels, so it may be
     // scheduled while this rank's candidate kernel still runs (its CTAs have all started by then) and has
     // its launch latency behind it when the first rows arrive
-    return launch_dependent(merge_and_sample_kernel, (unsigned)rows, (unsigned)threads, smem, st, "merge_and_sample", p);
+    // ... and does run beside it only on SMs that need not change the size of their shared memory in between: the
+    // candidate kernels' sizes are all of it for fewer than 256 rows and 64 % for more (1024 rows of 18992, k = 50, with
+    // their candidate kernel: 37.0 us, with the default 39.5 us)
+    const size_t need = (smem + 1024) * (size_t)((rows + 147) / 148 < 8 ? (rows + 147) / 148 : 8) * 100 / (228 << 10) + 1;
+    const int carveout = rows < 256 || need > 100 ? 100 : need < 64 ? 64 : (int)need;
+    return launch_dependent(merge_and_sample_kernel, (unsigned)rows, (unsigned)threads, smem, st, "merge_and_sample", carveout, p);
   }
   merge_and_sample_kernel<<<(unsigned)rows, threads, smem, st>>>(p);
   TLX_CHECK_LAUNCH("merge_and_sample");
