@@ -46,6 +46,9 @@ __device__ __forceinline__ uint32_t cl_ld_u16(uint32_t a) {
   asm volatile("ld.shared::cluster.u16 %0, [%1];" : "=h"(v) : "r"(a) : "memory");
   return v;
 }
+__device__ __forceinline__ void cl_st_u64(uint32_t addr, uint32_t lo, uint32_t hi) {
+  asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" :: "r"(addr), "r"(lo), "r"(hi) : "memory");
+}
 __device__ __forceinline__ void cl_st_u32(uint32_t a, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void cl_st_f32(uint32_t a, float v) { cl_st_u32(a, __float_as_uint(v)); }
 __device__ __forceinline__ void cl_st_u64(uint32_t a, uint64_t v) { asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }

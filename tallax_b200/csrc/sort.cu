@@ -249,12 +249,21 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
   const int64_t n_pad = next_pow2(n < 2 ? 2 : n);
   int rc;
   // Up to 1024 elements the network's few stages cost less than a pass's counters (f32 [1000, 512]: 13 us against 26).
-  // A CTA per row up to 16384: eight elements a thread, sixteen where the rows fill the GPU (fewer counters per element:
-  // f32 [1024, 4096] 77 us against 90); a cluster of CTAs of 16384 elements up to 131072.
+  // A CTA per row up to 8192: eight elements a thread, sixteen where the rows fill the GPU (fewer counters per element: f32
+  // [1024, 4096] 77 us against 90).  A cluster of CTAs beyond: of 4096 elements each where all of them run at once with an
+  // SM each (bf16 [4, 16384] 20 us, with 8192 elements 26, with one CTA per row 32), else of 8192, two to an SM, of which
+  // one works while the other waits at a barrier (f32 [128, 65536] 368 us against 385 with one of 16384), which rows of
+  // more than 65536 elements, eight CTAs being the most, take.
   if (n > 1024 && n <= kRadixMaxRow) {
-    if (n > kRadixTile)
-      return launch_radix<DT, 16, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, kRadixMaxThreads,
-                                        (int)((n + kRadixTile - 1) / kRadixTile));
+    if (n > kRadixTile) {
+      int cluster = (int)((n + 4095) / 4096);
+      if (cluster > 8 || rows * cluster > 148) cluster = (int)((n + kRadixTile - 1) / kRadixTile);
+      if (cluster > 8) cluster = rows * 8 <= 148 ? 8 : (int)((n + 2 * kRadixTile - 1) / (2 * kRadixTile));
+      if (cluster == 3) cluster = 4;   // clusters of three fill the GPU's groups of SMs badly (f32 [200, 20000] 179 us against 152)
+      int threads = (int)((n + cluster * 512 - 1) / (cluster * 512)) * 32;
+      if (threads < 256) threads = 256;
+      return launch_radix<DT, 16, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, cluster);
+    }
     const int ipt = n <= 8192 && rows <= 296 ? 8 : 16;
     int threads = (int)((n + 32 * ipt - 1) / (32 * ipt)) * 32;
     if (threads < 256) threads = 256;

@@ -1,7 +1,7 @@
 // Stable row-wise argsort by radix: least significant digit first, eight bits a pass, a row in the shared memory of one
-// CTA (up to 16384 elements) or of a cluster of CTAs (up to 131072).  Included by sort.cu.
+// CTA (up to 8192 elements) or of a cluster of CTAs (up to 131072).  Included by sort.cu.
 //
-// What bounds it: integer instructions, which issue at half rate, about 100 of them an element and pass; four passes for
+// What bounds it: integer instructions, which issue at half rate, about 130 of them an element and pass; four passes for
 // 32-bit keys and two for 16-bit ones, against 50 to 70 compare-exchanges of ten instructions an element of a bitonic
 // network on 64-bit composites.  Every pass keeps the order of equal digits, so the position need not be compared: it
 // travels beside the key.
@@ -20,8 +20,8 @@
 namespace tlx {
 
 constexpr int kRadixMaxThreads = 1024;
-constexpr int kRadixTile = 16384;            // elements per CTA at most
-constexpr int kRadixMaxRow = 8 * kRadixTile; // elements per row at most
+constexpr int kRadixTile = 8192;              // elements per CTA at most, of rows of up to eight of them
+constexpr int kRadixMaxRow = 16 * kRadixTile; // elements per row at most
 
 // Order-preserving key of a type in its own number of bits, and back (-0 comes back as +0, NaN as the one NaN).
 template <int DT> struct RadixKey {
@@ -84,6 +84,20 @@ __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p
                                                 RadixShared& s, unsigned short* count, uint32_t* sk, Pos* sp) {
   const int nt = blockDim.x, nw = nt >> 5, cap = nt * IPT;
   const int lane = lane_id(), w = warp_id();
+  uint2* pair = reinterpret_cast<uint2*>(sk);   // cluster: key and position side by side, one access for both
+  auto get = [&](int i, uint32_t& key, uint32_t& pos) {
+    if constexpr (CL) {
+      const uint2 e = pair[i];
+      key = e.x;
+      pos = e.y;
+    } else {
+      key = sk[i];
+      pos = sp[i];
+    }
+  };
+  // place / cap without an integer division: (place + 0.5) / cap is at least 0.5 / cap away from a whole number, and a place
+  // is below 2^17, far more than the product's rounding error
+  const float inv_cap = 1.0f / (float)cap;
   bool scattered = false;
 #pragma unroll 1
   for (int sh = 0; sh < kBits; sh += 8) {
@@ -91,9 +105,7 @@ __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p
     if (scattered) {
 #pragma unroll
       for (int j = 0; j < IPT; ++j) {
-        const int i = w * 32 * IPT + 32 * j + lane;
-        k[j] = sk[i];
-        p[j] = sp[i];
+        get(w * 32 * IPT + 32 * j + lane, k[j], p[j]);
       }
     }
     // ranks among the warp's equal digits
@@ -156,17 +168,19 @@ __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
       const int to = mine[(k[j] >> sh) & 255u] + at[j];
-      sk[to] = k[j];
-      sp[to] = (Pos)p[j];
+      if constexpr (CL) {
+        pair[to] = make_uint2(k[j], p[j]);
+      } else {
+        sk[to] = k[j];
+        sp[to] = (Pos)p[j];
+      }
     }
     __syncthreads();
     if constexpr (CL) {
       // read back in the CTA's order; then (nobody's area is needed any more) every element to its place in the row
 #pragma unroll
       for (int j = 0; j < IPT; ++j) {
-        const int i = threadIdx.x + j * nt;
-        k[j] = sk[i];
-        p[j] = sp[i];
+        get(threadIdx.x + j * nt, k[j], p[j]);
       }
       cl_sync();
       uint32_t all = 0, before = 0;
@@ -184,9 +198,8 @@ __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p
 #pragma unroll
       for (int j = 0; j < IPT; ++j) {
         const int to = threadIdx.x + j * nt + s.shift_by[(k[j] >> sh) & 255u];
-        const int r = to / cap, i = to - r * cap;
-        cl_st_u32(cl_map(sk + i, (uint32_t)r), k[j]);
-        cl_st_u32(cl_map(sp + i, (uint32_t)r), p[j]);
+        const int r = (int)(((float)to + 0.5f) * inv_cap), i = to - r * cap;
+        cl_st_u64(cl_map(pair + i, (uint32_t)r), k[j], p[j]);
       }
       cl_sync();
     }
@@ -194,11 +207,7 @@ __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p
   }
   if (scattered) {
 #pragma unroll
-    for (int j = 0; j < IPT; ++j) {
-      const int i = threadIdx.x + j * nt;
-      k[j] = sk[i];
-      p[j] = sp[i];
-    }
+    for (int j = 0; j < IPT; ++j) get(threadIdx.x + j * nt, k[j], p[j]);
   }
   return scattered;
 }
@@ -211,7 +220,7 @@ __device__ __forceinline__ uint32_t radix_diff(uint32_t diff, RadixShared& s) {
   return __reduce_or_sync(0xFFFFFFFFu, lane_id() < (int)(blockDim.x >> 5) ? s.warp[lane_id()] : 0u);
 }
 
-// Dynamic shared memory: RadixShared, counters [warps][256] u16, keys [cap] u32, positions [cap] u16 or (cluster) u32.
+// Dynamic shared memory (cluster: keys and positions in pairs): RadixShared, counters [warps][256] u16, keys [cap] u32, positions [cap] u16 or (cluster) u32.
 __host__ __device__ __forceinline__ size_t radix_smem(int threads, int cap, bool cluster) {
   return sizeof(RadixShared) + (size_t)(threads / 32) * 512 + (size_t)cap * (cluster ? 8 : 6);
 }

@@ -40,3 +40,15 @@ def test_radix_sort_row_counts(cuda, rows):
     x = np.random.default_rng(rows).standard_normal((rows, 3001)).astype(np.float32)
     keys, perm = tax.sort([to_dev(x, cuda)], num_keys=1, return_argsort=True)
     assert np.array_equal(to_np(perm), np.argsort(x, axis=1, kind="stable")) and np.array_equal(to_np(keys), np.sort(x, axis=1))
+
+
+# many rows: clusters of CTAs of 8192 elements (three become four), and of 16384 for the longest rows
+@pytest.mark.parametrize("dtype,rows,n", [("f32", 160, 8193), ("bf16", 80, 20001), ("f32", 40, 65536), ("i32", 24, 65537)])
+def test_radix_sort_many_rows(cuda, dtype, rows, n):
+    rng = np.random.default_rng(n)
+    x = np.round(rng.standard_normal((4, n)).astype(np.float32) * 300)
+    x = x.astype({"f32": np.float32, "bf16": o.bfloat16, "i32": np.int32}[dtype])
+    v, i = tax.sort([to_dev(np.tile(x, (rows // 4, 1)), cuda)], num_keys=1, is_stable=True, return_argsort=True)
+    ev, ei = o.sort([x], 1, is_stable=True, return_argsort=True)
+    assert np.array_equal(to_np(i), np.tile(ei, (rows // 4, 1)))
+    assert exact_match(to_np(v), np.tile(ev, (rows // 4, 1)))
