@@ -783,6 +783,7 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   p.error_flag = (int*)ws;
   p.item_counter = (int*)ws + 1;
   p.row_signals = (int*)ws + 2;
+  p.unit_counter = (int*)ws + 3;
   p.desc = (StreamDesc*)(ws + l.off_desc);
   p.counts = (int*)(ws + l.off_counts);
   p.wlump = (double*)(ws + l.off_lump);

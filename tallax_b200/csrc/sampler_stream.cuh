@@ -127,6 +127,7 @@ struct StreamParams {
   int* row_signals;          // 1 once the stream kernel has decided to count them (it does when the batch has
                              // wide rows, whose final items keep it busy long after the normal rows are done)
   int* item_counter;     // [1] next unclaimed item - gridDim.x (cleared by the prologue)
+  int* unit_counter;     // [1] next unclaimed unit of the finish kernel's final pass (cleared by the prologue)
   int* error_flag;       // [1] a bounded wait of the stream kernel gave up (cleared by the prologue)
   int debug;             // diagnostic switches, 0 in normal use
 };
@@ -395,7 +396,7 @@ __global__ void __launch_bounds__(kStProThreads) sample_prologue_kernel(StreamPa
     p.desc[row] = d;
     p.rowdone[row] = 0;
     if (p.sp.out_status) p.sp.out_status[row] = 0;
-    if (row == 0) { *p.error_flag = 0; *p.item_counter = 0; *p.row_signals = 0; }
+    if (row == 0) { *p.error_flag = 0; *p.item_counter = 0; *p.row_signals = 0; *p.unit_counter = 0; }
   }
   TLX_STAMP(p.sp, 1);
 }
@@ -1288,7 +1289,7 @@ __device__ __forceinline__ int st_finish_normal(const StreamParams& p, int row, 
 
 // One row of the finish kernel's row CTAs: normal rows are finished from their candidate lists; what that
 // cannot settle takes the whole-row routines.
-static __device__ __forceinline__ void st_finish_row(const StreamParams& p, int row, unsigned char* smem);
+static __device__ __forceinline__ bool st_finish_row(const StreamParams& p, int row, unsigned char* smem);
 
 // A row that the short paths left unanswered: exact whole-row routines (out of line: rare and slow, and
 // its stack frame and register needs stay out of the callers' way).  All threads call.
@@ -1476,11 +1477,26 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
   const int nwide = ctl.cnt;
   TLX_STAMP(sp, 1);
   if (nwide == 0) return;
-  int J = p.fin_ctas / nwide;   // ranges per row
+  // ranges per row: one per CTA that takes part (those below fin_ctas and the wide rows' own ones); if that leaves a row or
+  // more to a CTA, four units of work per CTA instead, so that the last ones to finish are not far apart
+  const int workers = p.fin_ctas + nwide;
+  int J = workers / nwide;
+  if (J < 2) J = (4 * workers + nwide - 1) / nwide;
   J = J < 1 ? 1 : (J > p.nfin ? p.nfin : J);
   J = J > kStThreads ? kStThreads : J;
-  // more wide rows than CTAs: a CTA takes several rows, one after the other
-  for (int unit = blockIdx.x; unit < nwide * J; unit += p.fin_ctas) {
+  // the CTAs below fin_ctas have their first unit; the others, and all further ones, are claimed
+  const int units = nwide * J;
+  bool first = (int)blockIdx.x < p.fin_ctas;
+  int unit = blockIdx.x;
+  for (;; first = false) {
+    if (!first) {
+      if (units <= p.fin_ctas) break;
+      __syncthreads();
+      if (threadIdx.x == 0) ctl.cnt = p.fin_ctas + atomicAdd(p.unit_counter, 1);
+      __syncthreads();
+      unit = ctl.cnt;
+    }
+    if (unit >= units) break;
     const int w = unit / J, j = unit - w * J;
     const int row = wlist[w];
     WideState* ws = p.wstate + row;
@@ -1518,7 +1534,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
       const float cb = key_f32(ctl.best_key);
       const float eps = expf(-(cb - 2.0f * (kGumbelSlack + 1e-5f * fabsf(cb)) - xtop)) * 1.000001f;
       const bool arrived = mbar_wait_suspended(&ctl.mbar[slot], phase);
-      if (c == c_begin && unit == (int)blockIdx.x) TLX_STAMP(sp, 2);
+      if (c == c_begin && first) TLX_STAMP(sp, 2);
       const unsigned char* buf = ring + (size_t)slot * kFinSlotBytes;
       const float* nbuf = reinterpret_cast<const float*>(buf + kFinChunk);
       const int nvec = (c == p.nfin - 1) ? last_nvec : kFinChunk / 16;
@@ -1644,7 +1660,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
       if (threadIdx.x == 0) fin_issue(p, row, c + kFinSlots, c_end, dense != 0, ring, ctl.mbar, slot);
       if (++slot == kFinSlots) { slot = 0; phase ^= 1u; }
     }
-    if (unit == (int)blockIdx.x) TLX_STAMP(sp, 3);
+    if (first) TLX_STAMP(sp, 3);
     if (p.debug & 4) continue;
     // the range's record
     const uint32_t key = f32_key(a1);
@@ -1673,7 +1689,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
       ctl.flag = (atomicAdd(&ws->done, 1) == J - 1) ? 1 : 0;
     }
     __syncthreads();
-    if (unit == (int)blockIdx.x) TLX_STAMP(sp, 4);
+    if (first) TLX_STAMP(sp, 4);
     if (ctl.flag) {
       __threadfence();
       TLX_STAMP(sp, 6);
@@ -1684,7 +1700,8 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
   TLX_STAMP(sp, 5);
 }
 
-static __device__ __forceinline__ void st_finish_row(const StreamParams& p, int row, unsigned char* smem) {
+// Returns whether the CTA is free to take part in the final pass: a wide row's, which has only its status to report.
+static __device__ __forceinline__ bool st_finish_row(const StreamParams& p, int row, unsigned char* smem) {
   TailShared& t = *reinterpret_cast<TailShared*>(smem);
   const SampleParams& sp = p.sp;
   for (int i = threadIdx.x; i < kTlBins; i += kStThreads) t.hist[i] = 0;
@@ -1742,6 +1759,7 @@ static __device__ __forceinline__ void st_finish_row(const StreamParams& p, int 
   // this kernel must not be complete before the stream kernel is: whatever follows on the stream may reuse
   // the workspace
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  return d.cls == kStWide && !slow && p.fin_items == 0;
 }
 
 constexpr size_t kStFinishRowSmem =
@@ -1749,11 +1767,15 @@ constexpr size_t kStFinishRowSmem =
 constexpr size_t kStFinishFixedSmem =
     kStFinishRowSmem > kFinFixedSmem ? kStFinishRowSmem : kFinFixedSmem;   // + one int per row (the final pass's list)
 
-// Grid: p.fin_ctas CTAs of the final pass, then one CTA per row.
+// Grid: p.fin_ctas CTAs of the final pass, then one CTA per row.  A wide row's CTA takes part in the final pass (256 rows of
+// 128256 without top-k, noise from a key: 147 us, without them 203, with a row at a time per CTA of the 188 others 252).
 __global__ void __launch_bounds__(kStThreads, 3) sample_finish_kernel(StreamParams p, int dense) {
   extern __shared__ __align__(128) unsigned char fin_smem[];
-  if ((int)blockIdx.x < p.fin_ctas) st_final_pass(p, dense, fin_smem);
-  else st_finish_row(p, (int)blockIdx.x - p.fin_ctas, fin_smem);
+  if ((int)blockIdx.x >= p.fin_ctas) {
+    if (!st_finish_row(p, (int)blockIdx.x - p.fin_ctas, fin_smem)) return;
+    __syncthreads();
+  }
+  st_final_pass(p, dense, fin_smem);
 }
 
 }  // namespace tlx
