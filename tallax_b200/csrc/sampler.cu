@@ -800,7 +800,8 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   const size_t fin_smem = kStFinishFixedSmem + (size_t)sp.rows * sizeof(int);
   int rc;
   if ((rc = ensure_smem((const void*)sample_stream_kernel, st_smem, "sample")) != TLX_OK) return rc;
-  if ((rc = ensure_smem((const void*)sample_finish_kernel, fin_smem, "sample")) != TLX_OK) return rc;
+  const auto finish = p.fin_ctas > 0 ? sample_finish_kernel<true> : sample_finish_kernel<false>;
+  if ((rc = ensure_smem((const void*)finish, fin_smem, "sample")) != TLX_OK) return rc;
   // An SM changes its split between L1 and shared memory only while idle: the three kernels ask for the same
   // split, so that each one's CTAs can move in beside those of the one before.
   {
@@ -812,7 +813,8 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
     if (dev >= 0 && dev < 64 && !done[dev]) {
       cudaFuncSetAttribute((const void*)sample_prologue_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       cudaFuncSetAttribute((const void*)sample_stream_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-      cudaFuncSetAttribute((const void*)sample_finish_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      cudaFuncSetAttribute((const void*)sample_finish_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      cudaFuncSetAttribute((const void*)sample_finish_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       done[dev] = true;
     }
   }
@@ -831,7 +833,7 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   if ((rc = launch_dependent(sample_stream_kernel, (unsigned)sgrid, kStThreads, st_smem, st, "sample (stream)", -1, p)) != TLX_OK) return rc;
   if (stages < 3) return TLX_OK;
   TLX_TIMELINE_KERNEL(2);
-  return launch_dependent(sample_finish_kernel, (unsigned)(p.fin_ctas + sp.rows), kStThreads, fin_smem, st,
+  return launch_dependent(finish, (unsigned)(p.fin_ctas + sp.rows), kStThreads, fin_smem, st,
                           "sample (finish)", -1, p, dense);
 }
 

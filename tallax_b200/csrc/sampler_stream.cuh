@@ -1769,13 +1769,19 @@ constexpr size_t kStFinishFixedSmem =
 
 // Grid: p.fin_ctas CTAs of the final pass, then one CTA per row.  A wide row's CTA takes part in the final pass (256 rows of
 // 128256 without top-k, noise from a key: 147 us, without them 203, with a row at a time per CTA of the 188 others 252).
+// kFinalPass false: the stream kernel has taken the final items, and there are no such CTAs.
+template <bool kFinalPass>
 __global__ void __launch_bounds__(kStThreads, 3) sample_finish_kernel(StreamParams p, int dense) {
   extern __shared__ __align__(128) unsigned char fin_smem[];
-  if ((int)blockIdx.x >= p.fin_ctas) {
-    if (!st_finish_row(p, (int)blockIdx.x - p.fin_ctas, fin_smem)) return;
-    __syncthreads();
+  if constexpr (kFinalPass) {
+    if ((int)blockIdx.x >= p.fin_ctas) {
+      if (!st_finish_row(p, (int)blockIdx.x - p.fin_ctas, fin_smem)) return;
+      __syncthreads();
+    }
+    st_final_pass(p, dense, fin_smem);
+  } else {
+    st_finish_row(p, (int)blockIdx.x, fin_smem);
   }
-  st_final_pass(p, dense, fin_smem);
 }
 
 }  // namespace tlx
