@@ -216,13 +216,16 @@ static int64_t next_pow2(int64_t n) {
   return p;
 }
 
-template <int DT, int IPT, bool CL>
+template <int DT, int IPT, bool CL, bool PAST = false>
 static int launch_radix(cudaStream_t st, const void* keys, int64_t rows, int64_t n, int descending, const int32_t* in_perm,
                         void* out_keys, int32_t* out_perm, int threads, int cluster) {
   using T = typename Elem<DT>::type;
+  // the kernel has a place for every element, or it writes outside its shared memory
+  if (threads < 256 || threads > kRadixMaxThreads || threads % 32 || (int64_t)threads * IPT * cluster < n || (!CL && cluster != 1))
+    return set_error(TLX_ERR_INVALID, "sort: no kernel for rows of %lld elements (%d threads)", (long long)n, threads);
   const size_t smem = radix_smem(threads, threads * IPT, CL);
   int rc;
-  if ((rc = sort_smem((const void*)sort_radix_kernel<DT, IPT, CL>, smem)) != TLX_OK) return rc;
+  if ((rc = sort_smem((const void*)sort_radix_kernel<DT, IPT, CL, PAST>, smem)) != TLX_OK) return rc;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(rows * cluster));
   cfg.blockDim = dim3((unsigned)threads);
@@ -234,7 +237,7 @@ static int launch_radix(cudaStream_t st, const void* keys, int64_t rows, int64_t
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = CL ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, sort_radix_kernel<DT, IPT, CL>, (const T*)keys, in_perm, n, descending, (T*)out_keys, out_perm,
+  cudaError_t e = cudaLaunchKernelEx(&cfg, sort_radix_kernel<DT, IPT, CL, PAST>, (const T*)keys, in_perm, n, descending, (T*)out_keys, out_perm,
                                      cluster);
   if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "sort: %s", cudaGetErrorString(e)); }
   count_launch();
@@ -249,8 +252,10 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
   const int64_t n_pad = next_pow2(n < 2 ? 2 : n);
   int rc;
   // Up to 1024 elements the network's few stages cost less than a pass's counters (f32 [1000, 512]: 13 us against 26).
-  // A CTA per row up to 8192: eight elements a thread, sixteen where the rows fill the GPU (fewer counters per element: f32
-  // [1024, 4096] 77 us against 90).  A cluster of CTAs beyond: of 4096 elements each where all of them run at once with an
+  // A CTA per row up to 8192: eight elements a thread, which wastes the fewest places, and sixteen, which need fewer counters per
+  // element, where the rows fill the GPU and the places (4096 at least) are used (f32 with a payload, eight / sixteen:
+  // [1024, 4096] 109 us / 90, [1024, 3000] 81 / 86, [1024, 2049] 67 / 87, [1024, 1025] 45 / 80; the network 129, 124, 124, 56).
+  // A cluster of CTAs beyond: of 4096 elements each where all of them run at once with an
   // SM each (bf16 [4, 16384] 20 us, with 8192 elements 26, with one CTA per row 32), else of 8192, two to an SM, of which
   // one works while the other waits at a barrier (f32 [128, 65536] 368 us against 385 with one of 16384), which rows of
   // more than 65536 elements, eight CTAs being the most, take.
@@ -264,9 +269,11 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
       if (threads < 256) threads = 256;
       return launch_radix<DT, 16, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, cluster);
     }
-    const int ipt = n <= 8192 && rows <= 296 ? 8 : 16;
+    const int ipt = n <= (rows <= 296 ? 8192 : 3072) ? 8 : 16;
     int threads = (int)((n + 32 * ipt - 1) / (32 * ipt)) * 32;
-    if (threads < 256) threads = 256;
+    if (threads < 256) threads = 256;   // (a pass needs 256 threads for its 256 digits)
+    if (rows > 296 && n <= 2048 - 32 * 8)   // at least one warp of the 256 threads has no element
+      return launch_radix<DT, 8, false, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, 1);
     if (ipt == 8) return launch_radix<DT, 8, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, 1);
     return launch_radix<DT, 16, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, 1);
   }

@@ -52,3 +52,28 @@ def test_radix_sort_many_rows(cuda, dtype, rows, n):
     ev, ei = o.sort([x], 1, is_stable=True, return_argsort=True)
     assert np.array_equal(to_np(i), np.tile(ei, (rows // 4, 1)))
     assert exact_match(to_np(v), np.tile(ev, (rows // 4, 1)))
+
+
+# many rows in one CTA each: rows that end in the first, a middle and the last warp, inside a group of 32 and at its end
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "i32"])
+@pytest.mark.parametrize("n", [1025, 1057, 1500, 2048, 2049, 3000, 3073, 4096, 4097])
+def test_radix_sort_places_past_the_end(cuda, dtype, n):
+    rng = np.random.default_rng(n)
+    x = np.round(rng.standard_normal((4, n)).astype(np.float32) * 300)
+    x[1] = x[1, 0]
+    if dtype == "i32":
+        x = x.astype(np.int32)
+        x[2, ::5] = 2**31 - 1                                  # the key that the places past the end carry
+        x[3, ::3] = -2**31
+    else:
+        x[2, ::5] = np.nan
+        x[3, ::3] = -np.inf
+        x = x.astype({"f32": np.float32, "bf16": o.bfloat16}[dtype])
+    rows = 300
+    payload = rng.integers(0, 1 << 30, x.shape).astype(np.int32)
+    for descending in (False, True):
+        got = tax.sort([to_dev(np.tile(a, (rows // 4, 1)), cuda) for a in (x, payload)], num_keys=1, is_stable=True,
+                       return_argsort=True, descending=descending)
+        exp = o.sort([x, payload], 1, is_stable=True, return_argsort=True, descending=descending)
+        for g, e in zip(got, exp):
+            assert exact_match(to_np(g), np.tile(e, (rows // 4, 1)))
