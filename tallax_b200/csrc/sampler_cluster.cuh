@@ -14,8 +14,10 @@
 // value plus the greatest Gumbel term there is would not do.  The survivors (a handful) go to the leader, and the
 // mass above its best ones comes from one more pass over the parts, which are still in shared memory.
 //
-// Anything these lists cannot hold (huge groups of equal values, top_k > 1024), and rows without a finite maximum,
-// takes rc_slow_row: exact, any top-k, by passes over the row in global memory.
+// Rows with 1024 < top_k < vocab are cut to their top-k set in shared memory (rc_cut_parts) and then taken as rows without.
+//
+// Anything these lists cannot hold (huge groups of equal values), rows without a finite maximum, and rows longer than a
+// cluster holds take rc_slow_row: exact, any top-k, by passes over the row in global memory.
 #pragma once
 #include "row_cluster.cuh"
 
@@ -718,6 +720,153 @@ __device__ __forceinline__ void rc_masses(const RcPart<DT>& part, float xmax, fl
   z = (zs[0] + zs[1]) + (zs[2] + zs[3]);
 }
 
+// Rows with 1024 < top_k < vocab: cuts the row, which lies in the parts, to its top-K set.  What is outside the set becomes
+// -inf, and the row is then one without top-k.
+//   The K-th greatest key comes from histograms of 2048 bins, eleven bits of the key at a time (two for bf16, three for f32, in
+// `bins`); the leader adds the CTAs' bins up and tells them which one holds the K-th key.  Of keys equal to it the lowest
+// columns belong to the set: the CTAs' own counts say how many of each part.
+//   Bound by latency: three reads of the part and four or six cluster barriers, about 15 us a row.  top_k 2000, a call: bf16
+// [8, 128256] 44 us, f32 [32, 128256] 70 us (by rc_slow_row, one CTA a row over global memory, 699 and 809 us).
+template <int DT>
+static __device__ __noinline__ void rc_cut_parts(uint4* vec, int off, int n, int nvec, int K, int cluster, uint32_t rank,
+                                                 RcShared& s, uint32_t* bins) {
+  using T = typename Elem<DT>::type;
+  constexpr int VEC = 16 / (int)sizeof(T), kBits = 8 * (int)sizeof(T), kDigit = 11;
+  static_assert(1 << kDigit == kRcBins && kRcBins == 8 * kRcThreads, "eight bins a thread");
+  auto key_of = [](T v) { return Elem<DT>::key(v) >> (32 - kBits); };   // (a bf16 is told by the upper half)
+  int need = K, in_bin = 0, bin = 0, top = kBits;
+  uint32_t vk = 0;   // the K-th key's bits from `top` on
+#pragma unroll 1
+  do {
+    const int sh = top > kDigit ? top - kDigit : 0;
+    const uint32_t least = vk, width_mask = top == 32 ? 0xFFFFFFFFu : (1u << top) - 1u;
+    uint4* b4 = reinterpret_cast<uint4*>(bins);
+    b4[threadIdx.x] = make_uint4(0, 0, 0, 0);
+    b4[threadIdx.x + kRcThreads] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+#pragma unroll 1
+    for (int v = threadIdx.x; v < nvec; v += kRcThreads) {
+      const uint4 w = vec[v];
+      const T* e = reinterpret_cast<const T*>(&w);
+      uint32_t at = 0;
+      uint32_t run = 0;   // equal neighbours are added at once
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const uint32_t d = key_of(e[j]) - least;   // (below `least`: wraps to a distance beyond the range)
+        if (d <= width_mask && (unsigned)(v * VEC + j - off) < (unsigned)n) {
+          if (run && (d >> sh) != at) { atomicAdd(&bins[at], run); run = 0; }
+          at = d >> sh;
+          ++run;
+        }
+      }
+      if (run) atomicAdd(&bins[at], run);
+    }
+    cl_sync();
+    if (rank == 0) {
+      // thread t: the bins 8 t' .. 8 t' + 7, t' = 255 - t, of all CTAs
+      const int t = kRcThreads - 1 - (int)threadIdx.x;
+      uint32_t c[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 2
+      for (int r = 0; r < cluster; ++r) {
+        const uint32_t a = cl_map(bins + 8 * t, (uint32_t)r);
+        const uint4 x = cl_ld_v4(a), y = cl_ld_v4(a + 16);
+        c[0] += x.x; c[1] += x.y; c[2] += x.z; c[3] += x.w;
+        c[4] += y.x; c[5] += y.y; c[6] += y.z; c[7] += y.w;
+      }
+      int sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sum += (int)c[j];
+      int incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane_id() >= o) incl += up;
+      }
+      if (lane_id() == 31) s.red_u32[0][warp_id()] = (uint32_t)incl;
+      __syncthreads();
+#pragma unroll 1
+      for (int w = 0; w < warp_id(); ++w) incl += (int)s.red_u32[0][w];
+      if (incl - sum < need && incl >= need) {
+        int run = incl - sum, found = 0, above = 0, count = 0;
+#pragma unroll
+        for (int j = 7; j >= 0; --j) {
+          if (run < need && run + (int)c[j] >= need) { found = 8 * t + j; above = run; count = (int)c[j]; }
+          run += (int)c[j];
+        }
+#pragma unroll 1
+        for (int r = 0; r < cluster; ++r) {
+          cl_st_u32(cl_map(&s.pick[0], (uint32_t)r), (uint32_t)found);
+          cl_st_u32(cl_map(&s.pick[1], (uint32_t)r), (uint32_t)above);
+          cl_st_u32(cl_map(&s.pick[2], (uint32_t)r), (uint32_t)count);
+        }
+      }
+    }
+    cl_sync();
+    bin = s.pick[0];
+    need -= s.pick[1];
+    in_bin = s.pick[2];
+    vk |= (uint32_t)bin << sh;
+    top = sh;
+  } while (top > 0 && in_bin != need);   // (a bin that belongs to the set as a whole needs no finer look)
+
+  // elements of this part among the `need` of the last bin: `allowed` of its `mine`, those of the lowest columns
+  int mine = 0, allowed = 0;
+  if (in_bin != need) {
+    const int lane = lane_id();
+    mine = (int)bins[bin];
+    const int c = lane < cluster && lane < (int)rank ? (int)cl_ld_u32(cl_map(bins + bin, (uint32_t)lane)) : 0;
+    allowed = min(max(need - (int)__reduce_add_sync(0xFFFFFFFFu, (unsigned)c), 0), mine);
+  }
+  const bool in_order = allowed > 0 && allowed < mine;
+  const bool above_only = in_bin != need && allowed == 0;
+  int seen = 0, tog = 2;
+#pragma unroll 1
+  for (int v0 = 0; v0 < nvec; v0 += kRcThreads) {
+    const int v = v0 + threadIdx.x;
+    uint32_t keep = 0, ties = 0;
+    if (v < nvec) {
+      const uint4 w = vec[v];
+      const T* e = reinterpret_cast<const T*>(&w);
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const uint32_t k = key_of(e[j]);
+        if (above_only ? k > vk : k >= vk) keep |= 1u << j;
+        if (in_order && k == vk && (unsigned)(v * VEC + j - off) < (unsigned)n) ties |= 1u << j;
+      }
+    }
+    if (in_order) {
+      int incl = __popc(ties);
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane_id() >= o) incl += up;
+      }
+      if (lane_id() == 31) s.red_u32[tog][warp_id()] = (uint32_t)incl;
+      __syncthreads();
+      int before = seen + incl - __popc(ties);
+#pragma unroll
+      for (int u = 0; u < kRcWarps; ++u) {
+        const int c = (int)s.red_u32[tog][u];
+        before += u < warp_id() ? c : 0;
+        seen += c;
+      }
+      tog ^= 1;
+      for (uint32_t m = ties; m; m &= m - 1, ++before)
+        if (before >= allowed) keep &= ~(m & (0u - m));
+    }
+    if (v < nvec && keep != (1u << VEC) - 1u) {
+      T* e = reinterpret_cast<T*>(vec + v);
+#pragma unroll
+      for (int j = 0; j < VEC; ++j)
+        if (!(keep >> j & 1u)) {
+          if constexpr (DT == TLX_F32) e[j] = -INFINITY;
+          else e[j] = __float2bfloat16_rn(-INFINITY);
+        }
+    }
+  }
+  __syncthreads();
+}
+
 // Rows with 1 <= top_k <= 1024 and greedy rows.  Returns the token in the leader (rank 0), -1 if the row has to be
 // answered by rc_slow_row; the other CTAs return -1 when they may leave.
 template <int DT>
@@ -1005,20 +1154,23 @@ __global__ void __launch_bounds__(kRcThreads, 4) sample_cluster_kernel(const __g
   int64_t K = p.sp.top_k[row];
   if (K <= 0 || K > n) K = n;
   if (T_ < kSamplingEps) K = 1;
-  const bool wide = K >= n && n > 1 && p.part_len > 0, large = !wide && (K > kRcMaxK || p.part_len == 0);
+  const bool resident = p.part_len > 0, wide = resident && n > 1 && (K >= n || K > kRcMaxK);
   if (threadIdx.x == 0) s.n_list = 0;
   part.copy_wait();
   __syncthreads();
   TLX_STAMP(p.sp, 1);
   const int64_t col0 = (int64_t)rank * p.part_len, nrow = row + p.sp.dim0_offset;
   int tok = -1, tog = 0;
-  if (wide) tok = rc_wide_row<DT>(p, part, col0, rank, pp, T_, nrow, s, l, smem, tog);
-  else if (!large) tok = rc_normal_row<DT>(p, part, col0, rank, (int)K, pp, T_, nrow, s, l, smem, tog);
+  if (wide) {
+    if (K < n)
+      rc_cut_parts<DT>(part.vec, part.off, part.n, part.nvec, (int)K, p.cluster, rank, s, reinterpret_cast<uint32_t*>(smem + l.off_x));
+    tok = rc_wide_row<DT>(p, part, col0, rank, pp, T_, nrow, s, l, smem, tog);
+  } else if (resident) tok = rc_normal_row<DT>(p, part, col0, rank, (int)K, pp, T_, nrow, s, l, smem, tog);
   if (rank != 0) return;
-  int status = wide || large ? kStatusGeneral : 0;
+  int status = wide || !resident ? kStatusGeneral : 0;
   if (tok < 0) {
     tok = rc_slow_row<DT>(rowp, n, K, pp, T_, p.sp.noise, nrow, s);
-    status |= large ? 0 : kStatusRedone;
+    status |= resident ? kStatusRedone : 0;
   }
   if (threadIdx.x == 0) {
     p.sp.out_tokens[row] = tok;

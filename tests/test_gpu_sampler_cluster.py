@@ -39,3 +39,33 @@ def test_cluster_sampler_sizes(cuda, dtype, V, from_key):
     bad = (to_np(tok) != exp) & ~flags
     assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
     assert (to_np(status) & 2 == 0).all()
+
+
+# 1024 < top_k < vocab: the row is cut to its top-k set in the parts.  The smallest and the largest such k; one, two, eight and
+# sixteen parts; parts that end inside a vector; ties at the k-th key that lie in one part, in several and in all of them
+@pytest.mark.parametrize("V", [1026, 2049, 6000, 40961, 131072, 200003])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("from_key", [False, True])
+def test_large_top_k_sizes(cuda, dtype, V, from_key):
+    B = 10
+    x, tk, tp, T, noise = o.make_sampling_inputs(B=B, V=V, seed=V, dtype=dtype)
+    xf = x.astype(np.float32)
+    tk[:] = [1025, V - 1, 1 + V // 2, 1025, 1025, V - 1, 1 + V // 2, 1025, 1 + V // 2, 1025]
+    tk[:] = np.clip(tk, 1025, V - 1)
+    xf[2] = np.round(xf[2])
+    xf[3] = np.round(xf[3])
+    xf[4] = 0.25 * (np.arange(V) % 2)                          # two values: the ties spread over all parts
+    xf[5] = -1.0                                               # one value: all but the last column
+    xf[6, V // 3:] = -np.inf                                   # fewer finite values than k
+    xf[7] = np.sort(xf[7])                                     # the set sits in the last part
+    xf[8] = 1.0 + 1e-3 * xf[8]                                 # (nearly) one bin of the first histogram
+    xf[9, :1500] = 7.0                                         # the ties sit in the first part
+    x = xf.astype(x.dtype)
+    kw = dict(rng_key=(23, V)) if from_key else dict(noise=noise)
+    exp, flags = o.sample(x, tk, tp, T, return_flags=True, **kw)
+    dkw = dict(rng_key=(23, V)) if from_key else dict(noise=to_dev(noise, cuda))
+    tok, status = ops.sample(to_dev(x, cuda), to_dev(tk, cuda), to_dev(tp, cuda), to_dev(T, cuda), return_status=True, **dkw)
+    bad = (to_np(tok) != exp) & ~flags
+    assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
+    assert (to_np(status) & 3 == 1).all()
+    assert (to_np(status)[[0, 1, 2]] == 1).all()               # decided from the parts
