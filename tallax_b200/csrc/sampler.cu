@@ -662,14 +662,19 @@ static bool stream_path_serves(int dtype, int64_t rows, int64_t vocab, int64_t r
   return stream_layout(rows, vocab).part_chunks <= kStMaxPartChunks;
 }
 
-// Whether it is the faster one for a call that both forms serve.  The clusters' time grows with the bytes (four CTAs an
-// SM take turns of about 10 us); the stream starts from the 25 us of its three kernels and then moves more bytes per
-// second.  Where they meet depends on the parameters, which the host does not know; us stream / cluster, requests with
-// mixed parameters, with one usual top_k and without top-k: a noise tensor, [64, 128256] 30/29, 21/13, 38/32 and
-// [96, 128256] 32/38, 24/22, 51/47; a key, [32, 128256] 31/34, 20/11, 36/33 and [64, 200064] 41/56, 27/22, 66/66.
-static bool stream_path_wanted(int64_t rows, int64_t vocab, bool dense) {
-  return rows * vocab * 2 > (dense ? (16ll << 20) : (9ll << 20));
-}
+// Whether it is the faster one for a call that both forms serve.  The clusters' time grows with the bytes (four CTAs an SM
+// take turns of about 10 us); the stream starts from the 20 to 25 us of its three kernels and then moves more bytes per second.
+// Where they meet depends on the parameters, which the host does not know.  us stream / cluster, requests with mixed
+// parameters, with one usual top_k and without top-k:
+//                      a noise tensor                     a key
+//   [32, 128256]   28/26  17/13  33/31            33/33  22/12  40/42
+//   [48, 151936]   30/34  22/14  38/41            35/42  27/14  49/56
+//   [64, 128256]   31/32  22/15  39/36            37/41  26/14  56/60
+//   [256, 32000]   33/41  34/25  40/47            39/49  31/23  66/61
+//   [72, 128256]   32/34  23/22  44/41            38/41  26/20  61/58
+// Up to 16 MB the cluster form saves more on the one usual setting than it loses on mixed ones; beyond, it runs in several waves.
+// One rule for both kinds of noise: the workspace's size is asked for before the noise is known.
+static bool stream_path_wanted(int64_t rows, int64_t vocab) { return rows * vocab * 2 > (16ll << 20); }
 
 // Diagnostic switch for timing the stages of the streaming path one by one (environment variable
 // TLX_SAMPLE_STAGES = 1..3: launch only the first n kernels; +16: the stream kernel only takes the
@@ -845,7 +850,7 @@ extern "C" {
 
 size_t tlx_sample_workspace_bytes(int64_t rows, int64_t vocab) {
   if (rows <= 0 || vocab <= 0) return 0;
-  return stream_path_wanted(rows, vocab, true) ? stream_layout(rows, vocab).bytes : 256;
+  return stream_path_wanted(rows, vocab) ? stream_layout(rows, vocab).bytes : 256;
 }
 
 // Key and row offset of a call: host values or device operands (see NoiseSrc).
@@ -877,7 +882,7 @@ static int sample_impl(void* stream, const void* logits, int dtype, int64_t rows
   p.noise.dense = noise; p.noise.stride = noise_stride; p.noise.k0 = key0; p.noise.k1 = key1; p.noise.vocab = vocab;
   p.noise.key_dev = op.key_dev; p.noise.row_offset_dev = op.dim0_offset_dev;
   p.dim0_offset = dim0_offset; p.out_tokens = out_tokens; p.out_status = out_status;
-  if (stream_path_serves(dtype, rows, vocab, row_stride, logits) && stream_path_wanted(rows, vocab, noise != nullptr) &&
+  if (stream_path_serves(dtype, rows, vocab, row_stride, logits) && stream_path_wanted(rows, vocab) &&
       workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && workspace_bytes >= stream_layout(rows, vocab).bytes)
     return launch_stream_path(st, p, workspace);
 #ifdef TLX_TIMELINE

@@ -69,3 +69,29 @@ def test_large_top_k_sizes(cuda, dtype, V, from_key):
     assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
     assert (to_np(status) & 3 == 1).all()
     assert (to_np(status)[[0, 1, 2]] == 1).all()               # decided from the parts
+
+
+# A call that needs a workspace for the form it would take has it reported: more scratch than that changes nothing.  Sizes
+# around 16 MB of logits, the rule's line, and below it
+@pytest.mark.parametrize("rows,V", [(33, 128256), (40, 128256), (48, 151936), (65, 128256), (66, 128256), (120, 128256)])
+@pytest.mark.parametrize("from_key", [False, True])
+def test_workspace_reported_is_the_workspace_used(cuda, rows, V, from_key):
+    import torch
+
+    from tallax_b200 import _lib
+    lib = _lib.load()
+    gen = torch.Generator(device=cuda).manual_seed(rows)
+    x = (torch.randn((rows, V), generator=gen, device=cuda) * 3).to(torch.bfloat16)
+    tk = torch.full((rows,), 50, dtype=torch.int32, device=cuda)
+    tp, T = torch.full((rows,), 0.9, device=cuda), torch.full((rows,), 0.8, device=cuda)
+    kw = dict(rng_key=(1, 2)) if from_key else dict(noise=torch.rand((rows, V), generator=gen, device=cuda))
+    reported = lib.tlx_sample_workspace_bytes(rows, V)
+    large = ops.SampleWorkspace(rows, V, cuda)
+    large.ws = torch.empty(64 << 20, dtype=torch.uint8, device=cuda)
+    launches, tokens = [], []
+    for w in (None, ops.SampleWorkspace(rows, V, cuda), large):
+        before = lib.tlx_kernel_launches()
+        tokens.append(ops.sample(x, tk, tp, T, workspace=w, **kw).clone())
+        launches.append(lib.tlx_kernel_launches() - before)
+    assert launches == [3 if reported > 256 else 1] * 3
+    assert torch.equal(tokens[0], tokens[1]) and torch.equal(tokens[0], tokens[2])
