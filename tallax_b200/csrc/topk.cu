@@ -152,10 +152,10 @@ constexpr int kShortThreads = 128;
 constexpr int kShortCap = 1024;
 constexpr int kShortMaxK = 128;
 
-// Row traversal by 16-byte vectors: fv(vector, first column) in the aligned body, kU loads in flight per
-// thread; fs(element, column) for the unaligned head and tail.
+// Row traversal by 16-byte vectors: fv(vector, first column) in the aligned body, of which one piece of a vector per thread
+// in `sub` is read, kU loads in flight per thread; fs(element, column) for the unaligned head and tail.
 template <int DT, int kU, typename FV, typename FS>
-__device__ __forceinline__ void for_each_vec(const typename Elem<DT>::type* __restrict__ row, int64_t n, FV&& fv,
+__device__ __forceinline__ void for_each_vec(const typename Elem<DT>::type* __restrict__ row, int64_t n, int sub, FV&& fv,
                                              FS&& fs) {
   using T = typename Elem<DT>::type;
   constexpr int VEC = 16 / (int)sizeof(T);
@@ -165,7 +165,7 @@ __device__ __forceinline__ void for_each_vec(const typename Elem<DT>::type* __re
   for (int64_t c = threadIdx.x; c < head; c += blockDim.x) fs(row[c], c);
   const int64_t nvec = (n - head) / VEC;
   const uint4* vp = reinterpret_cast<const uint4*>(row + head);
-  const int64_t step = (int64_t)blockDim.x;
+  const int64_t step = (int64_t)blockDim.x * sub;
   int64_t i = threadIdx.x;
   for (; i + (int64_t)(kU - 1) * step < nvec; i += (int64_t)kU * step) {
     uint4 v[kU];
@@ -451,7 +451,8 @@ __global__ void __launch_bounds__(TH, 1024 / TH) topk_sampled_kernel(TopkParams 
   }
 }
 
-template <int DT>
+// SUB: the bound comes from one piece in SUB of the row
+template <int DT, int SUB>
 __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams p) {
   using T = typename Elem<DT>::type;
   constexpr int kSlots = GroupMax<DT>::kSlots;
@@ -480,15 +481,15 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   if (head > n) head = n;
   const int64_t nvec = (n - head) / VEC;
   bool vec_maxima = false;
-  if constexpr (DT == TLX_BF16) vec_maxima = nvec <= kShortCap * 4;
+  if constexpr (DT == TLX_BF16 && SUB == 1) vec_maxima = nvec <= kShortCap * 4;
   __nv_bfloat16* vmax = reinterpret_cast<__nv_bfloat16*>(cand);
   GroupMax<DT> gm;
   gm.init();
-  if constexpr (DT == TLX_BF16) {
+  if constexpr (DT == TLX_BF16 && SUB == 1) {
     if (vec_maxima) {
       const __nv_bfloat16 ninf = __float2bfloat16_rn(-INFINITY);
       for (int64_t i = nvec + threadIdx.x; i < ((nvec + 7) & ~(int64_t)7); i += blockDim.x) vmax[i] = ninf;
-      for_each_vec<DT, kU>(row, n,
+      for_each_vec<DT, kU>(row, n, 1,
         [&](const uint4& v, int64_t cb) {
           gm.add(v);
           const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
@@ -499,7 +500,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
     }
   }
   if (!vec_maxima)
-    for_each_vec<DT, kU>(row, n, [&](const uint4& v, int64_t) { gm.add(v); }, [&](T x, int64_t) { gm.add_one(x); });
+    for_each_vec<DT, kU>(row, n, SUB, [&](const uint4& v, int64_t) { gm.add(v); }, [&](T x, int64_t) { gm.add_one(x); });
 #pragma unroll
   for (int j = 0; j < kSlots; ++j) gkeys[threadIdx.x * kSlots + j] = (uint16_t)(f32_key(gm.slot(j)) >> 16);
   if (threadIdx.x == 0) { s.fill = 0; s.bin = 0; s.above = 0; s.refinements = 0; }
@@ -546,7 +547,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
         }
       }
     } else {
-      for_each_vec<DT, kU>(row, n,
+      for_each_vec<DT, kU>(row, n, 1,
         [&](const uint4& v, int64_t cb) {
           const __nv_bfloat162* e = reinterpret_cast<const __nv_bfloat162*>(&v);
           // __hblt2: both halves less than the bound (false when either is a NaN)
@@ -555,7 +556,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
         push_one);
     }
   } else if constexpr (DT == TLX_F16) {
-    for_each_vec<DT, kU>(row, n,
+    for_each_vec<DT, kU>(row, n, 1,
       [&](const uint4& v, int64_t cb) {
         const __half2* e = reinterpret_cast<const __half2*>(&v);
         bool any = false;
@@ -568,7 +569,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
       },
       push_one);
   } else {
-    for_each_vec<DT, kU>(row, n,
+    for_each_vec<DT, kU>(row, n, 1,
       [&](const uint4& v, int64_t cb) {
         const float* e = reinterpret_cast<const float*>(&v);
         if (!(e[0] < thr) || !(e[1] < thr) || !(e[2] < thr) || !(e[3] < thr)) note(cb);
@@ -761,11 +762,18 @@ static int launch_topk_cluster(cudaStream_t st, const TopkParams& p) {
   return TLX_OK;
 }
 
-// Whether the two-pass kernel serves a call: K <= 128 and enough rows to fill the eight CTAs per SM.
+// Whether the two-pass kernel serves a call: K <= 128, enough rows to fill the eight CTAs per SM, and
+// - rows of up to 128 KB; or
+// - 16-bit rows of more vectors than the long-row kernel numbers (1 MB), if they are more than the two per SM that the one-pass
+//   kernel reads at once.  us two-pass / one-pass, k = 20: bf16 [300, 524296] 97/160, [1024, 600000] 228/397, [592, 1200000]
+//   269/364; f16 [592, 600000] 152/215, [256, 600000] 117/108.  32-bit rows, with half the elements a byte, gain only while they
+//   are short and no whole waves (f32 [300, 300000] 94/121, [592, 327680] 160/155, [592, 1000000] 418/371).
 static bool short_rows_apply(int dtype, const TopkParams& p) {
   if (!float_rows(dtype, p) || p.k_max > kShortMaxK) return false;
   if (forced_path()) return !strcmp(forced_path(), "short");
-  return p.rows >= 256 && p.n >= 2048 && p.n * dtype_bytes(dtype) <= (128 << 10);
+  const int64_t row = p.n * dtype_bytes(dtype);
+  if (row / 16 > kSampledVecs) return p.rows > 2 * 148 && dtype != TLX_F32;
+  return p.rows >= 256 && p.n >= 2048 && row <= (128 << 10);
 }
 
 // The shared memory that `ctas` CTAs of an SM need (1 KB each is the system's), asked for once per device, and not more: what
@@ -784,16 +792,24 @@ static cudaError_t ask_shared_memory(std::mutex& mu, bool (&asked)[64], F* kerne
   return e;
 }
 
-template <int DT>
-static int launch_topk_short(cudaStream_t st, const TopkParams& p) {
+template <int DT, int SUB>
+static int launch_topk_short_from(cudaStream_t st, const TopkParams& p) {
   const size_t smem = sizeof(SelectShared);
   static std::mutex mu;
   static bool asked[64] = {};
-  cudaError_t e = ask_shared_memory(mu, asked, topk_short_kernel<DT>, smem, 1024 / kShortThreads);
+  cudaError_t e = ask_shared_memory(mu, asked, topk_short_kernel<DT, SUB>, smem, 1024 / kShortThreads);
   if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  topk_short_kernel<DT><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
+  topk_short_kernel<DT, SUB><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
   TLX_CHECK_LAUNCH("top_k (short rows)");
   return TLX_OK;
+}
+// 16-bit rows of more than 1 MB, which L2 does not keep between the passes: the bound from a quarter of the row (bf16 [1024, 600000],
+// k = 20: 228 us against 355)
+template <int DT>
+static int launch_topk_short(cudaStream_t st, const TopkParams& p) {
+  if constexpr (DT != TLX_F32)
+    if (p.n * (int64_t)sizeof(typename Elem<DT>::type) / 16 > kSampledVecs) return launch_topk_short_from<DT, 4>(st, p);
+  return launch_topk_short_from<DT, 1>(st, p);
 }
 
 template <int DT, int TH>

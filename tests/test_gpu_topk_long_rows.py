@@ -17,7 +17,9 @@ pytestmark = pytest.mark.gpu
     ("bf16", 144, 65543, 100), ("f16", 112, 65541, 128),
     ("f32", 256, 32769, 128), ("f32", 288, 40964, 1), ("bf16", 160, 65537, 128), ("f16", 256, 65541, 128),
     ("f32", 400, 20484, 128), ("bf16", 304, 81920, 64), ("f16", 608, 49201, 20),
-    ("f32", 608, 24584, 64), ("bf16", 1184, 41001, 64), ("f32", 608, 30001, 65)])
+    ("f32", 608, 24584, 64), ("bf16", 1184, 41001, 64), ("f32", 608, 30001, 65),
+    # the shortest rows that the long-row kernel does not number: the bound from a quarter of the row
+    ("bf16", 304, 524296, 64), ("f16", 304, 524299, 128), ("f32", 304, 262149, 128)])
 def test_long_row_top_k_sizes(cuda, dtype, rows, n, k):
     rng = np.random.default_rng(n)
     x = rng.standard_normal((16, n)).astype(np.float32) * 2
