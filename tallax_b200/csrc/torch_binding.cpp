@@ -6,12 +6,15 @@
 // passed on directly, outputs come from torch's caching allocator, the stream is the current one.  A function returns
 // NotImplemented for anything else, and the Python wrapper of the same name converts the arguments and calls through
 // ctypes.  The library's functions are handed over as addresses (init), so the binding links to no particular build.
+// torch translates its own exceptions (HANDLE_TH_ERRORS): a declined allocation is a torch.OutOfMemoryError, as it is
+// where the wrapper allocates.
 #include <Python.h>
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <cstring>
@@ -82,13 +85,6 @@ bool finish(int rc) {
 }
 
 #define TLX_NOT_MINE Py_RETURN_NOTIMPLEMENTED
-#define TLX_TRY try {
-#define TLX_CATCH                                          \
-  }                                                        \
-  catch (const std::exception& e) {                        \
-    PyErr_SetString(PyExc_RuntimeError, e.what());         \
-    return nullptr;                                        \
-  }
 
 bool as_i64(PyObject* o, int64_t* v) {
   if (!PyLong_CheckExact(o)) return false;
@@ -110,7 +106,7 @@ bool as_key(PyObject* o, uint32_t* k) {
 
 // sample(logits, top_k, top_p, temperature, rng_key, noise, dim0_offset) -> tokens
 PyObject* py_sample(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  TLX_TRY
+  HANDLE_TH_ERRORS
   if (n != 7) TLX_NOT_MINE;
   const int dev = device_of(a[0]);
   if (dev < 0) TLX_NOT_MINE;
@@ -143,12 +139,12 @@ PyObject* py_sample(PyObject*, PyObject* const* a, Py_ssize_t n) {
                   ws.defined() ? ws_bytes : 0);
   Py_END_ALLOW_THREADS
   return finish(rc) ? THPVariable_Wrap(tokens) : nullptr;
-  TLX_CATCH
+  END_HANDLE_TH_ERRORS
 }
 
 // top_k(x, k, k_per_row or None, replace_val or None) -> (values, indices), exact
 PyObject* py_top_k(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  TLX_TRY
+  HANDLE_TH_ERRORS
   if (n != 4) TLX_NOT_MINE;
   const int dev = device_of(a[0]);
   if (dev < 0) TLX_NOT_MINE;
@@ -183,12 +179,12 @@ PyObject* py_top_k(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PyTuple_SET_ITEM(out, 0, THPVariable_Wrap(vals));
   PyTuple_SET_ITEM(out, 1, THPVariable_Wrap(idx));
   return out;
-  TLX_CATCH
+  END_HANDLE_TH_ERRORS
 }
 
 // argsort_rows(keys, descending, in_perm or None, want_keys, want_perm) -> (keys or None, perm or None)
 PyObject* py_argsort_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  TLX_TRY
+  HANDLE_TH_ERRORS
   if (n != 5) TLX_NOT_MINE;
   const int dev = device_of(a[0]);
   if (dev < 0) TLX_NOT_MINE;
@@ -221,12 +217,12 @@ PyObject* py_argsort_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
   PyTuple_SET_ITEM(out, 0, want_keys ? THPVariable_Wrap(keys) : Py_NewRef(Py_None));
   PyTuple_SET_ITEM(out, 1, want_perm ? THPVariable_Wrap(perm) : Py_NewRef(Py_None));
   return out;
-  TLX_CATCH
+  END_HANDLE_TH_ERRORS
 }
 
 // take_along_axis(values, indices, axis) -> out
 PyObject* py_take_along_axis(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  TLX_TRY
+  HANDLE_TH_ERRORS
   if (n != 3) TLX_NOT_MINE;
   const int dev = device_of(a[0]);
   if (dev < 0) TLX_NOT_MINE;
@@ -241,12 +237,12 @@ PyObject* py_take_along_axis(PyObject*, PyObject* const* a, Py_ssize_t n) {
                            i->size(1), (int)v->element_size(), (int)axis);
   Py_END_ALLOW_THREADS
   return finish(rc) ? THPVariable_Wrap(out) : nullptr;
-  TLX_CATCH
+  END_HANDLE_TH_ERRORS
 }
 
 // cumsum(x, axis, reverse) -> out
 PyObject* py_cumsum(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  TLX_TRY
+  HANDLE_TH_ERRORS
   if (n != 3) TLX_NOT_MINE;
   const int dev = device_of(a[0]);
   if (dev < 0) TLX_NOT_MINE;
@@ -262,13 +258,13 @@ PyObject* py_cumsum(PyObject*, PyObject* const* a, Py_ssize_t n) {
   rc = lib.cumsum(st, x->data_ptr(), out.data_ptr(), x->size(0), x->size(1), dt, (int)axis, reverse);
   Py_END_ALLOW_THREADS
   return finish(rc) ? THPVariable_Wrap(out) : nullptr;
-  TLX_CATCH
+  END_HANDLE_TH_ERRORS
 }
 
 // exchange_step(logits_shard, col_offset, vocab_total, rng_key, noise_shard, dim0_offset, k_cand, rank, world, peers
 // (address of the array of the ranks' buffers), own buffer, status, top_k, top_p, temperature, out or None) -> tokens
 PyObject* py_exchange_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
-  TLX_TRY
+  HANDLE_TH_ERRORS
   if (n != 16) TLX_NOT_MINE;
   const int dev = device_of(a[0]);
   if (dev < 0) TLX_NOT_MINE;
@@ -310,7 +306,7 @@ PyObject* py_exchange_step(PyObject*, PyObject* const* a, Py_ssize_t n) {
   Py_END_ALLOW_THREADS
   if (!finish(rc)) return nullptr;
   return given ? Py_NewRef(a[15]) : THPVariable_Wrap(tokens);
-  TLX_CATCH
+  END_HANDLE_TH_ERRORS
 }
 
 // init(check, {name: address})

@@ -45,3 +45,28 @@ def test_errors_keep_their_classes(cuda):
         tax.cumsum(x.half(), 1)
     with pytest.raises(ValueError):
         tumpy.take_along_axis(x, torch.zeros((3, 2), dtype=torch.int32, device=cuda), 1)
+
+
+@pytest.mark.parametrize("op", ["sample", "top_k", "sort", "take_along_axis", "cumsum"])
+def test_declined_allocation_is_torchs_own_error(cuda, op):
+    x = torch.zeros((128, 1 << 17), device=cuda)               # 64 MB; every call below wants more than 8 MB
+    index = torch.zeros((128, 1 << 17), dtype=torch.int32, device=cuda)
+    md = sampling.SamplingMetadata(torch.full((1024,), 5, dtype=torch.int32, device=cuda), torch.ones(1024, device=cuda),
+                                   torch.ones(1024, device=cuda))
+    logits = torch.zeros((1024, 1 << 15), dtype=torch.bfloat16, device=cuda)
+    call = {"sample": lambda: sampling.sample((1, 2), logits, md),
+            "top_k": lambda: tax.top_k(x.reshape(-1, 1 << 11), 1 << 11, block_token=1),
+            "sort": lambda: tax.sort([x], num_keys=1),
+            "take_along_axis": lambda: tumpy.take_along_axis(x, index, 1),
+            "cumsum": lambda: tax.cumsum(x, 1)}[op]
+    call()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(cuda).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (1 << 20)) / total)
+    try:
+        with pytest.raises(torch.OutOfMemoryError):
+            call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    call()
