@@ -594,23 +594,6 @@ __global__ void __launch_bounds__(256) gumbel_argmax_kernel(const float* __restr
   }
 }
 
-// Raises a kernel's dynamic shared memory limit once per (kernel, device).
-static int ensure_smem(const void* func, size_t bytes, const char* what) {
-  struct Entry { const void* func; int dev; size_t bytes; };
-  static Entry cache[256];
-  static int used = 0;
-  static std::mutex mu;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  for (int i = 0; i < used; ++i)
-    if (cache[i].func == func && cache[i].dev == dev && cache[i].bytes >= bytes) return TLX_OK;
-  cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "%s: cudaFuncSetAttribute(%zu): %s", what, bytes, cudaGetErrorString(e));
-  if (used < 256) cache[used++] = Entry{func, dev, bytes};
-  return TLX_OK;
-}
-
 static int device_sm_count() {
   static int cached[64];
   int dev = 0;
@@ -736,8 +719,9 @@ static int launch_cluster_path(cudaStream_t st, const SampleParams& sp) {
   size_t part_bytes = (size_t)p.part_len * es + 32;
   if (part_bytes < kRcMinPartBytes) part_bytes = kRcMinPartBytes;
   const size_t smem = RcLayout(p.cluster, true).off_part + part_bytes;
+  static SmemLimit limit;
   int rc;
-  if ((rc = ensure_smem((const void*)sample_cluster_kernel<DT>, smem, "sample")) != TLX_OK) return rc;
+  if ((rc = raise_smem(limit, (const void*)sample_cluster_kernel<DT>, smem, "sample")) != TLX_OK) return rc;
   {
     static std::mutex mu;
     static bool done[64] = {};
@@ -803,10 +787,11 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   const int64_t items = sp.rows * (int64_t)l.P;
   const size_t st_smem = kStFixedSmem + (size_t)sp.rows * 6;   // descriptor word and order entry per row
   const size_t fin_smem = kStFinishFixedSmem + (size_t)sp.rows * sizeof(int);
+  static SmemLimit stream_limit, finish_limits[2];
   int rc;
-  if ((rc = ensure_smem((const void*)sample_stream_kernel, st_smem, "sample")) != TLX_OK) return rc;
+  if ((rc = raise_smem(stream_limit, (const void*)sample_stream_kernel, st_smem, "sample")) != TLX_OK) return rc;
   const auto finish = p.fin_ctas > 0 ? sample_finish_kernel<true> : sample_finish_kernel<false>;
-  if ((rc = ensure_smem((const void*)finish, fin_smem, "sample")) != TLX_OK) return rc;
+  if ((rc = raise_smem(finish_limits[p.fin_ctas > 0], (const void*)finish, fin_smem, "sample")) != TLX_OK) return rc;
   // An SM changes its split between L1 and shared memory only while idle: the three kernels ask for the same
   // split, so that each one's CTAs can move in beside those of the one before.
   {
@@ -1032,8 +1017,9 @@ static int launch_merge(cudaStream_t st, const MergeParams& p, int64_t rows) {
   int P = 2;
   while (P < p.n_cand) P <<= 1;
   const size_t smem = kSharedHeader + (size_t)P * 8 + (size_t)p.n_cand * 12;   // candidates, merged order, list
+  static SmemLimit limit;
   int rc;
-  if ((rc = ensure_smem((const void*)merge_and_sample_kernel, smem, "merge_and_sample")) != TLX_OK) return rc;
+  if ((rc = raise_smem(limit, (const void*)merge_and_sample_kernel, smem, "merge_and_sample")) != TLX_OK) return rc;
   // one thread per two (padded) candidates: the sort's stages pair them up, the tail takes two items per thread
   int threads = P / 2;
   threads = threads < 64 ? 64 : (threads > kMergeThreads ? kMergeThreads : threads);

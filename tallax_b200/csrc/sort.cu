@@ -192,24 +192,6 @@ __global__ void __launch_bounds__(kSortThreads) sort_near_kernel(
   }
 }
 
-// Raises a kernel's dynamic shared memory limit once per (kernel, device).
-static int sort_smem(const void* func, size_t bytes) {
-  if (bytes <= 48 * 1024) return TLX_OK;
-  struct Entry { const void* func; int dev; size_t bytes; };
-  static Entry cache[64];
-  static int used = 0;
-  static std::mutex mu;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  std::lock_guard<std::mutex> lock(mu);
-  for (int i = 0; i < used; ++i)
-    if (cache[i].func == func && cache[i].dev == dev && cache[i].bytes >= bytes) return TLX_OK;
-  cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-  if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "sort: cudaFuncSetAttribute(%zu): %s", bytes, cudaGetErrorString(e));
-  if (used < 64) cache[used++] = Entry{func, dev, bytes};
-  return TLX_OK;
-}
-
 static int64_t next_pow2(int64_t n) {
   int64_t p = 1;
   while (p < n) p <<= 1;
@@ -224,8 +206,9 @@ static int launch_radix(cudaStream_t st, const void* keys, int64_t rows, int64_t
   if (threads < 256 || threads > kRadixMaxThreads || threads % 32 || (int64_t)threads * IPT * cluster < n || (!CL && cluster != 1))
     return set_error(TLX_ERR_INVALID, "sort: no kernel for rows of %lld elements (%d threads)", (long long)n, threads);
   const size_t smem = radix_smem(threads, threads * IPT, CL);
+  static SmemLimit limit;
   int rc;
-  if ((rc = sort_smem((const void*)sort_radix_kernel<DT, IPT, CL, PAST>, smem)) != TLX_OK) return rc;
+  if ((rc = raise_smem(limit, (const void*)sort_radix_kernel<DT, IPT, CL, PAST>, smem, "sort")) != TLX_OK) return rc;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(rows * cluster));
   cfg.blockDim = dim3((unsigned)threads);
@@ -280,7 +263,8 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
   if (n_pad <= kTile) {
     int threads = (int)(n_pad / 8);
     threads = threads < 64 ? 64 : (threads > kSortThreads ? kSortThreads : threads);
-    if ((rc = sort_smem((const void*)sort_small_kernel<DT>, padded_bytes((size_t)n_pad))) != TLX_OK) return rc;
+    static SmemLimit limit;
+    if ((rc = raise_smem(limit, (const void*)sort_small_kernel<DT>, padded_bytes((size_t)n_pad), "sort")) != TLX_OK) return rc;
     sort_small_kernel<DT><<<(unsigned)rows, threads, padded_bytes((size_t)n_pad), st>>>(
         (const T*)keys, in_perm, n, (int)n_pad, descending, (T*)out_keys, out_perm);
     TLX_CHECK_LAUNCH("sort (single tile)");
@@ -292,8 +276,9 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
   uint64_t* ws = (uint64_t*)workspace;
   const unsigned tiles = (unsigned)(rows * (n_pad / kTile));
   const size_t smem = padded_bytes((size_t)kTile);
-  if ((rc = sort_smem((const void*)sort_tiles_kernel<DT>, smem)) != TLX_OK) return rc;
-  if ((rc = sort_smem((const void*)sort_near_kernel<DT>, smem)) != TLX_OK) return rc;
+  static SmemLimit tiles_limit, near_limit;
+  if ((rc = raise_smem(tiles_limit, (const void*)sort_tiles_kernel<DT>, smem, "sort")) != TLX_OK) return rc;
+  if ((rc = raise_smem(near_limit, (const void*)sort_near_kernel<DT>, smem, "sort")) != TLX_OK) return rc;
   sort_tiles_kernel<DT><<<tiles, kSortThreads, smem, st>>>((const T*)keys, in_perm, n, n_pad, descending, ws);
   TLX_CHECK_LAUNCH("sort (tiles)");
   auto far_blocks = [&](int nsub) {

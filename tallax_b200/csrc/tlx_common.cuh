@@ -10,6 +10,7 @@
 #include <cstdio>
 
 #include "../../include/tallax_b200.h"
+#include "smem_limit.h"
 
 namespace tlx {
 
@@ -29,6 +30,16 @@ void count_launch();   // bumps the process-wide launch counter read by tlx_kern
     if (e_ != cudaSuccess)                                                             \
       return ::tlx::set_error(TLX_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e_));    \
   } while (0)
+
+// Lets `func` be launched with `bytes` of dynamic shared memory on the current device.
+inline int raise_smem(SmemLimit& limit, const void* func, size_t bytes, const char* what) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return limit.raise(dev, bytes, [&](size_t b) {
+    const cudaError_t e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b);
+    return e == cudaSuccess ? TLX_OK : set_error(TLX_ERR_CUDA, "%s: cudaFuncSetAttribute(%zu): %s", what, b, cudaGetErrorString(e));
+  });
+}
 
 inline int dtype_bytes(int dtype) {
   switch (dtype) {
