@@ -99,8 +99,11 @@ int tlx_argmax(void* stream, const void* keys, int dtype, int64_t rows, int64_t 
  * with it (least-significant-key-first chaining gives multi-key sorts).
  * out_keys (nullable): the sorted keys, canonicalised (-0 -> +0, one NaN).
  * out_perm (nullable): int32 source column of every output position.
+ * workspace: rows of up to TLX_SORT_NO_WORKSPACE_N elements need none (NULL, 0), longer ones
+ * tlx_sort_workspace_bytes(rows, n), which reports rows * next_pow2(n) * 8 for every n > 16384.
  * Replaces tallax/_src/sort.py:559-571 and :740-758 (the VMEM sort and the HBM
  * substage kernels behind `sort`, sort.py:768-929).                                 */
+#define TLX_SORT_NO_WORKSPACE_N 131072
 size_t tlx_sort_workspace_bytes(int64_t rows, int64_t n);
 int tlx_sort(void* stream, const void* keys, int dtype, int64_t rows, int64_t n, int descending,
              const int32_t* in_perm, void* out_keys, int32_t* out_perm, void* workspace,
@@ -113,8 +116,8 @@ int tlx_sort(void* stream, const void* keys, int dtype, int64_t rows, int64_t n,
  * for them).  The
  * scratch of the multi-tile path is a fixed area inside the library image (16 MiB, reported by
  * tlx_sort_static_max_bytes; every GPU that loads the library holds it until exit).
- *   - rows whose composites need more than that are rejected with TLX_ERR_INVALID and a
- *     message; nothing is launched;
+ *   - problems for which tlx_sort_workspace_bytes reports more than that are rejected with
+ *     TLX_ERR_INVALID and a message; nothing is launched;
  *   - the first call on a device looks up the area's device address (with that device
  *     current), a host-side query; later calls only launch kernels;
  *   - all calls share the one area and it keeps the previous call's contents; the kernels

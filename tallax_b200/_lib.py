@@ -13,6 +13,7 @@ LIB_PATH = os.path.join(_HERE, "lib", "libtallax_b200.so")
 TLX_F32, TLX_BF16, TLX_I32, TLX_F16, TLX_U32 = 0, 1, 2, 3, 4
 TLX_OK, TLX_ERR_INVALID, TLX_ERR_UNSUPPORTED, TLX_ERR_WORKSPACE, TLX_ERR_CUDA = 0, -1, -2, -3, -4
 TOPK_MAX_K = 2048
+SORT_NO_WORKSPACE_N = 131072
 
 _vp, _i64, _i32, _u32, _f32, _f64, _sz = (C.c_void_p, C.c_int64, C.c_int, C.c_uint32, C.c_float, C.c_double,
                                           C.c_size_t)

@@ -164,10 +164,9 @@ def argsort_rows(keys: torch.Tensor, descending: bool = False, in_perm: torch.Te
     lib = _lib.load()
     out_keys = torch.empty_like(keys) if want_keys else None
     out_perm = torch.empty((rows, n), dtype=torch.int32, device=keys.device) if want_perm else None
-    nbytes = lib.tlx_sort_workspace_bytes(rows, n)
-    ws = _ws(nbytes, keys.device)
+    ws = _ws(lib.tlx_sort_workspace_bytes(rows, n), keys.device) if n > _lib.SORT_NO_WORKSPACE_N else None
     check(lib.tlx_sort(_stream(), _ptr(keys), dtype_code(keys), rows, n, int(bool(descending)), _ptr(in_perm),
-                       _ptr(out_keys), _ptr(out_perm), _ptr(ws), ws.numel()))
+                       _ptr(out_keys), _ptr(out_perm), _ptr(ws), ws.numel() if ws is not None else 0))
     return out_keys, out_perm
 
 

@@ -192,6 +192,8 @@ __global__ void __launch_bounds__(kSortThreads) sort_near_kernel(
   }
 }
 
+static_assert(TLX_SORT_NO_WORKSPACE_N == kRadixMaxRow, "rows that the radix sort serves need no workspace");
+
 static int64_t next_pow2(int64_t n) {
   int64_t p = 1;
   while (p < n) p <<= 1;
@@ -313,6 +315,8 @@ using namespace tlx;
 
 extern "C" {
 
+// (What callers were told before rows of up to TLX_SORT_NO_WORKSPACE_N elements were sorted without a workspace: the limit of
+// tlx_sort_static and the sizes that programs have recorded stay what they were.)
 size_t tlx_sort_workspace_bytes(int64_t rows, int64_t n) {
   if (rows <= 0 || n <= 0) return 0;
   const int64_t n_pad = next_pow2(n < 2 ? 2 : n);

@@ -202,7 +202,7 @@ PyObject* py_argsort_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
   at::Tensor keys, perm, ws;
   if (want_keys) keys = empty({rows, cols}, x->scalar_type(), dev);
   if (want_perm) perm = empty({rows, cols}, at::kInt, dev);
-  const size_t ws_bytes = lib.sort_workspace_bytes(rows, cols);
+  const size_t ws_bytes = cols > TLX_SORT_NO_WORKSPACE_N ? lib.sort_workspace_bytes(rows, cols) : 0;
   if (ws_bytes) ws = empty({(int64_t)ws_bytes}, at::kByte, dev);
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
   int rc;

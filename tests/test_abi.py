@@ -118,3 +118,9 @@ def test_exchange_layout_and_argument_errors_need_no_gpu():
     assert rc == _lib.TLX_ERR_INVALID
     rc = lib.tlx_exchange_merge_and_sample(None, None, 4, 1024, 16, None, None, None, None, None)
     assert rc == _lib.TLX_ERR_UNSUPPORTED
+
+
+def test_sort_without_workspace_ends_where_the_header_says():
+    text = open(os.path.join(ROOT, "include", "tallax_b200.h")).read()
+    assert f"#define TLX_SORT_NO_WORKSPACE_N {_lib.SORT_NO_WORKSPACE_N}\n" in text
+    assert f"#define TLX_TOPK_MAX_K {_lib.TOPK_MAX_K}\n" in text

@@ -77,3 +77,25 @@ def test_radix_sort_places_past_the_end(cuda, dtype, n):
         exp = o.sort([x, payload], 1, is_stable=True, return_argsort=True, descending=descending)
         for g, e in zip(got, exp):
             assert exact_match(to_np(g), np.tile(e, (rows // 4, 1)))
+
+
+# no scratch is allocated that no kernel touches, by the binding or by the wrapper behind it; beyond 131072 elements it is needed
+@pytest.mark.parametrize("strided", [False, True])
+@pytest.mark.parametrize("rows,n,copies", [(64, 65536, 0), (32, 131072, 0), (8, 131073, 4)])
+def test_sort_allocates_what_it_uses(cuda, rows, n, copies, strided):
+    import torch
+
+    from tallax_b200._src import ops
+    x = torch.randn((rows, n), device=cuda)
+    if strided:
+        x = x.t().contiguous().t()
+    one = rows * n * 4
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    keys, perm = ops.argsort_rows(x)
+    used = torch.cuda.max_memory_allocated() - before
+    # keys, permutation, the contiguous copy of a strided operand, and the composites (8 bytes each, padded to a power of two)
+    assert (2 + strided + copies) * one <= used + 4096 and used <= (2 + strided + copies) * one * 1.01 + (1 << 20)
+    assert np.array_equal(to_np(perm), np.argsort(to_np(x), axis=1, kind="stable"))
