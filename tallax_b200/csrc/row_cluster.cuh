@@ -26,7 +26,6 @@ constexpr int kRcMaxPart = 49152;        // elements of a part (positions are 16
 
 // ---- cluster primitives -----------------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cl_rank() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r)); return r; }
-__device__ __forceinline__ uint32_t cl_size() { uint32_t r; asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r)); return r; }
 __device__ __forceinline__ void cl_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cl_sync() { cl_arrive(); cl_wait(); }
@@ -51,14 +50,8 @@ __device__ __forceinline__ void cl_st_u64(uint32_t addr, uint32_t lo, uint32_t h
 }
 __device__ __forceinline__ void cl_st_u32(uint32_t a, uint32_t v) { asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory"); }
 __device__ __forceinline__ void cl_st_f32(uint32_t a, float v) { cl_st_u32(a, __float_as_uint(v)); }
-__device__ __forceinline__ void cl_st_u64(uint32_t a, uint64_t v) { asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory"); }
 __device__ __forceinline__ void cl_st_f64(uint32_t a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
 __device__ __forceinline__ float cl_ld_f32(uint32_t a) { return __uint_as_float(cl_ld_u32(a)); }
-__device__ __forceinline__ double cl_ld_f64(uint32_t a) {
-  double v;
-  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
-  return v;
-}
 __device__ __forceinline__ uint4 cl_ld_v4(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
@@ -139,8 +132,6 @@ struct __align__(16) RcShared {
   uint32_t key_lo, key_hi;              // range of the candidates' keys (from the bound's search)
   int n_near;
   unsigned long long win;               // winner of a round of the decision
-  float win_x;
-  int fail;
 };
 
 // The dynamic shared memory of a CTA: state, the bound's words, the candidate list (position inside the part, value,
@@ -166,14 +157,6 @@ __device__ __forceinline__ uint32_t rc_max_u32(uint32_t v, RcShared& s, int& tog
   if (lane_id() == 0) s.red_u32[tog][warp_id()] = v;
   __syncthreads();
   v = __reduce_max_sync(0xFFFFFFFFu, s.red_u32[tog][lane_id() & (kRcWarps - 1)]);
-  tog ^= 1;
-  return v;
-}
-__device__ __forceinline__ uint32_t rc_sum_u32(uint32_t v, RcShared& s, int& tog) {
-  v = __reduce_add_sync(0xFFFFFFFFu, v);
-  if (lane_id() == 0) s.red_u32[tog][warp_id()] = v;
-  __syncthreads();
-  v = __reduce_add_sync(0xFFFFFFFFu, lane_id() < kRcWarps ? s.red_u32[tog][lane_id()] : 0u);
   tog ^= 1;
   return v;
 }

@@ -143,7 +143,7 @@ __device__ __forceinline__ uint32_t bf16_key16(uint32_t b) {
 __device__ __forceinline__ uint32_t key16_bf16_bits(uint32_t k) { return (k & 0x8000u) ? (k & 0x7FFFu) : (~k & 0xFFFFu); }
 __device__ __forceinline__ __nv_bfloat162 bf162_splat_bits(uint32_t b16) { return bf162_bits(b16 | (b16 << 16)); }
 // mbarrier wait that lets the hardware suspend the thread for up to about a microsecond per attempt
-// instead of spinning on the issue slots; bounded like mbar_wait.
+// instead of spinning on the issue slots.  Bounded: returns false if the barrier did not complete within 2^20 attempts.
 __device__ __forceinline__ bool mbar_wait_suspended(unsigned long long* bar, uint32_t parity) {
   for (uint32_t i = 0; i < (1u << 20); ++i) {
     uint32_t ok;

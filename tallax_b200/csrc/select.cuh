@@ -34,8 +34,6 @@ struct SelectShared {
   int above;      // elements in bins > B at the last refinement
   int refinements;
   int tmp_i[4];
-  unsigned long long tmp_u64[2];
-  float tmp_f[4];
 };
 
 // Real value at the lower edge of histogram bin b, clamped so that it is never a NaN

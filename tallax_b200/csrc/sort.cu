@@ -1,18 +1,16 @@
-// Stable row-wise argsort: bitonic network on 64-bit composites (key << 32 | position).
+// Stable row-wise argsort, by the length of the rows:
+//   up to 1024 elements       bitonic network on 64-bit composites (key << 32 | position) in the shared memory of one CTA
+//   up to 131072              radix sort in the shared memory of a CTA or of a cluster of CTAs (sort_radix.cuh)
+//   beyond                    the network on composites in the caller's workspace, in tiles of kTile elements
 //
-// The position in the low word makes every composite unique, so the (unstable) bitonic
-// network yields the stable order, and one u64 compare is the whole lexicographic test.
-// Rows up to kTile elements are sorted entirely in shared memory by one CTA.  Longer
-// rows keep the composites in the caller's workspace (L2-resident for the sizes of
-// interest): tiles are sorted in shared memory, every merge stage then runs its far
-// substages (partner distance >= kTile) over the workspace and its near substages in
+// The network.  The position in the low word makes every composite unique, so the (unstable) bitonic network yields the
+// stable order, and one u64 compare is the whole lexicographic test.  In the workspace, tiles are sorted in shared memory;
+// every merge stage then runs its far substages (partner distance >= kTile) over the workspace and its near substages in
 // shared memory again.
-// Substages are taken three at a time wherever possible: a thread brings eight elements
-// (spaced by the smallest of the three distances) into registers, does the twelve
-// compare-exchanges there and writes them back, which divides the shared-memory (or workspace)
-// traffic and the barriers by three.
+//   Substages are taken three at a time wherever possible: a thread brings eight elements (spaced by the smallest of the
+// three distances) into registers, does the twelve compare-exchanges there and writes them back, which divides the
+// shared-memory (or workspace) traffic and the barriers by three.
 #include <mutex>
-
 #include <type_traits>
 
 #include "sort_radix.cuh"
@@ -20,6 +18,7 @@
 namespace tlx {
 
 constexpr int kTile = 16384;    // composites per shared-memory tile (128 KB)
+constexpr int kSmallRow = 1024; // elements of a row at most that the network takes in one CTA
 constexpr int kSortThreads = 1024;
 constexpr uint64_t kPad = ~0ull;
 
@@ -110,7 +109,7 @@ __device__ __forceinline__ void emit(uint64_t v, int64_t c, int64_t n, bool desc
   if (operm) operm[c] = prow ? prow[pos] : pos;
 }
 
-// Whole row in one tile: build, sort, emit.  n_pad (power of two) <= kTile.
+// Whole row in one tile: build, sort, emit.  n_pad (power of two) <= kSmallRow.
 template <int DT>
 __global__ void __launch_bounds__(kSortThreads) sort_small_kernel(
     const typename Elem<DT>::type* __restrict__ keys, const int32_t* __restrict__ in_perm, int64_t n, int n_pad,
@@ -244,7 +243,7 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
   // SM each (bf16 [4, 16384] 20 us, with 8192 elements 26, with one CTA per row 32), else of 8192, two to an SM, of which
   // one works while the other waits at a barrier (f32 [128, 65536] 368 us against 385 with one of 16384), which rows of
   // more than 65536 elements, eight CTAs being the most, take.
-  if (n > 1024 && n <= kRadixMaxRow) {
+  if (n > kSmallRow && n <= kRadixMaxRow) {
     if (n > kRadixTile) {
       int cluster = (int)((n + 4095) / 4096);
       if (cluster > 8 || rows * cluster > 148) cluster = (int)((n + kRadixTile - 1) / kRadixTile);
@@ -262,11 +261,10 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
     if (ipt == 8) return launch_radix<DT, 8, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, 1);
     return launch_radix<DT, 16, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, 1);
   }
-  if (n_pad <= kTile) {
+  if (n <= kSmallRow) {
     int threads = (int)(n_pad / 8);
-    threads = threads < 64 ? 64 : (threads > kSortThreads ? kSortThreads : threads);
-    static SmemLimit limit;
-    if ((rc = raise_smem(limit, (const void*)sort_small_kernel<DT>, padded_bytes((size_t)n_pad), "sort")) != TLX_OK) return rc;
+    if (threads < 64) threads = 64;
+    static_assert(padded_bytes(kSmallRow) <= 48 * 1024, "no limit has to be raised");
     sort_small_kernel<DT><<<(unsigned)rows, threads, padded_bytes((size_t)n_pad), st>>>(
         (const T*)keys, in_perm, n, (int)n_pad, descending, (T*)out_keys, out_perm);
     TLX_CHECK_LAUNCH("sort (single tile)");

@@ -104,12 +104,6 @@ template <> struct Elem<TLX_U32> {
 __device__ __forceinline__ int lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ int warp_id() { return threadIdx.x >> 5; }
 
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-  return v;
-}
 __device__ __forceinline__ double shfl_up_f64(double v, int d) {
   int lo = __double2loint(v), hi = __double2hiint(v);
   lo = __shfl_up_sync(0xFFFFFFFFu, lo, d);
@@ -156,9 +150,7 @@ __device__ __forceinline__ T block_scan_incl(T v, T* scratch, T* total, ShflUp s
   __syncthreads();
   return v + base;
 }
-struct ShflUpI32 { __device__ int operator()(int v, int d) const { return __shfl_up_sync(0xFFFFFFFFu, v, d); } };
 struct ShflUpU32 { __device__ uint32_t operator()(uint32_t v, int d) const { return __shfl_up_sync(0xFFFFFFFFu, v, d); } };
-struct ShflUpF32 { __device__ float operator()(float v, int d) const { return __shfl_up_sync(0xFFFFFFFFu, v, d); } };
 struct ShflUpF64 { __device__ double operator()(double v, int d) const { return shfl_up_f64(v, d); } };
 
 // ---- in-shared-memory bitonic sort of `n` (power of two) u64 items, ascending -----
@@ -217,11 +209,7 @@ static __device__ __noinline__ float gumbel_exact(float u) {
   double d = (double)fmaxf(u, kF32Tiny);
   return (float)(-log(-log(d)));
 }
-// Screening form, f32; |gumbel_fast - gumbel_exact| is far below kGumbelSlack.
-__device__ __forceinline__ float gumbel_fast(float u) {
-  return -logf(-logf(fmaxf(u, kF32Tiny)));
-}
-// Cheapest screening form: hardware log2 for both logs.  -log(u) loses relative accuracy as u -> 1,
+// Screening form, far within kGumbelSlack of the exact one: hardware log2 for both logs.  -log(u) loses relative accuracy as u -> 1,
 // so the last percent takes the series of -log(1 - d), d = 1 - u (exact in f32), to the fourth
 // order (relative error below 1e-8); elsewhere the absolute error of the result stays below 5e-5.
 // Branch-free: a rare slow branch would be paid by the whole warp.
