@@ -634,19 +634,14 @@ __global__ void __launch_bounds__(kRcThreads, 4) topk_cluster_kernel(const __gri
   if (threadIdx.x == 0) s.n_list = 0;
   part.copy_wait();
   __syncthreads();
-  float thr = -INFINITY;
-  if (p.n > kRcListCap) {
-    uint32_t* bound = reinterpret_cast<uint32_t*>(smem + l.off_bound);
-    GroupMax<DT> gm;
-    gm.init();
+  uint32_t* bound = reinterpret_cast<uint32_t*>(smem + l.off_bound);
+  GroupMax<DT> gm;
+  gm.init();
 #pragma unroll 2
-    for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) gm.add(part.vec[v]);
-    rc_publish_maxima<DT>(gm, l.bound_words, bound);
-    cl_sync();
-    thr = key_f32(rc_bound_key16(bound, l.bound_words, K, s) << 16);
-  } else {
-    cl_sync();
-  }
+  for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) gm.add(part.vec[v]);
+  rc_publish_maxima<DT>(gm, l.bound_words, bound);
+  cl_sync();
+  const float thr = key_f32(rc_bound_key16(bound, l.bound_words, K, s) << 16);
   rc_filter<DT>(part, thr, s, lx, lpos);
   cl_sync();
   if (rank != 0) {
@@ -714,11 +709,12 @@ static bool long_rows_apply(int dtype, const TopkParams& p) {
   return row > (80 << 10) && all > ((p.rows > 4 * 148 ? 70ll : 30ll) << 20);
 }
 
-// Whether the cluster form serves a call: fewer rows than the kernels with a CTA per row want, rows that a cluster holds, and
-// not more than 64 MB, beyond which several waves of clusters take longer than the one-pass kernel.
+// Whether the cluster form serves a call: fewer rows than the kernels with a CTA per row want, rows that a cluster holds and that
+// are longer than a candidate list (all elements of a shorter row would be candidates, to be sorted: f16 [95, 1365], k = 4 25 us,
+// by the one-pass kernel 7), and not more than 64 MB, beyond which several waves of clusters take longer than the one-pass kernel.
 static bool cluster_rows_apply(int dtype, const TopkParams& p) {
   if (!float_rows(dtype, p) || p.k_max > kRcMaxK || forced_path() || long_rows_apply(dtype, p)) return false;
-  return p.rows < 256 && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart && p.rows * p.n * dtype_bytes(dtype) <= (64ll << 20);
+  return p.rows < 256 && p.n > kRcListCap && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart && p.rows * p.n * dtype_bytes(dtype) <= (64ll << 20);
 }
 
 template <int DT>
