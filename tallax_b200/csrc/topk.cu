@@ -711,10 +711,26 @@ static bool long_rows_apply(int dtype, const TopkParams& p) {
 
 // Whether the cluster form serves a call: fewer rows than the kernels with a CTA per row want, rows that a cluster holds and that
 // are longer than a candidate list (all elements of a shorter row would be candidates, to be sorted: f16 [95, 1365], k = 4 25 us,
-// by the one-pass kernel 7), and not more than 64 MB, beyond which several waves of clusters take longer than the one-pass kernel.
+// by the one-pass kernel 7), and, by the number of candidates that the leader has to order, against the one-pass kernel:
+// - k <= 128: not more than 64 MB, beyond which the clusters' several waves take longer
+// - k <= 200 (up to 256 candidates, ordered by counting): not more than 40 MB (us cluster / one-pass, f32, k = 200: [255, 32768]
+//   32/35, [255, 65536] 53/47)
+// - k <= 440 (512 in the bitonic network): rows of at least 12000 elements, not more than 16 MB, 40 MB of 16-bit ones (k = 300:
+//   [1, 8192] 14.0/12.7, [255, 8192] 22/17, [1, 12000] 14.4/16.8, [255, 16384] 26/27, [148, 32768] 30/29; bf16, k = 256:
+//   [255, 65536] 43/47)
+// - above: a few rows that are long enough for the leader's network not to matter (k = 1024: [1, 16384] 31/30, [1, 32768] 33/38,
+//   [32, 32768] 42/39, [32, 65536] 45/52, [148, 65536] 89/54; k = 512: [1, 12000] 20/20, [32, 32768] 24/29, [148, 32768] 39/33)
+static bool cluster_order_pays(int64_t rows, int64_t n, int k, int elem_bytes) {
+  const int64_t bytes = rows * n * elem_bytes;
+  if (k <= kShortMaxK) return bytes <= (64ll << 20);
+  if (k <= 200) return bytes <= (40ll << 20);
+  if (k <= 440) return n >= 12000 && bytes <= ((elem_bytes == 2 ? 40ll : 16ll) << 20);
+  return rows <= 64 && n >= (rows <= 8 ? 20ll : 40ll) * k;
+}
 static bool cluster_rows_apply(int dtype, const TopkParams& p) {
   if (!float_rows(dtype, p) || p.k_max > kRcMaxK || forced_path() || long_rows_apply(dtype, p)) return false;
-  return p.rows < 256 && p.n > kRcListCap && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart && p.rows * p.n * dtype_bytes(dtype) <= (64ll << 20);
+  return p.rows < 256 && p.n > kRcListCap && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart &&
+         cluster_order_pays(p.rows, p.n, p.k_max, dtype_bytes(dtype));
 }
 
 template <int DT>

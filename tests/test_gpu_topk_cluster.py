@@ -29,3 +29,17 @@ def test_cluster_top_k_sizes(cuda, dtype, n, k):
     ev, ei = o.top_k(x, k)
     assert np.array_equal(to_np(i), ei)
     assert exact_match(to_np(v), ev)
+
+
+# the lines between the cluster form and the one-pass kernel: lists of 128, 256, 512 and more candidates to order
+@pytest.mark.parametrize("rows,n,k", [(3, 2048, 128), (3, 2049, 128), (200, 2050, 200), (5, 11999, 201), (5, 12000, 201), (5, 12001, 440),
+                                      (8, 20 * 441 - 1, 441), (8, 20 * 441, 441), (9, 40 * 500 - 1, 500), (9, 40 * 500, 500)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16"])
+def test_top_k_at_the_lines_of_the_cluster_form(cuda, dtype, rows, n, k):
+    x = np.random.default_rng(n).standard_normal((rows, n)).astype(np.float32) * 2
+    x[1] = np.round(x[1])
+    x = x.astype({"f32": np.float32, "bf16": o.bfloat16}[dtype])
+    v, i = tax.top_k(to_dev(x, cuda), k, block_token=1)
+    ev, ei = o.top_k(x, k)
+    assert np.array_equal(to_np(i), ei)
+    assert exact_match(to_np(v), ev)
