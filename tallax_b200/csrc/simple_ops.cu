@@ -128,10 +128,10 @@ static int launch_gather(cudaStream_t st, const void* values, const int32_t* idx
 // CTA totals in distributed shared memory, and the sums go out from registers.  Reversed sums walk the same vectors
 // from the end.  f32 [64, 128256]: 143 us with one CTA per row and a block scan per 1024 elements.
 constexpr int kCumsumThreads = 256;
-template <typename T, typename Idx, int V, int kStages>
-__global__ void __launch_bounds__(kCumsumThreads)
+template <typename T, typename Idx, int V, int kStages, int kThreads>
+__global__ void __launch_bounds__(kThreads)
 cumsum_axis1_kernel(const T* __restrict__ in, T* __restrict__ out, Idx cols, int reverse, int cluster, int same_phase) {
-  constexpr int kThreads = kCumsumThreads, kWarps = kThreads / 32, kPer = kThreads * V;
+  constexpr int kWarps = kThreads / 32, kPer = kThreads * V;
   __shared__ __align__(16) uint4 ring[kStages][kPer];
   __shared__ T warp_total[2][kWarps];
   __shared__ T cta_total[2];           // alternating, so that a slow reader of the last turn is not overtaken
@@ -312,6 +312,21 @@ __global__ void __launch_bounds__(kAxis0Warps * 32) cumsum_axis0_kernel(const T*
   if (cluster > 1) cl_sync();   // nobody leaves while its totals may still be read
 }
 
+// The same for a few rows: a thread per column, a short loop.  The kernel above is straight-line code for sixteen rows a warp
+// and most of its time is then instruction fetch and idle warps.
+template <typename T>
+__global__ void __launch_bounds__(128) cumsum_axis0_few_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t rows, int64_t cols,
+                                                               int reverse) {
+  const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (c >= cols) return;
+  T acc = T(0);
+  for (int64_t r = 0; r < rows; ++r) {
+    const int64_t at = (reverse ? rows - 1 - r : r) * cols + c;
+    acc += in[at];
+    out[at] = acc;
+  }
+}
+
 template <typename... Params, typename... Args>
 static int launch_cluster(void (*kernel)(Params...), unsigned grid, unsigned block, int cluster, cudaStream_t st, const char* what,
                           Args... args) {
@@ -331,14 +346,15 @@ static int launch_cluster(void (*kernel)(Params...), unsigned grid, unsigned blo
   return TLX_OK;
 }
 
-template <typename T, typename Idx, int V, int kStages>
+template <typename T, typename Idx, int V, int kStages, int kThreads = kCumsumThreads>
 static int launch_cumsum_rows(cudaStream_t st, const T* in, T* out, int64_t rows, int64_t cols, int reverse, int cluster) {
   const int same = ((reinterpret_cast<uintptr_t>(in) ^ reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  return launch_cluster(cumsum_axis1_kernel<T, Idx, V, kStages>, (unsigned)(rows * cluster), kCumsumThreads, cluster, st, "cumsum", in,
+  return launch_cluster(cumsum_axis1_kernel<T, Idx, V, kStages, kThreads>, (unsigned)(rows * cluster), kThreads, cluster, st, "cumsum", in,
                         out, cols, reverse, cluster, same);
 }
 
-// One vector a thread for rows of up to 1024 elements; beyond that two tiles of 4096 elements (32 KB: six CTAs fit an SM)
+// One vector a thread for rows of up to 1024 elements, and a single warp for up to 128 (f32 [6000, 60] 4.7 us, with eight warps
+// 10.0); beyond that two tiles of 4096 elements (32 KB: six CTAs fit an SM)
 // and as many CTAs per row, up to eight and up to its tiles, as give 740 in all (five per SM): a barrier across CTAs
 // every turn costs more than it brings once the rows fill the GPU.  Measured, f32, with the ring: [64, 128256] 15.7 us,
 // [167, 27252] 10.1, [256, 128256] 54, [1024, 31000] 48 (5.3 TB/s).
@@ -347,6 +363,13 @@ static int launch_cumsum(cudaStream_t st, const void* in, void* out, int64_t row
   const T* x = (const T*)in;
   T* y = (T*)out;
   if (axis == 0) {
+    // us a thread per column / sixteen warps per 32 columns: [16, 500] 2.1/3.5, [40, 4096] 3.3/3.6, [48, 4096] 3.8/3.7, [48, 16384]
+    // 4.7/8.5, [64, 16384] 10.2/9.0, [64, 32768] 12/14, [96, 32768] 17/15, [128, 70000] 25/30, [192, 70000] 36/33
+    if (rows <= (cols < 8192 ? 40 : cols < 32768 ? 48 : cols < 65536 ? 64 : 128)) {
+      cumsum_axis0_few_kernel<T><<<(unsigned)((cols + 127) / 128), 128, 0, st>>>(x, y, rows, cols, reverse);
+      TLX_CHECK_LAUNCH("cumsum");
+      return TLX_OK;
+    }
     const int64_t strips = (cols + 31) / 32;
     int cluster = 1;
     while (cluster < 8 && strips * cluster * 2 <= 592 && (int64_t)cluster * kAxis0Turn < rows) cluster *= 2;
@@ -354,6 +377,7 @@ static int launch_cumsum(cudaStream_t st, const void* in, void* out, int64_t row
                           reverse, cluster);
   }
   const int64_t n = cols + 3;   // the first vector may be a partial one
+  if (n <= 128) return launch_cumsum_rows<T, int, 1, 2, 32>(st, x, y, rows, cols, reverse, 1);
   if (n <= 1024) return launch_cumsum_rows<T, int, 1, 2>(st, x, y, rows, cols, reverse, 1);
   int cluster = 1;
   while (cluster < 8 && rows * cluster * 2 <= 740 && cluster * 4096ll < n) cluster *= 2;

@@ -9,7 +9,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape,axis", [((5, 1021), 1), ((5, 1022), 1), ((3, 4095), 1), ((2, 4098), 1), ((7, 16385), 1), ((3, 70001), 1),
-                                        ((400, 5003), 1), ((1, 1), 1), ((256, 33), 0), ((257, 31), 0), ((2049, 5), 0), ((5000, 70), 0)])
+                                        ((400, 5003), 1), ((1, 1), 1), ((256, 33), 0), ((257, 31), 0), ((2049, 5), 0), ((5000, 70), 0),
+                                        # a warp per row and just not; a thread per column and just not
+                                        ((9, 125), 1), ((9, 126), 1), ((1, 7), 0), ((40, 129), 0), ((41, 129), 0), ((48, 8192), 0), ((49, 8192), 0),
+                                        ((128, 65537), 0)])
 @pytest.mark.parametrize("reverse", [False, True])
 def test_cumsum_sizes(cuda, shape, axis, reverse):
     rng = np.random.default_rng(shape[1])
