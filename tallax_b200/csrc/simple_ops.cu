@@ -95,10 +95,12 @@ static int launch_gather(cudaStream_t st, const void* values, const int32_t* idx
     if (total == 0) return TLX_OK;
     const int64_t want = (total + threads - 1) / threads;
     const int blocks = (int)(want < 148 * 64 ? want : 148 * 64);
-    // rows far longer than L1 could hold again: their lines are not kept there (84 against 88 us for f32 [1024, 4096]
-    // out of [1024, 262144])
+    // Many outputs out of rows of which hardly a line is read twice: the lines are not kept in L1.  us kept / not, rotating inputs,
+    // and with a cold L2: f32 [1024, 1000] out of [1024, 262144] 25.6/23.6, 39/33; [256, 4096] 22.2/21.5, 33/31.  A line's second
+    // reading, or a matrix that lies in L2, wants L1: [1024, 4096] out of [1024, 65537] 44.0/45.1, 59/74; [1024, 100] out of
+    // [1024, 262144] 4.1/5.8.
     if constexpr (sizeof(T) == 4) {
-      if (vc > (64 << 10)) {
+      if (vc > (64 << 10) && ic * 32 <= vc && ir * ic >= (1 << 18)) {
         gather_axis1_kernel<T, true><<<blocks, threads, 0, st>>>((const T*)values, idx, (T*)out, ir, vc, ic);
         TLX_CHECK_LAUNCH("take_along_axis");
         return TLX_OK;

@@ -28,6 +28,17 @@ def test_take_along_axis(cuda, num_tokens, vocab_size, k, axis):
     assert np.array_equal(to_np(out), o.take_along_axis(values, indices, axis))
 
 
+# many outputs out of long rows (lines not kept in L1), and the lines of that rule
+@pytest.mark.parametrize("rows,n,k", [(128, 70000, 2060), (128, 65536, 2050), (130, 65537, 2017), (64, 131104, 4097)])
+def test_take_along_axis_long_rows(cuda, rows, n, k):
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    values = torch.randn((rows, n), generator=gen, device=cuda)
+    indices = torch.randint(-3, n + 3, (rows, k), generator=gen, device=cuda, dtype=torch.int32)
+    inside = (indices >= 0) & (indices < n)
+    want = torch.where(inside, values.gather(1, indices.clamp(0, n - 1).long()), torch.zeros((), device=cuda))
+    assert torch.equal(tumpy.take_along_axis(values, indices, 1), want)
+
+
 @pytest.mark.parametrize("dtype", ["f32", "bf16", "i32"])
 def test_take_along_axis_large_and_out_of_range(cuda, dtype):
     rng = np.random.default_rng(1)
