@@ -373,9 +373,8 @@ __device__ __forceinline__ void rc_filter(const RcPart<DT>& part, float thr, RcS
   }
 }
 
-// Leader: prefix of the CTAs' counts (s.first), and the other CTAs' candidates behind its own ones in its own list.
-// Returns the number of candidates, or -1 if a list or the whole overflowed.
-__device__ __forceinline__ int rc_gather(RcShared& s, int cluster, float* lx, float* ls, unsigned short* lpos) {
+// Prefix of the CTAs' counts (s.first); whether a list or the whole overflowed, which every CTA that asks sees alike.
+__device__ __forceinline__ bool rc_count(RcShared& s, int cluster) {
   if (threadIdx.x < 32) {
     const int lane = lane_id();
     int c = lane < cluster ? (int)cl_ld_u32(cl_map(&s.n_list, (uint32_t)lane)) : 0;
@@ -390,8 +389,11 @@ __device__ __forceinline__ int rc_gather(RcShared& s, int cluster, float* lx, fl
     if (lane == 0) { s.first[0] = 0; s.pick[0] = over != 0; }
   }
   __syncthreads();
+  return s.pick[0] || s.first[cluster] > kRcListCap;
+}
+// Leader, lists that did not overflow: the other CTAs' candidates behind its own ones in its own list.  Returns their number.
+__device__ __forceinline__ int rc_collect(RcShared& s, int cluster, float* lx, float* ls, unsigned short* lpos) {
   const int m = s.first[cluster];
-  if (s.pick[0] || m > kRcListCap) return -1;
 #pragma unroll 1
   for (int i = s.first[1] + threadIdx.x; i < m; i += kRcThreads) {
     int r = 1;

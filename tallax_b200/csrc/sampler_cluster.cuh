@@ -14,10 +14,12 @@
 // value plus the greatest Gumbel term there is would not do.  The survivors (a handful) go to the leader, and the
 // mass above its best ones comes from one more pass over the parts, which are still in shared memory.
 //
-// Rows with 1024 < top_k < vocab are cut to their top-k set in shared memory (rc_cut_parts) and then taken as rows without.
+// Rows with 1024 < top_k < vocab, and rows whose lists overflow, are cut to their top-k set in shared memory (rc_cut_parts)
+// and then taken as rows without.
 //
-// Anything these lists cannot hold (huge groups of equal values), rows without a finite maximum, and rows longer than a
-// cluster holds take rc_slow_row: exact, any top-k, by passes over the row in global memory.
+// Rows without top-k whose survivors the lists cannot hold, greedy rows with huge groups of greatest values, rows without a
+// finite maximum, and rows longer than a cluster holds take rc_slow_row: exact, any top-k, by passes over the row in global
+// memory.
 #pragma once
 #include "row_cluster.cuh"
 
@@ -264,35 +266,36 @@ static __device__ __noinline__ void rc_cut_to_k(RcShared& s, int m, int K, int64
     __syncthreads();
     if (ties == need) break;   // everything in the bin belongs to the set: vk is its lower end
   }
-  // ties at the K-th key (vk is complete then): the `need` lowest columns stay.  Up to 256 ties are listed first.
-  const bool cut_ties = need < ties;
-  const bool listed = cut_ties && ties <= 256;
-  if (threadIdx.x == 0) s.pick[3] = 0;
-  __syncthreads();
-  if (listed) {
+  // ties at the K-th key (vk is complete then): the `need` lowest columns stay, found by the same descent over the columns
+  // (distinct and below 2^24), inverted.  Comparing every tie with every other one took 1.2 ms for 1500 equal values.
+  uint32_t from = 0;   // least inverted column that stays
+  if (need < ties) {
+    from = 0x7Fu << 24;
 #pragma unroll 1
-    for (int i = threadIdx.x; i < m; i += kRcThreads)
-      if (f32_key(lx[i]) == vk) s.hist[atomicAdd(&s.pick[3], 1)] = (uint32_t)rc_column(s, lpos, i, part_len);
-    __syncthreads();
+    for (int sh = 16; sh >= 0; sh -= 8) {
+      s.hist[threadIdx.x] = 0;
+      __syncthreads();
+#pragma unroll 1
+      for (int i = threadIdx.x; i < m; i += kRcThreads)
+        if (f32_key(lx[i]) == vk) {
+          const uint32_t c = 0x7FFFFFFFu - (uint32_t)rc_column(s, lpos, i, part_len);
+          if (((c ^ from) >> (sh + 8)) == 0) atomicAdd(&s.hist[(c >> sh) & 255u], 1u);
+        }
+      __syncthreads();
+      if (warp_id() == 0) rc_pick_bin(s.hist, need, s.pick);
+      __syncthreads();
+      from |= (uint32_t)s.pick[0] << sh;
+      need -= s.pick[1];
+      const bool whole = s.pick[2] == need;
+      __syncthreads();
+      if (whole) break;
+    }
   }
 #pragma unroll 1
   for (int i = threadIdx.x; i < m; i += kRcThreads) {
     const uint32_t k = f32_key(lx[i]);
-    bool out = k < vk;
-    if (cut_ties && k == vk) {
-      const uint32_t col = (uint32_t)rc_column(s, lpos, i, part_len);
-      int before = 0;
-#pragma unroll 1
-      for (int j = 0; j < (listed ? ties : m); ++j)
-        if (listed ? s.hist[j] < col : f32_key(lx[j]) == vk && (uint32_t)rc_column(s, lpos, j, part_len) < col) ++before;
-      out = before >= need;
-    }
-    if (out) ls[i] = __int_as_float(0x7FC00001);   // marked; the values are still being compared by other threads
+    if (k < vk || (k == vk && from != 0 && 0x7FFFFFFFu - (uint32_t)rc_column(s, lpos, i, part_len) < from)) { ls[i] = -INFINITY; lx[i] = -INFINITY; }
   }
-  __syncthreads();
-#pragma unroll 1
-  for (int i = threadIdx.x; i < m; i += kRcThreads)
-    if (__float_as_uint(ls[i]) == 0x7FC00001u) { ls[i] = -INFINITY; lx[i] = -INFINITY; }
   __syncthreads();
 }
 
@@ -720,7 +723,7 @@ __device__ __forceinline__ void rc_masses(const RcPart<DT>& part, float xmax, fl
   z = (zs[0] + zs[1]) + (zs[2] + zs[3]);
 }
 
-// Rows with 1024 < top_k < vocab: cuts the row, which lies in the parts, to its top-K set.  What is outside the set becomes
+// Rows with 1024 < top_k < vocab and rows whose lists overflowed: cuts the row, which lies in the parts, to its top-K set.  What is outside the set becomes
 // -inf, and the row is then one without top-k.
 //   The K-th greatest key comes from histograms of 2048 bins, eleven bits of the key at a time (two for bf16, three for f32, in
 // `bins`); the leader adds the CTAs' bins up and tells them which one holds the K-th key.  Of keys equal to it the lowest
@@ -868,11 +871,13 @@ static __device__ __noinline__ void rc_cut_parts(uint4* vec, int off, int n, int
 }
 
 // Rows with 1 <= top_k <= 1024 and greedy rows.  Returns the token in the leader (rank 0), -1 if the row has to be
-// answered by rc_slow_row; the other CTAs return -1 when they may leave.
+// answered by rc_slow_row; the other CTAs return -1 when they may leave.  kRcOver, in every CTA alike: the lists overflowed
+// (huge groups of equal values; fewer finite groups than top_k), and the row has to be cut in the parts.
+constexpr int kRcOver = -2;
 template <int DT>
 __device__ __forceinline__ int rc_normal_row(const RcSampleParams& p, const RcPart<DT>& part, int64_t col0, uint32_t rank, int K,
                                              float pp, float T_, int64_t nrow, RcShared& s, const RcLayout& l,
-                                             unsigned char* smem, int& tog) {
+                                             unsigned char* smem) {
   float* lx = reinterpret_cast<float*>(smem + l.off_x);
   float* ls = reinterpret_cast<float*>(smem + l.off_s);
   unsigned short* lpos = reinterpret_cast<unsigned short*>(smem + l.off_pos);
@@ -906,11 +911,13 @@ __device__ __forceinline__ int rc_normal_row(const RcSampleParams& p, const RcPa
   TLX_STAMP(p.sp, 5);
   cl_sync();
   TLX_STAMP(p.sp, 6);
+  const bool full = rc_count(s, p.cluster);
+  if (full && !greedy) return kRcOver;
   if (rank != 0) {
     cl_sync();
     return -1;
   }
-  const int m = rc_gather(s, p.cluster, lx, ls, lpos);
+  const int m = full ? -1 : rc_collect(s, p.cluster, lx, ls, lpos);
   cl_arrive();   // the other CTAs may leave
   TLX_STAMP(p.sp, 7);
   int tok = -1;
@@ -1161,13 +1168,17 @@ __global__ void __launch_bounds__(kRcThreads, 4) sample_cluster_kernel(const __g
   TLX_STAMP(p.sp, 1);
   const int64_t col0 = (int64_t)rank * p.part_len, nrow = row + p.sp.dim0_offset;
   int tok = -1, tog = 0;
-  if (wide) {
-    if (K < n)
+  if (resident && !wide) tok = rc_normal_row<DT>(p, part, col0, rank, (int)K, pp, T_, nrow, s, l, smem);
+  const bool over = tok == kRcOver;
+  if (wide || over) {
+    if (K < n) {
       rc_cut_parts<DT>(part.vec, part.off, part.n, part.nvec, (int)K, p.cluster, rank, s, reinterpret_cast<uint32_t*>(smem + l.off_x));
+      if (threadIdx.x == 0) s.n_list = 0;   // (read by the other CTAs before the barriers of the cut)
+    }
     tok = rc_wide_row<DT>(p, part, col0, rank, pp, T_, nrow, s, l, smem, tog);
-  } else if (resident) tok = rc_normal_row<DT>(p, part, col0, rank, (int)K, pp, T_, nrow, s, l, smem, tog);
+  }
   if (rank != 0) return;
-  int status = wide || !resident ? kStatusGeneral : 0;
+  int status = (wide || !resident ? kStatusGeneral : 0) | (over ? kStatusRedone : 0);
   if (tok < 0) {
     tok = rc_slow_row<DT>(rowp, n, K, pp, T_, p.sp.noise, nrow, s);
     status |= resident ? kStatusRedone : 0;

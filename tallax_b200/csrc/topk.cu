@@ -648,7 +648,7 @@ __global__ void __launch_bounds__(kRcThreads, 4) topk_cluster_kernel(const __gri
     cl_sync();
     return;
   }
-  int m = rc_gather(s, cluster, lx, nullptr, lpos);
+  int m = rc_count(s, cluster) ? -1 : rc_collect(s, cluster, lx, nullptr, lpos);
   cl_arrive();   // the other CTAs may leave
   uint64_t* cand = reinterpret_cast<uint64_t*>(smem + l.off_part);   // the part is not needed any more
   if (m < K) {   // (or -1)

@@ -95,3 +95,31 @@ def test_workspace_reported_is_the_workspace_used(cuda, rows, V, from_key):
         launches.append(lib.tlx_kernel_launches() - before)
     assert launches == [3 if reported > 256 else 1] * 3
     assert torch.equal(tokens[0], tokens[1]) and torch.equal(tokens[0], tokens[2])
+
+
+# rows with top-k whose candidates are hundreds of ties (cut by column) or more than the lists hold (cut in the parts)
+@pytest.mark.parametrize("V", [300, 1509, 2048, 2049, 12032, 80129])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("from_key", [False, True])
+def test_heavy_ties_and_masked_rows(cuda, dtype, V, from_key):
+    B = 12
+    x, tk, tp, T, noise = o.make_sampling_inputs(B=B, V=V, seed=V + 1, dtype=dtype)
+    xf = x.astype(np.float32)
+    tk[:] = np.minimum([50, 257, 1024, 50, 700, 1, 1024, 50, 1000, 3, 1024, 257], V - 1)
+    xf[:3] = 0.0                                               # one value
+    xf[3] = 0.5 * (np.arange(V) % 2)                           # two values, the cut inside the greater one's ties
+    xf[4] = np.where(np.arange(V) % 100 < 3, 1.0, 0.25 * (np.arange(V) % 3))
+    xf[5] = 2.0                                                # greedy: the first column of all
+    T[5] = 0.0
+    xf[6:9, V // 20:] = -np.inf                                # 95 % masked, together
+    xf[9] = np.round(xf[9] / 4)
+    xf[10, ::2] = -np.inf                                      # half masked, scattered
+    xf[11] = -7.0
+    x = xf.astype(x.dtype)
+    kw = dict(rng_key=(29, V)) if from_key else dict(noise=noise)
+    exp, flags = o.sample(x, tk, tp, T, return_flags=True, **kw)
+    dkw = dict(rng_key=(29, V)) if from_key else dict(noise=to_dev(noise, cuda))
+    tok, status = ops.sample(to_dev(x, cuda), to_dev(tk, cuda), to_dev(tp, cuda), to_dev(T, cuda), return_status=True, **dkw)
+    bad = (to_np(tok) != exp) & ~flags
+    assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
+    assert (to_np(status) & 2 == 0).all()
