@@ -121,7 +121,8 @@ struct __align__(16) RcShared {
   int n_list;                           // candidates of this CTA (may exceed kRcListCap: overflow)
   // rows without top-k
   float dom_x[2 * kRcMaxCluster], dom_s[2 * kRcMaxCluster];   // per CTA: its greatest element and its best-scored one
-  float cut_x[6], cut_s[6];             // an element is out if one of these has at least its value and a greater score
+  float cut_x[14], cut_s[14];           // an element is out if one of these has at least its value and a greater score
+  int n_cut;
   float query[4];                       // values whose mass above the leader asks for
   int n_query;
   int query_tok[4];                     // leader: their tokens

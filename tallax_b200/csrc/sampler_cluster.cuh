@@ -509,7 +509,7 @@ __device__ __forceinline__ void rc_keep_survivor(float x, float u, int i, const 
   const float a = fmaf(x, r.rt, gumbel_screen(u));
   bool out = !(a > -INFINITY);
 #pragma unroll 1
-  for (int j = 0; j < 6; ++j) out = out || (x <= s.cut_x[j] && a < s.cut_s[j]);
+  for (int j = 0; j < s.n_cut; ++j) out = out || (x <= s.cut_x[j] && a < s.cut_s[j]);
   if (!out) {
     const int slot = atomicAdd(&s.n_list, 1);
     if (slot < kRcWideCap) { w.x[slot] = x; w.s[slot] = a; w.pos[slot] = (unsigned short)i; }
@@ -1017,13 +1017,15 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
   // the same in every CTA: no finite maximum, or no score for it
   const bool lost = !(fabsf(xmax) < INFINITY) || !(fabsf(ms) < INFINITY) || !(fabsf(bs) < INFINITY);
   if (!lost) {
-    // [0]: the published element with the best score; [1]: the row's greatest element; [2..4]: filled below
-    if (threadIdx.x < 6) {
+    // [0]: the published element with the best score; [1]: the row's greatest element; the rest: filled below
+    if (threadIdx.x < 2) {
       s.cut_x[threadIdx.x] = threadIdx.x == 0 ? bx : xmax;
       s.cut_s[threadIdx.x] = rc_cut(threadIdx.x == 0 ? bs : ms);
     }
+    if (threadIdx.x == 0) s.n_cut = 2;
     __syncthreads();
     RcLow low{bx, rc_cut(bs), rc_cut(ms)};
+    float above = -INFINITY;
 #pragma unroll 1
     for (int attempt = 0;; ++attempt) {
       // from a key the greatest Gumbel term is that of 1 - 2^-23: 15.943
@@ -1032,25 +1034,28 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
       if (attempt == 0) { TLX_STAMP(p.sp, 10); }
       if (s.n_list <= kRcWideCap || attempt == 4) break;
       // too many (a flat row): the best of those that were kept, the best among the greater ones and the best
-      // among those that are greater again dominate nearly all of them
-      float above = -INFINITY;
+      // among those that are greater again dominate nearly all of them, as a rule; where the three lie close together,
+      // the next attempt goes on from the last of them
+      int cuts = s.n_cut;
 #pragma unroll 1
       for (int j = 0; j < 3; ++j) {
+        const bool first = attempt == 0 && j == 0;
         uint32_t bk = 0, xk = 0;
 #pragma unroll 1
-        for (int i = threadIdx.x; i < kRcWideCap; i += kRcThreads) if (j == 0 || l.x[i] > above) bk = max(bk, rc_score_key(l.s[i]));
+        for (int i = threadIdx.x; i < kRcWideCap; i += kRcThreads) if (first || l.x[i] > above) bk = max(bk, rc_score_key(l.s[i]));
         bk = rc_max_u32(bk, s, tog);
         if (bk == 0) break;
 #pragma unroll 1
         for (int i = threadIdx.x; i < kRcWideCap; i += kRcThreads)
-          if ((j == 0 || l.x[i] > above) && rc_score_key(l.s[i]) == bk) xk = max(xk, f32_key(l.x[i]));
+          if ((first || l.x[i] > above) && rc_score_key(l.s[i]) == bk) xk = max(xk, f32_key(l.x[i]));
         above = key_f32(rc_max_u32(xk, s, tog));
         const float cut = rc_cut(key_f32(bk));
-        if (threadIdx.x == 0) { s.cut_x[2 + j] = above; s.cut_s[2 + j] = cut; }
-        if (j == 0 && cut > low.bs) { low.bs = cut; low.bx = above; }
+        if (threadIdx.x == 0) { s.cut_x[cuts] = above; s.cut_s[cuts] = cut; }
+        ++cuts;
+        if (first && cut > low.bs) { low.bs = cut; low.bx = above; }
       }
       __syncthreads();
-      if (threadIdx.x == 0) s.n_list = 0;
+      if (threadIdx.x == 0) { s.n_list = 0; s.n_cut = cuts; }
       __syncthreads();
     }
     if (warp_id() == 0) {

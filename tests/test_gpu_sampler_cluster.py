@@ -123,3 +123,20 @@ def test_heavy_ties_and_masked_rows(cuda, dtype, V, from_key):
     bad = (to_np(tok) != exp) & ~flags
     assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
     assert (to_np(status) & 2 == 0).all()
+
+
+# flat rows without top-k: hundreds of elements of a part lie above the best-scored published one; the parts settle them all
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("from_key", [False, True])
+def test_flat_rows_without_top_k(cuda, dtype, from_key):
+    B, V = 32, 40001
+    x, tk, tp, T, noise = o.make_sampling_inputs(B=B, V=V, seed=3, dtype=dtype)
+    x = (x.astype(np.float32) * np.repeat(np.float32([0.1, 0.03, 0.01, 0.003]), B // 4)[:, None]).astype(x.dtype)
+    tk[:] = 0
+    kw = dict(rng_key=(31, 7)) if from_key else dict(noise=noise)
+    exp, flags = o.sample(x, tk, tp, T, return_flags=True, **kw)
+    dkw = dict(rng_key=(31, 7)) if from_key else dict(noise=to_dev(noise, cuda))
+    tok, status = ops.sample(to_dev(x, cuda), to_dev(tk, cuda), to_dev(tp, cuda), to_dev(T, cuda), return_status=True, **dkw)
+    bad = (to_np(tok) != exp) & ~flags
+    assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
+    assert (to_np(status) & 6 == 0).all()                      # none was answered by passes over global memory
