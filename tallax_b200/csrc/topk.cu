@@ -634,14 +634,19 @@ __global__ void __launch_bounds__(kRcThreads, 4) topk_cluster_kernel(const __gri
   if (threadIdx.x == 0) s.n_list = 0;
   part.copy_wait();
   __syncthreads();
-  uint32_t* bound = reinterpret_cast<uint32_t*>(smem + l.off_bound);
-  GroupMax<DT> gm;
-  gm.init();
+  float thr = -INFINITY;
+  if (p.n > kRcListCap) {
+    uint32_t* bound = reinterpret_cast<uint32_t*>(smem + l.off_bound);
+    GroupMax<DT> gm;
+    gm.init();
 #pragma unroll 2
-  for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) gm.add(part.vec[v]);
-  rc_publish_maxima<DT>(gm, l.bound_words, bound);
-  cl_sync();
-  const float thr = key_f32(rc_bound_key16(bound, l.bound_words, K, s) << 16);
+    for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) gm.add(part.vec[v]);
+    rc_publish_maxima<DT>(gm, l.bound_words, bound);
+    cl_sync();
+    thr = key_f32(rc_bound_key16(bound, l.bound_words, K, s) << 16);
+  } else {
+    cl_sync();
+  }
   rc_filter<DT>(part, thr, s, lx, lpos);
   cl_sync();
   if (rank != 0) {
@@ -710,8 +715,8 @@ static bool long_rows_apply(int dtype, const TopkParams& p) {
 }
 
 // Whether the cluster form serves a call: fewer rows than the kernels with a CTA per row want, rows that a cluster holds and that
-// are longer than a candidate list (all elements of a shorter row would be candidates, to be sorted: f16 [95, 1365], k = 4 25 us,
-// by the one-pass kernel 7), and, by the number of candidates that the leader has to order, against the one-pass kernel:
+// are longer than a candidate list (all elements of a shorter row are candidates: up to 256 are ordered by counting, f32 [60, 208]
+// 5.7 us against 9.0 of the one-pass kernel, but more would be sorted, f16 [95, 1365], k = 4 25 against 7), and, by the number of candidates that the leader has to order, against the one-pass kernel:
 // - k <= 128: not more than 64 MB, beyond which the clusters' several waves take longer
 // - k <= 200 (up to 256 candidates, ordered by counting): not more than 40 MB (us cluster / one-pass, f32, k = 200: [255, 32768]
 //   32/35, [255, 65536] 53/47)
@@ -722,14 +727,14 @@ static bool long_rows_apply(int dtype, const TopkParams& p) {
 //   [32, 32768] 42/39, [32, 65536] 45/52, [148, 65536] 89/54; k = 512: [1, 12000] 20/20, [32, 32768] 24/29, [148, 32768] 39/33)
 static bool cluster_order_pays(int64_t rows, int64_t n, int k, int elem_bytes) {
   const int64_t bytes = rows * n * elem_bytes;
-  if (k <= kShortMaxK) return bytes <= (64ll << 20);
+  if (k <= kShortMaxK || n <= kRcThreads) return bytes <= (64ll << 20);
   if (k <= 200) return bytes <= (40ll << 20);
   if (k <= 440) return n >= 12000 && bytes <= ((elem_bytes == 2 ? 40ll : 16ll) << 20);
   return rows <= 64 && n >= (rows <= 8 ? 20ll : 40ll) * k;
 }
 static bool cluster_rows_apply(int dtype, const TopkParams& p) {
   if (!float_rows(dtype, p) || p.k_max > kRcMaxK || forced_path() || long_rows_apply(dtype, p)) return false;
-  return p.rows < 256 && p.n > kRcListCap && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart &&
+  return p.rows < 256 && (p.n <= kRcThreads || p.n > kRcListCap) && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart &&
          cluster_order_pays(p.rows, p.n, p.k_max, dtype_bytes(dtype));
 }
 

@@ -32,7 +32,7 @@ def test_cluster_top_k_sizes(cuda, dtype, n, k):
 
 
 # the lines between the cluster form and the one-pass kernel: lists of 128, 256, 512 and more candidates to order
-@pytest.mark.parametrize("rows,n,k", [(3, 2048, 128), (3, 2049, 128), (200, 2050, 200), (5, 11999, 201), (5, 12000, 201), (5, 12001, 440),
+@pytest.mark.parametrize("rows,n,k", [(3, 256, 256), (3, 257, 256), (3, 2048, 128), (3, 2049, 128), (200, 2050, 200), (5, 11999, 201), (5, 12000, 201), (5, 12001, 440),
                                       (8, 20 * 441 - 1, 441), (8, 20 * 441, 441), (9, 40 * 500 - 1, 500), (9, 40 * 500, 500)])
 @pytest.mark.parametrize("dtype", ["f32", "bf16"])
 def test_top_k_at_the_lines_of_the_cluster_form(cuda, dtype, rows, n, k):
