@@ -714,24 +714,28 @@ static bool long_rows_apply(int dtype, const TopkParams& p) {
   return row > (80 << 10) && all > ((p.rows > 4 * 148 ? 70ll : 30ll) << 20);
 }
 
+// Whether the cluster form is faster than the one-pass kernel, by the number of candidates that the leader has to order and by how
+// many waves of clusters there are.  Few rows leave the one-pass kernel's SMs idle, so their clusters may take several waves (us
+// cluster / one-pass, f32, k = 256: [16, 300000] 31/71, [50, 262144] 61/66, [64, 262144] 74/66).
+// - k <= 128, or a row of which all elements are counted: not more than 64 MB
+// - k <= 200 (up to 256 candidates, ordered by counting): few rows, or not more than 40 MB (k = 200: [255, 32768] 32/35,
+//   [255, 65536] 53/47)
+// - k <= 440 (512 in the bitonic network): rows of at least 12000 elements, and few, or not more than 16 MB, 40 MB of 16-bit ones
+//   (k = 300: [1, 8192] 14.0/12.7, [255, 8192] 22/17, [1, 12000] 14.4/16.8, [255, 16384] 26/27, [148, 32768] 30/29; bf16, k = 256:
+//   [255, 65536] 43/47)
+// - above: few rows that are long enough for the leader's network not to matter (k = 1024: [1, 16384] 31/30, [1, 32768] 33/38,
+//   [32, 32768] 42/39, [32, 65536] 45/52, [64, 65536] 71/53, [50, 131072] 64/70; k = 512: [1, 12000] 20/20, [32, 32768] 24/29, [148, 32768] 39/33)
+static bool cluster_order_pays(int64_t rows, int64_t n, int k, int elem_bytes) {
+  const int64_t mb = (rows * n * elem_bytes + (1 << 20) - 1) >> 20;
+  const bool few = mb <= 64 && (rows <= 50 || (rows <= 64 && mb <= 40) || (rows <= 100 && elem_bytes == 2 && k <= 440));
+  if (k <= kShortMaxK || n <= kRcThreads) return mb <= 64;
+  if (k <= 200) return few || mb <= 40;
+  if (k <= 440) return n >= 12000 && (few || mb <= (elem_bytes == 2 ? 40 : 16));
+  return few && n >= (rows <= 8 ? 20ll : rows <= 32 ? 40ll : 120ll) * k;
+}
 // Whether the cluster form serves a call: fewer rows than the kernels with a CTA per row want, rows that a cluster holds and that
 // are longer than a candidate list (all elements of a shorter row are candidates: up to 256 are ordered by counting, f32 [60, 208]
-// 5.7 us against 9.0 of the one-pass kernel, but more would be sorted, f16 [95, 1365], k = 4 25 against 7), and, by the number of candidates that the leader has to order, against the one-pass kernel:
-// - k <= 128: not more than 64 MB, beyond which the clusters' several waves take longer
-// - k <= 200 (up to 256 candidates, ordered by counting): not more than 40 MB (us cluster / one-pass, f32, k = 200: [255, 32768]
-//   32/35, [255, 65536] 53/47)
-// - k <= 440 (512 in the bitonic network): rows of at least 12000 elements, not more than 16 MB, 40 MB of 16-bit ones (k = 300:
-//   [1, 8192] 14.0/12.7, [255, 8192] 22/17, [1, 12000] 14.4/16.8, [255, 16384] 26/27, [148, 32768] 30/29; bf16, k = 256:
-//   [255, 65536] 43/47)
-// - above: a few rows that are long enough for the leader's network not to matter (k = 1024: [1, 16384] 31/30, [1, 32768] 33/38,
-//   [32, 32768] 42/39, [32, 65536] 45/52, [148, 65536] 89/54; k = 512: [1, 12000] 20/20, [32, 32768] 24/29, [148, 32768] 39/33)
-static bool cluster_order_pays(int64_t rows, int64_t n, int k, int elem_bytes) {
-  const int64_t bytes = rows * n * elem_bytes;
-  if (k <= kShortMaxK || n <= kRcThreads) return bytes <= (64ll << 20);
-  if (k <= 200) return bytes <= (40ll << 20);
-  if (k <= 440) return n >= 12000 && bytes <= ((elem_bytes == 2 ? 40ll : 16ll) << 20);
-  return rows <= 64 && n >= (rows <= 8 ? 20ll : 40ll) * k;
-}
+// 5.7 us against 9.0 of the one-pass kernel, but more would be sorted, f16 [95, 1365], k = 4 25 against 7).
 static bool cluster_rows_apply(int dtype, const TopkParams& p) {
   if (!float_rows(dtype, p) || p.k_max > kRcMaxK || forced_path() || long_rows_apply(dtype, p)) return false;
   return p.rows < 256 && (p.n <= kRcThreads || p.n > kRcListCap) && p.n <= (int64_t)kRcMaxCluster * kRcMaxPart &&
