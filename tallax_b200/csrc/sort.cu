@@ -1,6 +1,6 @@
 // Stable row-wise argsort, by the length of the rows:
-//   up to 1024 elements       bitonic network on 64-bit composites (key << 32 | position) in the shared memory of one CTA
-//   up to 131072              radix sort in the shared memory of a CTA or of a cluster of CTAs (sort_radix.cuh)
+//   the shortest              bitonic network on 64-bit composites (key << 32 | position) in the shared memory of one CTA
+//   up to 131072              by estimated places in the shared memory of a CTA or of a cluster of CTAs (sort_places.cuh)
 //   beyond                    the network on composites in the caller's workspace, in tiles of kTile elements
 //
 // The network.  The position in the low word makes every composite unique, so the (unstable) bitonic network yields the
@@ -13,7 +13,7 @@
 #include <mutex>
 #include <type_traits>
 
-#include "sort_radix.cuh"
+#include "sort_places.cuh"
 
 namespace tlx {
 
@@ -199,17 +199,42 @@ static int64_t next_pow2(int64_t n) {
   return p;
 }
 
+// CTAs a row, of 16384 elements at most.
+//   Few rows: as many as run at once with an SM each, because a CTA's latency grows with its elements (f32 [1, 16384] in 1 / 2 / 4
+// CTAs 19.7 / 18.2 / 14.7 us, [20, 65536] in 4 / 6 / 8 34 / 30 / 35: 20 clusters of eight don't find room in the GPU's eight groups
+// of 18 SMs).  Up to 10000 elements the exchange costs more than it gives ([1, 8193] 12.2 / 13.8 / 13.0).
+//   Else CTAs of 8192, two to an SM, if all of them run at once ([40, 40000] in 4 / 5 CTAs 46 / 33).
+//   Else single CTAs ([400, 16384] in 1 / 2 60 / 81), and of clusters those that fill the groups of SMs: [128, 32768] in 2 / 3 / 4
+// 62 / 72 / 62, [256, 17000] 76 / 69 / 69; [256, 40000] in 4 / 5 / 8 184 / 162 / 181, [256, 49152] in 4 / 6 / 7 211 / 199 / 230,
+// [256, 65536] in 4 / 6 / 8 271 / 327 / 291.
+static int places_cluster(int64_t rows, int64_t n) {
+  auto ctas = [&](int64_t tile) { return (int)((n + tile - 1) / tile); };
+  auto at_once = [](int cluster, int an_sm) { return cluster == 1 ? 148 * an_sm : 8 * (18 * an_sm / cluster); };
+  const int least = ctas(16384);
+  if (n <= 10000) return 1;
+  for (int c = ctas(4096) < 8 ? ctas(4096) : 8; c >= least; --c)
+    if (rows <= at_once(c, 1)) return c;
+  if (least == 1) return 1;
+  const int half = ctas(8192);
+  if (half <= 8 && rows <= at_once(half, 2)) return half;
+  if (least == 2) return half == 3 ? 3 : 2;
+  return half <= 6 ? half : (least < 4 ? 4 : least);
+}
+
 template <int DT, int IPT, bool CL, bool PAST = false>
-static int launch_radix(cudaStream_t st, const void* keys, int64_t rows, int64_t n, int descending, const int32_t* in_perm,
-                        void* out_keys, int32_t* out_perm, int threads, int cluster) {
+static int launch_places(cudaStream_t st, const void* keys, int64_t rows, int64_t n, int descending, const int32_t* in_perm,
+                         void* out_keys, int32_t* out_perm, int cluster) {
   using T = typename Elem<DT>::type;
+  // the radix passes need 256 threads for their 256 digits
+  const int64_t share = (n + (int64_t)cluster * 32 * IPT - 1) / ((int64_t)cluster * 32 * IPT) * 32;
+  const int threads = share < 256 ? 256 : (int)(share < 4096 ? share : 4096);
   // the kernel has a place for every element, or it writes outside its shared memory
-  if (threads < 256 || threads > kRadixMaxThreads || threads % 32 || (int64_t)threads * IPT * cluster < n || (!CL && cluster != 1))
+  if (threads > kRadixMaxThreads || (int64_t)threads * IPT * cluster < n || cluster < 1 || cluster > (CL ? 8 : 1) || n > kRadixMaxRow)
     return set_error(TLX_ERR_INVALID, "sort: no kernel for rows of %lld elements (%d threads)", (long long)n, threads);
-  const size_t smem = radix_smem(threads, threads * IPT, CL);
+  const size_t smem = place_smem<IPT, CL>(threads);
   static SmemLimit limit;
   int rc;
-  if ((rc = raise_smem(limit, (const void*)sort_radix_kernel<DT, IPT, CL, PAST>, smem, "sort")) != TLX_OK) return rc;
+  if ((rc = raise_smem(limit, (const void*)sort_places_kernel<DT, IPT, CL, PAST>, smem, "sort")) != TLX_OK) return rc;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(rows * cluster));
   cfg.blockDim = dim3((unsigned)threads);
@@ -221,8 +246,7 @@ static int launch_radix(cudaStream_t st, const void* keys, int64_t rows, int64_t
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = CL ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, sort_radix_kernel<DT, IPT, CL, PAST>, (const T*)keys, in_perm, n, descending, (T*)out_keys, out_perm,
-                                     cluster);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, sort_places_kernel<DT, IPT, CL, PAST>, (const T*)keys, in_perm, n, descending, (T*)out_keys, out_perm, cluster);
   if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "sort: %s", cudaGetErrorString(e)); }
   count_launch();
   return TLX_OK;
@@ -235,31 +259,20 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
   using T = typename Elem<DT>::type;
   const int64_t n_pad = next_pow2(n < 2 ? 2 : n);
   int rc;
-  // Up to 1024 elements the network's few stages cost less than a pass's counters (f32 [1000, 512]: 13 us against 26).
-  // A CTA per row up to 8192: eight elements a thread, which wastes the fewest places, and sixteen, which need fewer counters per
-  // element, where the rows fill the GPU and the places (4096 at least) are used (f32 with a payload, eight / sixteen:
-  // [1024, 4096] 109 us / 90, [1024, 3000] 81 / 86, [1024, 2049] 67 / 87, [1024, 1025] 45 / 80; the network 129, 124, 124, 56).
-  // A cluster of CTAs beyond: of 4096 elements each where all of them run at once with an
-  // SM each (bf16 [4, 16384] 20 us, with 8192 elements 26, with one CTA per row 32), else of 8192, two to an SM, of which
-  // one works while the other waits at a barrier (f32 [128, 65536] 368 us against 385 with one of 16384), which rows of
-  // more than 65536 elements, eight CTAs being the most, take.
-  if (n > kSmallRow && n <= kRadixMaxRow) {
-    if (n > kRadixTile) {
-      int cluster = (int)((n + 4095) / 4096);
-      if (cluster > 8 || rows * cluster > 148) cluster = (int)((n + kRadixTile - 1) / kRadixTile);
-      if (cluster > 8) cluster = rows * 8 <= 148 ? 8 : (int)((n + 2 * kRadixTile - 1) / (2 * kRadixTile));
-      if (cluster == 3) cluster = 4;   // clusters of three fill the GPU's groups of SMs badly (f32 [200, 20000] 179 us against 152)
-      int threads = (int)((n + cluster * 512 - 1) / (cluster * 512)) * 32;
-      if (threads < 256) threads = 256;
-      return launch_radix<DT, 16, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, cluster);
-    }
-    const int ipt = n <= (rows <= 296 ? 8192 : 3072) ? 8 : 16;
-    int threads = (int)((n + 32 * ipt - 1) / (32 * ipt)) * 32;
-    if (threads < 256) threads = 256;   // (a pass needs 256 threads for its 256 digits)
+  // Short rows take the network while there are few of them to fill the GPU or while it has few stages (f32, network / places:
+  // [64, 64] 3.5 us / 3.3, [300, 128] 4.8 / 4.3, [1024, 128] 6.8 / 7.9, [1024, 256] 8.8 / 8.3, [5000, 128] 20 / 30, [1024, 512] 12.7 / 9.3).
+  if (n <= kRadixMaxRow && n > (rows <= 512 ? 64 : 256)) {
+    const int cluster = places_cluster(rows, n);
+    if (cluster > 1) return launch_places<DT, 16, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, cluster);
+    // Four, eight or sixteen elements a thread: the fewest that still let all rows run at once (1024 threads an SM), because a
+    // CTA's latency grows with them; with rows in several waves sixteen, which need less of everything else (f32, eight / sixteen:
+    // [64, 4096] 7.6 us / 9.5, [300, 2049] 9.3 / 11.2, [1024, 2049] 22.4 / 23.0, [1024, 3001] 29.5 / 27.1, [1024, 8192] 77 / 65).
+    if (n <= 1024) return launch_places<DT, 4, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, 1);
     if (rows > 296 && n <= 2048 - 32 * 8)   // at least one warp of the 256 threads has no element
-      return launch_radix<DT, 8, false, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, 1);
-    if (ipt == 8) return launch_radix<DT, 8, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, 1);
-    return launch_radix<DT, 16, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, threads, 1);
+      return launch_places<DT, 8, false, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, 1);
+    if (n <= 2048 || (n <= 8192 && rows * ((n + 255) / 256 * 32) <= 148 * 1024))
+      return launch_places<DT, 8, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, 1);
+    return launch_places<DT, 16, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, 1);
   }
   if (n <= kSmallRow) {
     int threads = (int)(n_pad / 8);

@@ -1,10 +1,8 @@
-// Stable row-wise argsort by radix: least significant digit first, eight bits a pass, a row in the shared memory of one
-// CTA (up to 8192 elements) or of a cluster of CTAs (up to 131072).  Included by sort.cu.
+// Radix passes over a row's keys and positions, least significant digit first, eight bits a pass, in the shared memory of one
+// CTA or of a cluster of CTAs: what sort_places.cuh falls back to.
 //
-// What bounds it: integer instructions, which issue at half rate, about 130 of them an element and pass; four passes for
-// 32-bit keys and two for 16-bit ones, against 50 to 70 compare-exchanges of ten instructions an element of a bitonic
-// network on 64-bit composites.  Every pass keeps the order of equal digits, so the position need not be compared: it
-// travels beside the key.
+// What bounds them: barriers and shared-memory latency, then integer instructions that issue at half rate, 128 per 32 elements
+// and pass.  Every pass keeps the order of equal digits, so the position need not be compared: it travels beside the key.
 //
 // A pass.  A warp owns consecutive elements, 32 at a time; lanes with the same digit find each other with one ballot per
 // digit bit (__match_any_sync took half as long again), their number goes into the warp's own counter of the digit and
@@ -20,8 +18,7 @@
 namespace tlx {
 
 constexpr int kRadixMaxThreads = 1024;
-constexpr int kRadixTile = 8192;              // elements per CTA at most, of rows of up to eight of them
-constexpr int kRadixMaxRow = 16 * kRadixTile; // elements per row at most
+constexpr int kRadixMaxRow = 131072;   // elements per row at most
 
 // Order-preserving key of a type in its own number of bits, and back (-0 comes back as +0, NaN as the one NaN).
 template <int DT> struct RadixKey {
@@ -218,74 +215,6 @@ __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p
     for (int j = 0; j < IPT; ++j) get(threadIdx.x + j * nt, k[j], p[j]);
   }
   return scattered;
-}
-
-// Digit-wise difference of the CTA's keys from the row's first one, in every thread.
-__device__ __forceinline__ uint32_t radix_diff(uint32_t diff, RadixShared& s) {
-  diff = __reduce_or_sync(0xFFFFFFFFu, diff);
-  if (lane_id() == 0) s.warp[warp_id()] = diff;
-  __syncthreads();
-  return __reduce_or_sync(0xFFFFFFFFu, lane_id() < (int)(blockDim.x >> 5) ? s.warp[lane_id()] : 0u);
-}
-
-// Dynamic shared memory (cluster: keys and positions in pairs): RadixShared, counters [warps][256] u16, keys [cap] u32, positions [cap] u16 or (cluster) u32.
-__host__ __device__ __forceinline__ size_t radix_smem(int threads, int cap, bool cluster) {
-  return sizeof(RadixShared) + (size_t)(threads / 32) * 512 + (size_t)cap * (cluster ? 8 : 6);
-}
-
-template <int DT, int IPT, bool CL, bool PAST>
-__global__ void __launch_bounds__(kRadixMaxThreads) sort_radix_kernel(
-    const typename Elem<DT>::type* __restrict__ keys, const int32_t* __restrict__ in_perm, int64_t n, int descending,
-    typename Elem<DT>::type* __restrict__ out_keys, int32_t* __restrict__ out_perm, int cluster) {
-  using RK = RadixKey<DT>;
-  using Pos = typename std::conditional<CL, uint32_t, unsigned short>::type;
-  extern __shared__ __align__(16) unsigned char radix_raw[];
-  const int nt = blockDim.x, nw = nt >> 5, cap = nt * IPT;
-  RadixShared& s = *reinterpret_cast<RadixShared*>(radix_raw);
-  unsigned short* count = reinterpret_cast<unsigned short*>(radix_raw + sizeof(RadixShared));
-  uint32_t* sk = reinterpret_cast<uint32_t*>(count + nw * 256);
-  Pos* sp = reinterpret_cast<Pos*>(sk + cap);
-  const int rank = CL ? (int)cl_rank() : 0;
-  const int64_t row = CL ? blockIdx.x / cluster : blockIdx.x;
-  const int64_t c0 = (int64_t)rank * cap;
-  const auto* krow = keys + row * n;
-  const int32_t* prow = in_perm ? in_perm + row * n : nullptr;
-  const uint32_t ones = RK::kBits == 32 ? 0xFFFFFFFFu : 0xFFFFu, flip = descending ? ones : 0u;
-
-  // element w * 32 * IPT + 32 j + lane of the CTA; those past the row's end carry the greatest key and stay last
-  const int i0 = warp_id() * 32 * IPT + lane_id();
-  uint32_t k[IPT], p[IPT];
-  const uint32_t first = RK::make(krow[prow ? prow[0] : 0]) ^ flip;
-  uint32_t diff = 0;
-#pragma unroll
-  for (int j = 0; j < IPT; ++j) {
-    const int64_t c = c0 + i0 + 32 * j;
-    k[j] = ones;
-    if (c < n) {
-      k[j] = RK::make(krow[prow ? (int64_t)prow[c] : c]) ^ flip;
-      diff |= k[j] ^ first;
-    }
-    p[j] = (uint32_t)c;
-  }
-  diff = radix_diff(diff, s);
-  if constexpr (CL) {
-    if (threadIdx.x == 0) s.total[0] = diff;
-    cl_sync();
-    diff = __reduce_or_sync(0xFFFFFFFFu, cl_ld_u32(cl_map(&s.total[0], (uint32_t)(lane_id() < cluster ? lane_id() : 0))));
-    cl_sync();
-  } else {
-    __syncthreads();
-  }
-  const bool scattered = radix_by_digits<IPT, RK::kBits, CL, PAST, Pos>(k, p, diff, (int)n, rank, cluster, s, count, sk, sp);
-  if constexpr (CL) cl_sync();   // (nobody leaves while another one may still read its counts)
-#pragma unroll
-  for (int j = 0; j < IPT; ++j) {
-    const int64_t c = c0 + (scattered ? (int)threadIdx.x + j * nt : i0 + 32 * j);
-    if (c < n) {
-      if (out_keys) out_keys[row * n + c] = RK::back(k[j] ^ flip);
-      if (out_perm) out_perm[row * n + c] = prow ? prow[p[j]] : (int32_t)p[j];
-    }
-  }
 }
 
 }  // namespace tlx

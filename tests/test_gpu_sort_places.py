@@ -1,0 +1,57 @@
+"""GPU: the sort by estimated places, one row of every kind that its branches tell apart, at the edges of its kernels' sizes.
+
+The expectation is numpy's stable argsort: sorting is exact, so there is no tolerance.
+"""
+import numpy as np
+import pytest
+import torch
+
+from tallax_b200 import tax
+
+pytestmark = pytest.mark.gpu
+
+
+def _rows(n, rng):
+    """Even keys; few values (the radix passes from the start); one value; a third of the row one value (more than its owner
+    has room for); in order, and in reverse order; keys over the whole range of exponents; values that occur dozens and
+    hundreds of times (large groups); every other element the same; a mask; two outliers that leave the rest one range."""
+    z = rng.standard_normal(n).astype(np.float32)
+    rare = np.clip(z, -4, 4) * np.float32(1e-6) + 1
+    rare[0], rare[-1] = 3e38, -3e38
+    return np.stack([z, np.round(z * 3), np.zeros(n, np.float32), np.where(rng.random(n) < 0.3, np.float32(np.inf), z),
+                     np.sort(z), -np.sort(z), np.exp(np.clip(z, -4, 4) * 20).astype(np.float32),
+                     rng.choice(z[:max(1, n // 40)], n), rng.choice(z[:max(1, n // 300)], n),
+                     np.where(np.arange(n) % 2 == 0, np.float32(3), z),
+                     np.where(np.arange(n) > n // 3, np.float32(-np.inf), z), rare])
+
+
+# (copies of the rows, elements): four, eight and sixteen elements a thread, warps past the end; clusters of CTAs of 4096, 8192
+# and 16384 elements; the rows that are too many for the shortest lengths
+@pytest.mark.parametrize("copies,n", [(1, 65), (1, 1024), (50, 65), (50, 256), (50, 257), (1, 1025), (30, 1792), (30, 1793), (30, 2049),
+                                      (1, 8192), (20, 8192), (1, 10000), (1, 10001), (15, 16384), (1, 16385), (6, 20000), (10, 24577),
+                                      (4, 65536), (12, 65536), (1, 131071), (2, 131072)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "i32"])
+def test_sort_by_places(cuda, dtype, copies, n):
+    rng = np.random.default_rng(n)
+    x = _rows(n, rng)
+    if dtype == "i32":
+        x = (np.clip(x, -1e4, 1e4) * 2e5).astype(np.int32)      # (the outliers are the type's limits, nearly)
+        t, a = torch.from_numpy(x), x.astype(np.int64)
+    else:
+        t = torch.from_numpy(x).to(torch.bfloat16 if dtype == "bf16" else torch.float32)
+        a = t.float().numpy()
+    for descending in (False, True):
+        v, p = tax.sort([t.to(cuda).repeat(copies, 1)], num_keys=1, is_stable=True, return_argsort=True, descending=descending)
+        e = np.argsort(-a if descending else a, axis=1, kind="stable")
+        assert np.array_equal(p.cpu().numpy(), np.tile(e, (copies, 1)))
+        assert torch.equal(v.cpu(), torch.take_along_dim(t, torch.from_numpy(e), 1).repeat(copies, 1))
+
+
+# through a permutation, which a second key does
+@pytest.mark.parametrize("n", [1000, 4097, 20000])
+def test_sort_by_places_of_two_keys(cuda, n):
+    rng = np.random.default_rng(n)
+    first, x = rng.integers(0, 3, (12, n)).astype(np.int32), _rows(n, rng)
+    out = tax.sort([torch.from_numpy(first).to(cuda), torch.from_numpy(x).to(cuda)], num_keys=2, is_stable=True, return_argsort=True)
+    e = np.stack([np.lexsort((x[r], first[r])) for r in range(12)])
+    assert np.array_equal(out[-1].cpu().numpy(), e)
