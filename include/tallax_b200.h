@@ -109,6 +109,22 @@ int tlx_sort(void* stream, const void* keys, int dtype, int64_t rows, int64_t n,
              const int32_t* in_perm, void* out_keys, int32_t* out_perm, void* workspace,
              size_t workspace_bytes);
 
+/* ---- sort of keys with payloads --------------------------------------------------
+ * tlx_sort, and arrays of the keys' shape that are brought into the same order by the kernel that ends the sort: payloads and
+ * further keys, up to TLX_SORT_MAX_CARRIED of them, of 2- or 4-byte elements.  key_dtype: -1, or the dtype of a further key,
+ * which leaves in canonical form as out_keys does.  No array may overlap another one's output.
+ * Replaces the operands beside the first key of tallax/_src/sort.py:768-929.        */
+#define TLX_SORT_MAX_CARRIED 4
+typedef struct {
+  const void* in;
+  void* out;
+  int32_t bytes;        /* 2 or 4 */
+  int32_t key_dtype;
+} tlx_sort_carried;
+int tlx_sort_carry(void* stream, const void* keys, int dtype, int64_t rows, int64_t n, int descending,
+                   const int32_t* in_perm, void* out_keys, int32_t* out_perm, const tlx_sort_carried* carried,
+                   int count, void* workspace, size_t workspace_bytes);
+
 /* ---- sort without any allocation ------------------------------------------------
  * Same operation and results as tlx_sort, for callers that have nowhere to get scratch
  * memory from: plugin hosts whose memory pool is owned by another runtime, or processes that

@@ -30,6 +30,7 @@ SIGNATURES = {
     "tlx_argmax": (_i32, [_vp, _vp, _i32, _i64, _i64, _i32, _vp]),
     "tlx_sort_workspace_bytes": (_sz, [_i64, _i64]),
     "tlx_sort": (_i32, [_vp, _vp, _i32, _i64, _i64, _i32, _vp, _vp, _vp, _vp, _sz]),
+    "tlx_sort_carry": (_i32, [_vp, _vp, _i32, _i64, _i64, _i32, _vp, _vp, _vp, _vp, _i32, _vp, _sz]),
     "tlx_sort_static_max_bytes": (_sz, []),
     "tlx_sort_static": (_i32, [_vp, _vp, _i32, _i64, _i64, _i32, _vp, _vp, _vp]),
     "tlx_top_k_workspace_bytes": (_sz, [_i64, _i64, _i32]),
@@ -69,8 +70,8 @@ SIGNATURES = {
 
 BINDING_PATH = os.path.join(_HERE, "lib", "_tlx_torch.so")
 # the library functions that the binding calls
-_BOUND = ("tlx_sample", "tlx_sample_workspace_bytes", "tlx_top_k", "tlx_top_k_workspace_bytes", "tlx_sort",
-          "tlx_sort_workspace_bytes", "tlx_take_along_axis", "tlx_cumsum", "tlx_exchange_shard_candidates",
+_BOUND = ("tlx_sample", "tlx_sample_workspace_bytes", "tlx_top_k", "tlx_top_k_workspace_bytes",
+          "tlx_sort_carry", "tlx_sort_workspace_bytes", "tlx_take_along_axis", "tlx_cumsum", "tlx_exchange_shard_candidates",
           "tlx_exchange_merge_and_sample")
 
 _lib = None

@@ -154,11 +154,20 @@ def argmax(keys: torch.Tensor, axis: int) -> torch.Tensor:
 
 
 def argsort_rows(keys: torch.Tensor, descending: bool = False, in_perm: torch.Tensor | None = None,
-                 want_keys: bool = True, want_perm: bool = True):
-    """Stable argsort of every row; returns (sorted_keys | None, perm | None)."""
-    out = _lib.native().argsort_rows(keys, descending, in_perm, want_keys, want_perm)
+                 want_keys: bool = True, want_perm: bool = True, carried: tuple = (), further_keys: int = 0):
+    """Stable argsort of every row; returns (sorted_keys | None, perm | None, *carried in the same order).
+
+    carried: operands of the keys' shape, the first `further_keys` of them keys, which leave in canonical form.
+    """
+    out = _lib.native().argsort_rows(keys, descending, in_perm, want_keys, want_perm, carried, further_keys)
     if out is not NotImplemented:
         return out
+    if carried:   # too many of them, or of a kind that the sort's kernels don't move
+        out_keys, out_perm = argsort_rows(keys, descending, in_perm, want_keys)
+        gathered = [take_along_axis(x, out_perm, 1) for x in carried]
+        for x in gathered[:further_keys]:
+            canonicalize_keys_(x)
+        return (out_keys, out_perm if want_perm else None, *gathered)
     keys = _dev(keys)
     rows, n = keys.shape
     lib = _lib.load()

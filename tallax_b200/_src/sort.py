@@ -17,12 +17,6 @@ def canonicalize_operand(operand):
     return operands, shapes[0]
 
 
-def _canonical_float(x):
-    # what a key looks like after the key-domain round trip (-0 -> +0, canonical NaN): in place, by the
-    # library's own kernel (x is the freshly gathered output)
-    return ops.canonicalize_keys_(x)
-
-
 def sort(operand, num_keys: int, is_stable: bool = False, return_argsort: bool = False, descending: bool = False,
          num_vmem_substages=None, block_token=None, interpret: bool = False):
     """Row-wise sort of one or several [rows, n] tensors.
@@ -35,19 +29,11 @@ def sort(operand, num_keys: int, is_stable: bool = False, return_argsort: bool =
     operands, shape = canonicalize_operand(operand)
     if not 1 <= num_keys <= len(operands):
         raise ValueError("num_keys must be between 1 and the number of operands")
-    # least-significant key first; each pass is a stable argsort composed with the previous permutation
+    # least-significant key first; each pass is a stable argsort composed with the previous permutation, and the last one,
+    # of the first key, brings the other operands into order
     perm = None
-    sorted_first = None
-    for j in reversed(range(num_keys)):
-        want_keys = j == 0
-        sorted_first, perm = ops.argsort_rows(operands[j], descending=descending, in_perm=perm, want_keys=want_keys)
-    outs = []
-    for i, x in enumerate(operands):
-        if i == 0:
-            outs.append(sorted_first)
-        else:
-            g = ops.take_along_axis(x, perm, 1)
-            outs.append(_canonical_float(g) if i < num_keys else g)
-    if return_argsort:
-        outs.append(perm)
-    return tuple(outs)
+    for j in reversed(range(1, num_keys)):
+        _, perm = ops.argsort_rows(operands[j], descending=descending, in_perm=perm, want_keys=False)
+    first, perm, *rest = ops.argsort_rows(operands[0], descending=descending, in_perm=perm, want_perm=return_argsort,
+                                          carried=tuple(operands[1:]), further_keys=num_keys - 1)
+    return (first, *rest, perm) if return_argsort else (first, *rest)

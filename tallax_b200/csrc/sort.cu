@@ -98,22 +98,25 @@ __device__ __forceinline__ void tile_substages(uint64_t* a, int tile, int64_t ba
 }
 
 template <int DT>
-__device__ __forceinline__ void emit(uint64_t v, int64_t c, int64_t n, bool descending,
-                                     const int32_t* __restrict__ prow, typename Elem<DT>::type* __restrict__ okeys,
-                                     int32_t* __restrict__ operm) {
+__device__ __forceinline__ void emit(uint64_t v, int64_t c, int64_t row0, int64_t n, bool descending,
+                                     const int32_t* __restrict__ prow, typename Elem<DT>::type* __restrict__ out_keys,
+                                     int32_t* __restrict__ out_perm, const SortCarry& carry) {
   if (c >= n) return;
   uint32_t k = (uint32_t)(v >> 32);
   if (descending) k = ~k;
-  const int32_t pos = (int32_t)(uint32_t)v;
-  if (okeys) okeys[c] = Elem<DT>::from_key(k);
-  if (operm) operm[c] = prow ? prow[pos] : pos;
+  int32_t pos = (int32_t)(uint32_t)v;
+  if (prow) pos = prow[pos];
+  if (out_keys) out_keys[row0 + c] = Elem<DT>::from_key(k);
+  if (out_perm) out_perm[row0 + c] = pos;
+  carry_one(carry, row0 + pos, row0 + c);
 }
 
 // Whole row in one tile: build, sort, emit.  n_pad (power of two) <= kSmallRow.
 template <int DT>
 __global__ void __launch_bounds__(kSortThreads) sort_small_kernel(
     const typename Elem<DT>::type* __restrict__ keys, const int32_t* __restrict__ in_perm, int64_t n, int n_pad,
-    int descending, typename Elem<DT>::type* __restrict__ out_keys, int32_t* __restrict__ out_perm) {
+    int descending, typename Elem<DT>::type* __restrict__ out_keys, int32_t* __restrict__ out_perm,
+    const __grid_constant__ SortCarry carry) {
   extern __shared__ uint64_t tile_smem[];
   const int64_t r = blockIdx.x;
   const auto* krow = keys + r * n;
@@ -123,8 +126,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_small_kernel(
   __syncthreads();
   for (int k = 2; k <= n_pad; k <<= 1) tile_substages(tile_smem, n_pad, 0, k, k >> 1);
   for (int c = threadIdx.x; c < n_pad; c += blockDim.x)
-    emit<DT>(tile_smem[pad_idx(c)], c, n, descending, prow, out_keys ? out_keys + r * n : nullptr,
-             out_perm ? out_perm + r * n : nullptr);
+    emit<DT>(tile_smem[pad_idx(c)], c, r * n, n, descending, prow, out_keys, out_perm, carry);
 }
 
 // Long rows, step 1: build composites of one tile and run stages 2..kTile on it.
@@ -172,7 +174,7 @@ template <int DT>
 __global__ void __launch_bounds__(kSortThreads) sort_near_kernel(
     uint64_t* __restrict__ ws, int64_t n, int64_t n_pad, int64_t k, int last, int descending,
     const int32_t* __restrict__ in_perm, typename Elem<DT>::type* __restrict__ out_keys,
-    int32_t* __restrict__ out_perm) {
+    int32_t* __restrict__ out_perm, const __grid_constant__ SortCarry carry) {
   extern __shared__ uint64_t tile_smem[];
   const int64_t tiles_per_row = n_pad / kTile;
   const int64_t r = blockIdx.x / tiles_per_row;
@@ -186,8 +188,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_near_kernel(
   } else {
     const int32_t* prow = in_perm ? in_perm + r * n : nullptr;
     for (int c = threadIdx.x; c < kTile; c += blockDim.x)
-      emit<DT>(tile_smem[pad_idx(c)], base + c, n, descending, prow, out_keys ? out_keys + r * n : nullptr,
-               out_perm ? out_perm + r * n : nullptr);
+      emit<DT>(tile_smem[pad_idx(c)], base + c, r * n, n, descending, prow, out_keys, out_perm, carry);
   }
 }
 
@@ -223,7 +224,7 @@ static int places_cluster(int64_t rows, int64_t n) {
 
 template <int DT, int IPT, bool CL, bool PAST = false>
 static int launch_places(cudaStream_t st, const void* keys, int64_t rows, int64_t n, int descending, const int32_t* in_perm,
-                         void* out_keys, int32_t* out_perm, int cluster) {
+                         void* out_keys, int32_t* out_perm, const SortCarry& carry, int cluster) {
   using T = typename Elem<DT>::type;
   // the radix passes need 256 threads for their 256 digits
   const int64_t share = (n + (int64_t)cluster * 32 * IPT - 1) / ((int64_t)cluster * 32 * IPT) * 32;
@@ -246,7 +247,7 @@ static int launch_places(cudaStream_t st, const void* keys, int64_t rows, int64_
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = CL ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, sort_places_kernel<DT, IPT, CL, PAST>, (const T*)keys, in_perm, n, descending, (T*)out_keys, out_perm, cluster);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, sort_places_kernel<DT, IPT, CL, PAST>, (const T*)keys, in_perm, n, descending, (T*)out_keys, out_perm, cluster, carry);
   if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "sort: %s", cudaGetErrorString(e)); }
   count_launch();
   return TLX_OK;
@@ -254,7 +255,7 @@ static int launch_places(cudaStream_t st, const void* keys, int64_t rows, int64_
 
 template <int DT>
 static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_t n, int descending,
-                         const int32_t* in_perm, void* out_keys, int32_t* out_perm, void* workspace,
+                         const int32_t* in_perm, void* out_keys, int32_t* out_perm, const SortCarry& carry, void* workspace,
                          size_t workspace_bytes) {
   using T = typename Elem<DT>::type;
   const int64_t n_pad = next_pow2(n < 2 ? 2 : n);
@@ -263,23 +264,23 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
   // [64, 64] 3.5 us / 3.3, [300, 128] 4.8 / 4.3, [1024, 128] 6.8 / 7.9, [1024, 256] 8.8 / 8.3, [5000, 128] 20 / 30, [1024, 512] 12.7 / 9.3).
   if (n <= kRadixMaxRow && n > (rows <= 512 ? 64 : 256)) {
     const int cluster = places_cluster(rows, n);
-    if (cluster > 1) return launch_places<DT, 16, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, cluster);
+    if (cluster > 1) return launch_places<DT, 16, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, carry, cluster);
     // Four, eight or sixteen elements a thread: the fewest that still let all rows run at once (1024 threads an SM), because a
     // CTA's latency grows with them; with rows in several waves sixteen, which need less of everything else (f32, eight / sixteen:
     // [64, 4096] 7.6 us / 9.5, [300, 2049] 9.3 / 11.2, [1024, 2049] 22.4 / 23.0, [1024, 3001] 29.5 / 27.1, [1024, 8192] 77 / 65).
-    if (n <= 1024) return launch_places<DT, 4, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, 1);
+    if (n <= 1024) return launch_places<DT, 4, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, carry, 1);
     if (rows > 296 && n <= 2048 - 32 * 8)   // at least one warp of the 256 threads has no element
-      return launch_places<DT, 8, false, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, 1);
+      return launch_places<DT, 8, false, true>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, carry, 1);
     if (n <= 2048 || (n <= 8192 && rows * ((n + 255) / 256 * 32) <= 148 * 1024))
-      return launch_places<DT, 8, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, 1);
-    return launch_places<DT, 16, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, 1);
+      return launch_places<DT, 8, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, carry, 1);
+    return launch_places<DT, 16, false>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, carry, 1);
   }
   if (n <= kSmallRow) {
     int threads = (int)(n_pad / 8);
     if (threads < 64) threads = 64;
     static_assert(padded_bytes(kSmallRow) <= 48 * 1024, "no limit has to be raised");
     sort_small_kernel<DT><<<(unsigned)rows, threads, padded_bytes((size_t)n_pad), st>>>(
-        (const T*)keys, in_perm, n, (int)n_pad, descending, (T*)out_keys, out_perm);
+        (const T*)keys, in_perm, n, (int)n_pad, descending, (T*)out_keys, out_perm, carry);
     TLX_CHECK_LAUNCH("sort (single tile)");
     return TLX_OK;
   }
@@ -310,7 +311,7 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
       j >>= nsub;
     }
     sort_near_kernel<DT><<<tiles, kSortThreads, smem, st>>>(ws, n, n_pad, k, k == n_pad, descending, in_perm,
-                                                             (T*)out_keys, out_perm);
+                                                             (T*)out_keys, out_perm, carry);
     TLX_CHECK_LAUNCH("sort (near substages)");
   }
   return TLX_OK;
@@ -335,23 +336,43 @@ size_t tlx_sort_workspace_bytes(int64_t rows, int64_t n) {
   return (size_t)rows * (size_t)n_pad * 8;
 }
 
-int tlx_sort(void* stream, const void* keys, int dtype, int64_t rows, int64_t n, int descending,
-             const int32_t* in_perm, void* out_keys, int32_t* out_perm, void* workspace, size_t workspace_bytes) {
+int tlx_sort_carry(void* stream, const void* keys, int dtype, int64_t rows, int64_t n, int descending, const int32_t* in_perm,
+                   void* out_keys, int32_t* out_perm, const tlx_sort_carried* carried, int count, void* workspace,
+                   size_t workspace_bytes) {
   cudaStream_t st = (cudaStream_t)stream;
   TLX_CHECK_ARG(rows >= 0 && n >= 0, "sort: negative extent");
   if (rows == 0 || n == 0) return TLX_OK;
   TLX_CHECK_ARG(keys, "sort: null keys");
-  TLX_CHECK_ARG(out_keys || out_perm, "sort: no output requested");
+  TLX_CHECK_ARG(count >= 0 && count <= TLX_SORT_MAX_CARRIED && (count == 0 || carried), "sort: 0 to %d arrays can be carried, got %d",
+                TLX_SORT_MAX_CARRIED, count);
+  TLX_CHECK_ARG(out_keys || out_perm || count, "sort: no output requested");
   TLX_CHECK_ARG(n < (1ll << 31), "sort: row length %lld does not fit an int32 position", (long long)n);
   TLX_CHECK_ARG(rows * (next_pow2(n) / (n > kTile ? kTile : next_pow2(n))) < (1ll << 31), "sort: too many tiles");
+  SortCarry c{};
+  c.count = count;
+  for (int i = 0; i < count; ++i) {
+    const tlx_sort_carried& a = carried[i];
+    TLX_CHECK_ARG(a.in && a.out, "sort: null pointer among the carried arrays");
+    TLX_CHECK_ARG((a.bytes == 2 || a.bytes == 4) && (a.key_dtype < 0 || dtype_bytes(a.key_dtype) == a.bytes),
+                  "sort: a carried array has elements of 2 or 4 bytes, its dtype's, got %d", (int)a.bytes);
+    c.in[i] = a.in;
+    c.out[i] = a.out;
+    c.bytes[i] = a.bytes;
+    c.key_dtype[i] = a.key_dtype;
+  }
   switch (dtype) {
-    case TLX_F32: return sort_dispatch<TLX_F32>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, workspace, workspace_bytes);
-    case TLX_BF16: return sort_dispatch<TLX_BF16>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, workspace, workspace_bytes);
-    case TLX_F16: return sort_dispatch<TLX_F16>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, workspace, workspace_bytes);
-    case TLX_I32: return sort_dispatch<TLX_I32>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, workspace, workspace_bytes);
-    case TLX_U32: return sort_dispatch<TLX_U32>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, workspace, workspace_bytes);
+    case TLX_F32: return sort_dispatch<TLX_F32>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, c, workspace, workspace_bytes);
+    case TLX_BF16: return sort_dispatch<TLX_BF16>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, c, workspace, workspace_bytes);
+    case TLX_F16: return sort_dispatch<TLX_F16>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, c, workspace, workspace_bytes);
+    case TLX_I32: return sort_dispatch<TLX_I32>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, c, workspace, workspace_bytes);
+    case TLX_U32: return sort_dispatch<TLX_U32>(st, keys, rows, n, descending, in_perm, out_keys, out_perm, c, workspace, workspace_bytes);
     default: return set_error(TLX_ERR_UNSUPPORTED, "sort: dtype %d not supported", dtype);
   }
+}
+
+int tlx_sort(void* stream, const void* keys, int dtype, int64_t rows, int64_t n, int descending,
+             const int32_t* in_perm, void* out_keys, int32_t* out_perm, void* workspace, size_t workspace_bytes) {
+  return tlx_sort_carry(stream, keys, dtype, rows, n, descending, in_perm, out_keys, out_perm, nullptr, 0, workspace, workspace_bytes);
 }
 
 size_t tlx_sort_static_max_bytes(void) { return kStaticSortBytes; }

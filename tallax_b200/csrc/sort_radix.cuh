@@ -46,6 +46,30 @@ template <> struct RadixKey<TLX_F16> {
   static __device__ __forceinline__ __half back(uint32_t k) { return __ushort_as_half(radix_half_back(k)); }
 };
 
+// What is brought into the keys' order: payloads, and further keys, which leave in canonical form.
+struct SortCarry {
+  const void* in[TLX_SORT_MAX_CARRIED];
+  void* out[TLX_SORT_MAX_CARRIED];
+  int bytes[TLX_SORT_MAX_CARRIED];
+  int key_dtype[TLX_SORT_MAX_CARRIED];   // -1: not a key
+  int count;
+};
+// Element `from` of the arrays to their element `to`.
+__device__ __forceinline__ void carry_one(const SortCarry& c, int64_t from, int64_t to) {
+#pragma unroll
+  for (int i = 0; i < TLX_SORT_MAX_CARRIED; ++i) {
+    if (i >= c.count) break;
+    const int key = c.key_dtype[i];
+    if (c.bytes[i] == 4) {
+      const uint32_t v = __ldg(reinterpret_cast<const uint32_t*>(c.in[i]) + from);
+      reinterpret_cast<uint32_t*>(c.out[i])[to] = key == TLX_F32 ? __float_as_uint(key_f32(f32_key(__uint_as_float(v)))) : v;
+    } else {
+      const uint32_t v = __ldg(reinterpret_cast<const unsigned short*>(c.in[i]) + from), inf = key == TLX_BF16 ? 0x7F80u : 0x7C00u;
+      reinterpret_cast<unsigned short*>(c.out[i])[to] = key >= 0 ? radix_half_back(radix_key_half(v, inf)) : (unsigned short)v;
+    }
+  }
+}
+
 struct __align__(16) RadixShared {
   uint32_t total[256];    // elements of every digit in this CTA
   int shift_by[256];      // cluster: place in the row - place in the CTA

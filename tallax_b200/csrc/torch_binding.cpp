@@ -28,7 +28,7 @@ struct Lib {
   decltype(&tlx_sample_workspace_bytes) sample_workspace_bytes;
   decltype(&tlx_top_k) top_k;
   decltype(&tlx_top_k_workspace_bytes) top_k_workspace_bytes;
-  decltype(&tlx_sort) sort;
+  decltype(&tlx_sort_carry) sort_carry;
   decltype(&tlx_sort_workspace_bytes) sort_workspace_bytes;
   decltype(&tlx_take_along_axis) take_along_axis;
   decltype(&tlx_cumsum) cumsum;
@@ -182,40 +182,60 @@ PyObject* py_top_k(PyObject*, PyObject* const* a, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-// argsort_rows(keys, descending, in_perm or None, want_keys, want_perm) -> (keys or None, perm or None)
+// argsort_rows(keys, descending, in_perm or None, want_keys, want_perm, carried, keys_among_them)
+//   -> (keys or None, perm or None, *carried in the same order)
+// carried: a tuple of tensors of the keys' shape, of which the first keys_among_them are further keys
 PyObject* py_argsort_rows(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  if (n != 5) TLX_NOT_MINE;
+  if (n != 7) TLX_NOT_MINE;
   const int dev = device_of(a[0]);
   if (dev < 0) TLX_NOT_MINE;
   const at::Tensor* x = plain(a[0], dev);
   if (!x || x->dim() != 2) TLX_NOT_MINE;
   const int64_t rows = x->size(0), cols = x->size(1);
   const int dt = dtype_code(x->scalar_type());
+  auto same_shape = [&](const at::Tensor* t) { return t && t->dim() == 2 && t->size(0) == rows && t->size(1) == cols; };
   const at::Tensor* perm_in = nullptr;
   if (a[2] != Py_None) {
     perm_in = plain(a[2], dev, at::kInt);
-    if (!perm_in || perm_in->dim() != 2 || perm_in->size(0) != rows || perm_in->size(1) != cols) TLX_NOT_MINE;
+    if (!same_shape(perm_in)) TLX_NOT_MINE;
   }
   const int desc = PyObject_IsTrue(a[1]), want_keys = PyObject_IsTrue(a[3]), want_perm = PyObject_IsTrue(a[4]);
-  if (dt < 0 || desc < 0 || want_keys < 0 || want_perm < 0 || rows == 0 || cols == 0) { PyErr_Clear(); TLX_NOT_MINE; }
-  at::Tensor keys, perm, ws;
+  int64_t further;
+  if (dt < 0 || desc < 0 || want_keys < 0 || want_perm < 0 || rows == 0 || cols == 0 || !PyTuple_CheckExact(a[5]) ||
+      !as_i64(a[6], &further)) { PyErr_Clear(); TLX_NOT_MINE; }
+  const Py_ssize_t count = PyTuple_GET_SIZE(a[5]);
+  if (count > TLX_SORT_MAX_CARRIED) TLX_NOT_MINE;
+  const at::Tensor* carried[TLX_SORT_MAX_CARRIED];
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    carried[i] = plain(PyTuple_GET_ITEM(a[5], i), dev);
+    if (!same_shape(carried[i]) || (carried[i]->element_size() != 2 && carried[i]->element_size() != 4)) TLX_NOT_MINE;
+    if (i < further && dtype_code(carried[i]->scalar_type()) < 0) TLX_NOT_MINE;
+  }
+  at::Tensor keys, perm, ws, outs[TLX_SORT_MAX_CARRIED];
+  tlx_sort_carried c[TLX_SORT_MAX_CARRIED];
   if (want_keys) keys = empty({rows, cols}, x->scalar_type(), dev);
   if (want_perm) perm = empty({rows, cols}, at::kInt, dev);
+  for (Py_ssize_t i = 0; i < count; ++i) {
+    outs[i] = empty({rows, cols}, carried[i]->scalar_type(), dev);
+    c[i] = {carried[i]->data_ptr(), outs[i].data_ptr(), (int32_t)carried[i]->element_size(),
+            i < further ? dtype_code(carried[i]->scalar_type()) : -1};
+  }
   const size_t ws_bytes = cols > TLX_SORT_NO_WORKSPACE_N ? lib.sort_workspace_bytes(rows, cols) : 0;
   if (ws_bytes) ws = empty({(int64_t)ws_bytes}, at::kByte, dev);
   void* st = c10::cuda::getCurrentCUDAStream(dev).stream();
   int rc;
   Py_BEGIN_ALLOW_THREADS
-  rc = lib.sort(st, x->data_ptr(), dt, rows, cols, desc, perm_in ? (const int32_t*)perm_in->data_ptr() : nullptr,
-                want_keys ? keys.data_ptr() : nullptr, want_perm ? (int32_t*)perm.data_ptr() : nullptr,
-                ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? ws_bytes : 0);
+  rc = lib.sort_carry(st, x->data_ptr(), dt, rows, cols, desc, perm_in ? (const int32_t*)perm_in->data_ptr() : nullptr,
+                      want_keys ? keys.data_ptr() : nullptr, want_perm ? (int32_t*)perm.data_ptr() : nullptr, c, (int)count,
+                      ws.defined() ? ws.data_ptr() : nullptr, ws.defined() ? ws_bytes : 0);
   Py_END_ALLOW_THREADS
   if (!finish(rc)) return nullptr;
-  PyObject* out = PyTuple_New(2);
+  PyObject* out = PyTuple_New(2 + count);
   if (!out) return nullptr;
   PyTuple_SET_ITEM(out, 0, want_keys ? THPVariable_Wrap(keys) : Py_NewRef(Py_None));
   PyTuple_SET_ITEM(out, 1, want_perm ? THPVariable_Wrap(perm) : Py_NewRef(Py_None));
+  for (Py_ssize_t i = 0; i < count; ++i) PyTuple_SET_ITEM(out, 2 + i, THPVariable_Wrap(outs[i]));
   return out;
   END_HANDLE_TH_ERRORS
 }
@@ -329,7 +349,7 @@ PyObject* py_init(PyObject*, PyObject* const* a, Py_ssize_t n) {
   TLX_BIND(sample_workspace_bytes)
   TLX_BIND(top_k)
   TLX_BIND(top_k_workspace_bytes)
-  TLX_BIND(sort)
+  TLX_BIND(sort_carry)
   TLX_BIND(sort_workspace_bytes)
   TLX_BIND(take_along_axis)
   TLX_BIND(cumsum)

@@ -55,3 +55,32 @@ def test_sort_by_places_of_two_keys(cuda, n):
     out = tax.sort([torch.from_numpy(first).to(cuda), torch.from_numpy(x).to(cuda)], num_keys=2, is_stable=True, return_argsort=True)
     e = np.stack([np.lexsort((x[r], first[r])) for r in range(12)])
     assert np.array_equal(out[-1].cpu().numpy(), e)
+
+
+# operands beside the first key, moved by the kernel that ends the sort: two and four bytes an element, further keys (whose -0
+# and NaNs become canonical), rows of the network, of the places and of the tiles; and the kinds that are gathered afterwards
+@pytest.mark.parametrize("n", [40, 1000, 4097, 20000, 131073])
+@pytest.mark.parametrize("payloads", [("i32",), ("bf16",), ("i32", "bf16", "f32", "f16"), ("i64",), ("i32",) * 5])
+@pytest.mark.parametrize("key", ["f32", "bf16", "i32"])
+def test_operands_beside_the_first_key(cuda, n, payloads, key):
+    types = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16, "i32": torch.int32, "i64": torch.int64}
+    gen = torch.Generator().manual_seed(n)
+    first = torch.randint(0, 3, (3, n), generator=gen, dtype=torch.int32)
+    second = torch.randn((3, n), generator=gen) * 100
+    if key != "i32":
+        second[:, ::5], second[:, 1::5], second[:, 2::9] = 0.0, -0.0, float("nan")
+    second = second.to(types[key])
+    rest = [torch.randint(0, 1000, (3, n), generator=gen).to(types[t]) for t in payloads]
+    out = tax.sort([t.to(cuda) for t in (first, second, *rest)], num_keys=2, is_stable=True)
+    v = second.float().numpy().astype(np.float64)
+    v = np.where(np.isnan(v), np.inf, v)
+    perm = torch.from_numpy(np.stack([np.lexsort((v[r], first[r].numpy())) for r in range(3)]))
+    want = [torch.take_along_dim(t, perm, 1) for t in (first, second, *rest)]
+    assert len(out) == len(want)
+    for i, (g, e) in enumerate(zip(out, want)):
+        g = g.cpu()
+        assert g.dtype == e.dtype
+        if i == 1 and key != "i32":
+            assert torch.equal(g.isnan(), e.isnan()) and not torch.signbit(g[g == 0]).any()
+            g, e = g.nan_to_num(nan=1e9), e.nan_to_num(nan=1e9)
+        assert torch.equal(g, e)
