@@ -373,6 +373,7 @@ __global__ void __launch_bounds__(kMergeThreads) merge_and_sample_kernel(MergePa
         if (p.status) atomicExch(p.status, 2);
         p.out[r] = -1;
       }
+      if (blockIdx.x == gridDim.x - 1) grid_wait();
       return;
     }
     if (threadIdx.x == 0) {
@@ -488,6 +489,8 @@ __global__ void __launch_bounds__(kMergeThreads) merge_and_sample_kernel(MergePa
       }
     }
   }
+  // (exchange mode: this kernel is not complete before the candidate kernel is, for what follows on the stream)
+  if (xh && blockIdx.x == gridDim.x - 1) grid_wait();
 }
 
 // ---------------------------------------------------------------------------------
@@ -650,40 +653,6 @@ static int debug_stages() {
   return v;
 }
 
-// Launches a kernel that may start while its predecessor on the stream still runs (programmatic dependent
-// launch): the kernel does whatever needs none of the predecessor's results and then executes
-// griddepcontrol.wait, which returns when the predecessor has finished and its writes are visible.  Where
-// the attribute is not accepted the kernel is launched in plain stream order (the wait is then a no-op).
-// carveout: the share of an SM's memory it prefers as shared memory, in percent; -1: as set for the kernel.
-template <typename... Params, typename... Args>
-static int launch_dependent(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t st,
-                            const char* what, int carveout, Args... args) {
-  static bool programmatic = getenv("TLX_NO_DEPENDENT_LAUNCH") == nullptr;
-  if (programmatic) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[2]{};
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
-    attr[1].val.sharedMemCarveout = (unsigned)carveout;
-    cfg.attrs = attr;
-    cfg.numAttrs = carveout >= 0 ? 2 : 1;
-    if (cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...) == cudaSuccess) {
-      count_launch();
-      return TLX_OK;
-    }
-    cudaGetLastError();
-    programmatic = false;
-  }
-  kernel<<<grid, block, smem, st>>>(static_cast<Params>(args)...);
-  TLX_CHECK_LAUNCH(what);
-  return TLX_OK;
-}
-
 // ---- cluster path (sampler_cluster.cuh) -----------------------------------------------------------------------
 template <int DT>
 static int launch_cluster_path(cudaStream_t st, const SampleParams& sp) {
@@ -712,21 +681,7 @@ static int launch_cluster_path(cudaStream_t st, const SampleParams& sp) {
       if (dev >= 0 && dev < 64) done[dev] = true;
     }
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(sp.rows * p.cluster));
-  cfg.blockDim = dim3(kRcThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)p.cluster;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, sample_cluster_kernel<DT>, p);
-  if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "sample: %s", cudaGetErrorString(e)); }
-  count_launch();
-  return TLX_OK;
+  return launch_dependent(sample_cluster_kernel<DT>, {(unsigned)(sp.rows * p.cluster), kRcThreads, smem, p.cluster}, st, "sample", p);
 }
 
 static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* workspace) {
@@ -792,16 +747,14 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
 #else
 #define TLX_TIMELINE_KERNEL(k) do {} while (0)
 #endif
-  sample_prologue_kernel<<<(unsigned)sp.rows, kStProThreads, 0, st>>>(p);
-  TLX_CHECK_LAUNCH("sample (prologue)");
+  if ((rc = launch_dependent(sample_prologue_kernel, {(unsigned)sp.rows, kStProThreads}, st, "sample (prologue)", p)) != TLX_OK) return rc;
   if (stages < 2) return TLX_OK;
   const int64_t sgrid = items < 4ll * sms ? items : 4ll * sms;
   TLX_TIMELINE_KERNEL(1);
-  if ((rc = launch_dependent(sample_stream_kernel, (unsigned)sgrid, kStThreads, st_smem, st, "sample (stream)", -1, p)) != TLX_OK) return rc;
+  if ((rc = launch_dependent(sample_stream_kernel, {(unsigned)sgrid, kStThreads, st_smem}, st, "sample (stream)", p)) != TLX_OK) return rc;
   if (stages < 3) return TLX_OK;
   TLX_TIMELINE_KERNEL(2);
-  return launch_dependent(finish, (unsigned)(p.fin_ctas + sp.rows), kStThreads, fin_smem, st,
-                          "sample (finish)", -1, p, dense);
+  return launch_dependent(finish, {(unsigned)(p.fin_ctas + sp.rows), kStThreads, fin_smem}, st, "sample (finish)", p, dense);
 }
 
 }  // namespace tlx
@@ -1011,7 +964,7 @@ static int launch_merge(cudaStream_t st, const MergeParams& p, int64_t rows) {
     // their candidate kernel: 37.0 us, with the default 39.5 us)
     const size_t need = (smem + 1024) * (size_t)((rows + 147) / 148 < 8 ? (rows + 147) / 148 : 8) * 100 / (228 << 10) + 1;
     const int carveout = rows < 256 || need > 100 ? 100 : need < 64 ? 64 : (int)need;
-    return launch_dependent(merge_and_sample_kernel, (unsigned)rows, (unsigned)threads, smem, st, "merge_and_sample", carveout, p);
+    return launch_dependent(merge_and_sample_kernel, {(unsigned)rows, (unsigned)threads, smem, 1, carveout}, st, "merge_and_sample", p);
   }
   merge_and_sample_kernel<<<(unsigned)rows, threads, smem, st>>>(p);
   TLX_CHECK_LAUNCH("merge_and_sample");

@@ -1160,6 +1160,7 @@ __global__ void __launch_bounds__(kRcThreads, 4) sample_cluster_kernel(const __g
   const int64_t n = p.sp.vocab;
   const T* rowp = reinterpret_cast<const T*>(p.sp.logits) + row * p.sp.row_stride;
   const RcPart<DT> part(rowp, n, p.part_len, rank, smem + l.off_part);
+  grid_wait();
   part.copy_in();
   TLX_STAMP(p.sp, 0);
   const float T_ = p.sp.temperature[row], pp = p.sp.top_p[row];

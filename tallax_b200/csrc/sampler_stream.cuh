@@ -306,8 +306,10 @@ __global__ void __launch_bounds__(kStProThreads) sample_prologue_kernel(StreamPa
   const int64_t V = p.sp.vocab;
   const __nv_bfloat16* rowp = reinterpret_cast<const __nv_bfloat16*>(p.sp.logits) + (int64_t)row * p.sp.row_stride;
   TLX_STAMP(p.sp, 0);
-  // the stream kernel may start now: it requests its first copies and then waits for this kernel's end
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // what precedes the call is complete, and the stream kernel may start now: it requests its first copies and then waits for
+  // this kernel's end
+  grid_wait();
+  grid_release();
   // the sample: 16 segments of 32 vectors, evenly spread over the row's full vectors
   const uint4* vp = reinterpret_cast<const uint4*>(rowp);
   const int64_t nv = V >> 3;

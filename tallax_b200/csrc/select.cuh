@@ -12,7 +12,7 @@
 // 3. sample_tail: softmax mass, top-p threshold, temperature, Gumbel arg-max over
 //    sorted candidates.
 #pragma once
-#include "tlx_common.cuh"
+#include "launch.cuh"
 
 namespace tlx {
 

@@ -34,6 +34,7 @@ template <typename T, bool kNoL1>
 __global__ void __launch_bounds__(256) gather_axis1_kernel(const T* __restrict__ values, const int32_t* __restrict__ idx,
                                                            T* __restrict__ out, int64_t rows, int64_t vcols, int64_t icols) {
   constexpr int kPer = 8;
+  grid_wait();
   const int64_t groups_per_row = (icols + kPer - 1) / kPer;
   const int64_t total = rows * groups_per_row;
   for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(256) gather_axis1_kernel(const T* __restrict__
 template <typename T>
 __global__ void gather_axis0_kernel(const T* __restrict__ values, const int32_t* __restrict__ idx,
                                     T* __restrict__ out, int64_t vrows, int64_t cols, int64_t irows) {
+  grid_wait();
   const int64_t total = irows * cols;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
@@ -94,28 +96,24 @@ static int launch_gather(cudaStream_t st, const void* values, const int32_t* idx
     const int64_t total = ir * ((ic + 7) >> 3);
     if (total == 0) return TLX_OK;
     const int64_t want = (total + threads - 1) / threads;
-    const int blocks = (int)(want < 148 * 64 ? want : 148 * 64);
+    const LaunchShape shape{(unsigned)(want < 148 * 64 ? want : 148 * 64), (unsigned)threads};
     // Many outputs out of rows of which hardly a line is read twice: the lines are not kept in L1.  us kept / not, rotating inputs,
     // and with a cold L2: f32 [1024, 1000] out of [1024, 262144] 25.6/23.6, 39/33; [256, 4096] 22.2/21.5, 33/31.  A line's second
     // reading, or a matrix that lies in L2, wants L1: [1024, 4096] out of [1024, 65537] 44.0/45.1, 59/74; [1024, 100] out of
     // [1024, 262144] 4.1/5.8.
     if constexpr (sizeof(T) == 4) {
       if (vc > (64 << 10) && ic * 32 <= vc && ir * ic >= (1 << 18)) {
-        gather_axis1_kernel<T, true><<<blocks, threads, 0, st>>>((const T*)values, idx, (T*)out, ir, vc, ic);
-        TLX_CHECK_LAUNCH("take_along_axis");
-        return TLX_OK;
+        return launch_dependent(gather_axis1_kernel<T, true>, shape, st, "take_along_axis", (const T*)values, idx, (T*)out, ir, vc, ic);
       }
     }
-    gather_axis1_kernel<T, false><<<blocks, threads, 0, st>>>((const T*)values, idx, (T*)out, ir, vc, ic);
+    return launch_dependent(gather_axis1_kernel<T, false>, shape, st, "take_along_axis", (const T*)values, idx, (T*)out, ir, vc, ic);
   } else {
     const int64_t total = ir * ic;
     if (total == 0) return TLX_OK;
     const int64_t want = (total + threads - 1) / threads;
-    const int blocks = (int)(want < 148 * 32 ? want : 148 * 32);
-    gather_axis0_kernel<T><<<blocks, threads, 0, st>>>((const T*)values, idx, (T*)out, vr, vc, ir);
+    const LaunchShape shape{(unsigned)(want < 148 * 32 ? want : 148 * 32), (unsigned)threads};
+    return launch_dependent(gather_axis0_kernel<T>, shape, st, "take_along_axis", (const T*)values, idx, (T*)out, vr, vc, ir);
   }
-  TLX_CHECK_LAUNCH("take_along_axis");
-  return TLX_OK;
 }
 
 // ---------------------------------------------------------------------------------
@@ -165,6 +163,7 @@ cumsum_axis1_kernel(const T* __restrict__ in, T* __restrict__ out, Idx cols, int
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
+  grid_wait();
   Idx v0 = (Idx)rank * kPer + slot0;   // in the order of summation
 #pragma unroll
   for (int i = 0; i < kStages - 1; ++i) fetch(v0 + i * stride, i);
@@ -272,6 +271,7 @@ __global__ void __launch_bounds__(kAxis0Warps * 32) cumsum_axis0_kernel(const T*
   const bool live = c < cols;
   T carry = T(0);
   int turn = 0;
+  grid_wait();
   for (int64_t base = 0; base < rows; base += (int64_t)kAxis0Turn * cluster, turn ^= 1) {
     const int64_t r0 = base + rank * kAxis0Turn + w * kAxis0Rows;
     T x[kAxis0Rows];
@@ -320,6 +320,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) cumsum_axis0_few_kernel(const T* __restrict__ in, T* __restrict__ out, int64_t rows, int64_t cols,
                                                                int reverse) {
   const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  grid_wait();
   if (c >= cols) return;
   T acc = T(0);
   for (int64_t r = 0; r < rows; ++r) {
@@ -329,30 +330,11 @@ __global__ void __launch_bounds__(128) cumsum_axis0_few_kernel(const T* __restri
   }
 }
 
-template <typename... Params, typename... Args>
-static int launch_cluster(void (*kernel)(Params...), unsigned grid, unsigned block, int cluster, cudaStream_t st, const char* what,
-                          Args... args) {
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(block);
-  cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)cluster;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = cluster > 1 ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
-  if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e)); }
-  count_launch();
-  return TLX_OK;
-}
-
 template <typename T, typename Idx, int V, int kStages, int kThreads = kCumsumThreads>
 static int launch_cumsum_rows(cudaStream_t st, const T* in, T* out, int64_t rows, int64_t cols, int reverse, int cluster) {
   const int same = ((reinterpret_cast<uintptr_t>(in) ^ reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  return launch_cluster(cumsum_axis1_kernel<T, Idx, V, kStages, kThreads>, (unsigned)(rows * cluster), kThreads, cluster, st, "cumsum", in,
-                        out, cols, reverse, cluster, same);
+  return launch_dependent(cumsum_axis1_kernel<T, Idx, V, kStages, kThreads>, {(unsigned)(rows * cluster), kThreads, 0, cluster}, st, "cumsum",
+                          in, out, cols, reverse, cluster, same);
 }
 
 // One vector a thread for rows of up to 1024 elements, and a single warp for up to 128 (f32 [6000, 60] 4.7 us, with eight warps
@@ -368,15 +350,13 @@ static int launch_cumsum(cudaStream_t st, const void* in, void* out, int64_t row
     // us a thread per column / sixteen warps per 32 columns: [16, 500] 2.1/3.5, [40, 4096] 3.3/3.6, [48, 4096] 3.8/3.7, [48, 16384]
     // 4.7/8.5, [64, 16384] 10.2/9.0, [64, 32768] 12/14, [96, 32768] 17/15, [128, 70000] 25/30, [192, 70000] 36/33
     if (rows <= (cols < 8192 ? 40 : cols < 32768 ? 48 : cols < 65536 ? 64 : 128)) {
-      cumsum_axis0_few_kernel<T><<<(unsigned)((cols + 127) / 128), 128, 0, st>>>(x, y, rows, cols, reverse);
-      TLX_CHECK_LAUNCH("cumsum");
-      return TLX_OK;
+      return launch_dependent(cumsum_axis0_few_kernel<T>, {(unsigned)((cols + 127) / 128), 128}, st, "cumsum", x, y, rows, cols, reverse);
     }
     const int64_t strips = (cols + 31) / 32;
     int cluster = 1;
     while (cluster < 8 && strips * cluster * 2 <= 592 && (int64_t)cluster * kAxis0Turn < rows) cluster *= 2;
-    return launch_cluster(cumsum_axis0_kernel<T>, (unsigned)(strips * cluster), kAxis0Warps * 32, cluster, st, "cumsum", x, y, rows, cols,
-                          reverse, cluster);
+    return launch_dependent(cumsum_axis0_kernel<T>, {(unsigned)(strips * cluster), kAxis0Warps * 32, 0, cluster}, st, "cumsum", x, y, rows,
+                            cols, reverse, cluster);
   }
   const int64_t n = cols + 3;   // the first vector may be a partial one
   if (n <= 128) return launch_cumsum_rows<T, int, 1, 2, 32>(st, x, y, rows, cols, reverse, 1);

@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(kSortThreads) sort_small_kernel(
     int descending, typename Elem<DT>::type* __restrict__ out_keys, int32_t* __restrict__ out_perm,
     const __grid_constant__ SortCarry carry) {
   extern __shared__ uint64_t tile_smem[];
+  grid_wait();
   const int64_t r = blockIdx.x;
   const auto* krow = keys + r * n;
   const int32_t* prow = in_perm ? in_perm + r * n : nullptr;
@@ -236,21 +237,8 @@ static int launch_places(cudaStream_t st, const void* keys, int64_t rows, int64_
   static SmemLimit limit;
   int rc;
   if ((rc = raise_smem(limit, (const void*)sort_places_kernel<DT, IPT, CL, PAST>, smem, "sort")) != TLX_OK) return rc;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(rows * cluster));
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)cluster;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = CL ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, sort_places_kernel<DT, IPT, CL, PAST>, (const T*)keys, in_perm, n, descending, (T*)out_keys, out_perm, cluster, carry);
-  if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "sort: %s", cudaGetErrorString(e)); }
-  count_launch();
-  return TLX_OK;
+  return launch_dependent(sort_places_kernel<DT, IPT, CL, PAST>, {(unsigned)(rows * cluster), (unsigned)threads, smem, cluster}, st, "sort",
+                          (const T*)keys, in_perm, n, descending, (T*)out_keys, out_perm, cluster, carry);
 }
 
 template <int DT>
@@ -279,10 +267,8 @@ static int sort_dispatch(cudaStream_t st, const void* keys, int64_t rows, int64_
     int threads = (int)(n_pad / 8);
     if (threads < 64) threads = 64;
     static_assert(padded_bytes(kSmallRow) <= 48 * 1024, "no limit has to be raised");
-    sort_small_kernel<DT><<<(unsigned)rows, threads, padded_bytes((size_t)n_pad), st>>>(
-        (const T*)keys, in_perm, n, (int)n_pad, descending, (T*)out_keys, out_perm, carry);
-    TLX_CHECK_LAUNCH("sort (single tile)");
-    return TLX_OK;
+    return launch_dependent(sort_small_kernel<DT>, {(unsigned)rows, (unsigned)threads, padded_bytes((size_t)n_pad)}, st, "sort (single tile)",
+                            (const T*)keys, in_perm, n, (int)n_pad, descending, (T*)out_keys, out_perm, carry);
   }
   const size_t need = (size_t)rows * (size_t)n_pad * 8;
   if (!workspace || workspace_bytes < need)

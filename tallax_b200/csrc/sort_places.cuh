@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(kRadixMaxThreads) sort_places_kernel(
     carry_one(carry, row * n64 + pos, to);
   };
 
+  grid_wait();
   // element w * 32 * IPT + 32 j + lane of the CTA
   const int i0 = w * 32 * IPT + lane, left = n - (c0 + i0);   // element j is there if 32 j < left
   uint32_t k[kRoom], p[kRoom];

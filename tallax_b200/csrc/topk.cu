@@ -113,6 +113,14 @@ __device__ __forceinline__ void emit_row(const TopkParams& p, int64_t r, const t
   }
 }
 
+// What every kernel here begins with.  Exchange mode (in which they are launched in plain order: 1024 rows of 18992, k = 50, with the
+// merge kernel 36.7 us, as dependents of the merge kernel before them 37.4): the merge kernel that follows waits for the rows' arrival counts, not for
+// this kernel, and may be scheduled now.
+__device__ __forceinline__ void topk_start(const TopkParams& p) {
+  grid_wait();
+  if (p.ex.world > 0) grid_release();
+}
+
 template <int DT, int CAP>
 __global__ void __launch_bounds__(kTopkThreads) topk_kernel(TopkParams p) {
   using T = typename Elem<DT>::type;
@@ -122,8 +130,7 @@ __global__ void __launch_bounds__(kTopkThreads) topk_kernel(TopkParams p) {
   const int64_t r = blockIdx.x;
   const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
   const int K = p.k_max;
-  // exchange mode: the merge kernel that follows waits for the rows' arrival counts, not for this kernel
-  if (p.ex.world > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  topk_start(p);
 
   bool ok = collect_row<DT, CAP>(row, p.n, K, s, cand);
   if (!ok) {
@@ -315,7 +322,7 @@ __global__ void __launch_bounds__(TH, 1024 / TH) topk_sampled_kernel(TopkParams 
   const int64_t r = blockIdx.x;
   const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
   const int K = p.k_max, n = (int)p.n, tid = threadIdx.x;
-  if (p.ex.world > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  topk_start(p);
   const int head = (int)(((16 - (reinterpret_cast<uintptr_t>(row) & 15)) & 15) / sizeof(T));
   const int nvec = (n - head) / VEC;
   const uint4* vp = reinterpret_cast<const uint4*>(row + head);
@@ -470,8 +477,7 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
   const int K = p.k_max;
   const int64_t n = p.n;
-  // exchange mode: the merge kernel that follows waits for the rows' arrival counts, not for this kernel
-  if (p.ex.world > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  topk_start(p);
 
   // bf16 rows of up to 4096 vectors (64 KB) read in full by pass 1: pass 1 also leaves every vector's greatest
   // element (NaN if it holds one) in shared memory, in the candidate list's space, and pass 2 reads those
@@ -625,9 +631,8 @@ __global__ void __launch_bounds__(kRcThreads, 4) topk_cluster_kernel(const __gri
   const int64_t r = blockIdx.x / cluster;
   const T* row = reinterpret_cast<const T*>(p.x) + r * p.row_stride;
   const RcPart<DT> part(row, p.n, part_len, rank, smem + l.off_part);
+  topk_start(p);
   part.copy_in();
-  // exchange mode: the merge kernel that follows waits for the rows' arrival counts, not for this kernel
-  if (p.ex.world > 0) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int K = p.k_max;
   float* lx = reinterpret_cast<float*>(smem + l.off_x);
   unsigned short* lpos = reinterpret_cast<unsigned short*>(smem + l.off_pos);
@@ -766,21 +771,7 @@ static int launch_topk_cluster(cudaStream_t st, const TopkParams& p) {
       if (dev >= 0 && dev < 64) raised[dev] = smem;
     }
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)(p.rows * cluster));
-  cfg.blockDim = dim3(kRcThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = (unsigned)cluster;
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, topk_cluster_kernel<DT>, p, cluster, part_len);
-  if (e != cudaSuccess) { cudaGetLastError(); return set_error(TLX_ERR_CUDA, "top_k: %s", cudaGetErrorString(e)); }
-  count_launch();
-  return TLX_OK;
+  return launch_dependent(topk_cluster_kernel<DT>, {(unsigned)(p.rows * cluster), kRcThreads, smem, cluster, -1, p.ex.world > 0}, st, "top_k", p, cluster, part_len);
 }
 
 // Whether the two-pass kernel serves a call: K <= 128, enough rows to fill the eight CTAs per SM, and
@@ -820,9 +811,7 @@ static int launch_topk_short_from(cudaStream_t st, const TopkParams& p) {
   static bool asked[64] = {};
   cudaError_t e = ask_shared_memory(mu, asked, topk_short_kernel<DT, SUB>, smem, 1024 / kShortThreads);
   if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  topk_short_kernel<DT, SUB><<<(unsigned)p.rows, kShortThreads, smem, st>>>(p);
-  TLX_CHECK_LAUNCH("top_k (short rows)");
-  return TLX_OK;
+  return launch_dependent(topk_short_kernel<DT, SUB>, {(unsigned)p.rows, kShortThreads, smem, 1, -1, p.ex.world > 0}, st, "top_k (short rows)", p);
 }
 // 16-bit rows of more than 1 MB, which L2 does not keep between the passes: the bound from a quarter of the row (bf16 [1024, 600000],
 // k = 20: 228 us against 355)
@@ -840,9 +829,7 @@ static int launch_topk_sampled_threads(cudaStream_t st, const TopkParams& p) {
   static bool asked[64] = {};
   cudaError_t e = ask_shared_memory(mu, asked, topk_sampled_kernel<DT, TH>, smem, 1024 / TH);
   if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  topk_sampled_kernel<DT, TH><<<(unsigned)p.rows, TH, smem, st>>>(p);
-  TLX_CHECK_LAUNCH("top_k (long rows)");
-  return TLX_OK;
+  return launch_dependent(topk_sampled_kernel<DT, TH>, {(unsigned)p.rows, TH, smem, 1, -1, p.ex.world > 0}, st, "top_k (long rows)", p);
 }
 // 1024 threads per SM in any case: one, two, four or eight rows at a time, by which of them has every row running at once (f32
 // [128, 262144]: 27.4 us with CTAs of 1024 threads, 31 of 512, 49 of 256; [200, 100000]: 32, 24, 30; [500, 100000]: 65, 47,
@@ -879,9 +866,7 @@ static int launch_topk_cap(cudaStream_t st, const TopkParams& p) {
     cudaError_t e = cudaMemcpyAsync(p.out_valid, &one, sizeof(one), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaMemcpyAsync: %s", cudaGetErrorString(e));
   }
-  topk_kernel<DT, CAP><<<(unsigned)p.rows, kTopkThreads, smem, st>>>(p);
-  TLX_CHECK_LAUNCH("top_k");
-  return TLX_OK;
+  return launch_dependent(topk_kernel<DT, CAP>, {(unsigned)p.rows, kTopkThreads, smem, 1, -1, p.ex.world > 0}, st, "top_k", p);
 }
 
 template <int DT>

@@ -1,0 +1,126 @@
+"""GPU: calls launched as programmatic dependents keep the stream's order, whatever precedes them, eager and in a graph.
+
+Every call reads what the operation before it on the stream has just written, over buffers that are used again at once; the
+expectation is the same call made after a synchronisation.
+"""
+import pytest
+import torch
+
+from tallax_b200 import sampling, tax, tumpy
+
+pytestmark = pytest.mark.gpu
+
+ROWS, N = 24, 40000
+
+
+def _calls(index, metadata, shape):
+    return {
+        "sample": lambda x: sampling.sample((3, 5), x, metadata),
+        "top_k": lambda x: tax.top_k(x, 20, block_token=1)[0],
+        "sort": lambda x: tax.sort([x], num_keys=1)[0],
+        "short_sort": lambda x: tax.sort([x[:, :40].contiguous()], num_keys=1)[0],
+        "gather": lambda x: tumpy.take_along_axis(x, index, 1),
+        "gather_rows": lambda x: tumpy.take_along_axis(x, index % ROWS, 0) if shape == index.shape else x,
+        "cumsum": lambda x: tax.cumsum(x, 1),
+        "cumsum_rows": lambda x: tax.cumsum(x, 0),
+    }
+
+
+def _setup(cuda):
+    gen = torch.Generator(device=cuda).manual_seed(11)
+    source = [torch.randn((ROWS, N), generator=gen, device=cuda) for _ in range(3)]
+    index = torch.randint(0, N, (ROWS, N), generator=gen, device=cuda, dtype=torch.int32)
+    metadata = sampling.SamplingMetadata(torch.full((ROWS,), 50, dtype=torch.int32, device=cuda), torch.full((ROWS,), 0.9, device=cuda),
+                                         torch.ones(ROWS, device=cuda))
+    return source, _calls(index, metadata, (ROWS, N))
+
+
+# what writes the input just before: an elementwise kernel, a copy, a fill and a copy, another of these calls
+def _write(x, source, how, calls):
+    if how == "kernel":
+        torch.add(source, 1.0, out=x)
+    elif how == "copy":
+        x.copy_(source)
+    elif how == "fill":
+        x.zero_()
+        x[:, ::3].copy_(source[:, ::3])
+    else:
+        x.copy_(calls["cumsum"](calls["sort"](source)))
+
+
+@pytest.mark.parametrize("how", ["kernel", "copy", "fill", "call"])
+@pytest.mark.parametrize("name", ["sample", "top_k", "sort", "short_sort", "gather", "gather_rows", "cumsum", "cumsum_rows"])
+def test_calls_wait_for_what_precedes_them(cuda, name, how):
+    source, calls = _setup(cuda)
+    x = torch.empty((ROWS, N), device=cuda)
+    want = []
+    for s in source:
+        _write(x, s, how, calls)
+        torch.cuda.synchronize()
+        want.append(calls[name](x).clone())
+        torch.cuda.synchronize()
+    got = []
+    for _ in range(3):
+        for s in source:                      # no synchronisation: the next write overwrites what the call before it reads
+            _write(x, s, how, calls)
+            got.append(calls[name](x))
+    torch.cuda.synchronize()
+    for i, g in enumerate(got):
+        assert torch.equal(g, want[i % 3])
+
+
+@pytest.mark.parametrize("how", ["kernel", "copy", "fill", "call"])
+def test_captured_calls_wait_for_what_precedes_them(cuda, how):
+    source, calls = _setup(cuda)
+    x, s = torch.empty((ROWS, N), device=cuda), torch.empty((ROWS, N), device=cuda)
+    side, other = torch.cuda.Stream(), torch.cuda.Stream()
+    want = []
+    for src in source:
+        _write(x, src, how, calls)
+        want.append([calls[c](x).clone() for c in ("top_k", "sort", "cumsum", "sample")])
+    torch.cuda.synchronize()
+    s.copy_(source[0])
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.stream(side):
+        for _ in range(2):
+            _write(x, s, how, calls)
+            [calls[c](x) for c in ("top_k", "sort", "cumsum", "sample")]
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            _write(x, s, how, calls)
+            first = calls["top_k"](x)
+            other.wait_stream(side)            # a fork and a join: two predecessors of the calls after it
+            with torch.cuda.stream(other):
+                second = calls["sort"](x)
+            third = calls["cumsum"](x)
+            side.wait_stream(other)
+            fourth = calls["sample"](x)
+    for _ in range(2):
+        for src, w in zip(source, want):
+            s.copy_(src)
+            graph.replay()
+            torch.cuda.synchronize()
+            for g, e in zip((first, second, third, fourth), w):
+                assert torch.equal(g, e)
+
+
+def test_steps_follow_each_other(cuda):
+    """A large sampler call (three kernels), a call of one kernel on the same buffers, and again, as a decode loop queues them."""
+    gen = torch.Generator(device=cuda).manual_seed(2)
+    rows, vocab = 160, 65536
+    logits = [(torch.randn((rows, vocab), generator=gen, device=cuda) * 3).bfloat16() for _ in range(2)]
+    k = torch.randint(0, 300, (rows,), generator=gen, device=cuda, dtype=torch.int32)
+    md = sampling.SamplingMetadata(k, torch.full((rows,), 0.9, device=cuda), torch.ones(rows, device=cuda))
+    want = []
+    for x in logits:
+        t = sampling.sample((1, 9), x, md)
+        torch.cuda.synchronize()
+        want.append((t, tax.top_k(x, 8, block_token=1)[1]))
+        torch.cuda.synchronize()
+    got, x = [], torch.empty_like(logits[0])
+    for i in range(12):
+        x.copy_(logits[i % 2])
+        got.append((sampling.sample((1, 9), x, md), tax.top_k(x, 8, block_token=1)[1]))
+    torch.cuda.synchronize()
+    for i, (t, v) in enumerate(got):
+        assert torch.equal(t, want[i % 2][0]) and torch.equal(v, want[i % 2][1])
