@@ -353,6 +353,9 @@ __global__ void __launch_bounds__(kMergeThreads) merge_and_sample_kernel(MergePa
   while (P < n_cand) P <<= 1;
   uint64_t* merged = cand + P;
   const int64_t r = blockIdx.x;
+  const float T_ = p.temperature[r], pp = p.top_p[r];   // (there before the candidates are)
+  int K = p.top_k[r];
+  if (K <= 0 || K > n_cand) K = n_cand;
 
   const float* v = p.cand_vals;
   const int32_t* id = p.cand_idx;
@@ -414,8 +417,6 @@ __global__ void __launch_bounds__(kMergeThreads) merge_and_sample_kernel(MergePa
   for (int i = threadIdx.x; i < n_cand; i += blockDim.x)
     if (i != block_of(i) * kpb && cand[i - 1] > cand[i]) unsorted = 1;
   unsorted = __syncthreads_or(unsorted);
-  int K = p.top_k[r];
-  if (K <= 0 || K > n_cand) K = n_cand;
   const uint64_t* top = cand;
   if (unsorted) {
     sort_candidates(cand, n_cand);
@@ -467,15 +468,13 @@ __global__ void __launch_bounds__(kMergeThreads) merge_and_sample_kernel(MergePa
     __syncthreads();
     top = merged;
   }
-  const float T_ = p.temperature[r];
-  int tok;
-  if (T_ < kSamplingEps) {
-    tok = id[at(cand_low(top[0]))];
-  } else {
-    tok = sample_tail<2>(
-        K, p.top_p[r], T_, s, [&](int i) { return key_f32(cand_key(top[i])); },
-        [&](int i) { return (int)id[at(cand_low(top[i]))]; }, [&](int i) { return un[at(cand_low(top[i]))]; });
-  }
+  int tok = 0;
+  const auto value_of = [&](int i) { return key_f32(cand_key(top[i])); };
+  const auto token_of = [&](int i) { return (int)id[at(cand_low(top[i]))]; };
+  const auto noise_of = [&](int i) { return un[at(cand_low(top[i]))]; };
+  if (T_ < kSamplingEps) tok = token_of(0);
+  else if (K > 128) tok = sample_tail<2>(K, pp, T_, s, value_of, token_of, noise_of);
+  else if (warp_id() == 0) tok = sample_tail_warp<4>(K, pp, T_, value_of, token_of, noise_of);
   if (threadIdx.x == 0) {
     p.out[r] = tok;
     if (xh) {

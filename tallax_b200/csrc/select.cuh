@@ -368,6 +368,71 @@ static __device__ __noinline__ int sample_tail_any(int K, float p, float T, Sele
   return b.tok;
 }
 
+// The same by one warp, K <= 32 * kMaxItems, without a barrier; every lane returns the token.  Contenders are only evaluated in f64
+// if there are several: the two logarithms take longer than all the rest.
+template <int kMaxItems, typename ValueOf, typename TokenOf, typename NoiseOf>
+static __device__ __forceinline__ int sample_tail_warp(int K, float p, float T, ValueOf value_of, TokenOf token_of, NoiseOf noise_of) {
+  const int per = (K + 31) / 32, i0 = lane_id() * per;
+  float x[kMaxItems], u[kMaxItems], a[kMaxItems];
+  double run[kMaxItems], acc = 0.0;
+#pragma unroll
+  for (int j = 0; j < kMaxItems; ++j)
+    if (j < per && i0 + j < K) u[j] = noise_of(i0 + j);
+  const float x0 = value_of(0);
+#pragma unroll
+  for (int j = 0; j < kMaxItems; ++j)
+    if (j < per && i0 + j < K) {
+      x[j] = value_of(i0 + j);
+      acc += (double)expf(x[j] - x0);
+      run[j] = acc;
+    }
+  double incl = acc;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const double up = shfl_up_f64(incl, o);
+    if (lane_id() >= o) incl += up;
+  }
+  const double base = incl - acc;
+  const double Z = __hiloint2double(__shfl_sync(0xFFFFFFFFu, __double2hiint(incl), 31), __shfl_sync(0xFFFFFFFFu, __double2loint(incl), 31));
+  int below = 0;
+#pragma unroll
+  for (int j = 0; j < kMaxItems; ++j)
+    if (j < per && i0 + j < K) below += (base + run[j]) / Z < (double)p ? 1 : 0;
+  below = __reduce_add_sync(0xFFFFFFFFu, below);
+  const float thr = value_of(min(below, K - 1));
+  float amax = -INFINITY;
+#pragma unroll
+  for (int j = 0; j < kMaxItems; ++j) {
+    a[j] = -INFINITY;
+    if (j < per && i0 + j < K && x[j] >= thr) {
+      a[j] = __fdiv_rn(x[j], T) + gumbel_screen(u[j]);
+      amax = fmaxf(amax, a[j]);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
+  const float cut = amax - (kGumbelSlack + 1e-5f * fabsf(amax));
+  int contenders = 0, tok = 0x7FFFFFFF;
+#pragma unroll
+  for (int j = 0; j < kMaxItems; ++j)
+    if (j < per && i0 + j < K && a[j] >= cut) {
+      ++contenders;
+      tok = token_of(i0 + j);
+    }
+  contenders = __reduce_add_sync(0xFFFFFFFFu, contenders);
+  if (contenders == 1) return __reduce_min_sync(0xFFFFFFFFu, tok);
+  Best best{-INFINITY, 0x7FFFFFFF};
+#pragma unroll 1
+  for (int j = 0; j < per; ++j) {
+    const int i = i0 + j;
+    if (i >= K) break;
+    const float xi = value_of(i), ui = noise_of(i);
+    if (xi >= thr && __fdiv_rn(xi, T) + gumbel_screen(ui) >= cut)
+      best = best_of(best, Best{__fdiv_rn(xi, T) + gumbel_exact(ui), token_of(i)});
+  }
+  return warp_best(best).tok;
+}
+
 template <int kMaxItems, typename ValueOf, typename TokenOf, typename NoiseOf>
 static __device__ __noinline__ int sample_tail(int K, float p, float T, SelectShared& s, ValueOf value_of,
                                            TokenOf token_of, NoiseOf noise_of) {
