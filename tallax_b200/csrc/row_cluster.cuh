@@ -52,6 +52,11 @@ __device__ __forceinline__ void cl_st_u32(uint32_t a, uint32_t v) { asm volatile
 __device__ __forceinline__ void cl_st_f32(uint32_t a, float v) { cl_st_u32(a, __float_as_uint(v)); }
 __device__ __forceinline__ void cl_st_f64(uint32_t a, double v) { asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory"); }
 __device__ __forceinline__ float cl_ld_f32(uint32_t a) { return __uint_as_float(cl_ld_u32(a)); }
+__device__ __forceinline__ double cl_ld_f64(uint32_t a) {
+  double v;
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint4 cl_ld_v4(uint32_t a) {
   uint4 v;
   asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
@@ -123,6 +128,8 @@ struct __align__(16) RcShared {
   float dom_x[2 * kRcMaxCluster], dom_s[2 * kRcMaxCluster];   // per CTA: its greatest element and its best-scored one
   float cut_x[14], cut_s[14];           // an element is out if one of these has at least its value and a greater score
   int n_cut;
+  float bin_mass[16];                   // softmax mass of this CTA's elements, by their distance from the row's greatest one
+  double z_part;                        // ... of all of them; later of those above a value
   float query[4];                       // values whose mass above the leader asks for
   int n_query;
   int query_tok[4];                     // leader: their tokens

@@ -8,8 +8,10 @@
 // be sorted: the best score of the set wins if the mass above its value is below top_p * Z; otherwise no lower
 // value is kept either, and the best score among the greater values is tried.  One or two rounds as a rule.
 //
-// Rows without top-k: every CTA publishes its greatest element and that element's score.  An element can only win if
-// no greater (or equal) element has a greater score, because a greater value is kept whenever the smaller one is;
+// Rows without top-k of which top_p leaves a share: the softmax denominator and the mass at sixteen distances from the
+// greatest element come first, and say from which value on elements can be kept; only those are scored (rc_pruned_row).
+//   The others, and what that leaves open: every CTA publishes its greatest element and that element's score.  An element can only
+// win if no greater (or equal) element has a greater score, because a greater value is kept whenever the smaller one is;
 // so what the published pairs dominate is out, and before its noise is even looked at an element is out if its
 // value plus the greatest Gumbel term there is would not do.  The survivors (a handful) go to the leader, and the
 // mass above its best ones comes from one more pass over the parts, which are still in shared memory.
@@ -723,6 +725,23 @@ __device__ __forceinline__ void rc_masses(const RcPart<DT>& part, float xmax, fl
   z = (zs[0] + zs[1]) + (zs[2] + zs[3]);
 }
 
+// The thread's share of the mass above a value alone.
+template <int DT>
+__device__ __forceinline__ void rc_masses_above(const RcPart<DT>& part, float xmax, float q, double& mass) {
+  using T = typename Elem<DT>::type;
+  constexpr int VEC = RcPart<DT>::VEC;
+#pragma unroll 1
+  for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) {
+    const uint4 w = part.vec[v];
+    if (!rc_any_at_least<DT>(w, q)) continue;
+#pragma unroll 1
+    for (int j = 0; j < VEC; ++j) {
+      const float x = elem_as_float<DT>(reinterpret_cast<const T*>(part.vec + v)[j]);
+      if (x > q) mass += (double)expf(x - xmax);
+    }
+  }
+}
+
 // Rows with 1024 < top_k < vocab and rows whose lists overflowed: cuts the row, which lies in the parts, to its top-K set.  What is outside the set becomes
 // -inf, and the row is then one without top-k.
 //   The K-th greatest key comes from histograms of 2048 bins, eleven bits of the key at a time (two for bf16, three for f32, in
@@ -942,6 +961,237 @@ __device__ __forceinline__ int rc_normal_row(const RcSampleParams& p, const RcPa
   return tok;
 }
 
+// ---- rows without top-k of which top-p leaves a share -----------------------------------------------------------------
+constexpr float kRcPruneBelow = 0.9999f;   // top_p from which on hardly anything is ruled out by it
+// Elements of a part from which on it is worth it; with noise from a tensor all it saves is the tensor's reading.  us without / with,
+// no top-k: tensor f32 [8, 32000] (parts of 2000) 13.8 / 15.7, [64, 50257] (6283) 28.8 / 25.4, [8, 151936] (9496) 23.6 / 22.1; key f32
+// [8, 32000] 15.5 / 15.9, bf16 [1, 128256] (8016) 16.0 / 14.1, f32 [64, 50257] 37.8 / 29.3, bf16 [32, 128256] 45 / 31.
+constexpr int kRcPruneTensorPart = 6000, kRcPruneKeyPart = 3000;
+constexpr int kRcMassBins = 16;
+constexpr int kRcScan = -3;                // rc_pruned_row: not settled here
+
+// A normal f32 that is not negative as f64, by integer operations (the conversion is an eighth-rate instruction).  Zero becomes
+// 2^-127, which no sum with an addend of 1 notices.
+__device__ __forceinline__ double rc_widen(float y) {
+  const uint32_t b = __float_as_uint(y);
+  return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+
+// The thread's share of the softmax denominator, and of the mass at the distances [i, i + 1), i < 16, below the greatest
+// element: bin i in acc[256 i + thread].  The bins only rule elements out, with a margin; they are f32.  A NaN makes the
+// denominator one.
+template <int DT>
+__device__ __forceinline__ double rc_mass_bins(const RcPart<DT>& part, float xmax, float* acc) {
+  using T = typename Elem<DT>::type;
+  constexpr int VEC = RcPart<DT>::VEC;
+  float* mine = acc + threadIdx.x;
+#pragma unroll
+  for (int i = 0; i < kRcMassBins; ++i) mine[kRcThreads * i] = 0.f;
+  double zs[4] = {0.0, 0.0, 0.0, 0.0};
+  bool nan = false;
+#pragma unroll 1
+  for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) {
+    const uint4 w = part.vec[v];
+    const T* e = reinterpret_cast<const T*>(&w);
+    const bool any = rc_any_at_least<DT>(w, xmax - (float)kRcMassBins);
+    float y[VEC];
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) {
+      y[j] = expf(elem_as_float<DT>(e[j]) - xmax);
+      nan = nan || y[j] != y[j];
+      zs[j & 3] += rc_widen(y[j]);
+    }
+    if (any) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const float d = xmax - elem_as_float<DT>(e[j]);
+        // (int)d without a conversion: the low bits of d + 2^23, rounded towards zero
+        if (d < (float)kRcMassBins) mine[kRcThreads * (__float_as_int(__fadd_rz(d, 8388608.0f)) & (kRcMassBins - 1))] += y[j];
+      }
+    }
+  }
+  const double z = (zs[0] + zs[1]) + (zs[2] + zs[3]);
+  return nan ? __longlong_as_double(0x7FF8000000000000ll) : z;
+}
+
+// The best screened score of the part's elements from `lo` on, per thread: score, place, and the second best score.  A warp
+// notes their positions and scores them 128 at a time, four interleaved chains a lane; what cannot reach the warp's best score so
+// far, less the screening slack, is passed over.
+struct RcTop {
+  float a1, a2;
+  int at;
+};
+template <int DT>
+__device__ __forceinline__ RcTop rc_best_from(const RcPart<DT>& part, float lo, const RcWideRow& r, unsigned short* queue) {
+  using T = typename Elem<DT>::type;
+  constexpr int VEC = RcPart<DT>::VEC;
+  const int lane = lane_id();
+  const uint32_t lt = (1u << lane) - 1u;
+  RcTop best{-INFINITY, -INFINITY, 0};
+  float reach = -INFINITY;
+  int waiting = 0;
+#pragma unroll 1
+  for (int v0 = 0; v0 < part.nvec; v0 += kRcThreads) {
+    const int v = v0 + threadIdx.x;
+    const bool last = v0 + kRcThreads >= part.nvec;
+    uint32_t mask = 0;
+    if (v < part.nvec) {
+      const uint4 w = part.vec[v];
+      const T* e = reinterpret_cast<const T*>(&w);
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) mask |= elem_as_float<DT>(e[j]) >= lo ? 1u << j : 0u;   // (outside the part: -inf)
+    }
+    // every lane's first element, every lane's second one, ...
+    for (uint32_t some = __ballot_sync(0xFFFFFFFFu, mask != 0); some; some = __ballot_sync(0xFFFFFFFFu, mask != 0)) {
+      if (mask) queue[waiting + __popc(some & lt)] = (unsigned short)(v * VEC + __ffs(mask) - 1 - part.off);
+      mask &= mask - 1;
+      waiting += __popc(some);
+    }
+    __syncwarp();
+    while (waiting >= 128 || (last && waiting > 0)) {
+      const int count = min(waiting, 128);
+      waiting -= count;
+      int at[4];
+      float u[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        at[k] = lane + 32 * k < count ? queue[waiting + lane + 32 * k] : -1;
+        if (r.dense) u[k] = at[k] >= 0 ? __ldg(r.dense + at[k]) : 0.f;
+      }
+      if (!r.dense) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) u[k] = fmaxf(threefry_uniform01(r.k0, r.k1, r.ctr0 + (uint32_t)at[k]), kF32Tiny);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (at[k] < 0) continue;
+        const float x = elem_as_float<DT>(part.elem(at[k]));
+        if (!rc_may_reach(x, u[k], r.rt, reach)) continue;
+        const float a = fmaf(x, r.rt, gumbel_screen(u[k]));
+        if (a > best.a1) { best.a2 = best.a1; best.a1 = a; best.at = at[k]; }
+        else if (a > best.a2) best.a2 = a;
+      }
+      const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, rc_score_key(best.a1));
+      if (top > 0x007FFFFFu) reach = rc_cut(key_f32(top));
+    }
+    __syncwarp();
+  }
+  return best;
+}
+
+// Top-p first: the denominator and the mass at sixteen distances from the greatest element say, in every CTA alike, from which
+// value on elements can be kept at all, within one unit of the logits; those are scored, and the best of them wins if the mass
+// above it is below top_p * Z.  If not, the best of the greater ones is next.  `x`: the thread's greatest element.
+//   Returns the token (in every CTA), -1 if there is no finite maximum, kRcScan if the row is left to the way without
+// bounds on the values: nothing is ruled out, no score, several scores within the screening slack of the best, or groups whose
+// greatest elements are all equal (`least`: the least of the thread's), as a rule a constant row.
+//   Four cluster barriers and three short loops over the part.  What bounds it: the denominator (5 of 20 us a row of bf16 [32, 128256]:
+// 24 instructions an element, two of them eighth-rate) and the scores (6 us).  us a call, without / with it: noise from a
+// key, bf16 [32, 128256] mixed parameters 32.5 / 23.3, no top-k 41 / 28.5, [40, 179328] 64 / 46; f32 [64, 50257] 34 / 25; tensor
+// bf16 [32, 128256] mixed 25.3 / 23.5, [40, 179328] 34 / 29; flat rows 134 / 74.
+//   Tried: the bins as 2^-23ths by integer atomics 6.6 us instead of 5.7; noise of a tensor read beside the values, two vectors a turn,
+// 9 us instead of 6 (the queue has 128 reads in flight a warp).
+template <int DT>
+__device__ __forceinline__ int rc_pruned_row(const RcSampleParams& p, const RcPart<DT>& part, int64_t col0, float x, float least, float pp,
+                                             const RcWideRow& r, RcShared& s, const RcLayout& layout, unsigned char* smem, int& tog) {
+  const int lane = lane_id(), of = lane < p.cluster ? lane : 0;
+  const bool asks = lane < p.cluster;
+  const uint32_t xm = rc_max_u32(f32_key(x), s, tog), lm = ~rc_max_u32(~f32_key(least), s, tog);
+  if (threadIdx.x == 0) { s.dom_x[0] = key_f32(xm); s.dom_x[1] = key_f32(lm); }
+  cl_sync();
+  TLX_STAMP(p.sp, 2);
+  const uint32_t at_x = cl_map(s.dom_x, (uint32_t)of);
+  const float xmax = key_f32(__reduce_max_sync(0xFFFFFFFFu, f32_key(cl_ld_f32(at_x))));
+  const float xleast = key_f32(__reduce_min_sync(0xFFFFFFFFu, f32_key(cl_ld_f32(at_x + 4))));
+  if (!(fabsf(xmax) < INFINITY) || xleast == xmax) {
+    cl_sync();
+    return xleast == xmax && fabsf(xmax) < INFINITY ? kRcScan : -1;
+  }
+  float* acc = reinterpret_cast<float*>(smem + layout.off_x);
+  double z = rc_mass_bins<DT>(part, xmax, acc), unused = 0.0;
+  rc_sum2_f64(z, unused, s, tog);
+  static_assert(kRcMassBins == 2 * kRcWarps && kRcMassBins * kRcThreads * 4 <= kRcListCap * 8, "two bins a warp, in the lists' space");
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int bin = 2 * warp_id() + h;
+    float m = 0.f;
+#pragma unroll
+    for (int i = 0; i < kRcThreads / 32; ++i) m += acc[kRcThreads * bin + 32 * i + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xFFFFFFFFu, m, o);
+    if (lane == 0) s.bin_mass[bin] = m;
+  }
+  if (threadIdx.x == 0) s.z_part = z;
+  cl_sync();
+  TLX_STAMP(p.sp, 3);
+  double Z = asks ? cl_ld_f64(cl_map(&s.z_part, (uint32_t)of)) : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) Z += shfl_xor_f64(Z, o);
+  float mass = 0.f;
+#pragma unroll 1
+  for (int i = 0; i < p.cluster; ++i) mass += cl_ld_f32(cl_map(&s.bin_mass[lane & (kRcMassBins - 1)], (uint32_t)i));
+#pragma unroll
+  for (int o = 1; o < kRcMassBins; o <<= 1) {
+    const float up = __shfl_up_sync(0xFFFFFFFFu, mass, o);
+    if (lane >= o) mass += up;
+  }
+  // an element is out if what is nearer to the greatest one than its unit's upper end has a share of top_p already
+  const unsigned enough = __ballot_sync(0xFFFFFFFFu, lane < kRcMassBins && (double)mass >= (double)pp * 1.0001 * Z);
+  int tok = kRcScan;
+  if (enough) {
+    float lo = xmax - (float)__ffs(enough);
+    lo -= 1e-5f * fmaxf(fabsf(lo), fabsf(xmax));   // (the distances are rounded)
+    unsigned short* queue = reinterpret_cast<unsigned short*>(smem + layout.off_s) + warp_id() * kRcQueue;
+#pragma unroll 1
+    for (int round = 0; round < 8; ++round) {
+      const RcTop best = rc_best_from<DT>(part, lo, r, queue);
+      if (round == 0) { TLX_STAMP(p.sp, 10); }
+      // of the CTA: the best score, its element, and the second best score
+      const uint32_t mine = rc_score_key(best.a1), ak = rc_max_u32(mine, s, tog);
+      if (mine == ak) s.pick[3] = (int)threadIdx.x;
+      __syncthreads();
+      const bool chosen = s.pick[3] == (int)threadIdx.x;
+      const uint32_t ak2 = rc_max_u32(rc_score_key(chosen ? best.a2 : best.a1), s, tog);
+      if (chosen) {
+        s.query[0] = key_f32(ak);
+        s.query[1] = elem_as_float<DT>(part.elem(best.at));
+        s.query[2] = key_f32(ak2);
+        s.query_tok[0] = (int)(col0 + best.at);
+      }
+      if (round == 0) { TLX_STAMP(p.sp, 5); }
+      cl_sync();
+      const uint32_t q = cl_map(s.query, (uint32_t)of);
+      const float a = asks ? cl_ld_f32(q) : -INFINITY, xa = cl_ld_f32(q + 4), a2 = asks ? cl_ld_f32(q + 8) : -INFINITY;
+      const int ta = (int)cl_ld_u32(cl_map(s.query_tok, (uint32_t)of));
+      const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, rc_score_key(a));
+      if (top <= 0x007FFFFFu) break;   // no score
+      const float cut = rc_cut(key_f32(top));
+      const unsigned near_ = __ballot_sync(0xFFFFFFFFu, a >= cut);
+      if (__popc(near_) > 1 || __any_sync(0xFFFFFFFFu, a2 >= cut)) break;
+      const int winner = __ffs(near_) - 1;
+      const float x1 = __shfl_sync(0xFFFFFFFFu, xa, winner);
+      const int t1 = __shfl_sync(0xFFFFFFFFu, ta, winner);
+      if (x1 == xmax) { tok = t1; break; }   // nothing lies above it: kept whatever top_p is
+      // the mass down to the lower end of its unit is below top_p, which settles it; else the mass above it is summed up
+      const float upto = __shfl_sync(0xFFFFFFFFu, mass, min((int)(xmax - x1), kRcMassBins - 1));
+      if ((double)upto < (double)pp * 0.9999 * Z) { tok = t1; break; }
+      double above = 0.0, none = 0.0;
+      rc_masses_above<DT>(part, xmax, x1, above);
+      rc_sum2_f64(above, none, s, tog);
+      if (threadIdx.x == 0) s.z_part = above;   // (the denominator's parts were read before the last barrier of the cluster)
+      if (round == 0) { TLX_STAMP(p.sp, 13); }
+      cl_sync();
+      double m = asks ? cl_ld_f64(cl_map(&s.z_part, (uint32_t)of)) : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m += shfl_xor_f64(m, o);
+      if (m == 0.0 || !(m / Z >= (double)pp)) { tok = t1; break; }
+      lo = key_f32(f32_key(x1) + 1u);
+    }
+  }
+  cl_sync();   // nobody leaves, or goes on, while its words may still be read
+  return tok;
+}
+
 // Rows without top-k.  Returns the token in the leader, -1 if the row has to be answered by rc_slow_row.
 template <int DT>
 __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart<DT>& part, int64_t col0, uint32_t rank, float pp,
@@ -962,14 +1212,24 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
     r.k1 = noise.key_dev ? __ldg(noise.key_dev + 1) : noise.k1;
     r.ctr0 = (uint32_t)(noise.row_of(nrow) * noise.vocab + col0);
   }
-  // every thread's greatest element and its score; of the CTA: the greatest element and the best-scored one of these
+  // every thread's greatest element
   GroupMax<DT> gm;
   gm.init();
 #pragma unroll 2
   for (int v = threadIdx.x; v < part.nvec; v += kRcThreads) gm.add(part.vec[v]);
-  float x = -INFINITY, a = -INFINITY;
+  float x = -INFINITY, least = INFINITY;   // (groups without a finite element are left out of the least)
 #pragma unroll
-  for (int j = 0; j < GroupMax<DT>::kSlots; ++j) x = fmaxf(x, gm.slot(j));
+  for (int j = 0; j < GroupMax<DT>::kSlots; ++j) {
+    const float g = gm.slot(j);
+    x = fmaxf(x, g);
+    if (g > -INFINITY) least = fminf(least, g);
+  }
+  if (pp < kRcPruneBelow && p.part_len >= (r.dense ? kRcPruneTensorPart : kRcPruneKeyPart)) {
+    const int tok = rc_pruned_row<DT>(p, part, col0, x, least, pp, r, s, layout, smem, tog);
+    if (tok != kRcScan) return tok;
+  }
+  // its score; of the CTA: the greatest element and the best-scored one of these
+  float a = -INFINITY;
   if (x > -INFINITY) {
     int at = 0;
 #pragma unroll 1

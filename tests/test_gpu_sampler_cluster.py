@@ -140,3 +140,46 @@ def test_flat_rows_without_top_k(cuda, dtype, from_key):
     bad = (to_np(tok) != exp) & ~flags
     assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
     assert (to_np(status) & 6 == 0).all()                      # none was answered by passes over global memory
+
+
+# rows without top-k whose values top-p bounds first: parts just long enough and just not, parts that end inside a vector, two
+# to sixteen CTAs; top_p from the least to what rules nothing out; what that way leaves to the other one: a constant row, equal
+# scores (constant noise), NaN, infinities; a threshold deep in the tail, several rounds (hot rows), a row in order
+@pytest.mark.parametrize("V", [8192, 23999, 24001, 50257, 96001, 131072])
+@pytest.mark.parametrize("dtype", ["bf16", "f32"])
+@pytest.mark.parametrize("noise_kind", ["key", "tensor", "constant"])
+def test_rows_bounded_by_top_p(cuda, dtype, V, noise_kind):
+    B = 16
+    x, tk, tp, T, noise = o.make_sampling_inputs(B=B, V=V, seed=V + 3, dtype=dtype)
+    xf = x.astype(np.float32)
+    tk[:] = 0
+    tp[:] = [0.0, 0.3, 0.6, 0.9, 0.95, 0.99, 0.9995, 0.99995, 1.0, 0.8, 0.8, 0.8, 0.8, 0.7, 0.9, 0.5]
+    T[:] = np.linspace(0.4, 1.6, B)
+    xf[9] = 0.5                                                # one value
+    xf[10] = np.round(xf[10])                                  # many equal values at the threshold
+    xf[11, V // 7:] = -np.inf                                  # masked
+    xf[12] *= 0.01                                             # flat: everything is scored
+    xf[13] = np.sort(xf[13])                                   # the kept ones sit in one part
+    xf[14] = np.where(np.arange(V) % 2 == 0, xf[14], xf[14] - 30)
+    T[15], tp[15] = 20.0, 0.2                                  # hot: the best score lies below the threshold, again and again
+    x = xf.astype(x.dtype)
+    if noise_kind == "constant":
+        noise = np.full_like(noise, 0.5)
+    kw = dict(rng_key=(41, V)) if noise_kind == "key" else dict(noise=noise)
+    exp, flags = o.sample(x, tk, tp, T, return_flags=True, **kw)
+    dkw = dict(rng_key=(41, V)) if noise_kind == "key" else dict(noise=to_dev(noise, cuda))
+    tok, status = ops.sample(to_dev(x, cuda), to_dev(tk, cuda), to_dev(tp, cuda), to_dev(T, cuda), return_status=True, **dkw)
+    bad = (to_np(tok) != exp) & ~flags
+    assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
+    assert (to_np(status) & 2 == 0).all()
+    # rows with NaNs and infinities give what they give by passes over the row in global memory, a longer row's way
+    xf[:4] = xf[13:14]
+    xf[0, 5], xf[1, V - 1], xf[2, 7], xf[3] = np.nan, np.inf, -np.inf, -np.inf
+    x = xf[:4].astype(x.dtype)
+    kw = dict(rng_key=(41, V)) if noise_kind == "key" else dict(noise=noise[:4])
+    exp, flags = o.sample(x[2:3], tk[2:3], tp[2:3], T[2:3], return_flags=True,
+                          **(dict(noise=noise[2:3]) if noise_kind != "key" else dict(rng_key=(41, V), dim0_offset=2)))
+    dkw = dict(rng_key=(41, V)) if noise_kind == "key" else dict(noise=to_dev(noise[:4], cuda))
+    tok = to_np(ops.sample(to_dev(x, cuda), to_dev(tk[:4], cuda), to_dev(tp[:4], cuda), to_dev(T[:4], cuda), **dkw))
+    assert ((tok >= 0) & (tok < V)).all()
+    assert flags[0] or tok[2] == exp[0]
