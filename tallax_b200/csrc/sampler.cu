@@ -693,11 +693,12 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   p.P = l.P; p.part_chunks = l.part_chunks; p.nchunks = l.nchunks; p.nfin = l.nfin; p.row_bytes = sp.vocab * 2;
   // the noise tensor can be streamed next to the logits if its rows start on 16-byte boundaries
   const int dense = sp.noise.dense && (reinterpret_cast<uintptr_t>(sp.noise.dense) & 15) == 0 && (sp.noise.stride & 3) == 0;
-  // Wide rows' arg-max over their kept elements: with such a noise tensor the stream kernel does it (final
-  // items, one record each; at most 128 per row); otherwise the finish kernel makes a final pass with the
-  // CTAs that three per SM leave beside one per row.
-  const int64_t fin_items = (sp.vocab + kStFinalElems - 1) / kStFinalElems;
-  const bool final_in_stream = dense && fin_items <= 128 && fin_items <= l.nfin && !getenv("TLX_FINAL_IN_FINISH");
+  // Wide rows' arg-max over their kept elements: the stream kernel does it (final items, one record each; at most 128 per row), but
+  // for a noise tensor that cannot be streamed, for which the finish kernel makes a final pass with the CTAs that three per SM leave
+  // beside one per row.  (With noise from a key it made that pass too, after the whole stream kernel: bf16 [256, 151936] mixed
+  // parameters 63 us, [256, 128256] without top-k 149; as final items 48 and 95.)
+  const int64_t fin_elems = sp.noise.dense ? StFinal<false>::kElems : StFinal<true>::kElems, fin_items = (sp.vocab + fin_elems - 1) / fin_elems;
+  const bool final_in_stream = (dense || !sp.noise.dense) && fin_items <= 128 && fin_items <= l.nfin && !getenv("TLX_FINAL_IN_FINISH");
   p.fin_items = final_in_stream ? (int)fin_items : 0;
   p.fin_ctas = final_in_stream ? 0 : (3 * sms - (int)sp.rows < sms ? sms : 3 * sms - (int)sp.rows);
   p.error_flag = (int*)ws;
@@ -718,9 +719,11 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   const int64_t items = sp.rows * (int64_t)l.P;
   const size_t st_smem = kStFixedSmem + (size_t)sp.rows * 6;   // descriptor word and order entry per row
   const size_t fin_smem = kStFinishFixedSmem + (size_t)sp.rows * sizeof(int);
-  static SmemLimit stream_limit, finish_limits[2];
+  static SmemLimit stream_limits[2], finish_limits[2];
   int rc;
-  if ((rc = raise_smem(stream_limit, (const void*)sample_stream_kernel, st_smem, "sample")) != TLX_OK) return rc;
+  const bool from_key = !sp.noise.dense;
+  const auto stream = from_key ? sample_stream_kernel<true> : sample_stream_kernel<false>;
+  if ((rc = raise_smem(stream_limits[from_key], (const void*)stream, st_smem, "sample")) != TLX_OK) return rc;
   const auto finish = p.fin_ctas > 0 ? sample_finish_kernel<true> : sample_finish_kernel<false>;
   if ((rc = raise_smem(finish_limits[p.fin_ctas > 0], (const void*)finish, fin_smem, "sample")) != TLX_OK) return rc;
   // An SM changes its split between L1 and shared memory only while idle: the three kernels ask for the same
@@ -733,7 +736,8 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
     std::lock_guard<std::mutex> lock(mu);
     if (dev >= 0 && dev < 64 && !done[dev]) {
       cudaFuncSetAttribute((const void*)sample_prologue_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-      cudaFuncSetAttribute((const void*)sample_stream_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      cudaFuncSetAttribute((const void*)sample_stream_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+      cudaFuncSetAttribute((const void*)sample_stream_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       cudaFuncSetAttribute((const void*)sample_finish_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       cudaFuncSetAttribute((const void*)sample_finish_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
       done[dev] = true;
@@ -750,7 +754,7 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   if (stages < 2) return TLX_OK;
   const int64_t sgrid = items < 4ll * sms ? items : 4ll * sms;
   TLX_TIMELINE_KERNEL(1);
-  if ((rc = launch_dependent(sample_stream_kernel, {(unsigned)sgrid, kStThreads, st_smem}, st, "sample (stream)", p)) != TLX_OK) return rc;
+  if ((rc = launch_dependent(stream, {(unsigned)sgrid, kStThreads, st_smem}, st, "sample (stream)", p)) != TLX_OK) return rc;
   if (stages < 3) return TLX_OK;
   TLX_TIMELINE_KERNEL(2);
   return launch_dependent(finish, {(unsigned)(p.fin_ctas + sp.rows), kStThreads, fin_smem}, st, "sample (finish)", p, dense);

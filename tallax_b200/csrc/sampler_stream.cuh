@@ -22,11 +22,13 @@
 //             window and sum of exp(x - window top) of everything below it, both added to the row's
 //             totals in the workspace; the CTA that delivers a wide row's last part takes the row's
 //             maximum, softmax denominator and top-p threshold key from the totals.
-//   finish    two kinds of CTA in one grid.  The first ones stream the wide rows again, one CTA per
-//             (row, range of 8 KB chunks), logits (from L2) and the chunk's noise side by side:
-//             screened Gumbel score of every kept element; each range leaves its best element as a
-//             record, and the CTA that delivers a row's last record decides the row on the
-//             f64-evaluated term among the records within the screening slack of the best one.  The
+//             Last come the wide rows' final items: ranges of a row's elements, logits (from L2) and the
+//             noise side by side, or logits alone where the noise comes from a key: the screened
+//             Gumbel score of every kept element that can still win; each item leaves its best
+//             element as a record, and the row's CTA of the next kernel decides the row on the
+//             f64-evaluated term among the records within the screening slack of the best one.
+//   finish    two kinds of CTA in one grid.  For a noise tensor that cannot be copied in bulk the first ones
+//             do the work of the final items, one CTA per (row, range of 8 KB chunks).  The
 //             other CTAs, one per row, finish the normal rows from their candidate lists (they were all
 //             taken with the same threshold, so "at least top_k of them" proves that they hold the
 //             top-k set): top-k boundary, softmax mass and top-p threshold from one histogram over the
@@ -59,11 +61,13 @@ constexpr int kStMinVocab = 16384;
 constexpr int kFinChunk = 8192;                      // final pass: bytes of logits per slot ...
 constexpr int kFinChunkElems = kFinChunk / 2;
 constexpr int kFinNoiseChunk = kFinChunkElems * 4;   // ... and of f32 noise
-// final items of the stream kernel: the logits and the noise of kStFinalElems elements of a wide row, in
-// chunks that fill a slot of the ring (2 + 4 bytes per element)
-constexpr int kStFinalChunkElems = kStChunk / 6;
-constexpr int kStFinalChunks = 4;
-constexpr int kStFinalElems = kStFinalChunks * kStFinalChunkElems;
+// final items of the stream kernel: the logits and the noise of some elements of a wide row, in chunks that fill a slot of the
+// ring: with a noise tensor four of 2 + 4 bytes per element, else two of the logits alone
+template <bool kKey> struct StFinal {
+  static constexpr int kChunkElems = kKey ? kStChunk / 2 : kStChunk / 6, kChunks = kKey ? 2 : 4, kElems = kChunks * kChunkElems;
+};
+constexpr int kStFinalQueue = 384;                   // final items, noise from a key: places a warp has noted (up to 127 + 32 lanes x 8)
+static_assert(kStWarps * kStFinalQueue * 2 <= (kWin + 512) * 4, "the queues lie in the window's space");
 constexpr int kFinSlots = 2;
 constexpr int kFinVecPerThread = kFinChunk / 16 / kStThreads;   // 2
 static_assert(kStMaxPartChunks * kStChunkElems <= 65536, "candidate positions are 16 bits");
@@ -121,8 +125,8 @@ struct StreamParams {
   int* wflag;            // [rows] wide rows: an element lay above the window
   WideState* wstate;     // [rows]
   FinRecord* records;    // [rows * nfin]
-  int fin_items;             // final items per wide row (kStFinalElems elements each); 0: the finish
-                             // kernel makes the final pass over the wide rows
+  int fin_items;             // final items per wide row (StFinal<noise from a key>::kElems elements each); 0: the
+                             // finish kernel makes the final pass over the wide rows
   int* rowdone;              // per row: parts of a normal row whose candidate lists are complete
   int* row_signals;          // 1 once the stream kernel has decided to count them (it does when the batch has
                              // wide rows, whose final items keep it busy long after the normal rows are done)
@@ -498,7 +502,7 @@ struct StProducer {
 };
 
 // Item codes: row << 8 | part for the logits of a part of a row; row << 8 | 0x80 | sub for a final item
-// (logits and noise of the elements [sub * kStFinalElems, (sub + 1) * kStFinalElems) of a wide row).
+// (logits, and noise of a tensor, of the sub-th StFinal::kElems elements of a wide row).
 struct StOrder {
   const unsigned short* rows;   // the wide rows, then the normal rows (each in row order)
   int nwide;
@@ -527,29 +531,34 @@ __device__ __forceinline__ int st_part_chunks(const StreamParams& p, int part) {
   const int rest = p.nchunks - part * p.part_chunks;
   return rest < p.part_chunks ? rest : p.part_chunks;
 }
+template <bool kKey>
 __device__ __forceinline__ int st_final_item_chunks(const StreamParams& p, int sub) {
-  const int64_t rest = p.sp.vocab - (int64_t)sub * kStFinalElems;
-  return rest >= kStFinalElems ? kStFinalChunks : (int)((rest + kStFinalChunkElems - 1) / kStFinalChunkElems);
+  using F = StFinal<kKey>;
+  const int64_t rest = p.sp.vocab - (int64_t)sub * F::kElems;
+  return rest >= F::kElems ? F::kChunks : (int)((rest + F::kChunkElems - 1) / F::kChunkElems);
 }
+template <bool kKey>
 __device__ __forceinline__ int st_code_chunks(const StreamParams& p, int code) {
-  return (code & 0x80) ? st_final_item_chunks(p, code & 0x7F) : st_part_chunks(p, code & 0x7F);
+  return (code & 0x80) ? st_final_item_chunks<kKey>(p, code & 0x7F) : st_part_chunks(p, code & 0x7F);
 }
 
+template <bool kKey>
 __device__ __forceinline__ void st_issue_chunk(const StreamParams& p, StProducer& ps, unsigned char* ring, StControl& ctl,
                                                int slot) {
   const unsigned char* src;
   uint32_t bytes;
   if (ps.part & 0x80) {
-    // logits to the front of the slot, noise behind them
-    const int64_t e0 = (int64_t)(ps.part & 0x7F) * kStFinalElems + (int64_t)ps.chunk * kStFinalChunkElems;
+    // logits to the front of the slot, noise (of a tensor) behind them
+    using F = StFinal<kKey>;
+    const int64_t e0 = (int64_t)(ps.part & 0x7F) * F::kElems + (int64_t)ps.chunk * F::kChunkElems;
     const int64_t rest = p.sp.vocab - e0;
-    const uint32_t elems = (uint32_t)(rest < kStFinalChunkElems ? rest : kStFinalChunkElems);
+    const uint32_t elems = (uint32_t)(rest < F::kChunkElems ? rest : F::kChunkElems);
     unsigned char* dst = ring + (size_t)slot * kStChunk;
-    mbar_expect_tx(&ctl.mbar[slot], elems * 6);
+    mbar_expect_tx(&ctl.mbar[slot], elems * (kKey ? 2 : 6));
     bulk_load(dst, reinterpret_cast<const __nv_bfloat16*>(p.sp.logits) + (int64_t)ps.row * p.sp.row_stride + e0, elems * 2,
               &ctl.mbar[slot]);
-    bulk_load(dst + kStFinalChunkElems * 2, p.sp.noise.dense_row(ps.row + p.sp.dim0_offset) + e0,
-              elems * 4, &ctl.mbar[slot]);
+    if constexpr (!kKey)
+      bulk_load(dst + F::kChunkElems * 2, p.sp.noise.dense_row(ps.row + p.sp.dim0_offset) + e0, elems * 4, &ctl.mbar[slot]);
     ps.chunk++;
     return;
   } else {
@@ -565,6 +574,7 @@ __device__ __forceinline__ void st_issue_chunk(const StreamParams& p, StProducer
 }
 
 // Requests the next chunk into `slot` (thread 0 only).
+template <bool kKey>
 __device__ __forceinline__ void st_issue(const StreamParams& p, StProducer& ps, const StOrder& order, unsigned char* ring,
                                          StControl& ctl, int slot) {
   for (;;) {
@@ -577,7 +587,7 @@ __device__ __forceinline__ void st_issue(const StreamParams& p, StProducer& ps, 
       ps.row = code >> 8;
       ps.part = code & 0xFF;
       ps.chunk = 0;
-      ps.nchunks = st_code_chunks(p, code);
+      ps.nchunks = st_code_chunks<kKey>(p, code);
       // The next item is claimed now, an item ahead, so that the counter's round trip stays off the path --
       // except behind a final item when there are fewer final items than CTAs: those are the last items of
       // the list and long ones, and a CTA that holds one must not sit on a second one while other CTAs run
@@ -588,7 +598,7 @@ __device__ __forceinline__ void st_issue(const StreamParams& p, StProducer& ps, 
     ctl.fifo[ps.pushed & 7] = code;
     ps.pushed++;
   }
-  st_issue_chunk(p, ps, ring, ctl, slot);
+  st_issue_chunk<kKey>(p, ps, ring, ctl, slot);
 }
 
 // A chunk of a final item: logits (front of the slot) and noise (behind them) of the elements [elem0,
@@ -610,7 +620,7 @@ __device__ __forceinline__ void st_final_chunk(const unsigned char* buf, int ngr
   if (__hblt2(m, tv2)) return;   // all eight below the threshold
   const float xg = fmaxf(__low2float(m), __high2float(m));   // NaN-propagating max: a NaN keeps the test open
   const float eps = xg == xg ? __expf(-(cbm - xg * inv_T)) * 1.00001f : INFINITY;
-  const float* nbuf = reinterpret_cast<const float*>(buf + kStFinalChunkElems * 2) + v * 8;
+  const float* nbuf = reinterpret_cast<const float*>(buf + StFinal<false>::kChunkElems * 2) + v * 8;
   const float4 n0 = *reinterpret_cast<const float4*>(nbuf);
   const float4 n1 = *reinterpret_cast<const float4*>(nbuf + 4);
   const float umax = fmaxf(fmaxf(fmaxf(n0.x, n0.y), fmaxf(n0.z, n0.w)), fmaxf(fmaxf(n1.x, n1.y), fmaxf(n1.z, n1.w)));
@@ -630,6 +640,63 @@ __device__ __forceinline__ void st_final_chunk(const unsigned char* buf, int ngr
   }
 }
 
+// The same with noise from a key, of the `elems` elements from elem0 on: a warp notes the places of the elements whose value
+// allows a winner with the greatest noise there is, and makes their noise 128 at a time, four interleaved chains a lane.  low: the
+// cbm above; ctr0: counter of element elem0.
+__device__ __forceinline__ void st_final_chunk_key(const unsigned char* buf, int elems, int elem0, float tvf, float inv_T, float T_,
+                                                   float low, uint32_t k0, uint32_t k1, uint32_t ctr0, unsigned short* queue,
+                                                   float& a1, float& a2, float& u1, uint32_t& b1, int& t1) {
+  const int lane = lane_id();
+  const uint32_t lt = (1u << lane) - 1u;
+  const float xcut = fmaxf(tvf, (low - 15.95f) * T_);   // (the Gumbel term of 1 - 2^-23: 15.943)
+  int waiting = 0;
+#pragma unroll 1
+  for (int g0 = 0; g0 * 8 < elems; g0 += kStThreads) {
+    const int g = g0 + (int)threadIdx.x;
+    const bool last = (g0 + kStThreads) * 8 >= elems;
+    uint32_t mask = 0;
+    if (g * 8 < elems) {
+      const uint4 x = *reinterpret_cast<const uint4*>(buf + (size_t)g * 16);
+      const uint32_t w[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float xf = __uint_as_float((e & 1) ? (w[e >> 1] & 0xFFFF0000u) : (w[e >> 1] << 16));
+        mask |= xf >= xcut ? 1u << e : 0u;
+      }
+    }
+    for (uint32_t some = __ballot_sync(0xFFFFFFFFu, mask != 0); some; some = __ballot_sync(0xFFFFFFFFu, mask != 0)) {
+      const int slot = waiting + __popc(some & lt);
+      if (mask && TLX_IN_BOUNDS(slot, kStFinalQueue, 11)) queue[slot] = (unsigned short)(g * 8 + __ffs(mask) - 1);
+      mask &= mask - 1;
+      waiting += __popc(some);
+    }
+    __syncwarp();
+    while (waiting >= 128 || (last && waiting > 0)) {
+      const int count = min(waiting, 128);
+      waiting -= count;
+      int at[4];
+      float u[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        at[k] = lane + 32 * k < count ? queue[waiting + lane + 32 * k] : -1;
+        u[k] = fmaxf(threefry_uniform01(k0, k1, ctr0 + (uint32_t)at[k]), kF32Tiny);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (at[k] < 0) continue;
+        const uint32_t bits = reinterpret_cast<const unsigned short*>(buf)[at[k]];
+        const float xf = __uint_as_float(bits << 16);
+        if (!(1.0f - u[k] <= __expf(fmaf(xf, inv_T, -low)) * 1.0001f)) continue;
+        const float a = fmaf(xf, inv_T, gumbel_screen(u[k]));
+        const int tok = elem0 + at[k];
+        if (a > a1 || (a == a1 && tok < t1)) { a2 = a1; a1 = a; u1 = u[k]; b1 = bits; t1 = tok; }
+        else if (a > a2) a2 = a;
+      }
+    }
+    __syncwarp();
+  }
+}
+
 // Counts the noted items in their rows' rowdone (thread 0): one fence for all of them, then plain adds.
 __device__ __forceinline__ int st_publish_rows(const StreamParams& p, StControl& ctl, int n) {
   if (n > 0) {
@@ -641,7 +708,10 @@ __device__ __forceinline__ int st_publish_rows(const StreamParams& p, StControl&
 
 // Shared memory beyond the fixed part: per row 4 bytes of descriptor (class << 16 | key) and 2 bytes of order.
 // The grid is a multiple of P (whole rows in the first wave) and at most rows * P.
+// kKey: the noise comes from a key.
+template <bool kKey>
 __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamParams p) {
+  using F = StFinal<kKey>;
   extern __shared__ __align__(128) unsigned char st_smem[];
   unsigned char* ring = st_smem;
   uint32_t* area = reinterpret_cast<uint32_t*>(st_smem + kStRingBytes);
@@ -701,12 +771,12 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
   ps.row = ps.item >> 8;
   ps.part = ps.item & 0xFF;
   ps.chunk = 0;
-  ps.nchunks = ps.item >= 0 ? st_code_chunks(p, ps.item) : 0;
+  ps.nchunks = ps.item >= 0 ? st_code_chunks<kKey>(p, ps.item) : 0;
   ps.next = 0;
   ps.pushed = 1;
   if (threadIdx.x == 0) {
     ctl.fifo[0] = ps.item;
-    for (int s = 0; s < kStSlots && s < ps.nchunks; ++s) st_issue_chunk(p, ps, ring, ctl, s);
+    for (int s = 0; s < kStSlots && s < ps.nchunks; ++s) st_issue_chunk<kKey>(p, ps, ring, ctl, s);
   }
   // everything below reads what the prologue kernel wrote
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -728,7 +798,7 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
   if (signal_rows && blockIdx.x == 0 && threadIdx.x == 0) *reinterpret_cast<volatile int*>(p.row_signals) = 1;
   if (threadIdx.x == 0) {
     // a first item shorter than the ring: go on into the claimed items
-    for (int s = ps.chunk; s < kStSlots; ++s) st_issue(p, ps, order, ring, ctl, s);
+    for (int s = ps.chunk; s < kStSlots; ++s) st_issue<kKey>(p, ps, order, ring, ctl, s);
   }
   __syncthreads();
 
@@ -774,8 +844,15 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
       const uint32_t tbits = key16_bf16_bits((uint32_t)wide_vstar16(res));
       const __nv_bfloat162 tv2 = bf162_splat_bits(tbits);
       const float tvf = __uint_as_float(tbits << 16);
-      const int nc = st_final_item_chunks(p, part);
-      const int64_t last_elems = p.sp.vocab - ((int64_t)part * kStFinalElems + (int64_t)(nc - 1) * kStFinalChunkElems);
+      const int nc = st_final_item_chunks<kKey>(p, part);
+      const int64_t last_elems = p.sp.vocab - ((int64_t)part * F::kElems + (int64_t)(nc - 1) * F::kChunkElems);
+      uint32_t k0 = 0, k1 = 0, row0 = 0;   // key, and counter of the row's first element
+      if constexpr (kKey) {
+        const NoiseSrc& ns = p.sp.noise;
+        k0 = ns.key_dev ? __ldg(ns.key_dev) : ns.k0;
+        k1 = ns.key_dev ? __ldg(ns.key_dev + 1) : ns.k1;
+        row0 = (uint32_t)(ns.row_of(row + p.sp.dim0_offset) * ns.vocab);
+      }
       float a1 = -INFINITY, a2 = -INFINITY, u1 = 0.5f, published = -INFINITY;
       uint32_t b1 = 0;
       int t1 = 0x7FFFFFFF;
@@ -785,17 +862,21 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
         const float cbm = cb - 2.0f * (kGumbelSlack + 1e-5f * fabsf(cb));
         const bool arrived = mbar_wait_suspended(&ctl.mbar[slot], phase);
         const unsigned char* buf = ring + (size_t)slot * kStChunk;
-        const int elem0 = part * kStFinalElems + ci * kStFinalChunkElems;
+        const int elem0 = part * F::kElems + ci * F::kChunkElems;
         if (res >= 0 && !(p.debug & 1)) {
-          const int ngroups = ci != nc - 1 || last_elems >= kStFinalChunkElems ? kStFinalChunkElems / 8 : (int)(last_elems >> 3);
-          st_final_chunk(buf, ngroups, elem0, tv2, tvf, inv_T, cbm, a1, a2, u1, b1, t1);
+          const int elems = ci != nc - 1 || last_elems >= F::kChunkElems ? F::kChunkElems : (int)last_elems;
+          if constexpr (kKey)
+            st_final_chunk_key(buf, elems, elem0, tvf, inv_T, ctl.fin_T, cbm, k0, k1, row0 + (uint32_t)elem0,
+                               reinterpret_cast<unsigned short*>(area) + warp * kStFinalQueue, a1, a2, u1, b1, t1);
+          else
+            st_final_chunk(buf, elems >> 3, elem0, tv2, tvf, inv_T, cbm, a1, a2, u1, b1, t1);
         }
         if (a1 > published) { atomicMax(&ctl.best_key, f32_key(a1)); published = a1; }
         if (__syncthreads_or(!arrived)) {
           if (threadIdx.x == 0) *p.error_flag = 1;
           return;
         }
-        if (threadIdx.x == 0) st_issue(p, ps, order, ring, ctl, slot);
+        if (threadIdx.x == 0) st_issue<kKey>(p, ps, order, ring, ctl, slot);
         if (++slot == kStSlots) { slot = 0; phase ^= 1u; }
       }
 #ifdef TLX_TIMELINE
@@ -873,7 +954,7 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
         return;
       }
       // the chunk is consumed, its slot is free
-      if (threadIdx.x == 0) st_issue(p, ps, order, ring, ctl, slot);
+      if (threadIdx.x == 0) st_issue<kKey>(p, ps, order, ring, ctl, slot);
       if (++slot == kStSlots) { slot = 0; phase ^= 1u; }
     }
 #ifdef TLX_TIMELINE
@@ -1751,7 +1832,7 @@ static __device__ __forceinline__ bool st_finish_row(const StreamParams& p, int 
       // the stream kernel has left a record per final item of the row: decide
       StControl& ctl = *reinterpret_cast<StControl*>(smem + kFinSlots * kFinSlotBytes);
       __syncthreads();
-      fin_decide_row(p, row, p.fin_items, kStFinalElems, ctl);
+      fin_decide_row(p, row, p.fin_items, sp.noise.dense ? StFinal<false>::kElems : StFinal<true>::kElems, ctl);
     }
     if (!slow && threadIdx.x == 0 && sp.out_status) atomicOr(sp.out_status + row, (int)kStatusGeneral | timeout);
   }

@@ -314,3 +314,29 @@ def test_streaming_path_row_counts(cuda, B):
     for _ in range(2):
         again, _ = ops.sample(*args, noise=dn, return_status=True)
         assert np.array_equal(to_np(again), got)
+
+
+# large calls with noise from a key: the stream kernel's final items take a wide row's elements in chunks of 6144, two an item; rows
+# that end eight elements into a chunk, inside one, and with an item
+@pytest.mark.parametrize("V", [73736, 65544, 147456])
+def test_stream_wide_rows_with_noise_from_a_key(cuda, V):
+    B, n = (17 << 20) // (2 * V) + 1, 24                       # (beyond 16 MB of logits; the first n rows are looked at)
+    x, tk, tp, T, _ = o.make_sampling_inputs(B=n, V=V, seed=V, dtype="bf16")
+    xf = x.astype(np.float32)
+    tk[:] = 0
+    tp[:] = np.tile(np.float32([0.05, 0.5, 0.8, 0.9, 0.97, 0.9999, 0.9, 0.7]), 3)
+    T[:] = np.linspace(0.4, 1.6, n)
+    xf[6] *= 0.01                                              # flat: everything is scored
+    xf[7] = np.round(xf[7])
+    xf[14, V // 9:] = -np.inf
+    xf[15] = np.sort(xf[15])                                   # the kept ones sit in the last items
+    T[22], tp[22] = 20.0, 0.3
+    tk[3], tk[11] = 40, 900                                    # normal rows among them
+    x = xf.astype(x.dtype)
+    exp, flags = o.sample(x, tk, tp, T, rng_key=(13, V), return_flags=True)
+    pad = lambda a: np.concatenate([a, np.tile(a, ((B - n + len(a) - 1) // len(a),) + (1,) * (a.ndim - 1))[:B - n]])
+    tok, status = ops.sample(to_dev(pad(x), cuda), to_dev(pad(tk), cuda), to_dev(pad(tp), cuda), to_dev(pad(T), cuda),
+                             rng_key=(13, V), return_status=True)
+    bad = (to_np(tok)[:n] != exp) & ~flags
+    assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[:n][bad], exp[bad])
+    assert (to_np(status) & 2 == 0).all()
