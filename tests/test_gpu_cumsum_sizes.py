@@ -23,3 +23,11 @@ def test_cumsum_sizes(cuda, shape, axis, reverse):
     f = (x % 8).astype(np.float32)
     g = np.flip(np.cumsum(np.flip(f, axis), axis=axis), axis) if reverse else np.cumsum(f, axis=axis)
     assert np.array_equal(to_np(tax.cumsum(to_dev(f, cuda), axis, reverse=reverse)), g)
+
+
+# rows over clusters, a turn ahead and (too many of them) not: one turn, several, one that ends with a vector's first element; rows
+# that begin at any element
+@pytest.mark.parametrize("shape", [(1, 4097), (65, 33001), (66, 33001), (260, 9001), (261, 9001), (2, 131075), (3, 32765), (5, 65537)])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_cumsum_over_clusters(cuda, shape, reverse):
+    test_cumsum_sizes(cuda, shape, 1, reverse)
