@@ -44,33 +44,52 @@ __device__ __forceinline__ typename Elem<DT>::type cast_replace(double v) {
   else return (uint32_t)v;
 }
 
+// What the exchange buffer's header says to a step: bit 0, which of its two sets the step uses; bit 1, whether the call's extents are
+// the buffer's.  It changes between steps only, when no candidate kernel runs.
+__device__ __forceinline__ uint32_t exchange_state(const TopkParams& p) {
+  const volatile ExchangeHeader* h = reinterpret_cast<const volatile ExchangeHeader*>(p.ex.peer[p.ex.rank]);
+  const uint32_t step = h->step, rows = h->rows, k = h->k_cand, world = h->world;
+  return (step & 1u) | (rows == (uint32_t)p.rows && k == (uint32_t)p.k_max && world == (uint32_t)p.ex.world ? 2u : 0u);
+}
+// Candidate stage: the noise of the row's element `col`.
+__device__ __forceinline__ float candidate_noise(const TopkParams& p, int64_t r, int32_t col) {
+  return p.noise.dense ? __ldg(p.noise.dense + r * p.noise.stride + col) : p.noise.at(r + p.dim0_offset, (int64_t)col + p.col_offset);
+}
+struct PlacedRow {         // a short list in order; candidate stage: with what was read while it was put in order
+  uint64_t cand[96];
+  float value[96], noise[96];
+  uint32_t state;          // exchange_state
+};
+
 // Writes a row's results from its sorted candidate list (m valid entries, the first K are the answer).
-template <int DT>
+// kStage: as the candidate stage (-1: as the call says).  kPlaced: `cand` is a PlacedRow's.
+template <int DT, int kStage = -1, bool kPlaced = false>
 __device__ __forceinline__ void emit_row(const TopkParams& p, int64_t r, const typename Elem<DT>::type* __restrict__ row,
                                          const uint64_t* cand, int m, int refinements = 0, int bin = 0) {
+  const PlacedRow* known = kPlaced ? reinterpret_cast<const PlacedRow*>(cand) : nullptr;
   using T = typename Elem<DT>::type;
   const int K = p.k_max;
   const int k_row = p.k_per_row ? p.k_per_row[r] : K;
   uint32_t par = 0;   // which of the exchange buffer's two sets this step uses
-  bool deliver = p.ex.world > 0;
-  if (p.ex.world > 0) {
+  const bool exchange = kStage != 0 && p.ex.world > 0;
+  bool deliver = exchange;
+  if (exchange) {
     // a call whose extents are not the buffer's stores nothing anywhere and leaves a mark
-    volatile ExchangeHeader* h = reinterpret_cast<volatile ExchangeHeader*>(p.ex.peer[p.ex.rank]);
-    par = h->step & 1u;
-    deliver = h->rows == (uint32_t)p.rows && h->k_cand == (uint32_t)K && h->world == (uint32_t)p.ex.world;
-    if (!deliver && threadIdx.x == 0) h->error = 2u;
+    const uint32_t state = kPlaced ? known->state : exchange_state(p);
+    par = state & 1u;
+    deliver = (state & 2u) != 0;
+    if (!deliver && threadIdx.x == 0) reinterpret_cast<volatile ExchangeHeader*>(p.ex.peer[p.ex.rank])->error = 2u;
   }
   for (int j = threadIdx.x; j < K; j += blockDim.x) {
     const uint64_t c = cand[j];
     const int32_t col = (int32_t)cand_low(c);
     const bool have = j < m;
-    if (p.cand_vals || p.ex.world > 0) {
+    if (kStage < 0 ? p.cand_vals || exchange : kStage == 1) {
       // candidate stage: f32 value, global token id, noise at that token
-      const float v = have ? elem_as_float<DT>(row[col]) : -INFINITY;
+      const float v = !have ? -INFINITY : kPlaced ? known->value[j] : elem_as_float<DT>(row[col]);
       const int64_t tok = (int64_t)col + p.col_offset;
-      float u = 0.5f;
-      if (have) u = p.noise.dense ? __ldg(p.noise.dense + r * p.noise.stride + col) : p.noise.at(r + p.dim0_offset, tok);
-      if (p.ex.world > 0) {
+      const float u = !have ? 0.5f : kPlaced ? known->noise[j] : candidate_noise(p, r, col);
+      if (exchange) {
         if (!deliver) continue;
         // slot `rank` of every rank's buffer, this rank's own included, starting with the next rank
         const size_t plane = (size_t)p.rows * K;
@@ -94,7 +113,7 @@ __device__ __forceinline__ void emit_row(const TopkParams& p, int64_t r, const t
       p.out_idx[r * K + j] = have ? col : 0;
     }
   }
-  if (p.ex.world > 0) {
+  if (exchange) {
     // the row's block is on its way to every rank: one arrival count each, released after the stores
     __syncthreads();
     if (deliver && (int)threadIdx.x < p.ex.world) {
@@ -458,8 +477,10 @@ __global__ void __launch_bounds__(TH, 1024 / TH) topk_sampled_kernel(TopkParams 
   }
 }
 
-// SUB: the bound comes from one piece in SUB of the row
-template <int DT, int SUB>
+// SUB: the bound comes from one piece in SUB of the row.  kStage: 1 the candidate stage, whose values, noise and exchange header are
+// read while the composites are counted, not one after the other behind it (1024 shard rows of 18 992, k = 50, with the merge: bf16
+// 36.1 -> 32.9 us, f16 38.2 -> 35.1, f32 41.5 -> 38.6); 0 not the stage; -1 as the call says.
+template <int DT, int SUB, int kStage>
 __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams p) {
   using T = typename Elem<DT>::type;
   constexpr int kSlots = GroupMax<DT>::kSlots;
@@ -601,18 +622,29 @@ __global__ void __launch_bounds__(kShortThreads, 8) topk_short_kernel(TopkParams
   if (m <= 96) {
     // a handful of candidates: every thread counts the composites below its own (they are distinct) and
     // puts it at that place; no network, no barriers in between
-    uint64_t* placed = reinterpret_cast<uint64_t*>(s.hist);
+    static_assert(sizeof(PlacedRow) <= sizeof(s.hist));
+    PlacedRow& placed = *reinterpret_cast<PlacedRow*>(s.hist);
+    if (kStage == 1 && p.ex.world > 0 && threadIdx.x == blockDim.x - 1) placed.state = exchange_state(p);
     if ((int)threadIdx.x < m) {
       const uint64_t c = cand[threadIdx.x];
+      float v = 0.f, u = 0.f;
+      if constexpr (kStage == 1) {
+        v = elem_as_float<DT>(row[cand_low(c)]);
+        u = candidate_noise(p, r, (int32_t)cand_low(c));
+      }
       int below = 0;
       for (int i = 0; i < m; ++i) below += cand[i] < c ? 1 : 0;
-      placed[below] = c;
+      placed.cand[below] = c;
+      if constexpr (kStage == 1) {
+        placed.value[below] = v;
+        placed.noise[below] = u;
+      }
     }
     __syncthreads();
-    emit_row<DT>(p, r, row, placed, m);
+    emit_row<DT, kStage, kStage == 1>(p, r, row, placed.cand, m);
   } else {
     sort_candidates(cand, m);
-    emit_row<DT>(p, r, row, cand, m);
+    emit_row<DT, kStage>(p, r, row, cand, m);
   }
 }
 
@@ -804,22 +836,26 @@ static cudaError_t ask_shared_memory(std::mutex& mu, bool (&asked)[64], F* kerne
   return e;
 }
 
-template <int DT, int SUB>
+template <int DT, int SUB, int kStage>
 static int launch_topk_short_from(cudaStream_t st, const TopkParams& p) {
   const size_t smem = sizeof(SelectShared);
   static std::mutex mu;
   static bool asked[64] = {};
-  cudaError_t e = ask_shared_memory(mu, asked, topk_short_kernel<DT, SUB>, smem, 1024 / kShortThreads);
+  cudaError_t e = ask_shared_memory(mu, asked, topk_short_kernel<DT, SUB, kStage>, smem, 1024 / kShortThreads);
   if (e != cudaSuccess) return set_error(TLX_ERR_CUDA, "top_k: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  return launch_dependent(topk_short_kernel<DT, SUB>, {(unsigned)p.rows, kShortThreads, smem, 1, -1, p.ex.world > 0}, st, "top_k (short rows)", p);
+  return launch_dependent(topk_short_kernel<DT, SUB, kStage>, {(unsigned)p.rows, kShortThreads, smem, 1, -1, p.ex.world > 0}, st, "top_k (short rows)", p);
 }
 // 16-bit rows of more than 1 MB, which L2 does not keep between the passes: the bound from a quarter of the row (bf16 [1024, 600000],
 // k = 20: 228 us against 355)
+// Without the stage's code the compiler fits bf16 rows into the 64 registers without a spill (bf16 [256, 30000], k = 64: 17.1 -> 16.3
+// us, [4096, 8192] 47.7 -> 46.7), the other forms only with it (f16 [1024, 18992], k = 50: 20.0 against 20.6, bf16 [592, 600000],
+// k = 20: 146 against 156).
 template <int DT>
 static int launch_topk_short(cudaStream_t st, const TopkParams& p) {
   if constexpr (DT != TLX_F32)
-    if (p.n * (int64_t)sizeof(typename Elem<DT>::type) / 16 > kSampledVecs) return launch_topk_short_from<DT, 4>(st, p);
-  return launch_topk_short_from<DT, 1>(st, p);
+    if (p.n * (int64_t)sizeof(typename Elem<DT>::type) / 16 > kSampledVecs) return launch_topk_short_from<DT, 4, -1>(st, p);
+  if (p.cand_vals || p.ex.world > 0) return launch_topk_short_from<DT, 1, 1>(st, p);
+  return launch_topk_short_from<DT, 1, DT == TLX_BF16 ? 0 : -1>(st, p);
 }
 
 template <int DT, int TH>

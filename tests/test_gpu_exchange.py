@@ -196,3 +196,42 @@ def test_merge_of_sorted_blocks_with_ties_and_every_top_k(cuda, world, k):
     exp, flags = o.merge_and_sample(cv, ci, cn, tk, tp, T, return_flags=True)
     assert not ((tok != exp) & ~flags).any()
     assert flags.mean() < 0.2
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "f16", "f32"])
+@pytest.mark.parametrize("n,k", [(2048, 1), (2051, 50), (9000, 96), (5003, 128)])
+def test_candidates_of_many_rows_are_read_while_they_are_put_in_order(cuda, dtype, n, k):
+    """At least 256 rows: up to 96 candidates are read as they are placed, more (ties, k = 128) after the network.  Values, tokens and
+    noise are exact, from a tensor and from a key, and the exchange gives the tokens of the gathered path."""
+    import torch
+    from tallax_b200._src import ops
+
+    rows, off, V = 260, 777, 777 + n
+    g = torch.Generator().manual_seed(n + k)
+    x = torch.randn(rows, n, generator=g)
+    x[1::7] = (x[1::7] * 4).round() / 4                # more than 96 candidates at one value
+    x[3, ::5] = float("-inf")
+    x = x.to({"bf16": torch.bfloat16, "f16": torch.float16, "f32": torch.float32}[dtype])
+    noise = torch.rand(rows, n, generator=g) * 0.98 + 0.01
+    order = torch.sort(x.float(), dim=1, descending=True, stable=True).indices[:, :k]
+    dx, dn = x.cuda(), noise.cuda()
+    got = ops.shard_candidates(dx, off, k, noise_shard=dn, vocab_total=V).cpu()
+    assert torch.equal(got[0], x.float().gather(1, order))
+    assert torch.equal(got[1].view(torch.int32), (order + off).int())
+    assert torch.equal(got[2], noise.gather(1, order))
+    key = (5, 9)
+    keyed = ops.shard_candidates(dx, off, k, rng_key=key, vocab_total=V, dim0_offset=3).cpu()
+    few = torch.cat([ops.shard_candidates(dx[a:a + 130], off, k, rng_key=key, vocab_total=V, dim0_offset=3 + a).cpu() for a in (0, 130)], 1)
+    assert torch.equal(keyed.view(torch.int32), few.view(torch.int32))
+
+    ex = ops.Exchange.local_group(rows, k, 1, dx.device)[0]
+    try:
+        tk = torch.full((rows,), k, dtype=torch.int32).cuda()
+        tp, T = torch.full((rows,), 0.9).cuda(), torch.full((rows,), 0.8).cuda()
+        for step in range(3):
+            ops.exchange_shard_candidates(dx, off, ex, noise_shard=dn, vocab_total=V)
+            tok = ops.exchange_merge_and_sample(ex, tk, tp, T)
+            assert torch.equal(tok, ops.merge_and_sample(got[None].cuda(), tk, tp, T))
+            assert ex.state() == (step + 1, 0)
+    finally:
+        ex.close()
