@@ -23,8 +23,9 @@
 // What bounds it: latency and barriers, then instruction issue (about 200 per 32 elements).
 // us, radix passes (up to 1024 elements: the bitonic network) / this, normal keys: f32 [128, 65536] 329 / 138, [128, 12000]
 // 53 / 17, [1024, 4096] 79 / 32, [64, 4097] 19.4 / 7.8, [1000, 700] 22 / 10.5, [1, 131072] 88 / 38; bf16, of two passes,
-// [128, 65536] 178 / 141, [1024, 4096] 46 / 34, [64, 4097] 11.4 / 8.1.  Rounded keys, which fall back: f32 [128, 65536] 290 / 302,
-// [1024, 1025] 38 / 40, bf16 [128, 65536] 170 / 188.
+// [128, 65536] 178 / 141, [1024, 4096] 46 / 34, [64, 4097] 11.4 / 8.1.  Rounded keys (27 values), which fall back, radix
+// kernel / the passes in this one: f32, of which two passes are left out, [128, 65536] 290 / 185, [1024, 4096] 90 / 53, [256, 50000]
+// 463 / 307; where none are, what was done before them is lost: bf16 [128, 65536] 171 / 191, [64, 4097] 11.2 / 11.9, i32 [300, 20000] 179 / 199.
 //   Tried: two places an element (groups of 1.5 elements) made nothing faster and a sort through in_perm a fifth slower, because
 // the shared memory it takes is the L1 that the reads through in_perm need.
 #pragma once
@@ -128,11 +129,15 @@ __global__ void __launch_bounds__(kRadixMaxThreads) sort_places_kernel(
   uint32_t least = k[0], greatest = k[0], diff = 0, equal = 0;
   uint32_t first = RK::make(krow[prow ? prow[0] : 0]) ^ flip;
   if (kHalf) first <<= 16;
+  // Float keys: of negative numbers all bits are turned round.  A bit that is the same in all of them once that is undone is the
+  // same in all keys of one sign, and the last pass parts the signs (f32 of few digits, of both signs: two passes, not four).
+  auto upright = [&](uint32_t key) { return DT == TLX_I32 || DT == TLX_U32 ? key : key ^ (~(uint32_t)((int32_t)key >> 31) & 0x7FFFFFFFu); };
+  first = upright(first);
 #pragma unroll
   for (int j = 0; j < IPT; ++j) {
     least = min(least, k[j]);
     greatest = max(greatest, k[j]);
-    diff |= k[j] ^ first;
+    diff |= upright(k[j]) ^ first;
   }
   if (kHalf) diff &= 0xFFFF0000u;
   {

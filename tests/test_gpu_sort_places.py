@@ -84,3 +84,24 @@ def test_operands_beside_the_first_key(cuda, n, payloads, key):
             assert torch.equal(g.isnan(), e.isnan()) and not torch.signbit(g[g == 0]).any()
             g, e = g.nan_to_num(nan=1e9), e.nan_to_num(nan=1e9)
         assert torch.equal(g, e)
+
+
+# keys of both signs whose lower digits only tell the sign (the passes leave them out), with the values whose bits are not their
+# key's: -0, NaNs of both signs, infinities; and rows of one sign
+@pytest.mark.parametrize("n", [300, 4097, 16385, 65536])
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "f16"])
+def test_keys_of_few_digits_and_both_signs(cuda, dtype, n):
+    rng = np.random.default_rng(n)
+    z = rng.standard_normal((5, n)).astype(np.float32)
+    z[0], z[1], z[2], z[3] = np.round(z[0] * 3), np.round(z[1] * 3) - 20, np.abs(np.round(z[2] * 3)), z[3].astype(np.float16)
+    z[4] = np.where(rng.random(n) < 0.5, np.float32(1.5), np.float32(-1.5))
+    z[::2, ::11], z[::2, 1::11], z[::4, 2::50], z[::4, 3::50] = 0.0, -0.0, np.inf, -np.inf
+    z[0, 4::50] = np.array([0x7FC00000, 0xFFC12300], np.uint32).view(np.float32)[rng.integers(0, 2, len(z[0, 4::50]))]
+    t = torch.from_numpy(z).to({"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16}[dtype])
+    a = t.float().numpy()
+    nan = np.isnan(a)
+    a = np.where(nan, 0, a)
+    for descending in (False, True):
+        p = tax.sort([t.to(cuda)], num_keys=1, is_stable=True, return_argsort=True, descending=descending)[1]
+        e = np.lexsort((-a, ~nan) if descending else (a, nan), axis=1)
+        assert np.array_equal(p.cpu().numpy(), e)
