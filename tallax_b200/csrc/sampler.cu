@@ -629,11 +629,12 @@ static bool stream_path_serves(int dtype, int64_t rows, int64_t vocab, int64_t r
 // Where they meet depends on the parameters, which the host does not know.  us stream / cluster, requests with mixed
 // parameters, with one usual top_k and without top-k:
 //                      a noise tensor                     a key
-//   [32, 128256]   28/26  17/13  33/31            33/33  22/12  40/42
-//   [48, 151936]   30/34  22/14  38/41            35/42  27/14  49/56
-//   [64, 128256]   31/32  22/15  39/36            37/41  26/14  56/60
-//   [256, 32000]   33/41  34/25  40/47            39/49  31/23  66/61
-//   [72, 128256]   32/34  23/22  44/41            38/41  26/20  61/58
+//   [32, 128256]   28/23  16/12  33/30            30/23  17/12  36/29
+//   [48, 151936]   30/28  21/14  38/39            33/28  22/14  40/40
+//   [64, 128256]   31/29  22/15  39/36            33/28  21/15  41/38
+//   [256, 32000]   33/39  34/25  41/38            34/38  28/23  44/40
+//   [72, 128256]   32/32  23/21  45/40            35/29  22/20  48/40
+//   [80, 128256]   33/35  23/22  46/40            37/32  25/21  50/42
 // Up to 16 MB the cluster form saves more on the one usual setting than it loses on mixed ones; beyond, it runs in several waves.
 // One rule for both kinds of noise: the workspace's size is asked for before the noise is known.
 static bool stream_path_wanted(int64_t rows, int64_t vocab) { return rows * vocab * 2 > (16ll << 20); }
