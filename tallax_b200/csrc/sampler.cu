@@ -231,7 +231,7 @@ static __device__ __noinline__ int tail_bf16_hist(const SampleParams& p, int64_t
   }
   TLX_STAMP(p, 6);
   const Best top = block_best(Best{a1, c1}, s);
-  const float cut = top.y - (kGumbelSlack + 1e-5f * fabsf(top.y));
+  const float cut = screen_cut(top.y);
   const int leaders = __syncthreads_count(a1 >= cut);
   const int crowded = __syncthreads_or(a2 >= cut);
   TLX_STAMP(p, 7);
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(256) gumbel_argmax_kernel(const float* __restr
   if (threadIdx.x == 0) {
     Best b{-INFINITY, 0x7FFFFFFF};
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) b = best_of(b, Best{sy[w], sp[w]});
-    out[line] = b.tok;
+    out[line] = b.tok != 0x7FFFFFFF ? b.tok : 0;   // nothing has a score: the line's first position
   }
 }
 

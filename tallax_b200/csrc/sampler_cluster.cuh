@@ -60,9 +60,6 @@ __device__ __forceinline__ void rc_pick_bin(const uint32_t* h, int need, int* ou
 
 // Key of a score for an unsigned maximum; NaN is below everything.
 __device__ __forceinline__ uint32_t rc_score_key(float a) { return a == a ? f32_key(a) : 0u; }
-__device__ __forceinline__ float rc_cut(float smax) {
-  return fabsf(smax) < INFINITY ? smax - (kGumbelSlack + 1e-5f * fabsf(smax)) : smax;
-}
 __device__ __forceinline__ unsigned long long rc_win_make(float y, int64_t tok) {
   return ((unsigned long long)rc_score_key(y) << 32) | (uint32_t)(0x7FFFFFFF - (int32_t)tok);
 }
@@ -131,7 +128,7 @@ static __device__ __noinline__ int rc_slow_row(const typename Elem<DT>::type* __
     });
     const uint32_t ak = rc_max_u32(a, s, tog);
     if (ak == 0) return top_col;   // nothing has a score
-    const float cut = rc_cut(key_f32(ak));
+    const float cut = screen_cut(key_f32(ak));
     uint64_t w = 0;
     for_each_elem<DT>(row, 0, n, [&](T v, int64_t c) {
       if (eligible(v, c)) {
@@ -326,7 +323,7 @@ static __device__ __noinline__ int rc_decide_large(RcShared& s, int m, float pp,
     a = __reduce_max_sync(0xFFFFFFFFu, s.red_u32[2][lane_id() & (kRcWarps - 1)]);
     if (first) x0 = key_f32(__reduce_max_sync(0xFFFFFFFFu, s.red_u32[3][lane_id() & (kRcWarps - 1)]));
     if (a <= 0x007FFFFFu) return -1;   // NaN or -inf
-    const float cut = rc_cut(key_f32(a));
+    const float cut = screen_cut(key_f32(a));
 #pragma unroll 1
     for (int i = threadIdx.x; i < m; i += kRcThreads)
       if ((first || lx[i] > above) && ls[i] >= cut) {
@@ -437,7 +434,7 @@ static __device__ __noinline__ int rc_decide_small(RcShared& s, int m, int K, fl
     best = __reduce_max_sync(0xFFFFFFFFu, best);
     int tok = -1;
     if (best > 0x007FFFFFu) {
-      const float cut = rc_cut(key_f32(best));
+      const float cut = screen_cut(key_f32(best));
       int near_ = 0;
       uint32_t hi = 0, lo = 0;
 #pragma unroll 1
@@ -631,7 +628,7 @@ __device__ __forceinline__ int rc_best_sent(int most, bool first, float above, c
     if (first || l.all_x[i] > above) a = max(a, rc_score_key(l.all_s[i]));
   a = __reduce_max_sync(0xFFFFFFFFu, a);
   if (a <= 0x007FFFFFu) return -1;
-  const float cut = rc_cut(key_f32(a));
+  const float cut = screen_cut(key_f32(a));
   int near_ = 0, at = -1;
 #pragma unroll 1
   for (int i = i0; i < i1; i += 2)
@@ -672,7 +669,7 @@ __device__ __forceinline__ int rc_thin_out(int m, float* lx, float* ls, unsigned
 #pragma unroll 1
     for (int i = lane; i < m; i += 32)
       if ((first || lx[i] > above) && rc_score_key(ls[i]) == a) xk = max(xk, f32_key(lx[i]));
-    const float x = key_f32(__reduce_max_sync(0xFFFFFFFFu, xk)), cut = rc_cut(key_f32(a));
+    const float x = key_f32(__reduce_max_sync(0xFFFFFFFFu, xk)), cut = screen_cut(key_f32(a));
 #pragma unroll 1
     for (int i = lane; i < m; i += 32)
       if ((first || lx[i] > above) && lx[i] <= x && ls[i] < cut) ls[i] = -INFINITY;
@@ -1072,7 +1069,7 @@ __device__ __forceinline__ RcTop rc_best_from(const RcPart<DT>& part, float lo, 
         else if (a > best.a2) best.a2 = a;
       }
       const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, rc_score_key(best.a1));
-      if (top > 0x007FFFFFu) reach = rc_cut(key_f32(top));
+      if (top > 0x007FFFFFu) reach = screen_cut(key_f32(top));
     }
     __syncwarp();
   }
@@ -1165,7 +1162,7 @@ __device__ __forceinline__ int rc_pruned_row(const RcSampleParams& p, const RcPa
       const int ta = (int)cl_ld_u32(cl_map(s.query_tok, (uint32_t)of));
       const uint32_t top = __reduce_max_sync(0xFFFFFFFFu, rc_score_key(a));
       if (top <= 0x007FFFFFu) break;   // no score
-      const float cut = rc_cut(key_f32(top));
+      const float cut = screen_cut(key_f32(top));
       const unsigned near_ = __ballot_sync(0xFFFFFFFFu, a >= cut);
       if (__popc(near_) > 1 || __any_sync(0xFFFFFFFFu, a2 >= cut)) break;
       const int winner = __ffs(near_) - 1;
@@ -1280,11 +1277,11 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
     // [0]: the published element with the best score; [1]: the row's greatest element; the rest: filled below
     if (threadIdx.x < 2) {
       s.cut_x[threadIdx.x] = threadIdx.x == 0 ? bx : xmax;
-      s.cut_s[threadIdx.x] = rc_cut(threadIdx.x == 0 ? bs : ms);
+      s.cut_s[threadIdx.x] = screen_cut(threadIdx.x == 0 ? bs : ms);
     }
     if (threadIdx.x == 0) s.n_cut = 2;
     __syncthreads();
-    RcLow low{bx, rc_cut(bs), rc_cut(ms)};
+    RcLow low{bx, screen_cut(bs), screen_cut(ms)};
     float above = -INFINITY;
 #pragma unroll 1
     for (int attempt = 0;; ++attempt) {
@@ -1309,7 +1306,7 @@ __device__ __forceinline__ int rc_wide_row(const RcSampleParams& p, const RcPart
         for (int i = threadIdx.x; i < kRcWideCap; i += kRcThreads)
           if ((first || l.x[i] > above) && rc_score_key(l.s[i]) == bk) xk = max(xk, f32_key(l.x[i]));
         above = key_f32(rc_max_u32(xk, s, tog));
-        const float cut = rc_cut(key_f32(bk));
+        const float cut = screen_cut(key_f32(bk));
         if (threadIdx.x == 0) { s.cut_x[cuts] = above; s.cut_s[cuts] = cut; }
         ++cuts;
         if (first && cut > low.bs) { low.bs = cut; low.bx = above; }

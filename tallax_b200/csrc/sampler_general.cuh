@@ -128,7 +128,7 @@ static __device__ __noinline__ int final_argmax(const typename Elem<DT>::type* _
     else if (a > a2) a2 = a;
   });
   const Best top = block_best(Best{a1, c1}, s);
-  const float cut = top.y - (kGumbelSlack + 1e-5f * fabsf(top.y));
+  const float cut = screen_cut(top.y);
   const int crowded = __syncthreads_or(a2 >= cut);
   Best best{-INFINITY, 0x7FFFFFFF};
   if (!crowded) {

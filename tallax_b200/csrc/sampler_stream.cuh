@@ -900,7 +900,7 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
         const bool any = btok != 0x7FFFFFFF;
         const bool mine = any ? (key == bkey && t1 == btok) : threadIdx.x == 0;
         const float amax = key_f32(bkey);
-        const float cut = amax - (kGumbelSlack + 1e-5f * fabsf(amax));
+        const float cut = screen_cut(amax);
         const int multi = __syncthreads_or(any && ((!mine && a1 >= cut) || a2 >= cut));
         if (mine) {
           FinRecord r;
@@ -1344,8 +1344,9 @@ __device__ __forceinline__ int st_finish_normal(const StreamParams& p, int row, 
   uint32_t bkey;
   int btok;
   tl_block_top(a1, t1, t, bkey, btok);
+  if (btok == 0x7FFFFFFF) return -1;   // no kept candidate has a score
   const float amax = key_f32(bkey);
-  const float cut = amax - (kGumbelSlack + 1e-5f * fabsf(amax));
+  const float cut = screen_cut(amax);
   const bool mine = f1 >= 0 && f32_key(a1) == bkey && t1 == btok;
   const int multi = __syncthreads_or((f1 >= 0 && !mine && a1 >= cut) || a2 >= cut);
   TLX_STAMP(sp, 7);
@@ -1426,6 +1427,8 @@ static __device__ __noinline__ void st_slow_row(const StreamParams& p, int row, 
       tok = general_row_bf16<kWin>(rowp, n, K, pp, T_, sp.noise, nrow, s, win, none);
     }
   }
+  // nothing in the row has a score (NaNs): its greatest element, as the cluster form answers it
+  if (tok == 0x7FFFFFFF) tok = 0x7FFFFFFF - (int)(uint32_t)row_argmax<TLX_BF16>(rowp, n, s);
   if (threadIdx.x == 0) {
     if (__ldcg(p.error_flag)) status |= kStatusTimeout;
     sp.out_tokens[row] = tok;
@@ -1483,7 +1486,7 @@ __device__ __forceinline__ void fin_decide_row(const StreamParams& p, int row, i
   amax = ctl.fbest[0];
 #pragma unroll
   for (int w = 1; w < kStWarps; ++w) amax = fmaxf(amax, ctl.fbest[w]);
-  const float cut = amax - (kGumbelSlack + 1e-5f * fabsf(amax));
+  const float cut = screen_cut(amax);
   const bool contender = tok != 0x7FFFFFFF && a >= cut;
   Best best{-INFINITY, 0x7FFFFFFF};
   if (contender && !(bits & 0x10000u)) best = Best{__fdiv_rn(__uint_as_float(bits << 16), T_) + gumbel_exact(u), tok};
@@ -1762,7 +1765,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
     const bool any = btok != 0x7FFFFFFF;
     const bool mine = any ? (key == bkey && t1 == btok) : threadIdx.x == 0;
     const float amax = key_f32(bkey);
-    const float cut = amax - (kGumbelSlack + 1e-5f * fabsf(amax));
+    const float cut = screen_cut(amax);
     const int multi = __syncthreads_or(any && ((!mine && a1 >= cut) || a2 >= cut));
     if (mine) {
       FinRecord r;

@@ -310,6 +310,8 @@ static __device__ __noinline__ int sort_candidates(uint64_t* cand, int m) {
 //   keep x_i >= x_t, y_i = x_i / T + gumbel(u_i), token = arg-max y (ties: lower token).
 // The arg-max is screened in f32 and decided on the f64-evaluated Gumbel term for the
 // contenders only.  All threads call; the result is valid in every thread.
+// A row in which nothing has a score (a NaN among the candidates is candidate 0 and makes the threshold one; a temperature
+// or noise that is a NaN) gets candidate 0's token.
 //
 // sample_tail<kMaxItems> keeps a thread's candidates in registers and serves K <= kMaxItems *
 // blockDim.x; above that it hands over to sample_tail_any, which serves any K by reading the
@@ -350,7 +352,7 @@ static __device__ __noinline__ int sample_tail_any(int K, float p, float T, Sele
   amax = -INFINITY;
   for (int w = 0; w < nw; ++w) amax = fmaxf(amax, (float)s.scan_f64[w]);
   __syncthreads();
-  const float cut = amax - (kGumbelSlack + 1e-5f * fabsf(amax));
+  const float cut = screen_cut(amax);
   Best best{-INFINITY, 0x7FFFFFFF};
   for (int i = i0; i < i1; ++i) {
     const float x = value_of(i);
@@ -365,7 +367,7 @@ static __device__ __noinline__ int sample_tail_any(int K, float p, float T, Sele
   Best b{-INFINITY, 0x7FFFFFFF};
   for (int w = 0; w < nw; ++w) b = best_of(b, Best{(float)s.scan_f64[w], (int)s.scan_u32[w]});
   __syncthreads();
-  return b.tok;
+  return b.tok != 0x7FFFFFFF ? b.tok : token_of(0);
 }
 
 // The same by one warp, K <= 32 * kMaxItems, without a barrier; every lane returns the token.  Contenders are only evaluated in f64
@@ -403,7 +405,7 @@ static __device__ __forceinline__ int sample_tail_warp(int K, float p, float T, 
   float amax = -INFINITY;
 #pragma unroll
   for (int j = 0; j < kMaxItems; ++j) {
-    a[j] = -INFINITY;
+    a[j] = NAN;   // (not kept: no contender, whatever the best score is)
     if (j < per && i0 + j < K && x[j] >= thr) {
       a[j] = __fdiv_rn(x[j], T) + gumbel_screen(u[j]);
       amax = fmaxf(amax, a[j]);
@@ -411,7 +413,7 @@ static __device__ __forceinline__ int sample_tail_warp(int K, float p, float T, 
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, o));
-  const float cut = amax - (kGumbelSlack + 1e-5f * fabsf(amax));
+  const float cut = screen_cut(amax);
   int contenders = 0, tok = 0x7FFFFFFF;
 #pragma unroll
   for (int j = 0; j < kMaxItems; ++j)
@@ -430,7 +432,8 @@ static __device__ __forceinline__ int sample_tail_warp(int K, float p, float T, 
     if (xi >= thr && __fdiv_rn(xi, T) + gumbel_screen(ui) >= cut)
       best = best_of(best, Best{__fdiv_rn(xi, T) + gumbel_exact(ui), token_of(i)});
   }
-  return warp_best(best).tok;
+  best = warp_best(best);
+  return best.tok != 0x7FFFFFFF ? best.tok : token_of(0);
 }
 
 template <int kMaxItems, typename ValueOf, typename TokenOf, typename NoiseOf>
@@ -472,7 +475,7 @@ static __device__ __noinline__ int sample_tail(int K, float p, float T, SelectSh
 #pragma unroll
   for (int j = 0; j < kMaxItems; ++j) {
     const int i = i0 + j;
-    a[j] = -INFINITY;
+    a[j] = NAN;   // (as above)
     if (j < per && i < K && x[j] >= thr) {
       u[j] = noise_of(i);
       a[j] = __fdiv_rn(x[j], T) + gumbel_screen(u[j]);
@@ -493,7 +496,7 @@ static __device__ __noinline__ int sample_tail(int K, float p, float T, SelectSh
     amax = m;
   }
   __syncthreads();
-  const float cut = amax - (kGumbelSlack + 1e-5f * fabsf(amax));
+  const float cut = screen_cut(amax);
   Best best{-INFINITY, 0x7FFFFFFF};
 #pragma unroll
   for (int j = 0; j < kMaxItems; ++j) {
@@ -513,7 +516,7 @@ static __device__ __noinline__ int sample_tail(int K, float p, float T, SelectSh
     best = b;
   }
   __syncthreads();
-  return best.tok;
+  return best.tok != 0x7FFFFFFF ? best.tok : token_of(0);
 }
 
 }  // namespace tlx

@@ -221,6 +221,10 @@ __device__ __forceinline__ float gumbel_screen(float u) {
   return -__logf(l);
 }
 constexpr float kGumbelSlack = 1e-3f;
+// Screened scores from here on may be the best exact one, `best` being the best screened one.  An infinite score has no slack.
+__device__ __forceinline__ float screen_cut(float best) {
+  return fabsf(best) < INFINITY ? best - (kGumbelSlack + 1e-5f * fabsf(best)) : best;
+}
 
 // ---- checked build ------------------------------------------------------------------------------
 // python -m tallax_b200.build --checked compiles with TLX_CHECKED: TLX_IN_BOUNDS(i, n, site) then tests an
