@@ -23,9 +23,13 @@
 // What bounds it: latency and barriers, then instruction issue (about 200 per 32 elements).
 // us, radix passes (up to 1024 elements: the bitonic network) / this, normal keys: f32 [128, 65536] 329 / 138, [128, 12000]
 // 53 / 17, [1024, 4096] 79 / 32, [64, 4097] 19.4 / 7.8, [1000, 700] 22 / 10.5, [1, 131072] 88 / 38; bf16, of two passes,
-// [128, 65536] 178 / 141, [1024, 4096] 46 / 34, [64, 4097] 11.4 / 8.1.  Rounded keys (27 values), which fall back, radix
-// kernel / the passes in this one: f32, of which two passes are left out, [128, 65536] 290 / 185, [1024, 4096] 90 / 53, [256, 50000]
-// 463 / 307; where none are, what was done before them is lost: bf16 [128, 65536] 171 / 191, [64, 4097] 11.2 / 11.9, i32 [300, 20000] 179 / 199.
+// [128, 65536] 178 / 141, [1024, 4096] 46 / 34, [64, 4097] 11.4 / 8.1.
+//   Rows that fall back take fewer passes than their digits where their keys have a shorter form: less the least one and without
+// the bits that are the same in all of them, or, of few different keys, their numbers, which are one digit.  us, a radix sort of all
+// digits / the passes of this kernel on the keys as they are / on the shorter form: rounded keys (27 values) bf16 [128, 65536] 170 / 191 / 140,
+// [1024, 4096] 46 / 50 / 41, [64, 4097] 11.2 / 12.0 / 10.0, [1000, 1500] 23.3 / 26.6 / 23.1, f16 [300, 20000] 109 / 120 / 92, f32 [128, 65536] 290 / 186 /
+// 136, [1024, 4096] 78 / 46 / 37; the same times a million, i32 [128, 65536] 295 / 303 / 249, [300, 20000] 179 / 199 / 160; two keys of which the first
+// has 50 values, bf16 [128, 65536] 456 / 420 / 367.
 //   Tried: two places an element (groups of 1.5 elements) made nothing faster and a sort through in_perm a fifth slower, because
 // the shared memory it takes is the L1 that the reads through in_perm need.
 #pragma once
@@ -43,12 +47,27 @@ constexpr uint32_t kPlaceMaxMean = 24;        // ... of an element's group on av
 constexpr int kPlaceWindow = 6;               // elements of a group that every element is compared with before any test
                                               // (six: one element in 1700 is in a larger group, one warp in fifty)
 
+constexpr int kMaxValues = 256;              // different keys of a row whose numbers are one digit
+// Entries of the table that numbers them, a byte each, at most: with more of them a pass over the CTA's `cap` elements is the cheaper one
+// (f32, with / without: 0..199, 17223 entries, [64, 4097], 4352 elements, 12.7 us / 11.7; [128, 65536], 16384 elements, 154 / 190; 0..49, 4241
+// entries, [1000, 1500], 2048 elements, 23.5 / 26.2).
+__host__ __device__ constexpr uint32_t value_table_max(uint32_t cap) { return cap < 4096 ? 8192 : 2 * cap; }
+
 struct __align__(16) PlaceShared {
   RadixShared radix;
   uint32_t red[4][32];     // of every warp: least key, greatest key, differing bits; groups' squares
   uint32_t row[4];         // this CTA's: least key, greatest key, differing bits
-  uint32_t to[32][8];      // of every warp: elements for every CTA of the cluster
+  union {
+    uint32_t to[32][8];            // of every warp: elements for every CTA of the cluster
+    uint32_t value[kMaxValues];    // a row of few keys: the keys by their numbers
+  };
   uint32_t count[8];       // of this CTA: the same
+  struct {
+    int encode;              // a row that is sorted by digits: it may have a shorter form
+    uint32_t base, most;     // its least and greatest key; shorter form: the base
+    uint32_t bits;           // of a key whose first bit is set, those that are the same in all keys
+    int shift, numbered;     // shorter form: (key >> shift) - base, or these keys' numbers (before: it may be a row of few keys)
+  } coded;
 };
 static_assert(sizeof(PlaceShared) % 16 == 0, "the counters behind it are cleared 16 bytes at a time");
 
@@ -63,8 +82,69 @@ template <int IPT> constexpr int kPlaceCounters = IPT > 8 ? IPT : 8;
 // ranges [2048] u16).
 template <int IPT, bool CL>
 __host__ __device__ __forceinline__ size_t place_smem(int threads) {
-  const size_t pairs = ((size_t)threads * kPlaceRoom<IPT, CL> + kPlaceWindow) * 8, ranges = (kPlaceRanges + 4) * 4 + kPlaceRanges * 2;
+  constexpr size_t ranges = (kPlaceRanges + 4) * 4 + kPlaceRanges * 2;
+  const size_t pairs = ((size_t)threads * kPlaceRoom<IPT, CL> + kPlaceWindow) * 8;
+  static_assert(IPT == 4 || value_table_max(256 * IPT) <= 256 * IPT * 8, "the table of a row of few keys lies in the pairs' place");
   return sizeof(PlaceShared) + (size_t)threads * kPlaceCounters<IPT> * 2 + (pairs > ranges ? pairs : ranges);
+}
+
+// Digits that the passes take of keys which differ in the bits `diff`.
+__device__ __forceinline__ int differing_digits(uint32_t diff) {
+  return (int)((diff & 0xFFu) != 0) + (int)((diff & 0xFF00u) != 0) + (int)((diff & 0xFF0000u) != 0) + (int)((diff >> 24) != 0);
+}
+
+// Rows of few different keys, of which every key has marked its entry of `table` [range] u8, the last one's among them: the marks become
+// the numbers of the keys in their order, and s.value[number] the key.  False if there are more than kMaxValues.
+//   In a cluster every CTA adds the others' marks to its own; the marks are summed up.  No atomics: a mark is the same whoever sets it.
+template <bool CL>
+static __device__ __forceinline__ bool number_marks(unsigned char* table, uint32_t range, int rank, int cluster, PlaceShared& s) {
+  const int nt = blockDim.x, vectors = (int)(range + 15) / 16;
+  uint4* t4 = reinterpret_cast<uint4*>(table);
+  if constexpr (CL) {
+    cl_sync();
+    for (int i = threadIdx.x; i < vectors; i += nt) {
+      uint4 q = t4[i];
+      for (int o = 1; o < cluster; ++o) {   // (what another one may have added by now are marks too)
+        const uint4 e = cl_ld_v4(cl_map(t4 + i, (uint32_t)(rank + o < cluster ? rank + o : rank + o - cluster)));
+        q.x |= e.x; q.y |= e.y; q.z |= e.z; q.w |= e.w;
+      }
+      t4[i] = q;
+    }
+    cl_sync();
+  } else {
+    __syncthreads();
+  }
+  // thread t < 256: `per` vectors from t * per on.  Marks -> marks before them (beyond the last mark the bytes may run over).
+  const int per = (vectors + 255) / 256, i0 = threadIdx.x * per, i1 = threadIdx.x < 256 ? min(i0 + per, vectors) : 0;
+  uint32_t marks = 0;
+  for (int i = i0; i < i1; ++i) {
+    const uint4 q = t4[i];
+    marks += __popc(q.x) + __popc(q.y) + __popc(q.z) + __popc(q.w);
+  }
+  uint32_t before = radix_scan256(marks, s.radix.warp);
+  if (threadIdx.x == 255) s.count[0] = before + marks;
+  for (int i = i0; i < i1; ++i) {
+    uint4 q = t4[i];
+    auto sums = [&](uint32_t& w) {
+      const uint32_t at = w * 0x01010101u;
+      w = before * 0x01010101u + (at << 8);
+      before += at >> 24;
+    };
+    sums(q.x); sums(q.y); sums(q.z); sums(q.w);
+    t4[i] = q;
+  }
+  __syncthreads();
+  if (s.count[0] > kMaxValues) return false;
+  // an entry is marked if the next one's number is another one (the last entry is)
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(table);
+  for (uint32_t i = threadIdx.x; 4 * i < range - 1; i += nt) {
+    const uint32_t w = words[i], next = w >> 8 | words[i + 1] << 24;
+#pragma unroll
+    for (uint32_t b = 0; b < 4; ++b)
+      if (((w ^ next) >> 8 * b & 255u) && 4 * i + b < range - 1) s.value[w >> 8 * b & 255u] = 4 * i + b;
+  }
+  if (threadIdx.x == 0) s.value[s.count[0] - 1] = range - 1;
+  return true;
 }
 
 template <int DT, int IPT, bool CL, bool PAST>
@@ -76,6 +156,7 @@ __global__ void __launch_bounds__(kRadixMaxThreads) sort_places_kernel(
   using T = typename Elem<DT>::type;
   constexpr bool kHalf = RK::kBits == 16;
   constexpr int kRoom = kPlaceRoom<IPT, CL>;
+  constexpr bool kShorter = IPT > 4;   // (four elements a thread: a pass costs little more than the search for a shorter form)
   extern __shared__ __align__(16) unsigned char place_raw[];
   const int nt = blockDim.x, nw = nt >> 5, cap = nt * IPT, n = (int)n64;
   const int lane = lane_id(), w = warp_id();
@@ -165,27 +246,45 @@ __global__ void __launch_bounds__(kRadixMaxThreads) sort_places_kernel(
   }
 
   // The radix passes of the whole row.  Rows that need two of them at most are done sooner that way.
-  auto whole_row_by_digits = [&]() {
+  auto whole_row_by_digits = [&](uint32_t passes, bool coded) {
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
       p[j] = (uint32_t)(c0 + i0 + 32 * j);
       if (32 * j >= left) k[j] = 0xFFFFFFFFu;
     }
     const bool scattered = radix_by_digits<IPT, 32, CL, PAST, uint32_t>(
-        reinterpret_cast<uint32_t(&)[IPT]>(k), reinterpret_cast<uint32_t(&)[IPT]>(p), diff, n, rank, cluster, s.radix, group_half,
+        reinterpret_cast<uint32_t(&)[IPT]>(k), reinterpret_cast<uint32_t(&)[IPT]>(p), passes, n, rank, cluster, s.radix, group_half,
         reinterpret_cast<uint32_t*>(pair), reinterpret_cast<uint32_t*>(pair) + cap);
     if constexpr (CL) cl_sync();   // (nobody leaves while another one may still read its counts)
+    if (coded) {
+      const int shift = s.coded.shift;
+      const uint32_t base = s.coded.base, bits = s.coded.bits, low = (1u << shift) - 1u;
+      const bool numbered = s.coded.numbered;
+#pragma unroll
+      for (int j = 0; j < IPT; ++j) {
+        const uint32_t top = ((numbered ? s.value[k[j] & 255u] : k[j]) + base) << shift;
+        k[j] = top | ((upright(top) == top ? bits : ~bits) & low);
+      }
+    }
 #pragma unroll
     for (int j = 0; j < IPT; ++j) {
       const int c = c0 + (scattered ? (int)threadIdx.x + j * nt : i0 + 32 * j);
       if (c < n) emit(c, k[j], p[j]);
     }
   };
-  const int digits = (int)((diff & 0xFFu) != 0) + (int)((diff & 0xFF00u) != 0) + (int)((diff & 0xFF0000u) != 0) + (int)((diff >> 24) != 0);
+  const int digits = differing_digits(diff);
   // Of 992 ordered pairs a warp, n / (32 IPT) warps, these are equal if an element's equals, with itself, are kPlaceMaxMean.
   // 16-bit keys, whose equals lie evenly: if one pair in 64 is, which are keys of a few dozen values.
   const uint32_t many = kHalf ? (uint32_t)n / (2 * IPT) : kPlaceMaxMean * 31 / IPT;
   bool by_digits = digits <= (kHalf ? 1 : 2) || equal > many;
+  // (what such a row needs later is left in shared memory: in registers it costs the rest of the kernel spilled ones)
+  if (kShorter && threadIdx.x == 0) {
+    s.coded.encode = by_digits && digits > 1;
+    s.coded.base = least;
+    s.coded.most = greatest;
+    s.coded.bits = first;
+    s.coded.numbered = equal * (8 * IPT) >= (uint32_t)n;   // one pair in 256 is equal, by the sample, as of 256 keys that are equally frequent
+  }
 
   int m = n, out0 = 0;   // CTA: elements that it puts right, and their first place in the row
   if (!by_digits) {
@@ -300,8 +399,46 @@ __global__ void __launch_bounds__(kRadixMaxThreads) sort_places_kernel(
     }
   }
   if (by_digits) {
-    if constexpr (!CL) __syncthreads();
-    whole_row_by_digits();
+    __syncthreads();
+    uint32_t passes = diff;
+    bool coded = false;
+    if (kShorter && s.coded.encode) {
+      const int low = __ffs(diff) - 1;
+      const uint32_t base = s.coded.base >> low, most = (s.coded.most >> low) - base;
+      const bool few = s.coded.numbered && most > 255 && most < value_table_max(cap);
+      bool numbered = false;
+      if (few || (39 - __clz(most)) / 8 < differing_digits(diff)) {
+#pragma unroll
+        for (int j = 0; j < IPT; ++j) k[j] = (k[j] >> low) - base;
+        if (few) {
+          unsigned char* table = reinterpret_cast<unsigned char*>(pair);
+          for (uint32_t i = threadIdx.x; i < most / 16 + 1; i += nt) reinterpret_cast<uint4*>(table)[i] = make_uint4(0, 0, 0, 0);
+          __syncthreads();
+#pragma unroll
+          for (int j = 0; j < IPT; ++j)
+            if (TLX_IN_BOUNDS(k[j], most + 1, 38)) table[k[j]] = 1;
+          numbered = number_marks<CL>(table, most + 1, rank, cluster, s);
+          if (numbered) {
+#pragma unroll
+            for (int j = 0; j < IPT; ++j) k[j] = table[k[j]];
+          }
+        }
+        passes = numbered ? 255 : 0xFFFFFFFFu >> __clz(most);
+        __syncthreads();   // (what is read above is overwritten)
+        if (threadIdx.x == 0) {
+          s.coded.base = base;
+          s.coded.shift = low;
+          s.coded.numbered = numbered;
+        }
+        // (passes of their own: where they meet the others' the kernel spills 70 bytes of registers, f32 [1024, 8192] 62.9 us against 61.6)
+        if constexpr (!CL) {
+          whole_row_by_digits(passes, true);
+          return;
+        }
+        coded = true;
+      }
+    }
+    whole_row_by_digits(passes, CL && coded);
     return;
   }
 

@@ -105,3 +105,41 @@ def test_keys_of_few_digits_and_both_signs(cuda, dtype, n):
         p = tax.sort([t.to(cuda)], num_keys=1, is_stable=True, return_argsort=True, descending=descending)[1]
         e = np.lexsort((-a, ~nan) if descending else (a, nan), axis=1)
         assert np.array_equal(p.cpu().numpy(), e)
+
+
+# rows of few values.  Near each other, they are numbered and sorted in one pass: two values, as many as fit one digit and one more; the
+# frequent one the least or the greatest; values that one CTA of a cluster sees and another does not, more in all than fit; as
+# far apart as the numbering's table reaches and further.  Others are sorted less the least one and without their common bits
+@pytest.mark.parametrize("copies,n", [(1, 300), (1, 1024), (50, 1500), (1, 4097), (3, 16385), (6, 20000), (1, 65536), (1, 131072)])
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "i32", "f16"])
+@pytest.mark.parametrize("spacing", ["scattered", "near", "far"])
+def test_rows_of_few_values(cuda, dtype, copies, n, spacing):
+    rng = np.random.default_rng(n)
+    types = {"f32": torch.float32, "bf16": torch.bfloat16, "f16": torch.float16, "i32": torch.int32}
+    at = np.arange(-300, 300) if spacing != "scattered" else np.unique(rng.integers(-2**31, 2**31, 600))
+    if dtype == "i32":
+        pool = (at * {"scattered": 1, "near": 6, "far": 7 << 20}[spacing]).astype(np.int32)
+    elif spacing == "scattered":
+        bits = np.arange(1, 30001, 100, dtype=np.int16)        # (positive, finite, and the same negative)
+        pool = torch.from_numpy(bits).view(types[dtype]).float().numpy() if dtype != "f32" else rng.random(300).astype(np.float32)
+        pool = np.unique(np.concatenate([pool, -pool]))
+    else:
+        pool = at.astype(np.float32) if spacing == "near" else np.sign(at) * 2.0 ** (np.abs(at) % 12) * (1 + np.abs(at) // 12 / 32)
+        pool = np.unique(torch.from_numpy(pool).to(types[dtype]).float().numpy())
+    rows = []
+    for count in (2, 3, 50, 200, 255, 256, 257, 258, 500):
+        for frequent in (0, -1):
+            v = pool[np.sort(rng.permutation(len(pool))[:count])]
+            v = pool[len(pool) // 2:][:count] if spacing == "near" and count < 256 else v
+            row = np.where(rng.random(n) < 0.5, v[frequent], rng.choice(v, n))
+            row[rng.permutation(n)[:min(n, len(v))]] = v[:n]     # each occurs
+            rows.append(row)
+    half = np.where(rng.random(n) < 0.6, pool[5], np.where(np.arange(n) < n // 2, rng.choice(pool[:150], n), rng.choice(pool[150:300], n)))
+    rows += [half, np.where(np.arange(n) < n // 2, pool[7], rng.choice(pool, n)), np.where(np.arange(n) % 2 == 0, pool[3], pool[4])]
+    a = np.stack(rows)
+    t, a = torch.from_numpy(a).to(types[dtype]), a.astype(np.float64)
+    for descending in (False, True):
+        v, p = tax.sort([t.to(cuda).repeat(copies, 1)], num_keys=1, is_stable=True, return_argsort=True, descending=descending)
+        e = np.argsort(-a if descending else a, axis=1, kind="stable")
+        assert np.array_equal(p.cpu().numpy(), np.tile(e, (copies, 1)))
+        assert torch.equal(v.cpu(), torch.take_along_dim(t, torch.from_numpy(e), 1).repeat(copies, 1))
