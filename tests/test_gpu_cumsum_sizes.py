@@ -31,3 +31,17 @@ def test_cumsum_sizes(cuda, shape, axis, reverse):
 @pytest.mark.parametrize("reverse", [False, True])
 def test_cumsum_over_clusters(cuda, shape, reverse):
     test_cumsum_sizes(cuda, shape, 1, reverse)
+
+
+# rounding errors along columns.  A large first element and ones that round up every time they are added to it alone: a running sum is off by
+# 0.4 units in the last place of the sum a row.  Sums of at most 16 rows, added up: their own additions, and those of their totals,
+# lose at most half a unit each, 2^-24 of the sum
+@pytest.mark.parametrize("rows,cols", [(9, 600), (40, 129), (41, 129), (48, 9000), (64, 33000), (128, 65537), (129, 65537)])
+@pytest.mark.parametrize("reverse", [False, True])
+def test_cumsum_of_few_rows_rounds_like_short_sums(cuda, rows, cols, reverse):
+    x = np.full((rows, cols), 1.2 * 2.0 ** -24, np.float32)
+    x[-1 if reverse else 0] = 1.0
+    got = to_np(tax.cumsum(to_dev(x, cuda), 0, reverse=reverse)).astype(np.float64)
+    want = np.cumsum(x[::-1] if reverse else x, axis=0, dtype=np.float64)
+    want = want[::-1] if reverse else want
+    assert np.abs(got - want).max() <= (16 + -(-rows // 8) + 1) * 2.0 ** -24 * want.max()
