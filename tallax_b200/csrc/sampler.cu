@@ -693,14 +693,14 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   p.sp = sp;
   p.P = l.P; p.part_chunks = l.part_chunks; p.nchunks = l.nchunks; p.nfin = l.nfin; p.row_bytes = sp.vocab * 2;
   // the noise tensor can be streamed next to the logits if its rows start on 16-byte boundaries
-  const int dense = sp.noise.dense && (reinterpret_cast<uintptr_t>(sp.noise.dense) & 15) == 0 && (sp.noise.stride & 3) == 0;
-  // Wide rows' arg-max over their kept elements: the stream kernel does it (final items, one record each; at most 128 per row), but
+  const bool dense = sp.noise.dense && (reinterpret_cast<uintptr_t>(sp.noise.dense) & 15) == 0 && (sp.noise.stride & 3) == 0;
+  // Wide rows' arg-max over their kept elements: the stream kernel does it (final items, one record each), but
   // for a noise tensor that cannot be streamed, for which the finish kernel makes a final pass with the CTAs that three per SM leave
   // beside one per row.  (With noise from a key it made that pass too, after the whole stream kernel: bf16 [256, 151936] mixed
   // parameters 63 us, [256, 128256] without top-k 149; as final items 48 and 95.)
-  const int64_t fin_elems = sp.noise.dense ? StFinal<false>::kElems : StFinal<true>::kElems, fin_items = (sp.vocab + fin_elems - 1) / fin_elems;
-  const bool final_in_stream = (dense || !sp.noise.dense) && fin_items <= 128 && fin_items <= l.nfin && !getenv("TLX_FINAL_IN_FINISH");
-  p.fin_items = final_in_stream ? (int)fin_items : 0;
+  const int64_t fin_elems = sp.noise.dense ? StFinal<false>::kElems : StFinal<true>::kElems;
+  const bool final_in_stream = dense || !sp.noise.dense;
+  p.fin_items = final_in_stream ? (int)((sp.vocab + fin_elems - 1) / fin_elems) : 0;
   p.fin_ctas = final_in_stream ? 0 : (3 * sms - (int)sp.rows < sms ? sms : 3 * sms - (int)sp.rows);
   p.error_flag = (int*)ws;
   p.item_counter = (int*)ws + 1;
@@ -758,7 +758,7 @@ static int launch_stream_path(cudaStream_t st, const SampleParams& sp, void* wor
   if ((rc = launch_dependent(stream, {(unsigned)sgrid, kStThreads, st_smem}, st, "sample (stream)", p)) != TLX_OK) return rc;
   if (stages < 3) return TLX_OK;
   TLX_TIMELINE_KERNEL(2);
-  return launch_dependent(finish, {(unsigned)(p.fin_ctas + sp.rows), kStThreads, fin_smem}, st, "sample (finish)", p, dense);
+  return launch_dependent(finish, {(unsigned)(p.fin_ctas + sp.rows), kStThreads, fin_smem}, st, "sample (finish)", p);
 }
 
 }  // namespace tlx

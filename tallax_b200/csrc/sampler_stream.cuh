@@ -58,9 +58,8 @@ constexpr int kStSampleVecs = 4;                     // 16-byte vectors per prol
 constexpr int kStProThreads = 128;
 constexpr int kStSample = kStProThreads * kStSampleVecs * 8;   // 4096 elements
 constexpr int kStMinVocab = 16384;
-constexpr int kFinChunk = 8192;                      // final pass: bytes of logits per slot ...
+constexpr int kFinChunk = 8192;                      // final pass: bytes of logits per slot
 constexpr int kFinChunkElems = kFinChunk / 2;
-constexpr int kFinNoiseChunk = kFinChunkElems * 4;   // ... and of f32 noise
 // final items of the stream kernel: the logits and the noise of some elements of a wide row, in chunks that fill a slot of the
 // ring: with a noise tensor four of 2 + 4 bytes per element, else two of the logits alone
 template <bool kKey> struct StFinal {
@@ -71,6 +70,9 @@ static_assert(kStWarps * kStFinalQueue * 2 <= (kWin + 512) * 4, "the queues lie 
 constexpr int kFinSlots = 2;
 constexpr int kFinVecPerThread = kFinChunk / 16 / kStThreads;   // 2
 static_assert(kStMaxPartChunks * kStChunkElems <= 65536, "candidate positions are 16 bits");
+constexpr int kStMaxVocab = kStMaxParts * kStMaxPartChunks * kStChunkElems;
+static_assert(kStMaxVocab <= 128 * StFinal<false>::kElems && kStMaxVocab <= 128 * StFinal<true>::kElems, "a final item's number is seven bits");
+static_assert(kFinChunkElems <= StFinal<false>::kElems && kFinChunkElems <= StFinal<true>::kElems, "a row's records have room for its final items");
 static_assert(kStChunkVecs % kStThreads == 0 && kFinChunk / 16 % kStThreads == 0, "whole vectors per thread");
 static_assert(kStMaxParts * kStWarps * (kStSpec / 16) <= kStThreads, "one round of speculative fetches per thread");
 
@@ -85,8 +87,7 @@ struct __align__(16) StreamDesc {
 
 struct __align__(16) WideState {
   int result;                // kWideNotReady until the row's threshold is settled; then -1 (the window did not
-                             // settle it) or (key of the greatest element - threshold key) << 16 | threshold key:
-                             // an element is kept if its value is not below the value of the threshold key
+                             // settle it) or the threshold key: an element is kept if its value is not below this key's
   uint32_t best_key;         // best screened score of a kept element of the row known so far (ordered key):
                              // seeded with the score of the row's greatest element when the threshold is
                              // published (one 8-byte store with `result`), raised by the final items
@@ -95,11 +96,6 @@ struct __align__(16) WideState {
 };
 static_assert(sizeof(WideState) == 16, "WideState layout");
 constexpr int kWideNotReady = (int)0x80000000;
-__device__ __forceinline__ int wide_result(int kmax16, int vstar16) {
-  return vstar16 < 0 ? -1 : ((kmax16 - vstar16) << 16) | vstar16;
-}
-__device__ __forceinline__ int wide_vstar16(int result) { return result < 0 ? -1 : (result & 0xFFFF); }
-__device__ __forceinline__ int wide_kmax16(int result) { return (result & 0xFFFF) + (result >> 16); }
 
 struct __align__(16) FinRecord {   // best element of one range of chunks of a wide row
   float a;          // its screened score
@@ -176,8 +172,7 @@ struct __align__(16) WideScratch {
   double dlump[16];
   int first[16];
   int vstar;
-  int kmax16;   // out: key of the greatest element
-  int pad[2];
+  int pad[3];
 };
 
 // Small per-CTA scratch shared by the kernels' block-wide steps.
@@ -246,7 +241,7 @@ __device__ __forceinline__ int wide_threshold_core(int wtop, float pp, const uin
     il += shfl_xor_f64(il, o);
   }
   if (lane == 31) { ws.dsum[warp] = im; ws.dlump[warp] = il; }
-  if (threadIdx.x == 0) { ws.vstar = -1; ws.kmax16 = kmax16; }
+  if (threadIdx.x == 0) ws.vstar = -1;
   __syncthreads();
   double total = 0.0, below = 0.0;
   for (int w = 0; w < kNW; ++w) {
@@ -841,7 +836,7 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
       __syncthreads();
       const int res = ctl.fin_result;
       const float inv_T = 1.0f / ctl.fin_T;
-      const uint32_t tbits = key16_bf16_bits((uint32_t)wide_vstar16(res));
+      const uint32_t tbits = key16_bf16_bits((uint32_t)res);
       const __nv_bfloat162 tv2 = bf162_splat_bits(tbits);
       const float tvf = __uint_as_float(tbits << 16);
       const int nc = st_final_item_chunks<kKey>(p, part);
@@ -1012,7 +1007,7 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
             const float u = p.sp.noise.at(row + p.sp.dim0_offset, pos);
             seed = f32_key(fmaf(__uint_as_float(bits << 16), 1.0f / T_, gumbel_screen(u)));
           }
-          const unsigned long long word = ((unsigned long long)seed << 32) | (unsigned long long)(uint32_t)wide_result(ctl.wide.kmax16, v);
+          const unsigned long long word = ((unsigned long long)seed << 32) | (unsigned long long)(uint32_t)v;
           *reinterpret_cast<volatile unsigned long long*>(&p.wstate[row]) = word;
         }
 #ifdef TLX_TIMELINE
@@ -1441,23 +1436,19 @@ static __device__ __noinline__ void st_slow_row(const StreamParams& p, int row, 
 // final-pass CTAs allows, so that the pass is a single wave.  A CTA keeps, per thread, the two best
 // screened scores of its range and leaves ONE record: its best element, and whether anything else of the
 // range comes within the screening slack of it.
-constexpr size_t kFinSlotBytes = (size_t)kFinChunk + kFinNoiseChunk;
+constexpr size_t kFinSlotBytes = (size_t)kFinChunk + kFinChunkElems * 2;   // logits, and the places that the warps have noted
 constexpr size_t kFinFixedSmem = kFinSlots * kFinSlotBytes + sizeof(StControl);   // + one int per row (the list)
 
-__device__ __forceinline__ void fin_issue(const StreamParams& p, int row, int c, int c_end, bool dense,
-                                          unsigned char* ring, unsigned long long* mbar, int slot) {
+__device__ __forceinline__ void fin_issue(const StreamParams& p, int row, int c, int c_end, unsigned char* ring, unsigned long long* mbar,
+                                          int slot) {
   if (c >= c_end) return;
   const int64_t off = (int64_t)c * kFinChunk;
   const int64_t rest = p.row_bytes - off;
   const uint32_t bytes = (uint32_t)(rest < kFinChunk ? rest : kFinChunk);
   unsigned char* dst = ring + (size_t)slot * kFinSlotBytes;
   const unsigned char* src = reinterpret_cast<const unsigned char*>(p.sp.logits) + (int64_t)row * p.sp.row_stride * 2 + off;
-  mbar_expect_tx(&mbar[slot], dense ? bytes * 3 : bytes);
+  mbar_expect_tx(&mbar[slot], bytes);
   bulk_load(dst, src, bytes, &mbar[slot]);
-  if (dense) {
-    const float* nsrc = p.sp.noise.dense_row(row + p.sp.dim0_offset) + (int64_t)c * kFinChunkElems;
-    bulk_load(dst + kFinChunk, nsrc, bytes * 2, &mbar[slot]);
-  }
 }
 
 // Decides a wide row from the records of its ranges (all threads of the CTA that delivered the last one;
@@ -1495,7 +1486,7 @@ __device__ __forceinline__ void fin_decide_row(const StreamParams& p, int row, i
   __syncthreads();
   if (lane == 0) ctl.wkey[warp] = again;
   __syncthreads();
-  const uint32_t vstar16 = (uint32_t)wide_vstar16(__ldcg(&p.wstate[row].result));
+  const uint32_t vstar16 = (uint32_t)__ldcg(&p.wstate[row].result);
   const float tvf = __uint_as_float(key16_bf16_bits(vstar16) << 16);
   const __nv_bfloat16* rowp = reinterpret_cast<const __nv_bfloat16*>(sp.logits) + (int64_t)row * sp.row_stride;
   for (int w = 0; w < kStWarps; ++w) {
@@ -1528,9 +1519,8 @@ __device__ __forceinline__ void fin_decide_row(const StreamParams& p, int row, i
 }
 
 // The final-pass CTAs of the finish kernel (block indices below p.fin_ctas).
-// dense != 0: the noise is a tensor whose rows can be bulk-copied (16-byte aligned); it is streamed next
-// to the logits.  Otherwise the noise of the kept elements is read (or generated from the key) one by one.
-static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int dense, unsigned char* smem) {
+// The noise is a tensor whose rows can't be bulk-copied (not 16-byte aligned): that of the elements that may win is read one by one.
+static __device__ __forceinline__ void st_final_pass(const StreamParams& p, unsigned char* smem) {
 #ifdef TLX_SIZE_PROBE2
   return;
 #endif
@@ -1586,12 +1576,10 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
     const int w = unit / J, j = unit - w * J;
     const int row = wlist[w];
     WideState* ws = p.wstate + row;
-    const int wres = __ldcg(&ws->result);
-    const int vstar = wide_vstar16(wres);
+    const int vstar = __ldcg(&ws->result);
     if (vstar < 0) continue;   // the row's own CTA answers it with the whole-row routines
     const int c_begin = (int)((int64_t)j * p.nfin / J), c_end = (int)((int64_t)(j + 1) * p.nfin / J);
     const uint32_t tbits = key16_bf16_bits((uint32_t)vstar);
-    const __nv_bfloat162 tv2 = bf162_splat_bits(tbits);
     const float tvf = __uint_as_float(tbits << 16);
     const float T_ = sp.temperature[row];
     const float inv_T = 1.0f / T_;
@@ -1602,7 +1590,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
       for (int s = 0; s < kFinSlots; ++s) mbar_init(&ctl.mbar[s], 1);
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       ctl.best_key = __ldcg(&ws->best_key);   // of the whole row so far
-      for (int s = 0; s < kFinSlots; ++s) fin_issue(p, row, c_begin + s, c_end, dense != 0, ring, ctl.mbar, s);
+      for (int s = 0; s < kFinSlots; ++s) fin_issue(p, row, c_begin + s, c_end, ring, ctl.mbar, s);
     }
     __syncthreads();
     float a1 = -INFINITY, a2 = -INFINITY, u1 = 0.5f;
@@ -1610,26 +1598,18 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
     int t1 = 0x7FFFFFFF;
     int slot = 0;
     uint32_t phase = 0;
-    // No element scores above (value of the row's maximum) / T + its own Gumbel term: once the CTA knows a
-    // score `cb`, an element whose noise u gives -log(-log u) < cb - xtop - margin cannot come within the
-    // screening slack of the best, and -log u <= 1 - u ... so the test is one comparison of 1 - u with
-    // eps = exp(-(cb - xtop - margin)) (1 - u >= 1 - exp(-eps') for the exact bound eps'; eps is looser).
-    const float xtop = key16_value(wide_kmax16(wres)) * inv_T;
     float published = -INFINITY;
     for (int c = c_begin; c < c_end; ++c) {
       const float cb = key_f32(ctl.best_key);
-      const float eps = expf(-(cb - 2.0f * (kGumbelSlack + 1e-5f * fabsf(cb)) - xtop)) * 1.000001f;
       const bool arrived = mbar_wait_suspended(&ctl.mbar[slot], phase);
       if (c == c_begin && first) TLX_STAMP(sp, 2);
       const unsigned char* buf = ring + (size_t)slot * kFinSlotBytes;
-      const float* nbuf = reinterpret_cast<const float*>(buf + kFinChunk);
       const int nvec = (c == p.nfin - 1) ? last_nvec : kFinChunk / 16;
-      if (!dense && !(p.debug & 2)) {
+      if (!(p.debug & 2)) {
         // noise element by element: only for values that could reach the best known score with the greatest noise
-        // there is (of 1 - 2^-23 from a key, 1 - 2^-24 in a tensor); the warp notes their places and then takes them
-        // 128 at a time, four a lane, so that the dependent rounds of four keys (or four reads) overlap
+        // there is, 1 - 2^-24; the warp notes their places and then takes them 128 at a time, four a lane, so that four reads overlap
         const float low = cb - 2.0f * (kGumbelSlack + 1e-5f * fabsf(cb));
-        const float xcut = fmaxf(tvf, (low - (sp.noise.dense ? 16.65f : 15.95f)) * T_);
+        const float xcut = fmaxf(tvf, (low - 16.65f) * T_);
         unsigned short* noted = reinterpret_cast<unsigned short*>(ring + (size_t)slot * kFinSlotBytes + kFinChunk) +
                                 warp * (kFinVecPerThread * 32 * 8);
         int n = 0;
@@ -1661,9 +1641,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
           n += __shfl_sync(0xFFFFFFFFu, incl, 31);
         }
         __syncwarp();
-        const uint32_t k0 = sp.noise.key_dev ? __ldg(sp.noise.key_dev) : sp.noise.k0;
-        const uint32_t k1 = sp.noise.key_dev ? __ldg(sp.noise.key_dev + 1) : sp.noise.k1;
-        const uint32_t ctr0 = (uint32_t)(sp.noise.row_of(nrow) * sp.noise.vocab) + (uint32_t)(c * kFinChunkElems);
+        const float* noise = sp.noise.dense_row(nrow) + c * kFinChunkElems;
 #pragma unroll 1
         for (int q0 = 0; q0 < n; q0 += 128) {
           int at[4];
@@ -1672,8 +1650,7 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
           for (int k = 0; k < 4; ++k) {
             const int q = q0 + lane + 32 * k;
             at[k] = q < n ? noted[q] : -1;
-            if (sp.noise.dense) un[k] = at[k] >= 0 ? __ldg(sp.noise.dense_row(nrow) + c * kFinChunkElems + at[k]) : 0.5f;
-            else un[k] = fmaxf(threefry_uniform01(k0, k1, ctr0 + (uint32_t)at[k]), kF32Tiny);
+            un[k] = at[k] >= 0 ? __ldg(noise + at[k]) : 0.5f;
           }
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
@@ -1687,63 +1664,13 @@ static __device__ __forceinline__ void st_final_pass(const StreamParams& p, int 
             else a2 = fmaxf(a2, a);
           }
         }
-      } else if (!(p.debug & 2)) {
-#pragma unroll 1
-        for (int jv = 0; jv < kFinVecPerThread; ++jv) {
-          const int v = (int)threadIdx.x + jv * kStThreads;
-          if (v < nvec) {
-            const uint4 x = *reinterpret_cast<const uint4*>(buf + (size_t)v * 16);
-            const __nv_bfloat162 m = __hmax2_nan(__hmax2_nan(bf162_bits(x.x), bf162_bits(x.y)),
-                                                 __hmax2_nan(bf162_bits(x.z), bf162_bits(x.w)));
-            if (!__hblt2(m, tv2)) {
-              // eight independent screened scores, then their best two
-              const uint32_t wd[4] = {x.x, x.y, x.z, x.w};
-              float un[8];
-              {
-                const float4 n0 = *reinterpret_cast<const float4*>(nbuf + v * 8);
-                const float4 n1 = *reinterpret_cast<const float4*>(nbuf + v * 8 + 4);
-                un[0] = n0.x; un[1] = n0.y; un[2] = n0.z; un[3] = n0.w;
-                un[4] = n1.x; un[5] = n1.y; un[6] = n1.z; un[7] = n1.w;
-                const float umax = fmaxf(fmaxf(fmaxf(un[0], un[1]), fmaxf(un[2], un[3])),
-                                         fmaxf(fmaxf(un[4], un[5]), fmaxf(un[6], un[7])));
-                if (1.0f - umax > eps) continue;   // none of the eight can matter
-              }
-              float sc[8];
-              float v1 = -INFINITY, v2 = -INFINITY;
-#pragma unroll
-              for (int e = 0; e < 8; ++e) {
-                const uint32_t hi = (e & 1) ? (wd[e >> 1] & 0xFFFF0000u) : (wd[e >> 1] << 16);
-                const float xf = __uint_as_float(hi);
-                bool keep = !(xf < tvf);
-                keep = keep && 1.0f - un[e] <= eps;
-                sc[e] = keep ? fmaf(xf, inv_T, gumbel_screen(un[e])) : -INFINITY;
-                const float lo = fminf(v1, sc[e]);
-                v1 = fmaxf(v1, sc[e]);
-                v2 = fmaxf(v2, lo);
-              }
-              if (v1 > a1) {
-                int ebest = 0;
-#pragma unroll
-                for (int e = 7; e >= 0; --e) if (sc[e] == v1) ebest = e;
-                u1 = un[0];
-                b1 = wd[0] & 0xFFFFu;
-#pragma unroll
-                for (int e = 1; e < 8; ++e)
-                  if (e == ebest) { u1 = un[e]; b1 = (e & 1) ? (wd[e >> 1] >> 16) : (wd[e >> 1] & 0xFFFFu); }
-                t1 = c * kFinChunkElems + v * 8 + ebest;
-              }
-              a2 = fmaxf(fminf(a1, v1), fmaxf(a2, v2));
-              a1 = fmaxf(a1, v1);
-            }
-          }
-        }
       }
       if (a1 > published) { atomicMax(&ctl.best_key, f32_key(a1)); published = a1; }
       if (__syncthreads_or(!arrived)) {   // a copy never arrived: give up, the row's status says so
         if (threadIdx.x == 0 && sp.out_status) atomicOr(sp.out_status + row, (int)kStatusTimeout);
         return;
       }
-      if (threadIdx.x == 0) fin_issue(p, row, c + kFinSlots, c_end, dense != 0, ring, ctl.mbar, slot);
+      if (threadIdx.x == 0) fin_issue(p, row, c + kFinSlots, c_end, ring, ctl.mbar, slot);
       if (++slot == kFinSlots) { slot = 0; phase ^= 1u; }
     }
     if (first) TLX_STAMP(sp, 3);
@@ -1853,18 +1780,17 @@ constexpr size_t kStFinishRowSmem =
 constexpr size_t kStFinishFixedSmem =
     kStFinishRowSmem > kFinFixedSmem ? kStFinishRowSmem : kFinFixedSmem;   // + one int per row (the final pass's list)
 
-// Grid: p.fin_ctas CTAs of the final pass, then one CTA per row.  A wide row's CTA takes part in the final pass (256 rows of
-// 128256 without top-k, noise from a key: 147 us, without them 203, with a row at a time per CTA of the 188 others 252).
+// Grid: p.fin_ctas CTAs of the final pass, then one CTA per row.  A wide row's CTA takes part in the final pass.
 // kFinalPass false: the stream kernel has taken the final items, and there are no such CTAs.
 template <bool kFinalPass>
-__global__ void __launch_bounds__(kStThreads, 3) sample_finish_kernel(StreamParams p, int dense) {
+__global__ void __launch_bounds__(kStThreads, 3) sample_finish_kernel(StreamParams p) {
   extern __shared__ __align__(128) unsigned char fin_smem[];
   if constexpr (kFinalPass) {
     if ((int)blockIdx.x >= p.fin_ctas) {
       if (!st_finish_row(p, (int)blockIdx.x - p.fin_ctas, fin_smem)) return;
       __syncthreads();
     }
-    st_final_pass(p, dense, fin_smem);
+    st_final_pass(p, fin_smem);
   } else {
     st_finish_row(p, (int)blockIdx.x, fin_smem);
   }

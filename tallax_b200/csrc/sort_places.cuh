@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kRadixMaxThreads) sort_places_kernel(
       p[j] = (uint32_t)(c0 + i0 + 32 * j);
       if (32 * j >= left) k[j] = 0xFFFFFFFFu;
     }
-    const bool scattered = radix_by_digits<IPT, 32, CL, PAST, uint32_t>(
+    const bool scattered = radix_by_digits<IPT, CL, PAST>(
         reinterpret_cast<uint32_t(&)[IPT]>(k), reinterpret_cast<uint32_t(&)[IPT]>(p), passes, n, rank, cluster, s.radix, group_half,
         reinterpret_cast<uint32_t*>(pair), reinterpret_cast<uint32_t*>(pair) + cap);
     if constexpr (CL) cl_sync();   // (nobody leaves while another one may still read its counts)
@@ -504,7 +504,7 @@ __global__ void __launch_bounds__(kRadixMaxThreads) sort_places_kernel(
       if (r0 + 32 * j >= m) k[j] = 0xFFFFFFFFu;
     }
     uint32_t* sk = reinterpret_cast<uint32_t*>(pair);
-    const bool scattered = radix_by_digits<kRoom, 32, false, false, uint32_t>(k, p, diff, m, 0, 1, s.radix, group_half, sk, sk + nt * kRoom);
+    const bool scattered = radix_by_digits<kRoom, false, false>(k, p, diff, m, 0, 1, s.radix, group_half, sk, sk + nt * kRoom);
 #pragma unroll
     for (int j = 0; j < kRoom; ++j) {
       const int i = scattered ? (int)threadIdx.x + j * nt : r0 + 32 * j;

@@ -104,9 +104,9 @@ __device__ __forceinline__ uint32_t radix_scan256(uint32_t v, uint32_t* warp_sum
 // PAST: warps that have no other, beyond the row's n elements, are passed over (f32 [1024, 1025] 45 us against 52).  Not
 // where every warp has elements: the branch costs 3 %.  A test per group of 32 elements keeps a warp's groups from
 // overlapping: f32 [1024, 4096] 105 us against 90.
-template <int IPT, int kBits, bool CL, bool PAST, typename Pos>
+template <int IPT, bool CL, bool PAST>
 __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p)[IPT], uint32_t diff, int n, int rank, int cluster,
-                                                RadixShared& s, unsigned short* count, uint32_t* sk, Pos* sp) {
+                                                RadixShared& s, unsigned short* count, uint32_t* sk, uint32_t* sp) {
   const int nt = blockDim.x, cap = nt * IPT;
   const int lane = lane_id(), w = warp_id();
   const int nw = PAST ? (n + 32 * IPT - 1) / (32 * IPT) : nt >> 5;   // warps that have elements
@@ -127,7 +127,7 @@ __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p
   const float inv_cap = 1.0f / (float)cap;
   bool scattered = false;
 #pragma unroll 1
-  for (int sh = 0; sh < kBits; sh += 8) {
+  for (int sh = 0; sh < 32; sh += 8) {
     if (((diff >> sh) & 255u) == 0) continue;
     if (scattered && mine_exist) {
 #pragma unroll
@@ -200,7 +200,7 @@ __device__ __forceinline__ bool radix_by_digits(uint32_t (&k)[IPT], uint32_t (&p
           pair[to] = make_uint2(k[j], p[j]);
         } else {
           sk[to] = k[j];
-          sp[to] = (Pos)p[j];
+          sp[to] = p[j];
         }
       }
     }
