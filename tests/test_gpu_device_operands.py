@@ -34,6 +34,28 @@ def test_sample_with_device_key_and_offset(cuda, dtype, V):
     assert not ((to_np(host) != exp) & ~flags).any()
 
 
+# the streaming form (more than 16 MB), rows without top-k among them: their noise is made in the stream kernel's final items
+@pytest.mark.parametrize("off", [0, 1000003])
+def test_streamed_sample_with_device_key_and_offset(cuda, off):
+    B, V = 72, 128256
+    x, tk, tp, T, noise = o.make_sampling_inputs(B=B, V=V, seed=13, dtype="bf16")
+    tk[::4] = 0
+    T[9] = 0.0                                             # greedy
+    args = [to_dev(a, cuda) for a in (x, tk, tp, T)]
+    off_dev = torch.tensor(off, dtype=torch.int32, device=cuda)
+    exp, flags = o.sample(x, tk, tp, T, rng_key=KEY, dim0_offset=off, return_flags=True)
+    for key, offset in ((KEY, off), (KEY, off_dev), (_key_dev(cuda), off), (_key_dev(cuda), off_dev)):
+        ws = ops.SampleWorkspace(B, V, cuda)
+        got, status = ops.sample(*args, rng_key=key, dim0_offset=offset, workspace=ws, return_status=True)
+        assert ws.ws.numel() > 256 and not ((to_np(got) != exp) & ~flags).any()
+        assert (to_np(status)[::4] & 1).all() and (to_np(status) & 2 == 0).all()
+    # a noise tensor's rows from a device offset on
+    wide = torch.cat([torch.rand((5, V), device=cuda), to_dev(noise, cuda)])
+    exp, flags = o.sample(x, tk, tp, T, noise=noise, return_flags=True)
+    got = ops.sample(*args, noise=wide, dim0_offset=torch.tensor(5, dtype=torch.int32, device=cuda))
+    assert not ((to_np(got) != exp) & ~flags).any()
+
+
 def test_sample_with_dense_noise_and_device_offset(cuda):
     B, V, off = 16, 128256, 8
     x, tk, tp, T, noise = o.make_sampling_inputs(B=B + off, V=V, seed=9, dtype="bf16")
