@@ -514,6 +514,9 @@ def exchange_step(logits_shard, col_offset: int, exchange: Exchange, top_k_, top
                                           exchange.status, top_k_, top_p, temperature, out)
         if got is not NotImplemented:
             return got
+    # nothing may write the parameters between the two stages: conversions come before both
+    dev, rows = logits_shard.device, exchange.rows
+    top_k_, top_p, temperature = _i32vec(top_k_, rows, dev), _f32vec(top_p, rows, dev), _f32vec(temperature, rows, dev)
     exchange_shard_candidates(logits_shard, col_offset, exchange, noise_shard=noise_shard, rng_key=rng_key,
                               vocab_total=vocab_total, dim0_offset=dim0_offset)
     return exchange_merge_and_sample(exchange, top_k_, top_p, temperature, out=out)
@@ -525,7 +528,12 @@ def exchange_merge_and_sample(exchange: Exchange, top_k_, top_p, temperature, ou
     dev = exchange.device
     if out is None:
         out = torch.empty(rows, dtype=torch.int32, device=dev)
+    given = top_k_, top_p, temperature
     top_k_, top_p, temperature = _i32vec(top_k_, rows, dev), _f32vec(top_p, rows, dev), _f32vec(temperature, rows, dev)
+    if any(isinstance(g, torch.Tensor) and g.is_cuda and v.data_ptr() != g.data_ptr() for g, v in zip(given, (top_k_, top_p, temperature))):
+        # The merge kernel may start, and read the parameters, while what precedes it ends: a kernel between the conversions
+        # and the merge is one that they have been waited for by.
+        torch.zeros(1, device=dev)
     check(_lib.load().tlx_exchange_merge_and_sample(
         _stream(), exchange.own, rows, exchange.k_cand, exchange.world, _ptr(top_k_),
         _ptr(top_p), _ptr(temperature), _ptr(out), _ptr(exchange.status)))

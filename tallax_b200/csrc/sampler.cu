@@ -353,8 +353,9 @@ __global__ void __launch_bounds__(kMergeThreads) merge_and_sample_kernel(MergePa
   while (P < n_cand) P <<= 1;
   uint64_t* merged = cand + P;
   const int64_t r = blockIdx.x;
-  const float T_ = p.temperature[r], pp = p.top_p[r];   // (there before the candidates are)
-  int K = p.top_k[r];
+  // (there before the candidates are; from L2: this kernel has not waited for anything yet)
+  const float T_ = __ldcg(p.temperature + r), pp = __ldcg(p.top_p + r);
+  int K = __ldcg(p.top_k + r);
   if (K <= 0 || K > n_cand) K = n_cand;
 
   const float* v = p.cand_vals;

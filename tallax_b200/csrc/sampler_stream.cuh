@@ -723,11 +723,12 @@ __global__ void __launch_bounds__(kStThreads, 4) sample_stream_kernel(StreamPara
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // The list of rows needs the rows' classes only as far as the parameters decide them (a row that the
-  // prologue downgrades is dropped when its items come up): it is built while the prologue kernel still runs.
+  // prologue downgrades is dropped when its items come up): it is built while the prologue kernel still runs, which has waited for
+  // what writes the parameters.  (They are read from L2: this kernel has not waited for anything yet.)
   uint32_t* pcls = dtab;   // parameter classes, replaced by the descriptors below
   for (int r = threadIdx.x; r < rows; r += kStThreads) {
     int K;
-    pcls[r] = (uint32_t)st_param_class(p.sp.top_k[r], p.sp.top_p[r], p.sp.temperature[r], p.sp.vocab, K);
+    pcls[r] = (uint32_t)st_param_class(__ldcg(p.sp.top_k + r), __ldcg(p.sp.top_p + r), __ldcg(p.sp.temperature + r), p.sp.vocab, K);
   }
   __syncthreads();
   int nlisted = 0, nwide = 0;

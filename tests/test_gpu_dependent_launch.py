@@ -1,12 +1,13 @@
 """GPU: calls launched as programmatic dependents keep the stream's order, whatever precedes them, eager and in a graph.
 
-Every call reads what the operation before it on the stream has just written, over buffers that are used again at once; the
-expectation is the same call made after a synchronisation.
+Every call reads what the operation before it on the stream has just written, over buffers that are used again at once: values,
+parameters, noise, keys, indices and permutations.  The expectation is the same call made after a synchronisation.
 """
 import pytest
 import torch
 
 from tallax_b200 import sampling, tax, tumpy
+from tallax_b200._src import ops
 
 pytestmark = pytest.mark.gpu
 
@@ -124,3 +125,96 @@ def test_steps_follow_each_other(cuda):
     torch.cuda.synchronize()
     for i, (t, v) in enumerate(got):
         assert torch.equal(t, want[i % 2][0]) and torch.equal(v, want[i % 2][1])
+
+
+def _versions(cuda, rows, n, dtype, vocab=None):
+    """Three sets of everything that a call reads."""
+    gen = torch.Generator(device=cuda).manual_seed(rows)
+    sets = []
+    for i in range(3):
+        k = torch.randint(1, 40, (rows,), generator=gen, device=cuda, dtype=torch.int32)
+        k[i::5] = 0 if vocab is None else 7
+        sets.append(dict(x=(torch.randn((rows, n), generator=gen, device=cuda) * 2).to(dtype), noise=torch.rand((rows, n), generator=gen, device=cuda),
+                         top_k=k, top_p=torch.rand(rows, generator=gen, device=cuda) * 0.6 + 0.4,
+                         temperature=(torch.rand(rows, generator=gen, device=cuda) + 0.5) * (torch.arange(rows, device=cuda) % 7 != i),
+                         index=torch.randint(0, n, (rows, n), generator=gen, device=cuda, dtype=torch.int32),
+                         perm=torch.argsort(torch.rand((rows, n), generator=gen, device=cuda), dim=1).int(),
+                         key=torch.randint(0, 1 << 30, (2,), generator=gen, device=cuda, dtype=torch.int32),
+                         offset=torch.tensor(3 * i, device=cuda, dtype=torch.int32)))
+    return sets
+
+
+# everything that a call reads is overwritten right before it, by kernels, the operand `last` at the very end; both forms of the sampler
+# (the streaming one lists its rows by their parameters before it waits), both kinds of noise, and the pair of the vocabulary shards
+READS = {"sample": "x noise top_k top_p temperature", "sample_key": "x key offset top_k top_p temperature", "gather": "x index",
+         "sort_through": "x perm", "shard": "x noise top_k top_p temperature"}
+READS["stream"], READS["stream_key"] = READS["sample"], READS["sample_key"]
+
+
+@pytest.mark.parametrize("name,last", [(name, last) for name, reads in READS.items() for last in reads.split()])
+def test_every_operand_may_change_between_queued_calls(cuda, name, last):
+    names = READS[name].split()
+    rows, n = (160, 65536) if name.startswith("stream") else (300, 4096) if name == "shard" else (24, 20000)
+    sets = _versions(cuda, rows, n, torch.float32 if name in ("gather", "sort_through") else torch.bfloat16, n if name == "shard" else None)
+    now = {k: torch.empty_like(v) for k, v in sets[0].items()}
+    ex = ops.Exchange.local_group(rows, 40, 1, cuda)[0] if name == "shard" else None
+    md = sampling.SamplingMetadata(now["top_k"], now["top_p"], now["temperature"])
+
+    def write(i):
+        for k in [k for k in names if k != last] + [last]:
+            v = sets[i][k]
+            if v.dtype in (torch.float32, torch.bfloat16):
+                torch.mul(v, 1.0, out=now[k])
+            else:
+                torch.add(v, 0, out=now[k])
+
+    def call():
+        if name in ("sample", "stream"):
+            return sampling.sample(None, now["x"], md, noise=now["noise"])
+        if name in ("sample_key", "stream_key"):
+            return ops.sample(now["x"], now["top_k"], now["top_p"], now["temperature"], rng_key=now["key"], dim0_offset=now["offset"])
+        if name == "gather":
+            return tumpy.take_along_axis(now["x"], now["index"], 1)
+        if name == "sort_through":
+            return ops.argsort_rows(now["x"], in_perm=now["perm"])[1]
+        return sampling.sample_vocab_sharded(None, now["x"], md, noise_shard=now["noise"], k_cand=40, exchange=ex)
+
+    try:
+        want = []
+        for i in range(3):
+            write(i)
+            torch.cuda.synchronize()
+            want.append(call().clone())
+            torch.cuda.synchronize()
+        got = []
+        for i in range(12):
+            write(i % 3)
+            got.append(call())
+        torch.cuda.synchronize()
+        for i, g in enumerate(got):
+            assert torch.equal(g, want[i % 3]), i
+    finally:
+        if ex is not None:
+            ex.close()
+
+
+# parameters of other types are converted: before both stages of a step, and, where the second one is called by itself, in order with it
+@pytest.mark.parametrize("by_stages", [False, True])
+def test_shard_parameters_of_other_types(cuda, by_stages):
+    rows, n = 300, 4096
+    sets = _versions(cuda, rows, n, torch.bfloat16, n)
+    ex = ops.Exchange.local_group(rows, 40, 1, cuda)[0]
+    try:
+        for i in range(12):
+            s = sets[i % 3]
+            args = s["top_k"].long(), s["top_p"].double(), s["temperature"].double()
+            if by_stages:
+                ops.exchange_shard_candidates(s["x"], 0, ex, noise_shard=s["noise"])
+                got = ops.exchange_merge_and_sample(ex, *args)
+            else:
+                got = ops.exchange_step(s["x"], 0, ex, *args, noise_shard=s["noise"])
+            block = ops.shard_candidates(s["x"], 0, 40, noise_shard=s["noise"], vocab_total=n)
+            torch.cuda.synchronize()
+            assert torch.equal(got, ops.merge_and_sample(block[None], s["top_k"], s["top_p"], s["temperature"])), i
+    finally:
+        ex.close()
