@@ -1138,6 +1138,7 @@ __device__ __forceinline__ int rc_pruned_row(const RcSampleParams& p, const RcPa
   if (enough) {
     float lo = xmax - (float)__ffs(enough);
     lo -= 1e-5f * fmaxf(fabsf(lo), fabsf(xmax));   // (the distances are rounded)
+    lo = fmaxf(lo, -FLT_MAX);                      // (finite also next to the type's least value: what lies outside the part is -inf)
     unsigned short* queue = reinterpret_cast<unsigned short*>(smem + layout.off_s) + warp_id() * kRcQueue;
 #pragma unroll 1
     for (int round = 0; round < 8; ++round) {

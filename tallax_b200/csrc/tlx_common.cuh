@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cfloat>
 #include <cstdarg>
 #include <cstdio>
 

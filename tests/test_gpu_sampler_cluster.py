@@ -183,3 +183,25 @@ def test_rows_bounded_by_top_p(cuda, dtype, V, noise_kind):
     tok = to_np(ops.sample(to_dev(x, cuda), to_dev(tk[:4], cuda), to_dev(tp[:4], cuda), to_dev(T[:4], cuda), **dkw))
     assert ((tok >= 0) & (tok < V)).all()
     assert flags[0] or tok[2] == exp[0]
+
+
+# f32 rows next to the type's least value (masked with it, and not all equal): what top-p bounds them by stays finite, so that nothing
+# outside the part, which holds -inf, is taken for an element; rows at every offset from a 16-byte boundary
+@pytest.mark.parametrize("V", [50257, 96003, 131070])
+@pytest.mark.parametrize("from_key", [False, True])
+def test_rows_next_to_the_least_value(cuda, V, from_key):
+    B = 16
+    rng = np.random.default_rng(V)
+    least = np.finfo(np.float32).max * np.float32(-1)
+    x = least * (1 - rng.integers(0, 64, (B, V)).astype(np.float32) * np.float32(2**-24)).astype(np.float32)
+    x[::2, V // 3] = least * np.float32(1 - 70 * 2.0**-24)     # the greatest once
+    x[5] = np.where(np.arange(V) == V - 1, np.float32(-1e38), least)
+    tk, tp = np.zeros(B, np.int32), np.linspace(0.05, 0.99, B).astype(np.float32)
+    T = np.linspace(1.0, 2.0, B).astype(np.float32)            # (from 1 on: every score is finite)
+    noise = rng.random((B, V), dtype=np.float32)
+    kw = dict(rng_key=(43, V)) if from_key else dict(noise=noise)
+    exp, flags = o.sample(x, tk, tp, T, return_flags=True, **kw)
+    dkw = kw if from_key else dict(noise=to_dev(noise, cuda))
+    tok = to_np(ops.sample(to_dev(x, cuda), to_dev(tk, cuda), to_dev(tp, cuda), to_dev(T, cuda), **dkw))
+    bad = (tok != exp) & ~flags
+    assert not bad.any(), (np.flatnonzero(bad), tok[bad], exp[bad])
