@@ -172,17 +172,21 @@ def test_rows_bounded_by_top_p(cuda, dtype, V, noise_kind):
     bad = (to_np(tok) != exp) & ~flags
     assert not bad.any(), (np.flatnonzero(bad), to_np(tok)[bad], exp[bad])
     assert (to_np(status) & 2 == 0).all()
-    # rows with NaNs and infinities give what they give by passes over the row in global memory, a longer row's way
+    # rows with NaNs and infinities are left to passes over the row in global memory.  A NaN has no score and makes every mass one, so that
+    # top-p rules nothing out: the row's token is that of the others at top_p 1.  An infinite logit wins, the first token of a masked row does,
+    # and one -inf is an element like others
     xf[:4] = xf[13:14]
     xf[0, 5], xf[1, V - 1], xf[2, 7], xf[3] = np.nan, np.inf, -np.inf, -np.inf
     x = xf[:4].astype(x.dtype)
-    kw = dict(rng_key=(41, V)) if noise_kind == "key" else dict(noise=noise[:4])
-    exp, flags = o.sample(x[2:3], tk[2:3], tp[2:3], T[2:3], return_flags=True,
-                          **(dict(noise=noise[2:3]) if noise_kind != "key" else dict(rng_key=(41, V), dim0_offset=2)))
     dkw = dict(rng_key=(41, V)) if noise_kind == "key" else dict(noise=to_dev(noise[:4], cuda))
     tok = to_np(ops.sample(to_dev(x, cuda), to_dev(tk[:4], cuda), to_dev(tp[:4], cuda), to_dev(T[:4], cuda), **dkw))
-    assert ((tok >= 0) & (tok < V)).all()
-    assert flags[0] or tok[2] == exp[0]
+    xf[0, 5], tp[0] = -np.inf, 1.0
+    x = xf[:4].astype(x.dtype)
+    for r in (0, 2):
+        kw = dict(noise=noise[r:r + 1]) if noise_kind != "key" else dict(rng_key=(41, V), dim0_offset=r)
+        exp, flags = o.sample(x[r:r + 1], tk[r:r + 1], tp[r:r + 1], T[r:r + 1], return_flags=True, **kw)
+        assert flags[0] or tok[r] == exp[0], r
+    assert tok[1] == V - 1 and tok[3] == 0
 
 
 # f32 rows next to the type's least value (masked with it, and not all equal): what top-p bounds them by stays finite, so that nothing
