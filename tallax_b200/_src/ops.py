@@ -530,7 +530,7 @@ def exchange_merge_and_sample(exchange: Exchange, top_k_, top_p, temperature, ou
         out = torch.empty(rows, dtype=torch.int32, device=dev)
     given = top_k_, top_p, temperature
     top_k_, top_p, temperature = _i32vec(top_k_, rows, dev), _f32vec(top_p, rows, dev), _f32vec(temperature, rows, dev)
-    if any(isinstance(g, torch.Tensor) and g.is_cuda and v.data_ptr() != g.data_ptr() for g, v in zip(given, (top_k_, top_p, temperature))):
+    if any(not isinstance(g, torch.Tensor) or v.data_ptr() != g.data_ptr() for g, v in zip(given, (top_k_, top_p, temperature))):
         # The merge kernel may start, and read the parameters, while what precedes it ends: a kernel between the conversions
         # and the merge is one that they have been waited for by.
         torch.zeros(1, device=dev)

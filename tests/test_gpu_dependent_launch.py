@@ -198,16 +198,27 @@ def test_every_operand_may_change_between_queued_calls(cuda, name, last):
             ex.close()
 
 
-# parameters of other types are converted: before both stages of a step, and, where the second one is called by itself, in order with it
+# parameters of other types, one number for all rows among them, are converted: before both stages of a step, and, where the second
+# one is called by itself, in order with it
 @pytest.mark.parametrize("by_stages", [False, True])
-def test_shard_parameters_of_other_types(cuda, by_stages):
+@pytest.mark.parametrize("kind", ["wider", "numbers", "of one row", "on the host"])
+def test_shard_parameters_of_other_types(cuda, kind, by_stages):
     rows, n = 300, 4096
     sets = _versions(cuda, rows, n, torch.bfloat16, n)
     ex = ops.Exchange.local_group(rows, 40, 1, cuda)[0]
     try:
         for i in range(12):
             s = sets[i % 3]
-            args = s["top_k"].long(), s["top_p"].double(), s["temperature"].double()
+            args = s["top_k"], s["top_p"], s["temperature"]
+            if kind in ("numbers", "of one row"):
+                args = [a[i:i + 1] for a in args]
+            same = [a.expand(rows).contiguous() for a in args]
+            if kind == "wider":
+                args = args[0].long(), args[1].double(), args[2].double()
+            elif kind == "numbers":
+                args = int(args[0]), float(args[1]), float(args[2])
+            elif kind == "on the host":
+                args = [a.cpu() for a in args]
             if by_stages:
                 ops.exchange_shard_candidates(s["x"], 0, ex, noise_shard=s["noise"])
                 got = ops.exchange_merge_and_sample(ex, *args)
@@ -215,6 +226,6 @@ def test_shard_parameters_of_other_types(cuda, by_stages):
                 got = ops.exchange_step(s["x"], 0, ex, *args, noise_shard=s["noise"])
             block = ops.shard_candidates(s["x"], 0, 40, noise_shard=s["noise"], vocab_total=n)
             torch.cuda.synchronize()
-            assert torch.equal(got, ops.merge_and_sample(block[None], s["top_k"], s["top_p"], s["temperature"])), i
+            assert torch.equal(got, ops.merge_and_sample(block[None], *same)), i
     finally:
         ex.close()
