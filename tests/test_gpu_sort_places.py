@@ -143,3 +143,115 @@ def test_rows_of_few_values(cuda, dtype, copies, n, spacing):
         e = np.argsort(-a if descending else a, axis=1, kind="stable")
         assert np.array_equal(p.cpu().numpy(), np.tile(e, (copies, 1)))
         assert torch.equal(v.cpu(), torch.take_along_dim(t, torch.from_numpy(e), 1).repeat(copies, 1))
+
+
+# ---- rows that get past the sample of equal keys: what the kernel decides later -------------------------------------------------
+def _cluster(rows, n):
+    """CTAs a row, as the dispatch chooses them; elements a thread; threads a CTA."""
+    ctas, at_once = (lambda tile: -(-n // tile)), (lambda c, an_sm: 148 * an_sm if c == 1 else 8 * (18 * an_sm // c))
+    least, half = ctas(16384), ctas(8192)
+    c = 1
+    if n > 10000:
+        c = next((c for c in range(min(ctas(4096), 8), least - 1, -1) if rows <= at_once(c, 1)), 0)
+        if c == 0:
+            c = (1 if least == 1 else half if half <= 8 and rows <= at_once(half, 2) else (3 if half == 3 else 2) if least == 2
+                 else half if half <= 6 else max(least, 4))
+    if c > 1 or n > 8192:
+        ipt = 16
+    else:
+        ipt = 4 if n <= 1024 else 8 if n <= 2048 or rows * ((n + 255) // 256 * 32) <= 148 * 1024 else 16
+    return c, ipt, max(256, -(-n // (c * 32 * ipt)) * 32)
+
+
+def _way(row, dtype, rows, descending):
+    """The way that a row takes, from the rules of the kernel: by digits from the start; by digits because an owner has no room; or, per
+    CTA, by places or by digits of its own elements."""
+    n, half = len(row), dtype == "bf16"
+    c, ipt, nt = _cluster(rows, n)
+    pos = np.arange(n, dtype=np.int64)
+    if dtype == "i32":
+        key = row.astype(np.int64) + 2**31
+    else:
+        bits = (row if dtype == "f32" else torch.from_numpy(row).to(torch.bfloat16).float().numpy()).view(np.uint32).astype(np.int64)
+        key = np.where(bits >> 31 == 1, bits ^ 0xFFFFFFFF, bits | 0x80000000)
+    if descending:
+        key = key ^ 0xFFFFFFFF
+    if half:
+        key = (key & 0xFFFF0000) | ((pos << 15) * (2 * (0xFFFFFFFF // n)) >> 32)
+    upright = key if dtype == "i32" else np.where(key >> 31 == 1, key, key ^ 0x7FFFFFFF)
+    diff = int(np.bitwise_or.reduce(upright ^ upright[0])) & (0xFFFF0000 if half else 0xFFFFFFFF)
+    digits = sum((diff >> s & 255) != 0 for s in (0, 8, 16, 24))
+    equal = 0
+    for start in range(0, n, 32 * ipt):
+        _, count = np.unique(key[start:start + 32] >> (16 if half else 0), return_counts=True)
+        equal += int((count * (count - 1)).sum())
+    if digits <= (1 if half else 2) or equal > (n // (2 * ipt) if half else 24 * 31 // ipt):
+        return ["digits"]
+    o = key - key.min()
+    sh = max(int(o.max()).bit_length() - 11, 0)
+    count = np.bincount(o >> sh, minlength=2049)
+    before = np.concatenate([[0], np.cumsum(count)])
+    at = before[o >> sh] + (((o << 1 & 0xFFFFFFFF) << (31 - sh) & 0xFFFFFFFF) * count[o >> sh] >> 32)
+    per = -(-n // c)
+    got = np.bincount(at // per, minlength=c)
+    if c > 1 and (got > nt * (ipt + ipt // 16)).any():
+        return ["no room"]
+    ways = []
+    for d in range(c):
+        group = np.bincount(at[at // per == d])
+        ways.append("own digits" if group.max(initial=0) > 512 or (np.minimum(group, 512)**2).sum() > 24 * got[d] else "places")
+    return ways
+
+
+def _crowded(n, dtype, rng):
+    """Clumps of 40, of 480 and of 1500 elements next to each other in value, evenly spread; clumps in a part of the values only; one dense
+    run, and nine tenths of the row a run.  Distinct keys; in bf16, of which there are not enough, equal ones side by side where the
+    sample does not look."""
+    rows, quiet = [], np.arange(n) % 128 >= 32
+    for clump, share in ((40, 1.0), (480, 1.0), (1500, 1.0), (300, 0.5), (0, 1.0), (0, 0.9)):
+        if dtype == "bf16":
+            z, at = rng.standard_normal(n).astype(np.float32), np.arange(n) // max(clump, 1)
+            v = rng.permutation(np.linspace(-9, 9, n // max(clump, 1) + 1).astype(np.float32))[at]
+            rows.append(np.where(quiet & (np.arange(n) < n * share), v if clump else np.float32(0.5), z))
+            continue
+        most, m = 0x7F000000, int(n * share)
+        k = 12345 + np.arange(m)
+        if clump:
+            k = (np.linspace(-most, most * (2 * share - 1) - 2 * clump, -(-m // clump)).astype(np.int64)[:, None] + np.arange(clump)).ravel()[:m]
+        k = np.unique(np.concatenate([k[:n - 2], [-most, most]]))
+        others = np.setdiff1d(rng.integers(-most, most, 2 * n), k)
+        k = rng.permutation(np.concatenate([k, rng.permutation(others)[:n - len(k)]])).astype(np.int32)
+        rows.append(k if dtype == "i32" else np.where(k < 0, -k | -2**31, k).astype(np.int32).view(np.float32))
+    return rows
+
+
+# a CTA, and clusters of two to eight; rows of which some CTAs' groups are large, on their own (the CTA's elements by digits), and rows
+# of which one owner would get more than it has room for; through a permutation too, and with a payload
+CROWDED = [(1, 700, 1), (1, 1500, 1), (1, 4097, 1), (80, 4097, 1), (11, 12000, 2), (1, 12000, 3), (1, 16384, 4), (1, 20000, 5),
+           (1, 24000, 6), (1, 28001, 7), (1, 32768, 8), (1, 131072, 8)]
+
+
+@pytest.mark.parametrize("copies,n,cluster", CROWDED)
+@pytest.mark.parametrize("dtype", ["f32", "bf16", "i32"])
+def test_crowded_keys(cuda, dtype, copies, n, cluster):
+    rng = np.random.default_rng(n)
+    a = np.stack(_crowded(n, dtype, rng))
+    assert _cluster(copies * len(a), n)[0] == cluster
+    t = torch.from_numpy(a).to(torch.bfloat16) if dtype == "bf16" else torch.from_numpy(a)
+    a = t.float().numpy() if dtype == "bf16" else a.astype(np.float64)
+    for descending in (False, True):
+        ways = [_way(r, dtype, copies * len(a), descending) for r in (t.float() if dtype == "bf16" else t).numpy()]
+        assert ["digits"] not in ways
+        assert any("own digits" in w for w in ways) and (cluster == 1 or ["no room"] in ways), ways
+        e = torch.from_numpy(np.argsort(-a if descending else a, axis=1, kind="stable"))
+        v, p = tax.sort([t.to(cuda).repeat(copies, 1)], num_keys=1, is_stable=True, return_argsort=True, descending=descending)
+        assert torch.equal(p.cpu().long(), e.repeat(copies, 1))
+        assert torch.equal(v.cpu(), torch.take_along_dim(t, e, 1).repeat(copies, 1))
+        # the second key brings the first one's row into this order before its pass
+        second = torch.from_numpy(np.stack([rng.permutation(n) for _ in range(len(a))]).astype(np.int32))
+        at = (n - 1 - second if descending else second).long()
+        first, payload = torch.take_along_dim(t, at, 1), torch.randint(0, 1 << 30, t.shape, dtype=torch.int32)
+        got = tax.sort([x.to(cuda).repeat(copies, 1) for x in (first, second, payload)], num_keys=2, is_stable=True, descending=descending)
+        order = torch.empty_like(at).scatter_(1, at, torch.arange(n).repeat(len(a), 1))   # where the second key puts which element
+        for g, x in zip(got, (first, second, payload)):
+            assert torch.equal(g.cpu(), torch.take_along_dim(torch.take_along_dim(x, order, 1), e, 1).repeat(copies, 1))
