@@ -5,7 +5,8 @@
 // calls before it are complete, which themselves began with the same wait, but the launch's own work, 1 to 2 us between two
 // kernels of a stream, is done by then.  A predecessor that knows nothing of this (any other kernel, a copy) is waited for in the
 // same way.  A kernel whose successor may start before it has finished (grid_release) is one whose successor waits for it,
-// in one CTA at least, before it ends.
+// in one CTA at least, before it ends.  The exchange's merge kernel alone reads and writes memory before it waits: the rows as they
+// arrive, and its parameters, which nothing may write between the candidate kernel and it (tlx_exchange_merge_and_sample).
 //   us a call, queued one after the other, plain launches / these: sampler bf16 [1, 128256] 10.6 / 9.3, [32, 128256] 26.0 / 24.2,
 // [256, 128256] 48.4 / 46.2; top-k f32 [8, 32768] 10.3 / 8.5; cumsum f32 [64, 128256] 18.6 / 17.2; gather 4096 of f32 [1024, 262144]
 // 78.4 / 76.8; sort bf16 [64, 4097] 10.2 / 7.7.

@@ -637,7 +637,8 @@ static bool stream_path_serves(int dtype, int64_t rows, int64_t vocab, int64_t r
 //   [72, 128256]   32/32  23/21  45/40            35/29  22/20  48/40
 //   [80, 128256]   33/35  23/22  46/40            37/32  25/21  50/42
 // Up to 16 MB the cluster form saves more on the one usual setting than it loses on mixed ones; beyond, it runs in several waves.
-// One rule for both kinds of noise: the workspace's size is asked for before the noise is known.
+// One line for both kinds of noise.  With a key it lies low for long rows (the last two lines: 9 to 17 % would be gained up to there at least)
+// and right for many short ones; the workspace is sized for the stream from 16 MB on in either case.
 static bool stream_path_wanted(int64_t rows, int64_t vocab) { return rows * vocab * 2 > (16ll << 20); }
 
 // Diagnostic switch for timing the stages of the streaming path one by one (environment variable
