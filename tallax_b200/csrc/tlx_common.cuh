@@ -232,7 +232,7 @@ __device__ __forceinline__ float screen_cut(float best) {
 // index that the code relies on being in range (it is false, and the access is skipped, when it is not) and
 // records the first violation in a device word that tlx_debug_check_status reads.  In other builds the
 // macro is the constant `true` and costs nothing.  It stands in for a memory checker where none can be
-// run; the sites are the shared-memory and workspace indices of the streaming sampler.
+// run; the sites are the shared-memory and workspace indices of the streaming sampler and of the sort by places.
 #ifdef TLX_CHECKED
 static __device__ int g_tlx_check_word[4];   // violations so far; site, index and bound of the first
 __device__ __forceinline__ bool tlx_check_fail(int site, long long i, long long n) {
